@@ -1,0 +1,442 @@
+"""Performance cases of the framework, through its public entry points.
+
+Each case is one call (or one short run of calls) as a program that uses the
+library makes it.  Shells, grids and physics are those of
+``calypso_b200.configs`` (the named workloads, the ensemble's shapes) and of
+the usual dealiased triangular truncations; the seeded start is the
+library's own (``init_fields(2, seed)``).
+
+``listed()`` are the cases, ``draw(rng)`` gives one more of the same ranges,
+``prepare`` builds what a program holds before the call, ``run`` makes the
+call, ``work`` counts the bytes and flops the call cannot do without, and
+``exact`` evaluates it in float64 with torch (transforms, products, closure
+network).  A whole time step has no ``exact`` value here: it would restate
+the solver.
+"""
+from __future__ import annotations
+
+import math
+
+import numpy as np
+import torch
+
+from calypso_b200 import PREC_FP64, PREC_MIXED, Ensemble, SphMHD, closure, configs, sph_tables
+from calypso_b200.sph_mhd import MAGNE, TEMP, VELO, CalypsoError, load_library, rlm_size, rtm_size
+
+PREC = {"fp64": PREC_FP64, "mixed": PREC_MIXED}
+STATE_SLOTS = (VELO, VELO + 1, VELO + 2, MAGNE, MAGNE + 1, MAGNE + 2, TEMP)
+
+
+def listed():
+    return [
+        # the headline workload: a production-size dynamo step on the mixed
+        # path, replayed from its graph, kernel variants as the autotuner
+        # picks them there
+        dict(name="step_mixed_L255", kind="step", prec="mixed", L=255, nr=129, nth=384, nph=768, E=1e-4, Ra=300.0,
+             dt=5e-6, steps=1, graph=True, tuned=True),
+        # the same shell on the plain float64 path, the default precision and
+        # the yardstick of the mixed one
+        dict(name="step_fp64_L255", kind="step", prec="fp64", L=255, nr=129, nth=384, nph=768, E=1e-4, Ra=300.0,
+             dt=5e-6, steps=1, graph=True, tuned=True),
+        # a medium shell stepped as the control-file program steps it: default
+        # kernel variants, eager launches
+        dict(name="step_mixed_L127_eager", kind="step", prec="mixed", L=127, nr=97, nth=192, nph=384, E=1e-3,
+             Ra=200.0, dt=2.5e-5, steps=2, graph=False, tuned=False),
+        # the reference's dynamo benchmark shell in float64 (its smallest real
+        # run), 10 eager steps between monitor rows
+        dict(name="step_fp64_L31_bench", kind="step", prec="fp64", L=31, nr=49, nth=48, nph=96, E=1e-3, Ra=100.0,
+             dt=5e-5, steps=10, graph=False, tuned=False),
+        # one more step of an ensemble of small and medium shells (parameter
+        # study), one graph launch for all of them
+        dict(name="ensemble_12_shells", kind="ensemble", prec="mixed", per_shape=4, steps=1),
+        # a host that keeps the restart set in (pinned) memory of its own and
+        # calls the library for each step
+        dict(name="step_host_L127", kind="host_step", prec="mixed", L=127, nr=97, nth=192, nph=384, E=1e-3, Ra=200.0,
+             dt=2.5e-5),
+        # the spherical transform of the round-trip workload, by the reference's
+        # routines on its own buffers: backward and forward Legendre, device
+        # buffers, 3 vectors + 2 scalars
+        dict(name="leg_bwd_mixed_L255", kind="leg_bwd", prec="mixed", L=255, nr=65, nth=384, nph=768, nvec=3,
+             nscal=2),
+        dict(name="leg_fwd_mixed_L170", kind="leg_fwd", prec="mixed", L=170, nr=49, nth=256, nph=512, nvec=4,
+             nscal=0),
+        # float64 Legendre transforms of a ragged truncation (T106)
+        dict(name="leg_fwd_fp64_L106", kind="leg_fwd", prec="fp64", L=106, nr=41, nth=162, nph=324, nvec=3, nscal=2),
+        # the grid products with their FFTs at a power-of-two zonal grid (T85)
+        dict(name="products_fp64_L85", kind="products", prec="fp64", L=85, nr=65, nth=128, nph=256),
+        # one minibatch of the closure's training, and its inference over a
+        # whole L63 shell
+        dict(name="closure_train_16k", kind="closure_train", rows=16384),
+        dict(name="closure_forward_L63", kind="closure_forward", rows=266240),
+    ]
+
+
+# zonal grids of the form 2^a 3^b and, for each, half as many colatitudes
+ZONAL = (48, 64, 72, 96, 108, 128, 144, 192, 216, 256, 288, 324, 384, 432, 512, 576, 648, 768)
+
+
+def _log_int(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def _draw_shell(rng, nph_max, points_max):
+    """A shell: zonal grid, truncation (dealiased by 3/2, the odd one, or a
+    lower one), radial points; at most points_max values of (L+1)^2 nr."""
+    nph = rng.choice([n for n in ZONAL if n <= nph_max])
+    nth = 2 * ((nph // 2 + 1) // 2)
+    top = nph // 3
+    L = rng.choice([top - 1, (nph - 1) // 3, rng.randint(max(8, top // 2), top - 1)])
+    L = min(L, 255)
+    nr = _log_int(rng, 9, min(129, max(10, points_max // ((L + 1) ** 2))))
+    return dict(L=L, nr=nr, nth=nth, nph=nph)
+
+
+def draw(rng):
+    kind = rng.choice(["step", "step", "step", "leg_bwd", "leg_fwd", "products", "closure_train", "closure_forward",
+                       "host_step"])
+    if kind == "closure_train":
+        return dict(kind=kind, rows=_log_int(rng, 500, 65536))
+    if kind == "closure_forward":
+        return dict(kind=kind, rows=_log_int(rng, 1000, 266240))
+    prec = rng.choice(["mixed", "fp64"])
+    if kind in ("step", "host_step"):
+        sh = _draw_shell(rng, 576, 2_000_000)
+        E = rng.choice([1e-3, 1e-4])
+        c = dict(kind=kind, prec=prec, **sh, E=E, Ra=float(rng.randint(80, 400)),
+                 dt=(3e-3 if E == 1e-3 else 8e-4) / (sh["L"] + 1))
+        if kind == "step":
+            c.update(steps=rng.randint(1, 8), graph=rng.random() < 0.5, tuned=rng.random() < 0.5)
+        return c
+    sh = _draw_shell(rng, 768, 3_000_000)
+    c = dict(kind=kind, prec=prec, **sh)
+    if kind != "products":
+        c.update(nvec=rng.randint(1, 4), nscal=rng.randint(0, 2))
+    return c
+
+
+# ---------------------------------------------------------------------------
+def _params(c):
+    return configs.shell_params(c["L"], c["nr"], c["nth"], c["nph"], E=c.get("E", 1e-3), Ra=c.get("Ra", 100.0),
+                                dt=c.get("dt", 1e-5))
+
+
+def _gen(seed):
+    return torch.Generator(device="cuda").manual_seed(int(seed))
+
+
+def _spectra(c, seed):
+    """rlm buffer [k][j][comp] of seeded spectra, power of degree l ~ l^-2"""
+    L, nr, nc = c["L"], c["nr"], 3 * c["nvec"] + c["nscal"]
+    l = torch.cat([torch.full((2 * q + 1,), float(q)) for q in range(L + 1)]).cuda().double()
+    amp = 1.0 / (l.clamp_min(1.0) * torch.sqrt(2.0 * l + 1.0))
+    x = torch.randn((nr, (L + 1) ** 2, nc), generator=_gen(seed), device="cuda", dtype=torch.float64)
+    x *= amp[None, :, None]
+    x[:, 0, :3 * c["nvec"]] = 0.0          # a vector has no l = 0 part
+    return x.contiguous()
+
+
+def _fourier(c, seed, nc):
+    """rtm buffer [m][theta][k][comp], m = -L..L, amplitudes falling with |m|
+    and towards the poles as the orders of a smooth field do"""
+    L, nr, nth = c["L"], c["nr"], c["nth"]
+    m = torch.arange(-L, L + 1, device="cuda").abs().double()
+    x = torch.randn((2 * L + 1, nth, nr, nc), generator=_gen(seed), device="cuda", dtype=torch.float64)
+    sin = torch.sin(math.pi * (torch.arange(nth, device="cuda").double() + 0.5) / nth)
+    x *= (1.0 / (1.0 + m))[:, None, None, None] * (sin[None, :] ** (m[:, None] / 4.0))[:, :, None, None]
+    return x.contiguous()
+
+
+def _mlp_params(seed, nin=closure.NIN, nhid=256, nout=closure.NOUT):
+    g = torch.Generator().manual_seed(1000 + int(seed))
+    parts = []
+    for rows, cols in ((nhid, nin), (nhid, nhid), (nout, nhid)):
+        parts += [(torch.rand(rows * cols, generator=g) * 2 - 1) * math.sqrt(3.0 / cols),
+                  (torch.rand(rows, generator=g) * 2 - 1) * 0.05]
+    return torch.cat(parts).numpy().astype(np.float32)
+
+
+def _closure_rows(c, seed):
+    g = _gen(seed)
+    x = torch.randn((c["rows"], closure.NIN), generator=g, device="cuda")
+    t = torch.randn((c["rows"], closure.NOUT), generator=g, device="cuda")
+    return x, t
+
+
+class _Step:
+    """A shell mid-run: past its Euler step, the step graph captured."""
+
+    def __init__(self, c, seed):
+        self.c = c
+        self.g = SphMHD(_params(c), PREC[c["prec"]])
+        if c["tuned"]:
+            # what the autotuner chooses on the large shells
+            self.g.tuning = [1, 2, 2, 384, 1]
+        self.g.init_fields(2, seed % (1 << 31))
+        self.g.step(2, graph=c["graph"])
+        self.out = torch.zeros((len(STATE_SLOTS), self.g.nr, self.g.jmax), device="cuda", dtype=torch.float64)
+
+    def run(self):
+        self.g.step(self.c["steps"], graph=self.c["graph"])
+        _read_state(self.g, self.out)
+        return self.out
+
+
+def _read_state(g, out):
+    """the evolved fields into device memory of the caller's"""
+    lib = load_library()
+    for q, slot in enumerate(STATE_SLOTS):
+        if lib.cb2_get_field_device(g._h, slot, out[q].data_ptr()):
+            raise CalypsoError("cb2_get_field_device failed")
+
+
+class _EnsembleStep:
+    def __init__(self, c, seed):
+        self.c = c
+        params = configs.ensemble(c["per_shape"], seed=seed % 1000)
+        self.e = Ensemble(params, PREC[c["prec"]], autotune=False)
+        self.e.init_fields(2, seed % (1 << 31))
+        self.e.step(2)
+        self.e.sync()
+        self.out = [torch.zeros((len(STATE_SLOTS), s.nr, s.jmax), device="cuda", dtype=torch.float64)
+                    for s in self.e.shells]
+
+    def run(self):
+        self.e.step(self.c["steps"])
+        self.e.sync()
+        for s, o in zip(self.e.shells, self.out):
+            _read_state(s, o)
+        return self.out
+
+
+class _HostStep:
+    def __init__(self, c, seed):
+        self.g = SphMHD(_params(c), PREC[c["prec"]])
+        self.g.init_fields(2, seed % (1 << 31))
+        self.g.step(2)
+        self.host = torch.from_numpy(self.g.get_restart_state()).pin_memory()
+
+    def run(self):
+        self.g.step_restart_state(self.host.numpy(), with_energies=False)
+        return self.host
+
+
+class _Routine:
+    """One of the reference's routines on device buffers of the caller's."""
+
+    def __init__(self, c, seed):
+        self.c, k = c, c["kind"]
+        self.g = SphMHD(_params(c), PREC[c["prec"]])
+        self.t = sph_tables(c["L"], c["nr"], c["nth"], c["nph"])
+        nc = 3 * c["nvec"] + c["nscal"] if k != "products" else 13
+        self.nc = nc
+        if k == "leg_bwd":
+            self.x, n = _spectra(c, seed), rtm_size(self.t, nc)
+        elif k == "leg_fwd":
+            self.x, n = _fourier(c, seed, nc), rlm_size(self.t, nc)
+        else:
+            self.x, n = _fourier(c, seed, 13), rtm_size(self.t, 12)
+        self.out = torch.zeros(n, device="cuda", dtype=torch.float64)
+
+    def run(self):
+        c, x, o = self.c, self.x.data_ptr(), self.out.data_ptr()
+        if c["kind"] == "leg_bwd":
+            self.g.sel_backward_legendre_trans(self.nc, c["nvec"], c["nscal"], x, self.t, o)
+        elif c["kind"] == "leg_fwd":
+            self.g.sel_forward_legendre_trans(self.nc, c["nvec"], c["nscal"], x, self.t, o)
+        else:
+            self.g.fft_products(x, self.t, o)
+        return self.out
+
+
+class _Closure:
+    def __init__(self, c, seed):
+        self.c = c
+        self.net = closure.MLP()
+        self.net.set_params(_mlp_params(seed))
+        self.x, self.t = _closure_rows(c, seed)
+
+    def run(self):
+        if self.c["kind"] == "closure_forward":
+            return self.net.forward(self.x)
+        loss, grad = self.net.loss_grad(self.x, self.t, want_grad=True)
+        self.net.adam_step(1e-3)
+        return [loss, grad]
+
+
+_KINDS = {"step": _Step, "ensemble": _EnsembleStep, "host_step": _HostStep, "leg_bwd": _Routine, "leg_fwd": _Routine,
+          "products": _Routine, "closure_train": _Closure, "closure_forward": _Closure}
+
+
+def prepare(case, seed):
+    state = _KINDS[case["kind"]](case, int(seed))
+    torch.cuda.synchronize()
+    return state
+
+
+def run(state):
+    return state.run()
+
+
+# ---------------------------------------------------------------------------
+def _step_work(L, nr, nth, nph):
+    """One step: the 12 fields it advances (7 of the state, 5 of the history)
+    read and written once; Legendre sums of 41 real columns a radius over one
+    hemisphere, 25 real FFTs a row."""
+    n = 8.0 * nr * (L + 1) ** 2
+    flops = 41 * 2.0 * (nth / 2) * nr * (L + 1) ** 2 + 25 * nth * nr * 2.5 * nph * math.log2(nph)
+    return {"bytes": 24 * n, "flops": flops}
+
+
+def work(case):
+    c, k = case, case["kind"]
+    if k in ("closure_forward", "closure_train"):
+        par = closure.NIN * 256 + 256 * 256 + closure.NOUT * 256
+        r = c["rows"]
+        if k == "closure_forward":
+            return {"bytes": r * 4.0 * (closure.NIN + closure.NOUT), "flops": 2.0 * r * par}
+        return {"bytes": r * 4.0 * (closure.NIN + closure.NOUT), "flops": 2.0 * r * (3 * par - closure.NIN * 256)}
+    if k == "ensemble":
+        w = [_step_work(L, nr, nth, nph) for (L, nr, nth, nph, _) in configs.ENSEMBLE_SHAPES]
+        return {q: c["steps"] * c["per_shape"] * sum(x[q] for x in w) for q in ("bytes", "flops")}
+    L, nr, nth, nph = c["L"], c["nr"], c["nth"], c["nph"]
+    if k == "step":
+        w = _step_work(L, nr, nth, nph)
+        return {q: c["steps"] * w[q] for q in w}
+    if k == "host_step":
+        return _step_work(L, nr, nth, nph)
+    four = 8.0 * nr * nth * (2 * L + 1)
+    if k == "products":
+        return {"bytes": 25 * four, "flops": 25 * nth * nr * 2.5 * nph * math.log2(nph)}
+    nc = 3 * c["nvec"] + c["nscal"]
+    return {"bytes": nc * (four + 8.0 * nr * (L + 1) ** 2),
+            "flops": (5 * c["nvec"] + c["nscal"]) * 2.0 * (nth / 2) * nr * (L + 1) ** 2}
+
+
+# ---------------------------------------------------------------------------
+# float64 values by plain torch
+def _radii(p, nr):
+    k = np.arange(nr)
+    r = p["r_icb"] + 0.5 * (p["r_cmb"] - p["r_icb"]) * (1.0 - np.cos(math.pi * k / (nr - 1)))
+    return torch.from_numpy(r).cuda()
+
+
+def _gauss(nth):
+    """cos(theta) and weights, the node nearest the south pole first"""
+    x, w = np.polynomial.legendre.leggauss(nth)
+    return torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+
+
+def _plm(L, m, x):
+    """Schmidt semi-normalised P_l^m and dP_l^m/dtheta, l = m..L, at x"""
+    s = torch.sqrt((1.0 - x) * (1.0 + x))
+    pmm = torch.ones_like(x)
+    for q in range(1, m + 1):
+        pmm = pmm * s * math.sqrt((2 * q - 1) / (2 * q)) * (math.sqrt(2.0) if q == 1 else 1.0)
+    p, dp = [pmm], [m * x / s * pmm]
+    for l in range(m + 1, L + 1):
+        prev2 = p[-2] if len(p) > 1 else torch.zeros_like(x)
+        p.append(((2 * l - 1) * x * p[-1] - math.sqrt((l - 1) ** 2 - m * m) * prev2) / math.sqrt(l * l - m * m))
+        dp.append((l * x * p[-1] - math.sqrt(l * l - m * m) * p[-2]) / s)
+    return torch.stack(p), torch.stack(dp), s
+
+
+def _exact_bwd(c, seed):
+    L, nr, nth, nv, ns = c["L"], c["nr"], c["nth"], c["nvec"], c["nscal"]
+    a = _spectra(c, seed)                                    # [k][j][c]
+    x, _ = _gauss(nth)
+    r = _radii(_params(c), nr)
+    out = torch.zeros((2 * L + 1, nth, nr, 3 * nv + ns), device="cuda", dtype=torch.float64)
+    for m in range(L + 1):
+        P, dP, s = _plm(L, m, x)
+        l = torch.arange(m, L + 1, device="cuda")
+        half = []
+        for mm in ((m, -m) if m else (0,)):
+            half.append(a[:, l * l + l + mm, :])              # [k][l][c]
+        mP = m * P / s
+        for q, mm in enumerate((m, -m) if m else (0,)):
+            here, other = half[q], half[1 - q] if m else half[0] * 0.0
+            sg = 1.0 if q == 0 else -1.0
+            o = out[L + mm]                                   # [theta][k][c]
+            for v in range(nv):
+                S = here[:, :, 3 * v] * (l * (l + 1.0)) / (r * r)[:, None]
+                D, T = here[:, :, 3 * v + 1] / r[:, None], here[:, :, 3 * v + 2] / r[:, None]
+                Do, To = other[:, :, 3 * v + 1] / r[:, None], other[:, :, 3 * v + 2] / r[:, None]
+                o[:, :, 3 * v] = (S @ P).T
+                o[:, :, 3 * v + 1] = (D @ dP + sg * (To @ mP)).T
+                o[:, :, 3 * v + 2] = (sg * (Do @ mP) - T @ dP).T
+            for q2 in range(ns):
+                o[:, :, 3 * nv + q2] = (here[:, :, 3 * nv + q2] @ P).T
+    return out.reshape(-1)
+
+
+def _exact_fwd(c, seed):
+    L, nr, nth, nv, ns = c["L"], c["nr"], c["nth"], c["nvec"], c["nscal"]
+    f = _fourier(c, seed, 3 * nv + ns)                        # [m][theta][k][c]
+    x, w = _gauss(nth)
+    r = _radii(_params(c), nr)
+    out = torch.zeros((nr, (L + 1) ** 2, 3 * nv + ns), device="cuda", dtype=torch.float64)
+    for m in range(L + 1):
+        P, dP, s = _plm(L, m, x)
+        l = torch.arange(m, L + 1, device="cuda").double()
+        ll = torch.where(l > 0, l * (l + 1), torch.ones_like(l))
+        g6 = (2 * l + 1) / (2.0 if m == 0 else 4.0)
+        g7 = torch.where(l > 0, g6 / ll, torch.ones_like(l))
+        Pw, dPw, mPw = P * w, dP * w, m * P / s * w
+        for mm in ((m, -m) if m else (0,)):
+            sg = 1.0 if mm >= 0 else -1.0
+            here, other = f[L + mm], f[L - mm]                # [theta][k][c]
+            j = (l * l + l + mm).long()
+            for v in range(nv):
+                R, T, F = (here[:, :, 3 * v + q] for q in range(3))
+                To, Fo = other[:, :, 3 * v + 1], other[:, :, 3 * v + 2]
+                out[:, j, 3 * v] = ((Pw @ R) * g7[:, None] * r * r).T
+                out[:, j, 3 * v + 1] = ((dPw @ T - sg * (mPw @ Fo)) * g7[:, None] * r).T
+                out[:, j, 3 * v + 2] = (-(sg * (mPw @ To) + dPw @ F) * g7[:, None] * r).T
+            for q in range(ns):
+                out[:, j, 3 * nv + q] = ((Pw @ here[:, :, 3 * nv + q]) * g6[:, None]).T
+    return out.reshape(-1)
+
+
+def _exact_products(c, seed):
+    L, nph, p = c["L"], c["nph"], _params(c)
+    x = _fourier(c, seed, 13)                                 # [m][theta][k][13]
+    z = torch.zeros((nph // 2 + 1,) + tuple(x.shape[1:]), device="cuda", dtype=torch.complex128)
+    z[0] = x[L]
+    z[1:L + 1] = 0.5 * (x[L + 1:] - 1j * x[:L].flip(0))
+    g = torch.fft.irfft(z * nph, n=nph, dim=0)
+    del z
+    u, w, b, j, t = (g[..., q:q + 3] for q in (0, 3, 6, 9, 12))
+    h = torch.cat([torch.linalg.cross(w, u) * p["coef_velo"], torch.linalg.cross(j, b) * p["coef_lor"],
+                   torch.linalg.cross(u, b) * p["coef_induct"], u * t[..., :1] * p["coef_temp"]], dim=-1)
+    del g
+    s = torch.fft.rfft(h, dim=0) / nph
+    out = torch.zeros((2 * L + 1,) + tuple(h.shape[1:]), device="cuda", dtype=torch.float64)
+    out[L] = s[0].real
+    out[L + 1:] = 2.0 * s[1:L + 1].real
+    out[:L] = -2.0 * s[1:L + 1].imag.flip(0)
+    return out.reshape(-1)
+
+
+def _exact_closure(c, seed):
+    par = torch.from_numpy(_mlp_params(seed)).cuda()
+    x, t = (v.double() for v in _closure_rows(c, seed))
+    nin, nh, no = closure.NIN, 256, closure.NOUT
+    size = [nh * nin, nh, nh * nh, nh, no * nh, no]
+    W1, b1, W2, b2, W3, b3 = torch.split(par, size)
+    W1, W2, W3 = (w.bfloat16().double() for w in (W1, W2, W3))
+    leaf = [v.double().clone().requires_grad_(c["kind"] == "closure_train") for v in (W1, b1, W2, b2, W3, b3)]
+    W1, b1, W2, b2, W3, b3 = leaf
+    act = torch.nn.functional.silu
+    y = act(act(x @ W1.view(nh, nin).T + b1) @ W2.view(nh, nh).T + b2) @ W3.view(no, nh).T + b3
+    if c["kind"] == "closure_forward":
+        return y
+    loss = ((y - t) ** 2).mean()
+    loss.backward()
+    return [float(loss), torch.cat([v.grad for v in leaf])]
+
+
+def exact(case, seed):
+    k = case["kind"]
+    fn = {"leg_bwd": _exact_bwd, "leg_fwd": _exact_fwd, "products": _exact_products,
+          "closure_train": _exact_closure, "closure_forward": _exact_closure}.get(k)
+    return fn(case, int(seed)) if fn else None
