@@ -79,11 +79,14 @@ def _log_int(rng, lo, hi):
     return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
 
 
-def _draw_shell(rng, nph_max, points_max):
+def _draw_shell(rng, prec, nph_max, points_max):
     """A shell: zonal grid, truncation (dealiased by 3/2, the odd one, or a
-    lower one), radial points; at most points_max values of (L+1)^2 nr."""
+    lower one), radial points; at most points_max values of (L+1)^2 nr.  The
+    mixed path takes colatitudes in multiples of 8, the float64 path any even
+    number."""
     nph = rng.choice([n for n in ZONAL if n <= nph_max])
-    nth = 2 * ((nph // 2 + 1) // 2)
+    step = 8 if prec == "mixed" else 2
+    nth = step * -(-nph // (2 * step))
     top = nph // 3
     L = rng.choice([top - 1, (nph - 1) // 3, rng.randint(max(8, top // 2), top - 1)])
     L = min(L, 255)
@@ -100,14 +103,14 @@ def draw(rng):
         return dict(kind=kind, rows=_log_int(rng, 1000, 266240))
     prec = rng.choice(["mixed", "fp64"])
     if kind in ("step", "host_step"):
-        sh = _draw_shell(rng, 576, 2_000_000)
+        sh = _draw_shell(rng, prec, 576, 2_000_000)
         E = rng.choice([1e-3, 1e-4])
         c = dict(kind=kind, prec=prec, **sh, E=E, Ra=float(rng.randint(80, 400)),
                  dt=(3e-3 if E == 1e-3 else 8e-4) / (sh["L"] + 1))
         if kind == "step":
             c.update(steps=rng.randint(1, 8), graph=rng.random() < 0.5, tuned=rng.random() < 0.5)
         return c
-    sh = _draw_shell(rng, 768, 3_000_000)
+    sh = _draw_shell(rng, prec, 768, 3_000_000)
     c = dict(kind=kind, prec=prec, **sh)
     if kind != "products":
         c.update(nvec=rng.randint(1, 4), nscal=rng.randint(0, 2))
