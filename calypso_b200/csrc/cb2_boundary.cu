@@ -47,11 +47,31 @@ int grow(void **buf, size_t *have, size_t need) {
   return 0;
 }
 
-// device table of one call: jj of each j_rlm, then (|m|, s) of each mp
+// Device tables of a call.  jo: (j_rlm, jj) in the order of jj, the library's
+// m-major index, so that consecutive entries are consecutive in the field
+// slots; mo: (mp, |m|, s, -) in the order of (|m|, s), so that the two orders
+// of a Fourier row follow each other; mpos: [|m|][s] -> mp (the last one the
+// table lists) or -1; jj and mq: by j_rlm and by mp.
 struct DevTab {
-  const int *jj = nullptr;   // nidx_rlm(2)
+  const int2 *jo = nullptr;  // nidx_rlm(2)
   const int *mq = nullptr;   // nidx_rtm(3) x 2: |m|, s (0 cos / order +m, 1 sin / order -m)
+  const int4 *mo = nullptr;  // nidx_rtm(3)
+  const int *mpos = nullptr; // (L + 1) x 2
 };
+
+// The device tables of the last call stay while a call's own tables hold the
+// same values: (l, m) of every j_rlm, m of every mp (the strides do not enter
+// the tables).  Checking, sorting and uploading 65536 modes took 0.35 ms of a
+// 1.6 ms call at L255; comparing the values takes about 0.02 ms.
+bool same_rlm(const Ctx &c, const cb2_sph_tables *t) {
+  const size_t n = 2 * (size_t)t->nidx_rlm[1];
+  return c.bnd_rlm_key.size() == n &&
+         std::memcmp(c.bnd_rlm_key.data(), t->idx_gl_1d_rlm_j + t->nidx_rlm[1], n * sizeof(int)) == 0;
+}
+bool same_rtm(const Ctx &c, const cb2_sph_tables *t) {
+  const size_t n = (size_t)t->nidx_rtm[2];
+  return c.bnd_rtm_key.size() == n && std::memcmp(c.bnd_rtm_key.data(), t->idx_gl_1d_rtm_m + n, n * sizeof(int)) == 0;
+}
 
 int check_tables(const Ctx &c, const cb2_sph_tables *t, bool need_rlm, bool need_rtp) {
   if (!t) { set_error("null index tables"); return CB2_ERR_ARG; }
@@ -62,7 +82,8 @@ int check_tables(const Ctx &c, const cb2_sph_tables *t, bool need_rlm, bool need
   }
   for (int q = 0; q < 3; q++)
     if (t->istep_rtm[q] < 1) { set_error("istep_rtm must be positive"); return CB2_ERR_ARG; }
-  for (int mp = 0; mp < t->nidx_rtm[2]; mp++) {
+  const bool known_m = same_rtm(c, t);
+  for (int mp = 0; !known_m && mp < t->nidx_rtm[2]; mp++) {
     const int m = t->idx_gl_1d_rtm_m[t->nidx_rtm[2] + mp];
     if (m < -c.L || m > c.L) { set_error("idx_gl_1d_rtm_m: order outside -L..L"); return CB2_ERR_ARG; }
   }
@@ -73,7 +94,8 @@ int check_tables(const Ctx &c, const cb2_sph_tables *t, bool need_rlm, bool need
       return CB2_ERR_ARG;
     }
     const int nj = t->nidx_rlm[1];
-    for (int j = 0; j < nj; j++) {
+    const bool known = same_rlm(c, t);
+    for (int j = 0; !known && j < nj; j++) {
       const int l = t->idx_gl_1d_rlm_j[nj + j], m = t->idx_gl_1d_rlm_j[2 * nj + j];
       if (l < 0 || l > c.L || m < -l || m > l) {
         set_error("idx_gl_1d_rlm_j: (l, m) outside the truncation");
@@ -113,20 +135,74 @@ int jj_host(const Ctx &c, int l, int m) {
   return c.h_moff[am] + ((m < 0) ? (c.L + 1 - am) : 0) + (l - am);
 }
 
-int upload_tables(Ctx &c, const cb2_sph_tables *t, bool rlm, DevTab *d) {
-  const int nj = rlm ? t->nidx_rlm[1] : 0, nm = t->nidx_rtm[2];
-  std::vector<int> h((size_t)nj + 2 * (size_t)nm);
-  for (int j = 0; j < nj; j++) h[j] = jj_host(c, t->idx_gl_1d_rlm_j[nj + j], t->idx_gl_1d_rlm_j[2 * nj + j]);
-  for (int mp = 0; mp < nm; mp++) {
-    const int m = t->idx_gl_1d_rtm_m[nm + mp];
-    h[nj + 2 * mp] = std::abs(m);
-    h[nj + 2 * mp + 1] = (m < 0) ? 1 : 0;
+int upload_rlm(Ctx &c, const cb2_sph_tables *t) {
+  const int nj = t->nidx_rlm[1];
+  const int *lm = t->idx_gl_1d_rlm_j + nj;   // l of every j, then m
+  // entries of equal key keep the table's order (a table may list a mode twice)
+  std::vector<int> head(c.jmax, -1), next(nj), h;
+  for (int j = nj - 1; j >= 0; j--) {
+    const int jj = jj_host(c, lm[j], lm[nj + j]);
+    next[j] = head[jj];
+    head[jj] = j;
   }
+  h.reserve(2 * (size_t)nj);
+  for (int jj = 0; jj < c.jmax; jj++)
+    for (int j = head[jj]; j >= 0; j = next[j]) { h.push_back(j); h.push_back(jj); }
+  c.bnd_rlm_key.clear();   // no key while the device table changes
   if (int rc = grow((void **)&c.d_bnd_tab, &c.bnd_tab_bytes, h.size() * sizeof(int))) return rc;
   CB2_CUDA(cudaMemcpyAsync(c.d_bnd_tab, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
-  d->jj = c.d_bnd_tab;
-  d->mq = c.d_bnd_tab + nj;
+  c.bnd_rlm_key.assign(lm, lm + 2 * (size_t)nj);
   return 0;
+}
+
+// [mo: nm x 4][mq: nm x 2][mpos: (L + 1) x 2]
+int upload_rtm(Ctx &c, const cb2_sph_tables *t) {
+  const int nm = t->nidx_rtm[2], M1 = c.L + 1;
+  const int *om = t->idx_gl_1d_rtm_m + nm;
+  std::vector<int> head(2 * M1, -1), next(nm), mpos(2 * (size_t)M1, -1), h;
+  for (int mp = nm - 1; mp >= 0; mp--) {
+    const int key = 2 * std::abs(om[mp]) + (om[mp] < 0);
+    next[mp] = head[key];
+    head[key] = mp;
+    if (mpos[key] < 0) mpos[key] = mp;
+  }
+  h.reserve(6 * (size_t)nm + mpos.size());
+  for (int key = 0; key < 2 * M1; key++)
+    for (int mp = head[key]; mp >= 0; mp = next[mp]) {
+      h.push_back(mp); h.push_back(key >> 1); h.push_back(key & 1); h.push_back(0);
+    }
+  for (int mp = 0; mp < nm; mp++) { h.push_back(std::abs(om[mp])); h.push_back((om[mp] < 0) ? 1 : 0); }
+  h.insert(h.end(), mpos.begin(), mpos.end());
+  c.bnd_rtm_key.clear();
+  if (int rc = grow((void **)&c.d_bnd_mtab, &c.bnd_mtab_bytes, h.size() * sizeof(int))) return rc;
+  CB2_CUDA(cudaMemcpyAsync(c.d_bnd_mtab, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
+  c.bnd_rtm_key.assign(om, om + nm);
+  return 0;
+}
+
+int device_tables(Ctx &c, const cb2_sph_tables *t, bool rlm, DevTab *d) {
+  if (rlm && !same_rlm(c, t))
+    if (int rc = upload_rlm(c, t)) return rc;
+  if (!same_rtm(c, t))
+    if (int rc = upload_rtm(c, t)) return rc;
+  const int nm = t->nidx_rtm[2];
+  d->jo = reinterpret_cast<const int2 *>(c.d_bnd_tab);
+  d->mo = reinterpret_cast<const int4 *>(c.d_bnd_mtab);
+  d->mq = c.d_bnd_mtab + 4 * (size_t)nm;
+  d->mpos = d->mq + 2 * (size_t)nm;
+  return 0;
+}
+
+// nidx x istep cover 0 .. product - 1 without a gap or an overlap
+bool dense3(const int *n, const int *st) {
+  int q[3] = {0, 1, 2};
+  std::sort(q, q + 3, [&](int a, int b) { return st[a] != st[b] ? st[a] < st[b] : n[a] < n[b]; });
+  long long want = 1;
+  for (int i = 0; i < 3; i++) {
+    if (n[q[i]] > 1 && st[q[i]] != want) return false;
+    want *= n[q[i]];
+  }
+  return true;
 }
 
 // the caller's buffer on the device: itself, or a copy in staging buffer `which`
@@ -149,9 +225,11 @@ int device_out(Ctx &c, double *p, size_t n, int which, double **out) {
   return 0;
 }
 
-int finish_out(Ctx &c, double *host, const double *dev, size_t n) {
+// result to the caller's buffer; the stream drains here unless the caller
+// reads the status word next, which waits for it anyway
+int finish_out(Ctx &c, double *host, const double *dev, size_t n, bool drain = true) {
   if (host != dev) CB2_CUDA(cudaMemcpyAsync(host, dev, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-  CB2_CUDA(cudaStreamSynchronize(c.stream));
+  if (drain) CB2_CUDA(cudaStreamSynchronize(c.stream));
   return 0;
 }
 
@@ -183,23 +261,125 @@ std::vector<Chunk> chunks(int prec, int nvec, int nscal) {
 
 constexpr int kBnd = 256;
 
-// rlm buffer -> work slots (device order), one thread per (j_rlm, k)
-__global__ void k_rlm_to_slots(int nj, int nr, int ncomp, int is0, int is1, int comp0, int nq, int slot0,
-                               const int *jj, const double *WR, double *f, size_t fs, int jmax) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
-  if (j >= nj || k >= nr) return;
-  const size_t src = (size_t)ncomp * ((size_t)k * is0 + (size_t)j * is1) + comp0;
-  const size_t dst = (size_t)k * jmax + jj[j];
-  for (int q = 0; q < nq; q++) f[(size_t)(slot0 + q) * fs + dst] = WR[src + q];
+// e / n for 0 <= e < 2^16 and 1 <= n <= 2^15: (e * ceil(2^32 / n)) >> 32
+struct FastDiv {
+  unsigned n, mul;
+  explicit FastDiv(int d) : n((unsigned)d), mul((unsigned)((0x100000000ull + d - 1) / d)) {}
+  __device__ __forceinline__ int div(int e) const { return n == 1 ? e : (int)__umulhi((unsigned)e, mul); }
+};
+
+// rlm buffer <-> work slots (device order).  The slots run along jj, the
+// rlm buffer along the nq components of a mode (a run of 8 nq bytes): a block
+// takes JT modes of consecutive jj at one radial level and turns them round
+// in shared memory, so both sides move in whole runs: bound by the runs'
+// partial sectors.  At L255 / Nr65 / 11 components 198 us inwards (3.8 TB/s);
+// a thread per mode, whose 8-byte slot writes scattered over the orders, took
+// 482 us.  Outwards at L170 / Nr49 / 12 components 73 us against 176.
+constexpr int JT = 64;
+
+template <bool TO_SLOTS>
+__global__ void __launch_bounds__(kBnd)
+k_rlm_slots(int nj, int ncomp, int is0, int is1, int comp0, FastDiv nq, int slot0, const int2 *__restrict__ jo,
+            double *__restrict__ rlm, double *__restrict__ f, size_t fs, int jmax) {
+  extern __shared__ double tile[];   // [JT][nq | 1]
+  __shared__ int2 ent[JT];
+  const int i0 = blockIdx.x * JT, k = blockIdx.y, nt = min(JT, nj - i0), n = (int)nq.n, pitch = n | 1;
+  if (threadIdx.x < nt) ent[threadIdx.x] = jo[i0 + threadIdx.x];
+  __syncthreads();
+  double *r0 = rlm + (size_t)ncomp * ((size_t)k * is0) + comp0;
+  double *f0 = f + (size_t)slot0 * fs + (size_t)k * jmax;
+  if (TO_SLOTS) {
+    for (int e = threadIdx.x; e < nt * n; e += kBnd) {
+      const int i = nq.div(e), q = e - i * n;
+      tile[i * pitch + q] = __ldg(r0 + (size_t)ncomp * ent[i].x * is1 + q);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < JT * n; e += kBnd) {
+      const int q = e / JT, i = e % JT;
+      if (i < nt) f0[(size_t)q * fs + ent[i].y] = tile[i * pitch + q];
+    }
+  } else {
+    for (int e = threadIdx.x; e < JT * n; e += kBnd) {
+      const int q = e / JT, i = e % JT;
+      if (i < nt) tile[i * pitch + q] = __ldg(f0 + (size_t)q * fs + ent[i].y);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nt * n; e += kBnd) {
+      const int i = nq.div(e), q = e - i * n;
+      r0[(size_t)ncomp * ent[i].x * is1 + q] = tile[i * pitch + q];
+    }
+  }
 }
 
-__global__ void k_slots_to_rlm(int nj, int nr, int ncomp, int is0, int is1, int comp0, int nq, int slot0,
-                               const int *jj, const double *f, size_t fs, int jmax, double *WS) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
-  if (j >= nj || k >= nr) return;
-  const size_t dst = (size_t)ncomp * ((size_t)k * is0 + (size_t)j * is1) + comp0;
-  const size_t src = (size_t)k * jmax + jj[j];
-  for (int q = 0; q < nq; q++) WS[dst + q] = f[(size_t)(slot0 + q) * fs + src];
+// Order-major Fourier rows <-> rtm buffer where the radius runs faster than
+// the order (istep_rtm(1) <= istep_rtm(3), the reference's own order): a
+// block takes one colatitude of one order, the lanes along the buffer's
+// (k, component) runs.  One thread per (theta, k) and order with its
+// components in a loop (k_four_to_rtm / k_rtm_to_four, which stay for the
+// other stride orders) wrote 8 bytes of every line at a time: 1112 us
+// outwards at L255 / Nr65 / 11 components, now 295 us (5.6 TB/s); 323 us
+// inwards at L170 / Nr49 / 12, now 140 us.  Bound by HBM.
+struct CompOff {
+  int off[13];     // element offset of component c (s = 0) within its block's radial level
+  int inD;         // bit c: component c sits in the D block
+};
+
+constexpr int RTH = 8;   // colatitudes a block: that many independent loads a thread
+
+__global__ void __launch_bounds__(kBnd)
+k_rows_to_rtm(MLayout ml, CompOff co, FastDiv nc, int ncomp, int is0, int is1, int is2, int comp0,
+              const int4 *__restrict__ mo, double *__restrict__ WS) {
+  __shared__ int off[13];
+  const int4 me = mo[blockIdx.x];   // mp, |m|, s
+  const int th0 = blockIdx.y * RTH, nt = min(RTH, ml.nth - th0), n = (int)nc.n;
+  if (threadIdx.x < 13) off[threadIdx.x] = co.off[threadIdx.x];
+  __syncthreads();
+  const float *P = ml.P + ((size_t)me.y * ml.nth + th0) * ml.sP() + me.z;
+  const float *D = ml.D + ((size_t)me.y * ml.nth + th0) * ml.sD() + me.z;
+  const int rP = ml.rpP(), rD = ml.rpD();
+  double *w = WS + (size_t)ncomp * ((size_t)th0 * is1 + (size_t)me.x * is2) + comp0;
+  const size_t wt = (size_t)ncomp * is1;
+  for (int e = threadIdx.x; e < ml.nr * n; e += kBnd) {
+    const int k = nc.div(e), c = e - k * n;
+    const bool d = co.inD >> c & 1;
+    const float *src = d ? D + k * rD + off[c] : P + k * rP + off[c];
+    const size_t st = d ? ml.sD() : ml.sP();
+    double *o = w + (size_t)ncomp * k * is0 + c;
+    float v[RTH];
+#pragma unroll
+    for (int i = 0; i < RTH; i++) v[i] = (i < nt) ? __ldg(src + i * st) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < RTH; i++)
+      if (i < nt) o[i * wt] = (double)v[i];
+  }
+}
+
+// every element of the order's rows, both signs: an order the table does not
+// list is zero, as are the sine part of m = 0 and the padding
+__global__ void __launch_bounds__(kBnd)
+k_rtm_to_rows(MLayout ml, int ncomp, int is0, int is1, int is2, int comp0, FastDiv rP, FastDiv rD,
+              const int *__restrict__ mpos, const double *__restrict__ WR) {
+  const int m = blockIdx.x, th = blockIdx.y, nr = ml.nr, nv = ml.nvec;
+  const int mp0 = mpos[2 * m], mp1 = (m > 0) ? mpos[2 * m + 1] : -1;
+  const double *w0 = WR + (size_t)ncomp * ((size_t)th * is1 + (size_t)max(mp0, 0) * is2) + comp0;
+  const double *w1 = WR + (size_t)ncomp * ((size_t)th * is1 + (size_t)max(mp1, 0) * is2) + comp0;
+  const size_t ks = (size_t)ncomp * is0;
+  float *P = ml.P + ((size_t)m * ml.nth + th) * ml.sP();
+  const int eP = nr * (int)rP.n, eP4 = (int)ml.sP(), eD = nr * (int)rD.n, eD4 = (int)ml.sD();
+  for (int e = threadIdx.x; e < eP4; e += kBnd) {
+    const int k = rP.div(e), x = e - k * (int)rP.n, fl = x >> 1, c = (fl < nv) ? 3 * fl : 2 * nv + fl;
+    float v = 0.0f;
+    if (e < eP && ((x & 1) ? mp1 : mp0) >= 0) v = (float)__ldg(((x & 1) ? w1 : w0) + k * ks + c);
+    P[e] = v;
+  }
+  if (nv == 0) return;
+  float *D = ml.D + ((size_t)m * ml.nth + th) * ml.sD();
+  for (int e = threadIdx.x; e < eD4; e += kBnd) {
+    const int k = rD.div(e), x = e - k * (int)rD.n, c = 3 * (x >> 2) + 1 + ((x & 3) >> 1);
+    float v = 0.0f;
+    if (e < eD && ((x & 1) ? mp1 : mp0) >= 0) v = (float)__ldg(((x & 1) ? w1 : w0) + k * ks + c);
+    D[e] = v;
+  }
 }
 
 // Fourier rows of the context (float64 [theta][k][c][slot] with nc
@@ -281,6 +461,58 @@ size_t four_bytes(const Ctx &c) {
                                    : mlayout_floats(c) * sizeof(float);
 }
 
+// Fourier rows -> rtm buffer of one chunk
+void rows_out(Ctx &c, const cb2_sph_tables *t, const DevTab &dt, const FourView &fv, int ncomp, int comp0, double *dWS) {
+  const int *is = t->istep_rtm, nm = t->nidx_rtm[2];
+  if (!fv.f64 && is[0] <= is[2] && c.nr * fv.nc < (1 << 16) && c.nth < (1 << 16)) {
+    CompOff co{};
+    const MLayout &ml = fv.ml;
+    for (int q = 0; q < fv.nc; q++) {
+      const int v = q / 3, cc = q - 3 * v;
+      if (q >= 3 * ml.nvec) co.off[q] = 2 * (ml.nvec + q - 3 * ml.nvec);
+      else if (cc == 0) co.off[q] = 2 * v;
+      else { co.off[q] = 4 * v + 2 * (cc - 1); co.inD |= 1 << q; }
+    }
+    k_rows_to_rtm<<<dim3(nm, cdiv(c.nth, RTH)), kBnd, 0, c.stream>>>(ml, co, FastDiv(fv.nc), ncomp, is[0], is[1], is[2], comp0,
+                                                          dt.mo, dWS);
+    return;
+  }
+  k_four_to_rtm<<<dim3(cdiv((long)c.nth * c.nr, kBnd), nm), kBnd, 0, c.stream>>>(fv, c.nth, c.nr, ncomp, is[0], is[1],
+                                                                                 is[2], comp0, dt.mq, dWS);
+}
+
+// rtm buffer -> every element of the Fourier rows of one chunk
+int rows_in(Ctx &c, const cb2_sph_tables *t, const DevTab &dt, const FourView &fv, int ncomp, int comp0,
+            const double *dWR) {
+  const int *is = t->istep_rtm, nm = t->nidx_rtm[2];
+  if (!fv.f64 && is[0] <= is[2] && fv.ml.sP() < (1u << 16) && fv.ml.sD() < (1u << 16) && c.nth < (1 << 16)) {
+    const MLayout &ml = fv.ml;
+    k_rtm_to_rows<<<dim3(c.L + 1, c.nth), kBnd, 0, c.stream>>>(ml, ncomp, is[0], is[1], is[2], comp0, FastDiv(ml.rpP()),
+                                                               FastDiv(std::max(1, ml.rpD())), dt.mpos, dWR);
+    return 0;
+  }
+  CB2_CUDA(cudaMemsetAsync(fv.f64 ? (void *)fv.f64 : (void *)fv.ml.P, 0, four_bytes(c), c.stream));
+  k_rtm_to_four<<<dim3(cdiv((long)c.nth * c.nr, kBnd), nm), kBnd, 0, c.stream>>>(fv, c.nth, c.nr, ncomp, is[0], is[1],
+                                                                                 is[2], comp0, dt.mq, dWR);
+  return 0;
+}
+
+// clears what a call will not write of an rtm (rlm) buffer of n values: the
+// whole buffer, or only its tail where the tables cover the rest densely
+int clear_rtm(Ctx &c, const cb2_sph_tables *t, int ncomp, int nwritten, size_t n, double *dWS) {
+  const size_t ext = rtm_extent(t, ncomp);
+  const size_t from = (ncomp == nwritten && dense3(t->nidx_rtm, t->istep_rtm)) ? ext : 0;
+  if (from < n) CB2_CUDA(cudaMemsetAsync(dWS + from, 0, (n - from) * sizeof(double), c.stream));
+  return 0;
+}
+int clear_rlm(Ctx &c, const cb2_sph_tables *t, int ncomp, int nwritten, size_t n, double *dWS) {
+  const size_t ext = rlm_extent(t, ncomp);
+  const int nn[3] = {t->nidx_rlm[0], t->nidx_rlm[1], 1}, st[3] = {t->istep_rlm[0], t->istep_rlm[1], 1 << 30};
+  const size_t from = (ncomp == nwritten && dense3(nn, st)) ? ext : 0;
+  if (from < n) CB2_CUDA(cudaMemsetAsync(dWS + from, 0, (n - from) * sizeof(double), c.stream));
+  return 0;
+}
+
 int leg_args_ok(const Ctx &c, int ncomp, int nvec, int nscal) {
   if (nvec < 0 || nscal < 0 || nvec + nscal == 0 || ncomp < 3 * nvec + nscal) {
     set_error("Legendre transform: need nvector, nscalar >= 0, at least one field, ncomp >= 3 nvector + nscalar");
@@ -314,11 +546,11 @@ int cb2_leg_bwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, int nvector, int
   const double *dWR;
   double *dWS;
   int rc;
-  if ((rc = upload_tables(*c, t, true, &dt)) || (rc = device_in(*c, WR, n_WR, 0, &dWR)) ||
+  if ((rc = device_tables(*c, t, true, &dt)) || (rc = device_in(*c, WR, n_WR, 0, &dWR)) ||
       (rc = device_out(*c, WS, n_WS, 1, &dWS)))
     return rc;
   // the callee clears WS, as the reference's backward transforms do
-  CB2_CUDA(cudaMemsetAsync(dWS, 0, n_WS * sizeof(double), c->stream));
+  if ((rc = clear_rtm(*c, t, ncomp, 3 * nvector + nscalar, n_WS, dWS))) return rc;
   const int nj = t->nidx_rlm[1];
   for (const Chunk &ch : chunks(c->prec, nvector, nscalar)) {
     const int nc = ch.nc();
@@ -329,21 +561,19 @@ int cb2_leg_bwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, int nvector, int
     // modes the table leaves out are zero
     if (nj < c->jmax)
       CB2_CUDA(cudaMemsetAsync(c->fld(MADV), 0, (size_t)nc * c->fsize() * sizeof(double), c->stream));
-    k_rlm_to_slots<<<dim3(cdiv(nj, kBnd), c->nr), kBnd, 0, c->stream>>>(
-        nj, c->nr, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, nc, MADV, dt.jj, dWR, c->d_f, c->fsize(),
-        c->jmax);
+    k_rlm_slots<true><<<dim3(cdiv(nj, JT), c->nr), kBnd, JT * (nc | 1) * sizeof(double), c->stream>>>(
+        nj, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, FastDiv(nc), MADV, dt.jo, const_cast<double *>(dWR),
+        c->d_f, c->fsize(), c->jmax);
     if (c->prec == CB2_PREC_FP64) {
       leg_bwd_f64(*c, ch.nv, ch.ns, slots, (double *)c->d_four);
     } else {
       const MLayout l = mlayout(*c, c->d_four, ch.nv, ch.ns);
       if ((rc = leg_bwd_mixed(*c, slots, l))) return rc;
     }
-    k_four_to_rtm<<<dim3(cdiv((long)c->nth * c->nr, kBnd), t->nidx_rtm[2]), kBnd, 0, c->stream>>>(
-        four_view(*c, ch.nv, ch.ns), c->nth, c->nr, ncomp, t->istep_rtm[0], t->istep_rtm[1], t->istep_rtm[2],
-        ch.comp0, dt.mq, dWS);
+    rows_out(*c, t, dt, four_view(*c, ch.nv, ch.ns), ncomp, ch.comp0, dWS);
   }
   CB2_CUDA(cudaGetLastError());
-  if ((rc = finish_out(*c, WS, dWS, n_WS))) return rc;
+  if ((rc = finish_out(*c, WS, dWS, n_WS, false))) return rc;
   return check_status(*c);
 }
 
@@ -360,32 +590,29 @@ int cb2_leg_fwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, int nvector, int
   const double *dWR;
   double *dWS;
   int rc;
-  if ((rc = upload_tables(*c, t, true, &dt)) || (rc = device_in(*c, WR, n_WR, 0, &dWR)) ||
+  if ((rc = device_tables(*c, t, true, &dt)) || (rc = device_in(*c, WR, n_WR, 0, &dWR)) ||
       (rc = device_out(*c, WS, n_WS, 1, &dWS)))
     return rc;
-  CB2_CUDA(cudaMemsetAsync(dWS, 0, n_WS * sizeof(double), c->stream));
+  if ((rc = clear_rlm(*c, t, ncomp, 3 * nvector + nscalar, n_WS, dWS))) return rc;
   const int nj = t->nidx_rlm[1];
   for (const Chunk &ch : chunks(c->prec, nvector, nscalar)) {
     const int nc = ch.nc();
     int slots[13];
     for (int g = 0; g < ch.nv; g++) slots[g] = MADV + 3 * g;
     for (int s = 0; s < ch.ns; s++) slots[ch.nv + s] = MADV + 3 * ch.nv + s;
-    CB2_CUDA(cudaMemsetAsync(c->d_four, 0, four_bytes(*c), c->stream));
-    k_rtm_to_four<<<dim3(cdiv((long)c->nth * c->nr, kBnd), t->nidx_rtm[2]), kBnd, 0, c->stream>>>(
-        four_view(*c, ch.nv, ch.ns), c->nth, c->nr, ncomp, t->istep_rtm[0], t->istep_rtm[1], t->istep_rtm[2],
-        ch.comp0, dt.mq, dWR);
+    if ((rc = rows_in(*c, t, dt, four_view(*c, ch.nv, ch.ns), ncomp, ch.comp0, dWR))) return rc;
     if (c->prec == CB2_PREC_FP64) {
       leg_fwd_f64(*c, ch.nv, ch.ns, (const double *)c->d_four, slots);
     } else {
       const MLayout l = mlayout(*c, c->d_four, ch.nv, ch.ns);
       if ((rc = leg_fwd_mixed(*c, l, slots))) return rc;
     }
-    k_slots_to_rlm<<<dim3(cdiv(nj, kBnd), c->nr), kBnd, 0, c->stream>>>(
-        nj, c->nr, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, nc, MADV, dt.jj, c->d_f, c->fsize(),
-        c->jmax, dWS);
+    k_rlm_slots<false><<<dim3(cdiv(nj, JT), c->nr), kBnd, JT * (nc | 1) * sizeof(double), c->stream>>>(
+        nj, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, FastDiv(nc), MADV, dt.jo, dWS, c->d_f, c->fsize(),
+        c->jmax);
   }
   CB2_CUDA(cudaGetLastError());
-  if ((rc = finish_out(*c, WS, dWS, n_WS))) return rc;
+  if ((rc = finish_out(*c, WS, dWS, n_WS, false))) return rc;
   return check_status(*c);
 }
 
@@ -398,16 +625,14 @@ int cb2_fft_bwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, size_t n_WR, con
   const double *dWR;
   double *dF;
   int rc;
-  if ((rc = upload_tables(*c, t, false, &dt)) || (rc = device_in(*c, WR, n_WR, 0, &dWR)) ||
+  if ((rc = device_tables(*c, t, false, &dt)) || (rc = device_in(*c, WR, n_WR, 0, &dWR)) ||
       (rc = device_out(*c, fld_rtp, nout, 1, &dF)))
     return rc;
   if ((rc = grow((void **)&c->d_bnd_grid, &c->bnd_grid_bytes, 13 * nnod * sizeof(double)))) return rc;
   for (int c0 = 0; c0 < ncomp; c0 += 13) {
     const int nc = std::min(13, ncomp - c0);
-    CB2_CUDA(cudaMemsetAsync(c->d_four, 0, four_bytes(*c), c->stream));
     FourView fv = four_view(*c, 0, nc);
-    k_rtm_to_four<<<dim3(cdiv((long)c->nth * c->nr, kBnd), t->nidx_rtm[2]), kBnd, 0, c->stream>>>(
-        fv, c->nth, c->nr, ncomp, t->istep_rtm[0], t->istep_rtm[1], t->istep_rtm[2], c0, dt.mq, dWR);
+    if ((rc = rows_in(*c, t, dt, fv, ncomp, c0, dWR))) return rc;
     if (c->prec == CB2_PREC_FP64) fft_backward_grid<double>(*c, nc, (const double *)c->d_four, c->d_bnd_grid);
     else fft_backward_grid_m(*c, fv.ml, c->d_bnd_grid);
     k_grid_to_rtp<<<cdiv((long)nnod, kBnd), kBnd, 0, c->stream>>>(nc, c->nr, c->nth, c->nph, t->istep_rtp[0],
@@ -430,19 +655,15 @@ int cb2_fft_products(cb2_ctx *c, const cb2_sph_tables *t, size_t n_WR, const dou
   const double *dWR;
   double *dWS;
   int rc;
-  if ((rc = upload_tables(*c, t, false, &dt)) || (rc = device_in(*c, WR, n_WR, 0, &dWR)) ||
+  if ((rc = device_tables(*c, t, false, &dt)) || (rc = device_in(*c, WR, n_WR, 0, &dWR)) ||
       (rc = device_out(*c, WS, n_WS, 1, &dWS)))
     return rc;
-  CB2_CUDA(cudaMemsetAsync(dWS, 0, n_WS * sizeof(double), c->stream));
-  CB2_CUDA(cudaMemsetAsync(c->d_four, 0, four_bytes(*c), c->stream));
+  if ((rc = clear_rtm(*c, t, 12, 12, n_WS, dWS))) return rc;
   const FourView fin = four_view(*c, 4, 1), fout = four_view(*c, 4, 0, c->d_four2);
-  const dim3 grid(cdiv((long)c->nth * c->nr, kBnd), t->nidx_rtm[2]);
-  k_rtm_to_four<<<grid, kBnd, 0, c->stream>>>(fin, c->nth, c->nr, 13, t->istep_rtm[0], t->istep_rtm[1],
-                                             t->istep_rtm[2], 0, dt.mq, dWR);
+  if ((rc = rows_in(*c, t, dt, fin, 13, 0, dWR))) return rc;
   if (c->prec == CB2_PREC_FP64) fft_products<double>(*c, (const double *)c->d_four, (double *)c->d_four2);
   else fft_products_m(*c, fin.ml, fout.ml);
-  k_four_to_rtm<<<grid, kBnd, 0, c->stream>>>(fout, c->nth, c->nr, 12, t->istep_rtm[0], t->istep_rtm[1],
-                                             t->istep_rtm[2], 0, dt.mq, dWS);
+  rows_out(*c, t, dt, fout, 12, 0, dWS);
   CB2_CUDA(cudaGetLastError());
   return finish_out(*c, WS, dWS, n_WS);
 }
@@ -456,11 +677,11 @@ int cb2_fft_fwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, const double *fr
   const double *dF;
   double *dWS;
   int rc;
-  if ((rc = upload_tables(*c, t, false, &dt)) || (rc = device_in(*c, frc_rtp, nin, 0, &dF)) ||
+  if ((rc = device_tables(*c, t, false, &dt)) || (rc = device_in(*c, frc_rtp, nin, 0, &dF)) ||
       (rc = device_out(*c, WS, n_WS, 1, &dWS)))
     return rc;
   if ((rc = grow((void **)&c->d_bnd_grid, &c->bnd_grid_bytes, 13 * nnod * sizeof(double)))) return rc;
-  CB2_CUDA(cudaMemsetAsync(dWS, 0, n_WS * sizeof(double), c->stream));
+  if ((rc = clear_rtm(*c, t, ncomp, ncomp, n_WS, dWS))) return rc;
   for (int c0 = 0; c0 < ncomp; c0 += 13) {
     const int nc = std::min(13, ncomp - c0);
     k_rtp_to_grid<<<cdiv((long)nnod, kBnd), kBnd, 0, c->stream>>>(nc, c->nr, c->nth, c->nph, t->istep_rtp[0],
@@ -469,8 +690,7 @@ int cb2_fft_fwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, const double *fr
     FourView fv = four_view(*c, 0, nc);
     if (c->prec == CB2_PREC_FP64) fft_forward_grid<double>(*c, nc, c->d_bnd_grid, (double *)c->d_four);
     else fft_forward_grid_m(*c, c->d_bnd_grid, fv.ml);
-    k_four_to_rtm<<<dim3(cdiv((long)c->nth * c->nr, kBnd), t->nidx_rtm[2]), kBnd, 0, c->stream>>>(
-        fv, c->nth, c->nr, ncomp, t->istep_rtm[0], t->istep_rtm[1], t->istep_rtm[2], c0, dt.mq, dWS);
+    rows_out(*c, t, dt, fv, ncomp, c0, dWS);
   }
   CB2_CUDA(cudaGetLastError());
   return finish_out(*c, WS, dWS, n_WS);
