@@ -272,6 +272,612 @@ k_tc_gemm(int M, int N, int NT, int K, const TAT *__restrict__ A, int lda, const
   if (warp == 0) tc::tmem_dealloc(tmem, tmem_cols);
 }
 
+// ---------------------------------------------------------------------------
+// The network in one kernel a pass (k_mlp_fwd), its data gradient in one
+// (k_mlp_bwd) and every weight and bias gradient in one (k_mlp_wgrad), for
+// the sizes of fused_ok: F <= 32 inputs, H a multiple of 32 up to 256, O <= 8.
+// Three GEMMs with the activations between them in memory moved 1.6 GB for
+// 266240 rows (2031 us: the GEMMs, whose threads read a row each, 1510, bias
+// and SiLU 505); kept in tensor and shared memory the pass reads 64 and
+// writes 20 bytes a row and takes 189 us, bound by the SiLU epilogue (an
+// __expf and a divide per unit and layer) and the operand split.  A training
+// pass of 16384 rows: 35 + 45 + 69 us of kernels, before 500 us.
+//
+// A CTA keeps the bfloat16 weights in shared memory and walks tiles of 128
+// rows.  Warps 0-7 are the epilogue: warp w reads tensor-memory lanes
+// 32 (w & 3) .. + 31, one row a thread, the warps 0-3 (group 0) the even and
+// 4-7 (group 1) the odd chunks of 32 columns.  A chunk of an activation is
+// split into bfloat16 hi + lo and written as the next product's A operand
+// into one of ML_ST stages; warp 8 issues the MMAs of a chunk as soon as it
+// is there, so the second product runs behind the first one's epilogue.  The
+// last layer (O <= 8 columns) is float32 FMAs on the thread's row.
+constexpr int ML_EPI = 256, ML_THREADS = ML_EPI + 32, ML_ST = 3, ML_O = 8;
+constexpr uint32_t ML_STAGE = 2 * GA_BYTES;   // hi and lo of 128 rows x 32 columns
+
+struct MlpArgs {
+  long long n;
+  int F, H, O, vec;              // vec: rows of X can be read 16 bytes at a time
+  const float *X, *b1, *b2, *b3;
+  const __nv_bfloat16 *W1, *W2, *W3;
+  float *Y;                      // forward output, n x O
+  // training: targets, 2 / (n O), pre-activations, dL/dY, loss partial sums
+  // (4 a tile), and the data gradients of the hidden layers
+  const float *T;
+  float scale;
+  float *Z1, *Z2, *dY, *dZ2, *dZ1;
+  double *part;
+  int *status;
+  unsigned long long wait_ns;
+};
+
+struct MlpBars {
+  uint64_t full[ML_ST], empty[ML_ST], d1, d2, fin;
+  uint32_t tmem;
+  int abort;
+};
+
+struct MlpLayout {
+  uint32_t w2, w1, st, b1, b2, w3, yp, bar, total;
+};
+__host__ __device__ inline MlpLayout mlp_layout(int H) {
+  MlpLayout o;
+  uint32_t p = 0;
+  o.w2 = p; p += (uint32_t)H * H * 2;
+  o.w1 = p; p += (uint32_t)H * 64;
+  o.st = p; p += ML_ST * ML_STAGE;
+  o.b1 = p; p += (uint32_t)H * 4;
+  o.b2 = p; p += (uint32_t)H * 4;
+  o.w3 = p; p += (uint32_t)H * ML_O * 4;
+  o.yp = p; p += 128 * ML_O * 4;
+  o.bar = p; p += 128;
+  o.total = p;
+  return o;
+}
+
+__device__ inline float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
+__device__ inline float dsilu(float z) {
+  const float s = __fdividef(1.0f, 1.0f + __expf(-z));
+  return s * (1.0f + z * (1.0f - s));
+}
+
+// barrier of the 256 epilogue threads; true when any of them passes true
+__device__ inline bool epi_any(bool v) {
+  int r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.s32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred q, 1, 256, p;\n\t"
+      "selp.s32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((int)v)
+      : "memory");
+  return r != 0;
+}
+
+__device__ inline void tmem_ld32(uint32_t ta, float v[32]) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(ta)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 32 columns of one row into a stage, hi at 0 and lo at GA_BYTES
+__device__ inline void put_chunk(unsigned char *stage, int row, const float v[32]) {
+#pragma unroll
+  for (int c = 0; c < 4; c++) put_row8<2>(stage, GA_BYTES, row, c, v + 8 * c);
+}
+
+__device__ inline void store32(float *dst, const float v[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+}
+__device__ inline void load32(const float *src, float v[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    const float4 x = *reinterpret_cast<const float4 *>(src + j);
+    v[j] = x.x; v[j + 1] = x.y; v[j + 2] = x.z; v[j + 3] = x.w;
+  }
+}
+
+// one thread: acc (+)= (hi + lo) of `stage` times the bfloat16 tile `b`, ks
+// steps of 16 columns
+__device__ inline void mma_chunk(uint32_t acc, const unsigned char *stage, const unsigned char *b, uint32_t idesc, int ks,
+                                 bool first) {
+  const uint64_t ah = tc::smem_desc_sw64(stage), al = tc::smem_desc_sw64(stage + GA_BYTES), bd = tc::smem_desc_sw64(b);
+  for (int q = 0; q < ks; q++) {
+    const uint64_t o = (uint64_t)(q * 2);
+    tc::mma_f16(acc, ah + o, bd + o, idesc, (first && q == 0) ? 0u : 1u);
+    tc::mma_f16(acc, al + o, bd + o, idesc, 1u);
+  }
+}
+
+// shared set-up of the two row kernels: barriers, 512 tensor-memory columns,
+// biases and the last layer's weights
+__device__ inline void mlp_setup(const MlpArgs &a, unsigned char *base, const MlpLayout &lay, MlpBars *sb) {
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    for (int q = 0; q < ML_ST; q++) { tc::mbar_init(&sb->full[q], 4); tc::mbar_init(&sb->empty[q], 1); }
+    tc::mbar_init(&sb->d1, 1); tc::mbar_init(&sb->d2, 1); tc::mbar_init(&sb->fin, 1);
+    sb->abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  float *b1 = reinterpret_cast<float *>(base + lay.b1), *b2 = reinterpret_cast<float *>(base + lay.b2);
+  float *w3 = reinterpret_cast<float *>(base + lay.w3);
+  for (int c = tid; c < a.H; c += ML_THREADS) {
+    b1[c] = a.b1[c];
+    b2[c] = a.b2[c];
+#pragma unroll
+    for (int o = 0; o < ML_O; o++) w3[c * ML_O + o] = (o < a.O) ? __bfloat162float(a.W3[(size_t)o * a.H + c]) : 0.0f;
+  }
+}
+
+// releases tensor memory once every MMA has completed; a wait that ran out
+// is reported in *status
+__device__ inline void mlp_finish(const MlpArgs &a, MlpBars *sb, uint32_t tmem, bool bad) {
+  if (bad) sb->abort = 1;
+  tc::tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && sb->abort) atomicOr(a.status, CB2_STATUS_PIPE_TIMEOUT);
+  if (threadIdx.x >> 5 == 0) tc::tmem_dealloc(tmem, 512);
+}
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(ML_THREADS, 1)
+k_mlp_fwd(const __grid_constant__ MlpArgs a) {
+  extern __shared__ unsigned char g_smem_raw[];
+  unsigned char *base = tc::smem_base_1024(g_smem_raw);
+  const MlpLayout lay = mlp_layout(a.H);
+  MlpBars *sb = reinterpret_cast<MlpBars *>(base + lay.bar);
+  unsigned char *W2s = base + lay.w2, *W1s = base + lay.w1, *st0 = base + lay.st;
+  const float *b1 = reinterpret_cast<float *>(base + lay.b1), *b2 = reinterpret_cast<float *>(base + lay.b2);
+  const float *w3 = reinterpret_cast<float *>(base + lay.w3);
+  float *yp = reinterpret_cast<float *>(base + lay.yp);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = a.H, nch = H / 32;
+  mlp_setup(a, base, lay, sb);
+  if (warp == 0) tc::tmem_alloc(&sb->tmem, 512);
+  // W1 [n = unit][k = input] as one chunk, W2 [n][k] as H / 32 chunks
+  for (int e = tid; e < H * 4; e += ML_THREADS) {
+    const int r = e >> 2, c = e & 3;
+    __nv_bfloat16 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = (c * 8 + u < a.F) ? a.W1[(size_t)r * a.F + c * 8 + u] : __float2bfloat16_rn(0.0f);
+    *reinterpret_cast<uint4 *>(W1s + tc::sw64_chunk(r, c)) = *reinterpret_cast<const uint4 *>(v);
+  }
+  for (int e = tid; e < H * (H / 8); e += ML_THREADS) {
+    const int r = e / (H / 8), c8 = e - r * (H / 8);
+    *reinterpret_cast<uint4 *>(W2s + (size_t)(c8 >> 2) * H * 64 + tc::sw64_chunk(r, c8 & 3)) =
+        *reinterpret_cast<const uint4 *>(a.W2 + (size_t)r * H + c8 * 8);
+  }
+  tc::fence_proxy_async();
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = sb->tmem;
+  const long long ntile = (a.n + 127) / 128;
+  bool bad = false;
+  if (warp == ML_EPI / 32) {
+    if (lane == 0) {
+      const uint32_t idesc = tc::idesc_bf16_f32(128, H);
+      uint32_t q = 0;
+      for (long long t = blockIdx.x; t < ntile && !bad; t += gridDim.x)
+        for (int c = -1; c < nch; c++, q++) {   // c = -1: the input rows
+          const uint32_t s = q % ML_ST;
+          if (!tc::mbar_wait(&sb->full[s], (q / ML_ST) & 1, a.wait_ns)) { bad = true; break; }
+          tc::tc_fence_after();
+          if (c < 0) mma_chunk(tmem, st0 + s * ML_STAGE, W1s, idesc, (a.F + 15) / 16, true);
+          else mma_chunk(tmem + 256, st0 + s * ML_STAGE, W2s + (size_t)c * H * 64, idesc, 2, c == 0);
+          tc::mma_commit(&sb->empty[s]);
+          if (c < 0) tc::mma_commit(&sb->d1);
+          else if (c == nch - 1) tc::mma_commit(&sb->d2);
+        }
+      tc::mma_commit(&sb->fin);
+      if (!tc::mbar_wait(&sb->fin, 0)) bad = true;
+    }
+  } else {
+    const int qd = warp & 3, g = warp >> 2, r = qd * 32 + lane;
+    const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
+    // stage of sequence number q, once its last MMAs have read it
+    auto stage = [&](uint32_t q) {
+      if (q >= ML_ST && !bad && !tc::mbar_wait(&sb->empty[q % ML_ST], ((q / ML_ST) - 1) & 1, a.wait_ns)) bad = true;
+      bad = __any_sync(0xffffffffu, bad);
+      return st0 + (q % ML_ST) * ML_STAGE;
+    };
+    auto publish = [&](uint32_t q) {
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&sb->full[q % ML_ST]);
+    };
+    auto put_input = [&](long long t, uint32_t q) {
+      const long long row = t * 128 + r;
+      float x[32];
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (row < a.n && j < a.F) {
+          const float *p = a.X + row * a.F + j;
+          if (a.vec) v = __ldg(reinterpret_cast<const float4 *>(p));
+          else v = make_float4(p[0], j + 1 < a.F ? p[1] : 0.0f, j + 2 < a.F ? p[2] : 0.0f, j + 3 < a.F ? p[3] : 0.0f);
+        }
+        x[j] = v.x; x[j + 1] = v.y; x[j + 2] = v.z; x[j + 3] = v.w;
+      }
+      unsigned char *s = stage(q);
+      if (!bad) put_chunk(s, r, x);
+      publish(q);
+    };
+    uint32_t q0 = 0;
+    if (g == 0) put_input(blockIdx.x, 0);
+    int i = 0;
+    for (long long t = blockIdx.x; t < ntile; t += gridDim.x, i++, q0 += nch + 1) {
+      const long long row = t * 128 + r;
+      const bool in = row < a.n;
+      if (!bad && !tc::mbar_wait(&sb->d1, i & 1, a.wait_ns)) bad = true;
+      bad = __any_sync(0xffffffffu, bad);
+      tc::tc_fence_after();
+      for (int c = g; c < nch; c += 2) {
+        float z[32];
+        tmem_ld32(tl + c * 32, z);
+#pragma unroll
+        for (int j = 0; j < 32; j++) z[j] += b1[c * 32 + j];
+        if (TRAIN && in) store32(a.Z1 + row * H + c * 32, z);
+#pragma unroll
+        for (int j = 0; j < 32; j++) z[j] = silu(z[j]);
+        unsigned char *s = stage(q0 + 1 + c);
+        if (!bad) put_chunk(s, r, z);
+        tc::tc_fence_before();
+        publish(q0 + 1 + c);
+      }
+      // the next tile's input goes in front of this tile's last epilogue
+      if (g == 0 && t + gridDim.x < ntile) put_input(t + gridDim.x, q0 + nch + 1);
+      if (!bad && !tc::mbar_wait(&sb->d2, i & 1, a.wait_ns)) bad = true;
+      bad = __any_sync(0xffffffffu, bad);
+      tc::tc_fence_after();
+      float y[ML_O];
+#pragma unroll
+      for (int o = 0; o < ML_O; o++) y[o] = 0.0f;
+      for (int c = g; c < nch; c += 2) {
+        float z[32];
+        tmem_ld32(tl + 256 + c * 32, z);
+#pragma unroll
+        for (int j = 0; j < 32; j++) z[j] += b2[c * 32 + j];
+        if (TRAIN && in) store32(a.Z2 + row * H + c * 32, z);
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+          const float h = silu(z[j]);
+          const float4 wa = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O);
+          y[0] += h * wa.x; y[1] += h * wa.y; y[2] += h * wa.z; y[3] += h * wa.w;
+          if (a.O > 4) {
+            const float4 wb = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O + 4);
+            y[4] += h * wb.x; y[5] += h * wb.y; y[6] += h * wb.z; y[7] += h * wb.w;
+          }
+        }
+      }
+      if (g == 1) {
+#pragma unroll
+        for (int o = 0; o < ML_O; o++) yp[r * ML_O + o] = y[o];
+      }
+      // both groups have read the accumulators: the next tile may refill them
+      tc::tc_fence_before();
+      bad = epi_any(bad);
+      if (bad) break;
+      if (g == 0) {
+        double e = 0.0;
+#pragma unroll
+        for (int o = 0; o < ML_O; o++)
+          if (in && o < a.O) {
+            const float v = y[o] + yp[r * ML_O + o] + a.b3[o];
+            if (!TRAIN) {
+              a.Y[row * a.O + o] = v;
+            } else {
+              const float d = v - a.T[row * a.O + o];
+              a.dY[row * a.O + o] = d * a.scale;
+              e += (double)d * (double)d;
+            }
+          }
+        if (TRAIN) {
+          for (int u = 16; u > 0; u >>= 1) e += __shfl_xor_sync(0xffffffffu, e, u);
+          if (lane == 0) a.part[t * 4 + qd] = e;
+        }
+      }
+    }
+  }
+  mlp_finish(a, sb, tmem, bad);
+}
+
+// Data gradients of the hidden layers: dZ2 = (dY W3) SiLU'(Z2), written out
+// and, a chunk of 32 columns at a time, the A operand of dH1 = dZ2 W2 (the
+// CTA holds W2 transposed: [n = input unit][k = output unit]); then
+// dZ1 = dH1 SiLU'(Z1).  The same roles as k_mlp_fwd; tile i accumulates in
+// half i & 1 of tensor memory.
+__global__ void __launch_bounds__(ML_THREADS, 1)
+k_mlp_bwd(const __grid_constant__ MlpArgs a) {
+  extern __shared__ unsigned char g_smem_raw[];
+  unsigned char *base = tc::smem_base_1024(g_smem_raw);
+  const MlpLayout lay = mlp_layout(a.H);
+  MlpBars *sb = reinterpret_cast<MlpBars *>(base + lay.bar);
+  unsigned char *W2s = base + lay.w2, *st0 = base + lay.st;
+  const float *w3 = reinterpret_cast<float *>(base + lay.w3);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = a.H, nch = H / 32;
+  mlp_setup(a, base, lay, sb);
+  if (warp == 0) tc::tmem_alloc(&sb->tmem, 512);
+  for (int e = tid; e < H * (H / 8); e += ML_THREADS) {
+    const int r = e % H, c8 = e / H;   // lanes along the input units: coalesced reads of W2's rows
+    __nv_bfloat16 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = a.W2[(size_t)(c8 * 8 + u) * H + r];
+    *reinterpret_cast<uint4 *>(W2s + (size_t)(c8 >> 2) * H * 64 + tc::sw64_chunk(r, c8 & 3)) =
+        *reinterpret_cast<const uint4 *>(v);
+  }
+  tc::fence_proxy_async();
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = sb->tmem;
+  const long long ntile = (a.n + 127) / 128;
+  bool bad = false;
+  if (warp == ML_EPI / 32) {
+    if (lane == 0) {
+      const uint32_t idesc = tc::idesc_bf16_f32(128, H);
+      uint32_t q = 0;
+      int i = 0;
+      for (long long t = blockIdx.x; t < ntile && !bad; t += gridDim.x, i++)
+        for (int c = 0; c < nch; c++, q++) {
+          const uint32_t s = q % ML_ST;
+          if (!tc::mbar_wait(&sb->full[s], (q / ML_ST) & 1, a.wait_ns)) { bad = true; break; }
+          tc::tc_fence_after();
+          mma_chunk(tmem + (i & 1) * 256, st0 + s * ML_STAGE, W2s + (size_t)c * H * 64, idesc, 2, c == 0);
+          tc::mma_commit(&sb->empty[s]);
+          if (c == nch - 1) tc::mma_commit(&sb->d1);
+        }
+      tc::mma_commit(&sb->fin);
+      if (!tc::mbar_wait(&sb->fin, 0)) bad = true;
+    }
+  } else {
+    const int qd = warp & 3, g = warp >> 2, r = qd * 32 + lane;
+    uint32_t q0 = 0;
+    int i = 0;
+    for (long long t = blockIdx.x; t < ntile; t += gridDim.x, i++, q0 += nch) {
+      const long long row = t * 128 + r;
+      const bool in = row < a.n;
+      const uint32_t tl = tmem + (i & 1) * 256 + ((uint32_t)(qd * 32) << 16);
+      float dy[ML_O];
+#pragma unroll
+      for (int o = 0; o < ML_O; o++) dy[o] = (in && o < a.O) ? a.dY[row * a.O + o] : 0.0f;
+      for (int c = g; c < nch; c += 2) {
+        float z[32];
+        if (in) load32(a.Z2 + row * H + c * 32, z);
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+          const float4 wa = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O);
+          float d = dy[0] * wa.x + dy[1] * wa.y + dy[2] * wa.z + dy[3] * wa.w;
+          if (a.O > 4) {
+            const float4 wb = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O + 4);
+            d += dy[4] * wb.x + dy[5] * wb.y + dy[6] * wb.z + dy[7] * wb.w;
+          }
+          z[j] = in ? d * dsilu(z[j]) : 0.0f;
+        }
+        if (in) store32(a.dZ2 + row * H + c * 32, z);
+        const uint32_t q = q0 + c;
+        if (q >= ML_ST && !bad && !tc::mbar_wait(&sb->empty[q % ML_ST], ((q / ML_ST) - 1) & 1, a.wait_ns)) bad = true;
+        bad = __any_sync(0xffffffffu, bad);
+        if (!bad) put_chunk(st0 + (q % ML_ST) * ML_STAGE, r, z);
+        tc::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&sb->full[q % ML_ST]);
+      }
+      if (!bad && !tc::mbar_wait(&sb->d1, i & 1, a.wait_ns)) bad = true;
+      bad = __any_sync(0xffffffffu, bad);
+      tc::tc_fence_after();
+      for (int c = g; c < nch; c += 2) {
+        float d[32], z[32];
+        tmem_ld32(tl + c * 32, d);
+        if (in) {
+          load32(a.Z1 + row * H + c * 32, z);
+#pragma unroll
+          for (int j = 0; j < 32; j++) d[j] *= dsilu(z[j]);
+          store32(a.dZ1 + row * H + c * 32, d);
+        }
+      }
+      // both groups have read this half before the tile after next refills it
+      tc::tc_fence_before();
+      bad = epi_any(bad);
+      if (bad) break;
+    }
+  }
+  mlp_finish(a, sb, tmem, bad);
+}
+
+// Weight and bias gradients: sums over the rows of dZ2^T H1 (W2), dZ1^T X
+// (W1) and H2^T dY (W3, transposed), H1 = SiLU(Z1), H2 = SiLU(Z2).  CTA
+// (x, y): rows [x kchunk, (x + 1) kchunk), units 128 y .. of the M side.  Per
+// block of 32 rows thread m transposes column m of an operand into the
+// K-major tiles (the lanes along the columns, so every read is a whole line),
+// float32 values as bfloat16 hi + lo: products hi hi', hi lo', lo hi' as in
+// k_tc_gemm.  The partial sums are added with 16-byte float32 atomics.
+// One launch for what three k_tc_gemm launches (96 us at 16384 rows) and
+// three column-sum launches (63 us, one block a column) did.
+constexpr int WG_THREADS = 256;
+struct WgradArgs {
+  long long n;
+  int F, H, O, kchunk;
+  const float *X, *Z1, *Z2, *dY, *dZ1, *dZ2;
+  float *gW1, *gb1, *gW2, *gb2, *gW3, *gb3;
+  int *status;
+  unsigned long long wait_ns;
+};
+// stage: A tiles dZ2, dZ1, H2 (128 units), B tiles H1 (H units), X and dY
+// (32 columns each)
+__host__ __device__ inline uint32_t wg_b_bytes(int H) { return (uint32_t)H * 64; }
+__host__ __device__ inline uint32_t wg_stage(int H) { return 3 * 2 * GA_BYTES + 2 * wg_b_bytes(H) + 4 * 32 * 64; }
+
+__global__ void __launch_bounds__(WG_THREADS, 1)
+k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
+  extern __shared__ unsigned char g_smem_raw[];
+  unsigned char *base = tc::smem_base_1024(g_smem_raw);
+  const int H = a.H, F = a.F, O = a.O, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t bb = wg_b_bytes(H), stage = wg_stage(H);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(base + 2 * stage);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 3);
+  if (tid == 0) {
+    tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init(&bar[2], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) tc::tmem_alloc(tslot, 512);
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = *tslot;   // W2 at 0 (H columns), W1 at 256 and W3 at 288 (32 each)
+  const int m0 = blockIdx.y * 128;
+  const long long k0 = (long long)blockIdx.x * a.kchunk, k1 = min(a.n, k0 + a.kchunk);
+  const int nblk = (int)((k1 - k0 + GK - 1) / GK);
+  const int NF = ((F + 15) / 16) * 16, NO16 = 16;
+  const uint32_t id2 = tc::idesc_bf16_f32(128, H), id1 = tc::idesc_bf16_f32(128, NF), id3 = tc::idesc_bf16_f32(128, NO16);
+  float sb1 = 0.0f, sb2 = 0.0f, sb3 = 0.0f;   // column sums of dZ1, dZ2 (thread = unit m0 + tid) and dY
+  bool bad = false;
+  for (int ib = 0; ib < nblk; ib++) {
+    const int s = ib & 1;
+    const long long kb = k0 + (long long)ib * GK;
+    unsigned char *st = base + s * stage;
+    if (ib >= 2 && !tc::mbar_wait(&bar[s], ((ib - 2) >> 1) & 1, a.wait_ns)) bad = true;
+    if (__syncthreads_or(bad)) { bad = true; break; }
+    unsigned char *tB = st + 6 * GA_BYTES, *tX = tB + 2 * bb, *tY = tX + 2 * 32 * 64;
+    // A tiles: thread = (unit, half of the 32 rows)
+    {
+      const int m = tid & 127, h = tid >> 7, u = m0 + m;
+      const bool ok = u < H;
+#pragma unroll
+      for (int c = 2 * h; c < 2 * h + 2; c++) {
+        float v2[8], v1[8], hh[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+          const long long k = kb + c * 8 + e;
+          const bool in = ok && k < k1;
+          const size_t at = in ? (size_t)k * H + u : 0;
+          v2[e] = in ? __ldg(a.dZ2 + at) : 0.0f;
+          v1[e] = in ? __ldg(a.dZ1 + at) : 0.0f;
+          hh[e] = in ? __ldg(a.Z2 + at) : 0.0f;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) { sb2 += v2[e]; sb1 += v1[e]; hh[e] = silu(hh[e]); }
+        put_row8<2>(st, GA_BYTES, m, c, v2);
+        put_row8<2>(st + 2 * GA_BYTES, GA_BYTES, m, c, v1);
+        put_row8<2>(st + 4 * GA_BYTES, GA_BYTES, m, c, hh);
+      }
+    }
+    // B tile H1: thread = unit
+    for (int u = tid; u < H; u += WG_THREADS) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+          const long long k = kb + c * 8 + e;
+          v[e] = (k < k1) ? __ldg(a.Z1 + (size_t)k * H + u) : 0.0f;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[e] = silu(v[e]);
+        put_row8<2>(tB, bb, u, c, v);
+      }
+    }
+    // B tiles X and dY: thread = (chunk of 8 rows, column)
+    {
+      const int c = (tid >> 5) & 3, u = tid & 31;
+      const bool isx = tid < 128;
+      const int w = isx ? F : O;
+      const float *src = isx ? a.X : a.dY;
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        const long long k = kb + c * 8 + e;
+        v[e] = (u < w && k < k1) ? __ldg(src + (size_t)k * w + u) : 0.0f;
+      }
+      if (!isx) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) sb3 += v[e];
+      }
+      put_row8<2>(isx ? tX : tY, 32 * 64, u, c, v);
+    }
+    tc::fence_proxy_async();
+    __syncthreads();
+    if (tid == 0) {
+      tc::tc_fence_after();
+#pragma unroll
+      for (int ks = 0; ks < GK / 16; ks++) {
+        const uint64_t o = (uint64_t)(ks * 2);
+        const uint32_t first = (ib == 0 && ks == 0) ? 0u : 1u;
+        auto mul = [&](uint32_t acc, const unsigned char *A, const unsigned char *B, uint32_t lo, uint32_t idesc) {
+          const uint64_t ah = tc::smem_desc_sw64(A) + o, al = tc::smem_desc_sw64(A + GA_BYTES) + o;
+          const uint64_t bh = tc::smem_desc_sw64(B) + o, bl = tc::smem_desc_sw64(B + lo) + o;
+          tc::mma_f16(acc, ah, bh, idesc, first);
+          tc::mma_f16(acc, ah, bl, idesc, 1u);
+          tc::mma_f16(acc, al, bh, idesc, 1u);
+        };
+        mul(tmem, st, tB, bb, id2);
+        mul(tmem + 256, st + 2 * GA_BYTES, tX, 32 * 64, id1);
+        mul(tmem + 288, st + 4 * GA_BYTES, tY, 32 * 64, id3);
+      }
+      tc::mma_commit(&bar[s]);
+    }
+  }
+  if (tid == 0) tc::mma_commit(&bar[2]);
+  if (!tc::mbar_wait(&bar[2], 0)) bad = true;
+  bad = __syncthreads_or(bad);
+  tc::tc_fence_after();
+  if (bad) {
+    if (tid == 0) atomicOr(a.status, CB2_STATUS_PIPE_TIMEOUT);
+  } else if (nblk > 0) {
+    const int qd = warp & 3, g = warp >> 2, u = m0 + qd * 32 + lane;
+    const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
+    float v[32];
+    for (int c = g; c < H / 32; c += 2) {
+      tmem_ld32(tl + c * 32, v);
+      if (u < H) {
+        float4 *d = reinterpret_cast<float4 *>(a.gW2 + (size_t)u * H + c * 32);
+#pragma unroll
+        for (int j = 0; j < 8; j++) atomicAdd(d + j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+      }
+    }
+    if (g == 0) {
+      tmem_ld32(tl + 256, v);
+#pragma unroll
+      for (int j = 0; j < 32; j++)
+        if (u < H && j < F) atomicAdd(a.gW1 + (size_t)u * F + j, v[j]);
+    } else {
+      tmem_ld32(tl + 288, v);
+#pragma unroll
+      for (int j = 0; j < ML_O; j++)
+        if (u < H && j < O) atomicAdd(a.gW3 + (size_t)j * H + u, v[j]);
+    }
+    if (m0 + (tid & 127) < H) {
+      atomicAdd(a.gb1 + m0 + (tid & 127), sb1);
+      atomicAdd(a.gb2 + m0 + (tid & 127), sb2);
+    }
+    if (blockIdx.y == 0 && tid >= 128 && (tid & 31) < O) atomicAdd(a.gb3 + (tid & 31), sb3);
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, 512);
+}
+
+// loss = sum of the partial sums / (n O) (one block, fixed order)
+__global__ void __launch_bounds__(256)
+k_loss_sum(long long np, const double *part, double inv, double *out) {
+  __shared__ double sh[256];
+  double s = 0.0;
+  for (long long i = threadIdx.x; i < np; i += 256) s += part[i];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  for (int q = 128; q > 0; q >>= 1) {
+    if (threadIdx.x < q) sh[threadIdx.x] += sh[threadIdx.x + q];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[0] = sh[0] * inv;
+}
+
 __device__ inline float sigm(float z) { return 1.0f / (1.0f + __expf(-z)); }
 
 // Z += b (per column); H = SiLU(Z) (act != 0) or Z
@@ -325,15 +931,18 @@ __global__ void k_colsum(size_t n, int w, const float *X, float *out) {
   if (threadIdx.x == 0) out[c] = (float)sh[0];
 }
 
+// one Adam step of the float32 master parameters and their bfloat16 copy
 __global__ void k_adam(size_t n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2,
-                       float eps, float c1, float c2) {
+                       float eps, float c1, float c2, __nv_bfloat16 *w) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
   const float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
   m[i] = mi;
   v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  p[i] = pi;
+  w[i] = __float2bfloat16_rn(pi);
 }
 
 __global__ void k_to_bf16(size_t n, const float *src, __nv_bfloat16 *dst) {
@@ -361,29 +970,81 @@ struct cb2_mlp {
   float *dH = nullptr, *dZ = nullptr;
   double *part = nullptr;       // loss partial sums
   int *status = nullptr;        // device status word of the GEMMs (bit 2: a wait ran out)
-  size_t part_cap = 0;
+  double *loss = nullptr;       // loss of the last fused training pass
+  size_t ycap = 0;              // rows of Yp
   cudaStream_t stream = nullptr;
 };
 
 namespace cb2 {
 namespace {
 
-int mlp_reserve(cb2_mlp *n, size_t rows) {
+// the sizes the one-kernel passes take: tensor memory holds two accumulators
+// of 256 columns, shared memory W2 and the operand stages (208 KB at H = 256),
+// the last layer sits in registers; W2's rows are copied 16 bytes at a time
+bool fused_ok(const cb2_mlp *n) {
+  return n->F <= 32 && n->H % 32 == 0 && n->H >= 64 && n->H <= 256 && n->O <= ML_O && n->oW2 % 8 == 0;
+}
+
+int grow(float **p, size_t count) {
+  if (*p) cudaFree(*p);
+  *p = nullptr;
+  CB2_CUDA(cudaMalloc(p, count * sizeof(float)));
+  return 0;
+}
+
+// Work buffers of `rows` rows.  The fused passes keep the activations on the
+// chip: inference needs none of these, training Z1, Z2 and the gradients dY,
+// dZ2 (in dZ) and dZ1 (in dH).
+int mlp_reserve(cb2_mlp *n, size_t rows, bool train) {
+  int rc = 0;
+  if (fused_ok(n) && !train) return 0;
   if (rows <= n->cap) return 0;
-  float **bufs[8] = {&n->Z1, &n->H1, &n->Z2, &n->H2, &n->Yp, &n->dY, &n->dH, &n->dZ};
-  const size_t width[8] = {(size_t)n->H, (size_t)n->H, (size_t)n->H, (size_t)n->H, (size_t)n->O, (size_t)n->O,
-                           (size_t)n->H, (size_t)n->H};
-  for (int q = 0; q < 8; q++) {
-    if (*bufs[q]) cudaFree(*bufs[q]);
-    *bufs[q] = nullptr;
-    CB2_CUDA(cudaMalloc(bufs[q], rows * width[q] * sizeof(float)));
-  }
-  const size_t pc = blocks(rows * n->O) + 1;
+  n->cap = 0;
+  const size_t w = (size_t)n->H;
+  if ((rc = grow(&n->Z1, rows * w)) || (rc = grow(&n->Z2, rows * w)) || (rc = grow(&n->dH, rows * w)) ||
+      (rc = grow(&n->dZ, rows * w)) || (rc = grow(&n->dY, rows * n->O)))
+    return rc;
+  if (!fused_ok(n) && ((rc = grow(&n->H1, rows * w)) || (rc = grow(&n->H2, rows * w)))) return rc;
+  const size_t pc = std::max((size_t)blocks(rows * n->O), 4 * ((rows + 127) / 128)) + 1;
   if (n->part) cudaFree(n->part);
   n->part = nullptr;
   CB2_CUDA(cudaMalloc(&n->part, pc * sizeof(double)));
-  n->part_cap = pc;
   n->cap = rows;
+  return 0;
+}
+
+// the output buffer of passes that have none of the caller's
+int mlp_reserve_y(cb2_mlp *n, size_t rows) {
+  if (rows <= n->ycap) return 0;
+  n->ycap = 0;
+  if (int rc = grow(&n->Yp, rows * n->O)) return rc;
+  n->ycap = rows;
+  return 0;
+}
+
+MlpArgs mlp_args(const cb2_mlp *n, const float *X, size_t rows, int *status) {
+  MlpArgs a{};
+  a.n = (long long)rows; a.F = n->F; a.H = n->H; a.O = n->O;
+  a.X = X;
+  a.vec = n->F % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+  a.b1 = n->master + n->ob1; a.b2 = n->master + n->ob2; a.b3 = n->master + n->ob3;
+  a.W1 = n->w + n->oW1; a.W2 = n->w + n->oW2; a.W3 = n->w + n->oW3;
+  a.scale = 2.0f / (float)(rows * (size_t)n->O);
+  a.status = status;
+  a.wait_ns = kWaitNsGemm;
+  return a;
+}
+
+// one CTA per SM over the row tiles
+template <typename K>
+int launch_rows(K *kernel, const MlpArgs &a, cudaStream_t st) {
+  const size_t smem = mlp_layout(a.H).total + 1024;
+  CB2_CUDA(raise_smem_limit(kernel, smem));
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  kernel<<<(unsigned)std::min<long long>(sms, (a.n + 127) / 128), ML_THREADS, smem, st>>>(a);
+  CB2_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -418,20 +1079,52 @@ void gemm(cudaStream_t st, int *status, int M, int N, int K, const TAT *A, int l
                                                         split_k ? 1 : 0, cols, status, kWaitNsGemm);
 }
 
-// forward pass of n rows of X (normalised features) into n->Yp, on stream st
-int mlp_forward(cb2_mlp *nt, const float *X, size_t n, cudaStream_t st, int *status = nullptr) {
-  int rc = mlp_reserve(nt, n);
-  if (rc) return rc;
+// forward pass of n rows of X (normalised features) into Y, on stream st
+int mlp_forward(cb2_mlp *nt, const float *X, size_t n, float *Y, cudaStream_t st, int *status = nullptr) {
   if (!status) status = nt->status;
+  if (fused_ok(nt)) {
+    MlpArgs a = mlp_args(nt, X, n, status);
+    a.Y = Y;
+    return launch_rows(k_mlp_fwd<false>, a, st);
+  }
+  int rc = mlp_reserve(nt, n, false);
+  if (rc) return rc;
   const int F = nt->F, H = nt->H, O = nt->O;
   gemm<float, __nv_bfloat16, false, true>(st, status, (int)n, H, F, X, F, nt->w + nt->oW1, F, nt->Z1, H, false);
   k_bias_act<<<blocks(n * H), 256, 0, st>>>(n, H, nt->Z1, nt->master + nt->ob1, nt->H1, 1);
   gemm<float, __nv_bfloat16, false, true>(st, status, (int)n, H, H, nt->H1, H, nt->w + nt->oW2, H, nt->Z2, H,
                                           false);
   k_bias_act<<<blocks(n * H), 256, 0, st>>>(n, H, nt->Z2, nt->master + nt->ob2, nt->H2, 1);
-  gemm<float, __nv_bfloat16, false, true>(st, status, (int)n, O, H, nt->H2, H, nt->w + nt->oW3, H, nt->Yp, O,
+  gemm<float, __nv_bfloat16, false, true>(st, status, (int)n, O, H, nt->H2, H, nt->w + nt->oW3, H, Y, O,
                                           false);
-  k_bias_act<<<blocks(n * O), 256, 0, st>>>(n, O, nt->Yp, nt->master + nt->ob3, nt->Yp, 0);
+  k_bias_act<<<blocks(n * O), 256, 0, st>>>(n, O, Y, nt->master + nt->ob3, Y, 0);
+  CB2_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// the fused training pass: loss (left in nt->loss) and gradients
+int mlp_backward_fused(cb2_mlp *nt, const float *X, const float *T, size_t n) {
+  cudaStream_t st = nt->stream;
+  MlpArgs a = mlp_args(nt, X, n, nt->status);
+  a.T = T; a.Z1 = nt->Z1; a.Z2 = nt->Z2; a.dY = nt->dY; a.dZ2 = nt->dZ; a.dZ1 = nt->dH; a.part = nt->part;
+  CB2_CUDA(cudaMemsetAsync(nt->grad, 0, nt->np * sizeof(float), st));
+  int rc = launch_rows(k_mlp_fwd<true>, a, st);
+  if (rc) return rc;
+  k_loss_sum<<<1, 256, 0, st>>>(4 * ((a.n + 127) / 128), nt->part, 1.0 / ((double)n * nt->O), nt->loss);
+  if ((rc = launch_rows(k_mlp_bwd, a, st))) return rc;
+  WgradArgs w{};
+  w.n = a.n; w.F = a.F; w.H = a.H; w.O = a.O;
+  w.X = X; w.Z1 = nt->Z1; w.Z2 = nt->Z2; w.dY = nt->dY; w.dZ1 = nt->dH; w.dZ2 = nt->dZ;
+  w.gW1 = nt->grad + nt->oW1; w.gb1 = nt->grad + nt->ob1; w.gW2 = nt->grad + nt->oW2; w.gb2 = nt->grad + nt->ob2;
+  w.gW3 = nt->grad + nt->oW3; w.gb3 = nt->grad + nt->ob3;
+  w.status = nt->status; w.wait_ns = kWaitNsGemm;
+  // about one CTA an SM: 74 row chunks x 2 halves of the units
+  const int ny = (a.H + 127) / 128;
+  const long long want = std::max<long long>(1, 148 / ny);
+  w.kchunk = (int)(((a.n + want - 1) / want + GK - 1) / GK * GK);
+  const size_t smem = 2 * (size_t)wg_stage(a.H) + 64 + 1024;
+  CB2_CUDA(raise_smem_limit(k_mlp_wgrad, smem));
+  k_mlp_wgrad<<<dim3((unsigned)((a.n + w.kchunk - 1) / w.kchunk), ny), WG_THREADS, smem, st>>>(w);
   CB2_CUDA(cudaGetLastError());
   return 0;
 }
@@ -439,8 +1132,15 @@ int mlp_forward(cb2_mlp *nt, const float *X, size_t n, cudaStream_t st, int *sta
 // loss and gradients of the mean squared error over n rows (grad <- dL/dparams)
 int mlp_backward(cb2_mlp *nt, const float *X, const float *T, size_t n, double *loss) {
   cudaStream_t st = nt->stream;
-  int rc = mlp_forward(nt, X, n, st);
+  int rc = mlp_reserve(nt, n, true);
   if (rc) return rc;
+  if (fused_ok(nt)) {
+    if ((rc = mlp_backward_fused(nt, X, T, n))) return rc;
+    // the caller waits for the stream (mlp_status) before it reads the loss
+    if (loss) CB2_CUDA(cudaMemcpyAsync(loss, nt->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
+    return 0;
+  }
+  if ((rc = mlp_reserve_y(nt, n)) || (rc = mlp_forward(nt, X, n, nt->Yp, st))) return rc;
   const int F = nt->F, H = nt->H, O = nt->O;
   const unsigned nb = blocks(n * O);
   k_mse<<<nb, 256, 0, st>>>(n, O, nt->Yp, T, nt->dY, nt->part);
@@ -490,7 +1190,7 @@ int closure_apply(Ctx &c) {
                                               c.h_r[c.kout], c.d_f, c.fsize(), feat_slots(), cs->X);
   const size_t nn = (size_t)c.nr * NF;
   k_normalise<<<blocks(n * NF), 256, 0, c.stream>>>(n, c.jmax, cs->X, cs->norm, cs->norm + nn, cs->Xn);
-  int rc = mlp_forward(cs->net, cs->Xn, n, c.stream, c.d_status);
+  int rc = mlp_forward(cs->net, cs->Xn, n, cs->net->Yp, c.stream, c.d_status);
   if (rc) return rc;
   k_add_tendency<<<blocks(n), 256, 0, c.stream>>>(n, c.nr, c.jmax, cs->net->Yp, cs->norm + 2 * nn, c.d_f, c.fsize(),
                                                   out_slots());
@@ -542,7 +1242,7 @@ int cb2_mlp_create(int nin, int nhid, int nout, unsigned seed, cb2_mlp **out) {
       cudaMalloc(&n->m, n->np * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&n->v, n->np * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&n->w, n->np * sizeof(__nv_bfloat16)) != cudaSuccess ||
-      cudaMalloc(&n->status, sizeof(int)) != cudaSuccess)
+      cudaMalloc(&n->loss, sizeof(double)) != cudaSuccess || cudaMalloc(&n->status, sizeof(int)) != cudaSuccess)
     return fail(cuda_fail(cudaGetLastError(), "cb2_mlp_create"));
   cudaMemcpy(n->master, p.data(), n->np * sizeof(float), cudaMemcpyHostToDevice);
   cudaMemset(n->grad, 0, n->np * sizeof(float));
@@ -559,7 +1259,7 @@ int cb2_mlp_destroy(cb2_mlp *n) {
   if (!n) return 0;
   if (n->stream) cudaStreamSynchronize(n->stream);
   void *ptrs[] = {n->master, n->grad, n->m, n->v, n->w, n->Z1, n->H1, n->Z2, n->H2, n->Yp, n->dY, n->dH, n->dZ,
-                  n->part, n->status};
+                  n->part, n->loss, n->status};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   if (n->stream) cudaStreamDestroy(n->stream);
@@ -600,9 +1300,7 @@ static int mlp_status(cb2_mlp *n) {
 
 int cb2_mlp_forward(cb2_mlp *n, const float *dev_x, long long rows, float *dev_y) {
   if (!n || !dev_x || !dev_y || rows <= 0) return CB2_ERR_ARG;
-  int rc = mlp_forward(n, dev_x, (size_t)rows, n->stream);
-  if (rc) return rc;
-  CB2_CUDA(cudaMemcpyAsync(dev_y, n->Yp, (size_t)rows * n->O * sizeof(float), cudaMemcpyDeviceToDevice, n->stream));
+  if (int rc = mlp_forward(n, dev_x, (size_t)rows, dev_y, n->stream)) return rc;
   return mlp_status(n);
 }
 
@@ -623,8 +1321,7 @@ int cb2_mlp_adam_step(cb2_mlp *n, float lr, float beta1, float beta2, float eps)
   if (!n) return CB2_ERR_ARG;
   n->t += 1;
   const float c1 = 1.0f - std::pow(beta1, (float)n->t), c2 = 1.0f - std::pow(beta2, (float)n->t);
-  k_adam<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->grad, n->m, n->v, lr, beta1, beta2, eps, c1, c2);
-  k_to_bf16<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->w);
+  k_adam<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->grad, n->m, n->v, lr, beta1, beta2, eps, c1, c2, n->w);
   CB2_CUDA(cudaGetLastError());
   return 0;
 }
@@ -730,7 +1427,8 @@ int cb2_closure_attach(cb2_ctx *c, cb2_mlp *net, const float *norm) {
   CB2_CUDA(cudaMemcpy(cs->norm, hn.data(), hn.size() * sizeof(float), cudaMemcpyHostToDevice));
   CB2_CUDA(cudaMalloc(&cs->X, cs->rows * NF * sizeof(float)));
   CB2_CUDA(cudaMalloc(&cs->Xn, cs->rows * NF * sizeof(float)));
-  return mlp_reserve(net, cs->rows);
+  if (int rc = mlp_reserve(net, cs->rows, false)) return rc;
+  return mlp_reserve_y(net, cs->rows);
 }
 
 }  // extern "C"
