@@ -849,7 +849,14 @@ k_fft_products_t(int L, MLayout fin, MLayout fout, const float2 *__restrict__ tw
 // (R2 values, DFT over n2).  The Hermitian pair rows are built on the fly
 // from the staged (a_m, b_m) without the 1/2 of z = x + i y: the products
 // are bilinear, so their coefficients carry the 1/4 instead (exact).
-constexpr int F4_THREADS = 384;
+// A group is R2 threads, one per column of the first step; in the second
+// each takes R1 / R2 rows, so every thread of the 21 (18) groups holds R1
+// values in both steps.  With 16 threads a group whatever R1 and R2, half to
+// three quarters of them idled at M < 256, in CTAs of 384 threads: float32
+// M = 128 (18624 rows) 477 -> 379 us, M = 64 (6240 rows) 110 -> 70, float64
+// M = 32 (2352 rows) 116 -> 36.
+constexpr int F4_THREADS = 384;   // the tuning value that selects these kernels
+template <int R2> __host__ __device__ constexpr int f4_threads() { return 24 * R2; }
 
 template <int R1, int R2>
 struct F4Plan {
@@ -876,10 +883,12 @@ __device__ __forceinline__ T2 cmulc(T2 a, T2 w) {   // a * conj(w)
 // orders, [theta][m / 16][element] with the elements of the output layout
 // (P block k 8 + j, then D block sP + k 16 + j).
 template <int R1, int R2>
-__global__ void __launch_bounds__(F4_THREADS, 2)
+__global__ void __launch_bounds__(f4_threads<R2>(), R2 == 16 ? 2 : R1 == 16 ? 4 : R2 == 8 ? 5 : 10)
 k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, ProdCoef pc,
                   float *__restrict__ pmax, const float *__restrict__ wgt) {
   using P = F4Plan<R1, R2>;
+  constexpr int NT = f4_threads<R2>(), RU = R1 / R2;
+  static_assert(R1 % R2 == 0, "rows of the second step");
   constexpr int M = P::M, N = P::N, TP = P::TP, TG = P::TG, MP2 = P::MP2, WP = P::WP;
   extern __shared__ __align__(16) unsigned char smraw[];
   // input staging [7 pairs][MP2][2]: the (a_m, b_m) of components 2p and
@@ -889,16 +898,16 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
   float2 *TW3 = X + P::X;                                          // [3][M]
   float2 *TWM = TW3 + 3 * M;                                       // [R2][WP]
   const int th = blockIdx.x / fin.nr, k = blockIdx.x % fin.nr;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = F4_THREADS / 32;
-  const int grp = tid >> 4, lt = tid & 15;
-  for (int e = tid; e < 14; e += F4_THREADS) S2[((e >> 1) * MP2 + M) * 2 + (e & 1)] = float2{0.0f, 0.0f};
-  for (int e = tid; e < M; e += F4_THREADS) S2[(6 * MP2 + e) * 2 + 1] = float2{0.0f, 0.0f};
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = NT / 32;
+  const int grp = tid / R2, lt = tid % R2;
+  for (int e = tid; e < 14; e += NT) S2[((e >> 1) * MP2 + M) * 2 + (e & 1)] = float2{0.0f, 0.0f};
+  for (int e = tid; e < M; e += NT) S2[(6 * MP2 + e) * 2 + 1] = float2{0.0f, 0.0f};
   // input and tables by asynchronous 8-byte copies, all in flight at once.
   // At one (theta, k) an order m has 13 (cos, sin) pairs: a run of 5 in the
   // P block and one of 8 in the D block; half-warp h of warp w copies the
   // orders 2 (w + nwarp i) + h, lane j < 13 of the half pair j into the
   // staging row of its component
-  for (int e = tid; e < P::NTW; e += F4_THREADS) {
+  for (int e = tid; e < P::NTW; e += NT) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(TW3 + e);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(tables + e) : "memory");
   }
@@ -927,7 +936,7 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
   __syncthreads();
   const int gp = grp / 3, gr = grp - 3 * gp;   // pair, residue of this group
   // ---- backward, step 1: column n2 = lt, pair rows built from the staging
-  if (grp < 21 && lt < R2) {
+  if (grp < 21) {
     const float4 *xy = reinterpret_cast<const float4 *>(S2) + gp * MP2;   // (x_m, y_m) of the pair
     const float2 om = (gr == 0) ? float2{1.0f, 0.0f}
                     : float2{-0.5f, (gr == 1) ? -0.86602540378443864676f : 0.86602540378443864676f};
@@ -949,28 +958,34 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
     for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = (k1 == 0) ? v[0] : cmulf(v[k1], TWM[lt * WP + k1]);
   }
   // the transpose block T of a group is written and read by the group's own
-  // 16 threads, half of one warp
+  // R2 threads, which sit in one warp
   __syncwarp();
   // ---- backward, step 2: row k1 = lt -> grid samples j = 3 (k1 + R1 k2) + r
-  float2 w[R2];
-  if (grp < 21 && lt < R1) {
-    const float2 *T = X + grp * TG + lt * TP;
+  float2 w[RU][R2];
+  if (grp < 21) {
 #pragma unroll
-    for (int n2 = 0; n2 < R2; n2++) w[n2] = T[n2];
-    dftr<R2, +1>(w);
+    for (int u = 0; u < RU; u++) {
+      const float2 *T = X + grp * TG + (lt + R2 * u) * TP;
+#pragma unroll
+      for (int n2 = 0; n2 < R2; n2++) w[u][n2] = T[n2];
+      dftr<R2, +1>(w[u]);
+    }
   }
   __syncthreads();
-  if (grp < 21 && lt < R1) {
-    float2 *G = X + gp * N + 3 * lt + gr;
+  if (grp < 21) {
 #pragma unroll
-    for (int k2 = 0; k2 < R2; k2++) G[3 * R1 * k2] = w[k2];
+    for (int u = 0; u < RU; u++) {
+      float2 *G = X + gp * N + 3 * (lt + R2 * u) + gr;
+#pragma unroll
+      for (int k2 = 0; k2 < R2; k2++) G[3 * R1 * k2] = w[u][k2];
+    }
   }
   __syncthreads();
   // ---- products at every grid point (in place: 7 pair rows in, 6 out)
   {
     const float cv = 0.25f * (float)pc.cv, cl = 0.25f * (float)pc.cl, ci = 0.25f * (float)pc.ci,
                 ct = 0.25f * (float)pc.ct;
-    for (int q = tid; q < N; q += F4_THREADS) {
+    for (int q = tid; q < N; q += NT) {
       const float2 p0 = X[0 * N + q], p1 = X[1 * N + q], p2 = X[2 * N + q], p3 = X[3 * N + q];
       const float2 p4 = X[4 * N + q], p5 = X[5 * N + q], p6 = X[6 * N + q];
       const float ur = p0.x, ut = p0.y, up = p1.x, wr = p1.y, wt = p2.x, wp = p2.y;
@@ -986,7 +1001,7 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
   __syncthreads();
   // ---- forward, step 1: column n2 = lt of the samples j = 3 (n1 R2 + n2) + r
   float2 v[R1];
-  if (grp < 18 && lt < R2) {
+  if (grp < 18) {
     const float2 *G = X + gp * N + 3 * lt + gr;
 #pragma unroll
     for (int n1 = 0; n1 < R1; n1++) v[n1] = G[3 * R2 * n1];
@@ -995,24 +1010,30 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
     for (int k1 = 1; k1 < R1; k1++) v[k1] = cmulc(v[k1], TWM[lt * WP + k1]);
   }
   __syncthreads();
-  if (grp < 18 && lt < R2) {
+  if (grp < 18) {
     float2 *T = X + grp * TG;
 #pragma unroll
     for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = v[k1];
   }
   __syncwarp();   // the group's own transpose block, as in the backward steps
   // ---- forward, step 2: row k1 = lt -> F_r[k1 + R1 k2]
-  if (grp < 18 && lt < R1) {
-    const float2 *T = X + grp * TG + lt * TP;
+  if (grp < 18) {
 #pragma unroll
-    for (int n2 = 0; n2 < R2; n2++) w[n2] = T[n2];
-    dftr<R2, -1>(w);
+    for (int u = 0; u < RU; u++) {
+      const float2 *T = X + grp * TG + (lt + R2 * u) * TP;
+#pragma unroll
+      for (int n2 = 0; n2 < R2; n2++) w[u][n2] = T[n2];
+      dftr<R2, -1>(w[u]);
+    }
   }
   __syncthreads();
-  if (grp < 18 && lt < R1) {
-    float2 *F = X + grp * M + lt;   // [pair][r][M]: grp = 3 p + r
+  if (grp < 18) {
 #pragma unroll
-    for (int k2 = 0; k2 < R2; k2++) F[R1 * k2] = w[k2];
+    for (int u = 0; u < RU; u++) {
+      float2 *F = X + grp * M + lt + R2 * u;   // [pair][r][M]: grp = 3 p + r
+#pragma unroll
+      for (int k2 = 0; k2 < R2; k2++) F[R1 * k2] = w[u][k2];
+    }
   }
   __syncthreads();
   // ---- combine the residues: Z[m], Z[N - m] -> (a_m, b_m) of both
@@ -1031,7 +1052,7 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
         o1[m] = float2{an * (zk.y + zn.y), an * (zk.x - zn.x)};
       }
     };
-    for (int idx = tid; idx < 6 * MH; idx += F4_THREADS) {
+    for (int idx = tid; idx < 6 * MH; idx += NT) {
       const int p = idx / MH, m = idx - p * MH, mm = (M - m) & (M - 1);
       const float2 *F = X + p * 3 * M;
       float2 *o0 = O2 + (2 * p) * MP2, *o1 = o0 + MP2;
@@ -1079,7 +1100,7 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
     const float wt = __ldg(wgt + th);
     const size_t E = fout.sP() + fout.sD();
     float *pm = pmax + (size_t)th * MB * E;
-    for (int t = tid; t < 24 * MB; t += F4_THREADS) {
+    for (int t = tid; t < 24 * MB; t += NT) {
       const int j = t % 24, mb = t / 24;
       int c, sg;
       m_comp_of_out(j, c, sg);
@@ -1115,12 +1136,13 @@ struct F4Plan64 {
 };
 
 template <int R1, int R2>
-__global__ void __launch_bounds__(F4_THREADS, 1)
+__global__ void __launch_bounds__(f4_threads<R2>(), R2 == 16 ? 1 : R1 == 16 ? 2 : R2 == 8 ? 4 : 8)
 k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2, int NS,
                     const double2 *__restrict__ tables, ProdCoef pc) {
   using P = F4Plan64<R1, R2>;
   using PB = PairBits<double>;
   using U = PB::U;
+  constexpr int NT = f4_threads<R2>(), RU = R1 / R2;
   constexpr int M = P::M, N = P::N, TP = P::TP, TG = P::TG, MP2 = P::MP2, WP = P::WP;
   extern __shared__ __align__(16) unsigned char smraw[];
   double2 *S2 = reinterpret_cast<double2 *>(smraw);   // [14][MP2] (a_m, b_m); later [12][MP2] out
@@ -1131,12 +1153,12 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
   const size_t row = blockIdx.x;
   const double *fin = four + row * 13 * (size_t)NS;
   double *fout = four2 + row * 12 * (size_t)NS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = F4_THREADS / 32;
-  const int grp = tid >> 4, lt = tid & 15;
-  for (int e = tid; e < P::NTW; e += F4_THREADS) TW3[e] = tables[e];
-  for (int e = tid; e < 14; e += F4_THREADS) S2[e * MP2 + M] = double2{0.0, 0.0};
-  for (int e = tid; e < M; e += F4_THREADS) S2[13 * MP2 + e] = double2{0.0, 0.0};
-  for (int e = tid; e < 13 * M; e += F4_THREADS) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = NT / 32;
+  const int grp = tid / R2, lt = tid % R2;
+  for (int e = tid; e < P::NTW; e += NT) TW3[e] = tables[e];
+  for (int e = tid; e < 14; e += NT) S2[e * MP2 + M] = double2{0.0, 0.0};
+  for (int e = tid; e < M; e += NT) S2[13 * MP2 + e] = double2{0.0, 0.0};
+  for (int e = tid; e < 13 * M; e += NT) {
     const int c = e / M, m = e - c * M;
     S2[c * MP2 + m] = __ldg(reinterpret_cast<const double2 *>(fin + (size_t)c * NS) + m);
   }
@@ -1156,7 +1178,7 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
   const int gp = grp / 3, gr = grp - 3 * gp;
   // ---- backward, step 1: column n2 = lt, pair rows from the staging (the
   // second row of the pair scaled by sy)
-  if (grp < 21 && lt < R2) {
+  if (grp < 21) {
     const double2 *x0 = S2 + (2 * gp) * MP2, *y0 = S2 + (2 * gp + 1) * MP2;
     const double sy = (2 * gp + 1 < 13) ? PB::factor(cmx[2 * gp], cmx[2 * gp + 1], false) : 1.0;
     const double2 om = (gr == 0) ? double2{1.0, 0.0}
@@ -1178,21 +1200,27 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
 #pragma unroll
     for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = (k1 == 0) ? v[0] : cmulf(v[k1], TWM[lt * WP + k1]);
   }
-  __syncthreads();
+  __syncwarp();   // the group's own transpose block
   // ---- backward, step 2: row k1 = lt -> grid samples j = 3 (k1 + R1 k2) + r
   {
-    double2 w[R2];
-    if (grp < 21 && lt < R1) {
-      const double2 *T = X + grp * TG + lt * TP;
+    double2 w[RU][R2];
+    if (grp < 21) {
 #pragma unroll
-      for (int n2 = 0; n2 < R2; n2++) w[n2] = T[n2];
-      dftr<R2, +1>(w);
+      for (int u = 0; u < RU; u++) {
+        const double2 *T = X + grp * TG + (lt + R2 * u) * TP;
+#pragma unroll
+        for (int n2 = 0; n2 < R2; n2++) w[u][n2] = T[n2];
+        dftr<R2, +1>(w[u]);
+      }
     }
     __syncthreads();
-    if (grp < 21 && lt < R1) {
-      double2 *G = X + gp * N + 3 * lt + gr;
+    if (grp < 21) {
 #pragma unroll
-      for (int k2 = 0; k2 < R2; k2++) G[3 * R1 * k2] = w[k2];
+      for (int u = 0; u < RU; u++) {
+        double2 *G = X + gp * N + 3 * (lt + R2 * u) + gr;
+#pragma unroll
+        for (int k2 = 0; k2 < R2; k2++) G[3 * R1 * k2] = w[u][k2];
+      }
     }
   }
   __syncthreads();
@@ -1206,7 +1234,7 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
     U hm[12];
 #pragma unroll
     for (int c = 0; c < 12; c++) hm[c] = 0;
-    for (int q = tid; q < N; q += F4_THREADS) {
+    for (int q = tid; q < N; q += NT) {
       const double2 p0 = X[0 * N + q], p1 = X[1 * N + q], p2 = X[2 * N + q], p3 = X[3 * N + q];
       const double2 p4 = X[4 * N + q], p5 = X[5 * N + q], p6 = X[6 * N + q];
       const double ur = p0.x, ut = p0.y * iy[0], up = p1.x, wr = p1.y * iy[1], wt = p2.x, wp = p2.y * iy[2];
@@ -1233,7 +1261,7 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
     }
   }
   __syncthreads();
-  for (int idx = tid; idx < 6 * N; idx += F4_THREADS) {
+  for (int idx = tid; idx < 6 * N; idx += NT) {
     const int p = idx / N;
     X[idx].y *= PB::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], false);
   }
@@ -1241,7 +1269,7 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
   // ---- forward, step 1: column n2 = lt of the samples j = 3 (n1 R2 + n2) + r
   {
     double2 v[R1];
-    if (grp < 18 && lt < R2) {
+    if (grp < 18) {
       const double2 *G = X + gp * N + 3 * lt + gr;
 #pragma unroll
       for (int n1 = 0; n1 < R1; n1++) v[n1] = G[3 * R2 * n1];
@@ -1250,27 +1278,33 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
       for (int k1 = 1; k1 < R1; k1++) v[k1] = cmulc(v[k1], TWM[lt * WP + k1]);
     }
     __syncthreads();
-    if (grp < 18 && lt < R2) {
+    if (grp < 18) {
       double2 *T = X + grp * TG;
 #pragma unroll
       for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = v[k1];
     }
   }
-  __syncthreads();
+  __syncwarp();
   // ---- forward, step 2: row k1 = lt -> F_r[k1 + R1 k2]
   {
-    double2 w[R2];
-    if (grp < 18 && lt < R1) {
-      const double2 *T = X + grp * TG + lt * TP;
+    double2 w[RU][R2];
+    if (grp < 18) {
 #pragma unroll
-      for (int n2 = 0; n2 < R2; n2++) w[n2] = T[n2];
-      dftr<R2, -1>(w);
+      for (int u = 0; u < RU; u++) {
+        const double2 *T = X + grp * TG + (lt + R2 * u) * TP;
+#pragma unroll
+        for (int n2 = 0; n2 < R2; n2++) w[u][n2] = T[n2];
+        dftr<R2, -1>(w[u]);
+      }
     }
     __syncthreads();
-    if (grp < 18 && lt < R1) {
-      double2 *F = X + grp * M + lt;   // [pair][r][M]: grp = 3 p + r
+    if (grp < 18) {
 #pragma unroll
-      for (int k2 = 0; k2 < R2; k2++) F[R1 * k2] = w[k2];
+      for (int u = 0; u < RU; u++) {
+        double2 *F = X + grp * M + lt + R2 * u;   // [pair][r][M]: grp = 3 p + r
+#pragma unroll
+        for (int k2 = 0; k2 < R2; k2++) F[R1 * k2] = w[u][k2];
+      }
     }
   }
   __syncthreads();
@@ -1278,7 +1312,7 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
   // second unscaled), into the staging rows [c][MP2]
   {
     const double an = 1.0 / (double)N;
-    for (int idx = tid; idx < 6 * M; idx += F4_THREADS) {
+    for (int idx = tid; idx < 6 * M; idx += NT) {
       const int p = idx / M, m = idx - p * M, mm = (M - m) & (M - 1);
       const double2 *F = X + p * 3 * M;
       const double2 t1 = TW3[M + m], t2 = TW3[2 * M + m];
@@ -1296,7 +1330,7 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
     }
   }
   __syncthreads();
-  for (int e = tid; e < 12 * M; e += F4_THREADS) {
+  for (int e = tid; e < 12 * M; e += NT) {
     const int c = e / M, m = e - c * M;
     reinterpret_cast<double2 *>(fout + (size_t)c * NS)[m] = S2[c * MP2 + m];
   }
@@ -1557,7 +1591,7 @@ static const typename C2<T>::t *twid(Ctx &c) {
 
 template <int R1, int R2>
 static void launch_fft_4s64(Ctx &c, const double *four, double *four2, const ProdCoef &pc) {
-  k_fft_products_4s64<R1, R2><<<(unsigned)(c.nth * c.nr), F4_THREADS, F4Plan64<R1, R2>::smem(), c.stream>>>(
+  k_fft_products_4s64<R1, R2><<<(unsigned)(c.nth * c.nr), f4_threads<R2>(), F4Plan64<R1, R2>::smem(), c.stream>>>(
       four, four2, c.NS, (const double2 *)c.d_twf4_64, pc);
 }
 
@@ -1613,7 +1647,7 @@ static void launch_fft_t(Ctx &c, const MLayout &in, const MLayout &out, const Pr
 
 template <int R1, int R2>
 static bool launch_fft_4s(Ctx &c, const MLayout &in, const MLayout &out, const ProdCoef &pc, float *pmax) {
-  k_fft_products_4s<R1, R2><<<(unsigned)(c.nth * c.nr), F4_THREADS, F4Plan<R1, R2>::smem(), c.stream>>>(
+  k_fft_products_4s<R1, R2><<<(unsigned)(c.nth * c.nr), f4_threads<R2>(), F4Plan<R1, R2>::smem(), c.stream>>>(
       in, out, (const float2 *)c.d_twf4, pc, pmax, pmax ? mixed_weights32(c) : nullptr);
   return pmax != nullptr;
 }
