@@ -64,14 +64,13 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   // host tables
   std::vector<int> h_jl, h_jm;          // per jj
-  std::vector<int> h_perm;              // jj -> j = l(l+1)+m
   std::vector<int> h_moff;              // offset of block (m, +) for m = 0..L
   std::vector<size_t> h_poff;           // offset of order m in the P tables
   std::vector<double> h_r, h_colat, h_wgt;
   BCW bc{};
   double cev = 0, cet = 0, ceb = 0, temp_icb_fld = 0, temp_cmb_fld = 0;
   // device tables
-  int *d_jl = nullptr, *d_jm = nullptr, *d_perm = nullptr, *d_moff = nullptr;
+  int *d_jl = nullptr, *d_jm = nullptr, *d_moff = nullptr;
   double *d_g3 = nullptr, *d_g3rlm = nullptr, *d_gl = nullptr, *d_g6 = nullptr;
   double *d_g7 = nullptr, *d_g11 = nullptr, *d_g12 = nullptr;
   double *d_r = nullptr, *d_ar1 = nullptr, *d_ar2 = nullptr, *d_d1 = nullptr, *d_d2 = nullptr;

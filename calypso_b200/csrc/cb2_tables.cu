@@ -214,7 +214,6 @@ int setup_tables(Ctx &c) {
   if (off != c.jmax) { set_error("index table size mismatch"); return CB2_ERR_ARG; }
   c.h_jl.assign(c.jmax, 0);
   c.h_jm.assign(c.jmax, 0);
-  c.h_perm.assign(c.jmax, 0);
   for (int m = 0; m <= L; m++)
     for (int s = 0; s < (m == 0 ? 1 : 2); s++)
       for (int l = m; l <= L; l++) {
@@ -222,7 +221,6 @@ int setup_tables(Ctx &c) {
         int mm = s ? -m : m;
         c.h_jl[jj] = l;
         c.h_jm[jj] = mm;
-        c.h_perm[jj] = l * (l + 1) + mm;
       }
   // normalisations (reference: SERIAL_src/spherical_harmonics/spherical_harmonics.f90:92-141)
   std::vector<double> g3(c.jmax), g3rlm(c.jmax), gl(c.jmax), g6(c.jmax), g7(c.jmax), g11(c.jmax),
@@ -382,7 +380,7 @@ int setup_tables(Ctx &c) {
     po += (size_t)(L + 1 - m) * c.nh;
   }
   c.h_poff[L + 1] = po;
-  UP(c.d_jl, c.h_jl); UP(c.d_jm, c.h_jm); UP(c.d_perm, c.h_perm); UP(c.d_moff, c.h_moff);
+  UP(c.d_jl, c.h_jl); UP(c.d_jm, c.h_jm); UP(c.d_moff, c.h_moff);
   UP(c.d_g3, g3); UP(c.d_g3rlm, g3rlm); UP(c.d_gl, gl); UP(c.d_g6, g6); UP(c.d_g7, g7);
   UP(c.d_g11, g11); UP(c.d_g12, g12);
   UP(c.d_r, r); UP(c.d_ar1, ar1); UP(c.d_ar2, ar2); UP(c.d_d1, d1); UP(c.d_d2, d2);
@@ -408,7 +406,7 @@ int setup_tables(Ctx &c) {
 }
 
 void free_tables(Ctx &c) {
-  void *ptrs[] = {c.d_jl, c.d_jm, c.d_perm, c.d_moff, c.d_g3, c.d_g3rlm, c.d_gl, c.d_g6, c.d_g7,
+  void *ptrs[] = {c.d_jl, c.d_jm, c.d_moff, c.d_g3, c.d_g3rlm, c.d_gl, c.d_g6, c.d_g7,
                   c.d_g11, c.d_g12, c.d_r, c.d_ar1, c.d_ar2, c.d_d1, c.d_d2, c.d_reft0, c.d_reft1,
                   c.d_om, c.d_colat, c.d_wgt, c.d_asin, c.d_poff, c.d_Plt, c.d_dPlt, c.d_Ptl,
                   c.d_dPtl, c.d_jgi1, c.d_jgi2, c.d_jei1, c.d_sw, c.d_tw};
