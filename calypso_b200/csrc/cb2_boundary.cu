@@ -272,43 +272,55 @@ struct FastDiv {
 // rlm buffer along the nq components of a mode (a run of 8 nq bytes): a block
 // takes JT modes of consecutive jj at one radial level and turns them round
 // in shared memory, so both sides move in whole runs: bound by the runs'
-// partial sectors.  At L255 / Nr65 / 11 components 198 us inwards (3.8 TB/s);
+// partial sectors.  At L255 / Nr65 / 11 components 150 us inwards (5.0 TB/s);
 // a thread per mode, whose 8-byte slot writes scattered over the orders, took
 // 482 us.  Outwards at L170 / Nr49 / 12 components 73 us against 176.
 constexpr int JT = 64;
+constexpr int JK = 4;   // radial levels a block: that many independent loads a thread and mode
 
 template <bool TO_SLOTS>
 __global__ void __launch_bounds__(kBnd)
-k_rlm_slots(int nj, int ncomp, int is0, int is1, int comp0, FastDiv nq, int slot0, const int2 *__restrict__ jo,
-            double *__restrict__ rlm, double *__restrict__ f, size_t fs, int jmax) {
-  extern __shared__ double tile[];   // [JT][nq | 1]
+k_rlm_slots(int nj, int nr, int ncomp, int is0, int is1, int comp0, FastDiv nq, int slot0,
+            const int2 *__restrict__ jo, double *__restrict__ rlm, double *__restrict__ f, size_t fs, int jmax) {
+  extern __shared__ double tile[];   // [JK][JT][nq | 1]
   __shared__ int2 ent[JT];
-  const int i0 = blockIdx.x * JT, k = blockIdx.y, nt = min(JT, nj - i0), n = (int)nq.n, pitch = n | 1;
+  const int i0 = blockIdx.x * JT, k0 = blockIdx.y * JK, nt = min(JT, nj - i0), nk = min(JK, nr - k0);
+  const int n = (int)nq.n, pitch = n | 1, kp = JT * pitch;
   if (threadIdx.x < nt) ent[threadIdx.x] = jo[i0 + threadIdx.x];
   __syncthreads();
-  double *r0 = rlm + (size_t)ncomp * ((size_t)k * is0) + comp0;
-  double *f0 = f + (size_t)slot0 * fs + (size_t)k * jmax;
-  if (TO_SLOTS) {
+  const size_t rk = (size_t)ncomp * is0;
+  double *r0 = rlm + (size_t)k0 * rk + comp0;
+  double *f0 = f + (size_t)slot0 * fs + (size_t)k0 * jmax;
+  auto along_rlm = [&](bool load) {
     for (int e = threadIdx.x; e < nt * n; e += kBnd) {
       const int i = nq.div(e), q = e - i * n;
-      tile[i * pitch + q] = __ldg(r0 + (size_t)ncomp * ent[i].x * is1 + q);
+      double *g = r0 + (size_t)ncomp * ent[i].x * is1 + q, *t = tile + i * pitch + q;
+#pragma unroll
+      for (int k = 0; k < JK; k++)
+        if (k < nk) {
+          if (load) t[k * kp] = __ldg(g + k * rk);
+          else g[k * rk] = t[k * kp];
+        }
     }
-    __syncthreads();
+  };
+  auto along_slots = [&](bool load) {
     for (int e = threadIdx.x; e < JT * n; e += kBnd) {
       const int q = e / JT, i = e % JT;
-      if (i < nt) f0[(size_t)q * fs + ent[i].y] = tile[i * pitch + q];
+      if (i >= nt) continue;
+      double *g = f0 + (size_t)q * fs + ent[i].y, *t = tile + i * pitch + q;
+#pragma unroll
+      for (int k = 0; k < JK; k++)
+        if (k < nk) {
+          if (load) t[k * kp] = __ldg(g + (size_t)k * jmax);
+          else g[(size_t)k * jmax] = t[k * kp];
+        }
     }
-  } else {
-    for (int e = threadIdx.x; e < JT * n; e += kBnd) {
-      const int q = e / JT, i = e % JT;
-      if (i < nt) tile[i * pitch + q] = __ldg(f0 + (size_t)q * fs + ent[i].y);
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < nt * n; e += kBnd) {
-      const int i = nq.div(e), q = e - i * n;
-      r0[(size_t)ncomp * ent[i].x * is1 + q] = tile[i * pitch + q];
-    }
-  }
+  };
+  if (TO_SLOTS) along_rlm(true);
+  else along_slots(true);
+  __syncthreads();
+  if (TO_SLOTS) along_slots(false);
+  else along_rlm(false);
 }
 
 // Order-major Fourier rows <-> rtm buffer where the radius runs faster than
@@ -561,8 +573,8 @@ int cb2_leg_bwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, int nvector, int
     // modes the table leaves out are zero
     if (nj < c->jmax)
       CB2_CUDA(cudaMemsetAsync(c->fld(MADV), 0, (size_t)nc * c->fsize() * sizeof(double), c->stream));
-    k_rlm_slots<true><<<dim3(cdiv(nj, JT), c->nr), kBnd, JT * (nc | 1) * sizeof(double), c->stream>>>(
-        nj, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, FastDiv(nc), MADV, dt.jo, const_cast<double *>(dWR),
+    k_rlm_slots<true><<<dim3(cdiv(nj, JT), cdiv(c->nr, JK)), kBnd, JK * JT * (nc | 1) * sizeof(double), c->stream>>>(
+        nj, c->nr, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, FastDiv(nc), MADV, dt.jo, const_cast<double *>(dWR),
         c->d_f, c->fsize(), c->jmax);
     if (c->prec == CB2_PREC_FP64) {
       leg_bwd_f64(*c, ch.nv, ch.ns, slots, (double *)c->d_four);
@@ -607,8 +619,8 @@ int cb2_leg_fwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, int nvector, int
       const MLayout l = mlayout(*c, c->d_four, ch.nv, ch.ns);
       if ((rc = leg_fwd_mixed(*c, l, slots))) return rc;
     }
-    k_rlm_slots<false><<<dim3(cdiv(nj, JT), c->nr), kBnd, JT * (nc | 1) * sizeof(double), c->stream>>>(
-        nj, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, FastDiv(nc), MADV, dt.jo, dWS, c->d_f, c->fsize(),
+    k_rlm_slots<false><<<dim3(cdiv(nj, JT), cdiv(c->nr, JK)), kBnd, JK * JT * (nc | 1) * sizeof(double), c->stream>>>(
+        nj, c->nr, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, FastDiv(nc), MADV, dt.jo, dWS, c->d_f, c->fsize(),
         c->jmax);
   }
   CB2_CUDA(cudaGetLastError());
