@@ -281,7 +281,7 @@ k_tc_gemm(int M, int N, int NT, int K, const TAT *__restrict__ A, int lda, const
 // and SiLU 505); kept in tensor and shared memory the pass reads 64 and
 // writes 20 bytes a row and takes 189 us, bound by the SiLU epilogue (an
 // __expf and a divide per unit and layer) and the operand split.  A training
-// pass of 16384 rows: 35 + 45 + 69 us of kernels, before 500 us.
+// pass of 16384 rows: 35 + 45 + 51 us of kernels, before 500 us.
 //
 // A CTA keeps the bfloat16 weights in shared memory and walks tiles of 128
 // rows.  Warps 0-7 are the epilogue: warp w reads tensor-memory lanes
@@ -700,7 +700,7 @@ k_mlp_bwd(const __grid_constant__ MlpArgs a) {
 // k_tc_gemm.  The partial sums are added with 16-byte float32 atomics.
 // One launch for what three k_tc_gemm launches (96 us at 16384 rows) and
 // three column-sum launches (63 us, one block a column) did.
-constexpr int WG_THREADS = 256;
+constexpr int WG_THREADS = 512;
 struct WgradArgs {
   long long n;
   int F, H, O, kchunk;
@@ -745,46 +745,41 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
     if (ib >= 2 && !tc::mbar_wait(&bar[s], ((ib - 2) >> 1) & 1, a.wait_ns)) bad = true;
     if (__syncthreads_or(bad)) { bad = true; break; }
     unsigned char *tB = st + 6 * GA_BYTES, *tX = tB + 2 * bb, *tY = tX + 2 * 32 * 64;
-    // A tiles: thread = (unit, half of the 32 rows)
+    // A tiles: thread = (unit, chunk of 8 rows)
     {
-      const int m = tid & 127, h = tid >> 7, u = m0 + m;
+      const int m = tid & 127, c = tid >> 7, u = m0 + m;
       const bool ok = u < H;
+      float v2[8], v1[8], hh[8];
 #pragma unroll
-      for (int c = 2 * h; c < 2 * h + 2; c++) {
-        float v2[8], v1[8], hh[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-          const long long k = kb + c * 8 + e;
-          const bool in = ok && k < k1;
-          const size_t at = in ? (size_t)k * H + u : 0;
-          v2[e] = in ? __ldg(a.dZ2 + at) : 0.0f;
-          v1[e] = in ? __ldg(a.dZ1 + at) : 0.0f;
-          hh[e] = in ? __ldg(a.Z2 + at) : 0.0f;
-        }
-#pragma unroll
-        for (int e = 0; e < 8; e++) { sb2 += v2[e]; sb1 += v1[e]; hh[e] = silu(hh[e]); }
-        put_row8<2>(st, GA_BYTES, m, c, v2);
-        put_row8<2>(st + 2 * GA_BYTES, GA_BYTES, m, c, v1);
-        put_row8<2>(st + 4 * GA_BYTES, GA_BYTES, m, c, hh);
+      for (int e = 0; e < 8; e++) {
+        const long long k = kb + c * 8 + e;
+        const bool in = ok && k < k1;
+        const size_t at = in ? (size_t)k * H + u : 0;
+        v2[e] = in ? __ldg(a.dZ2 + at) : 0.0f;
+        v1[e] = in ? __ldg(a.dZ1 + at) : 0.0f;
+        hh[e] = in ? __ldg(a.Z2 + at) : 0.0f;
       }
+#pragma unroll
+      for (int e = 0; e < 8; e++) { sb2 += v2[e]; sb1 += v1[e]; hh[e] = silu(hh[e]); }
+      put_row8<2>(st, GA_BYTES, m, c, v2);
+      put_row8<2>(st + 2 * GA_BYTES, GA_BYTES, m, c, v1);
+      put_row8<2>(st + 4 * GA_BYTES, GA_BYTES, m, c, hh);
     }
-    // B tile H1: thread = unit
-    for (int u = tid; u < H; u += WG_THREADS) {
+    // B tile H1: thread = (unit, chunks of 8 rows)
+    for (int e0 = tid; e0 < 4 * H; e0 += WG_THREADS) {
+      const int u = e0 % H, c = e0 / H;
+      float v[8];
 #pragma unroll
-      for (int c = 0; c < 4; c++) {
-        float v[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-          const long long k = kb + c * 8 + e;
-          v[e] = (k < k1) ? __ldg(a.Z1 + (size_t)k * H + u) : 0.0f;
-        }
-#pragma unroll
-        for (int e = 0; e < 8; e++) v[e] = silu(v[e]);
-        put_row8<2>(tB, bb, u, c, v);
+      for (int e = 0; e < 8; e++) {
+        const long long k = kb + c * 8 + e;
+        v[e] = (k < k1) ? __ldg(a.Z1 + (size_t)k * H + u) : 0.0f;
       }
+#pragma unroll
+      for (int e = 0; e < 8; e++) v[e] = silu(v[e]);
+      put_row8<2>(tB, bb, u, c, v);
     }
     // B tiles X and dY: thread = (chunk of 8 rows, column)
-    {
+    if (tid < 256) {
       const int c = (tid >> 5) & 3, u = tid & 31;
       const bool isx = tid < 128;
       const int w = isx ? F : O;
@@ -833,7 +828,7 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
     const int qd = warp & 3, g = warp >> 2, u = m0 + qd * 32 + lane;
     const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
     float v[32];
-    for (int c = g; c < H / 32; c += 2) {
+    for (int c = g; c < H / 32; c += WG_THREADS / 128) {
       tmem_ld32(tl + c * 32, v);
       if (u < H) {
         float4 *d = reinterpret_cast<float4 *>(a.gW2 + (size_t)u * H + c * 32);
@@ -846,7 +841,7 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
 #pragma unroll
       for (int j = 0; j < 32; j++)
         if (u < H && j < F) atomicAdd(a.gW1 + (size_t)u * F + j, v[j]);
-    } else {
+    } else if (g == 1) {
       tmem_ld32(tl + 288, v);
 #pragma unroll
       for (int j = 0; j < ML_O; j++)
@@ -856,7 +851,7 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
       atomicAdd(a.gb1 + m0 + (tid & 127), sb1);
       atomicAdd(a.gb2 + m0 + (tid & 127), sb2);
     }
-    if (blockIdx.y == 0 && tid >= 128 && (tid & 31) < O) atomicAdd(a.gb3 + (tid & 31), sb3);
+    if (blockIdx.y == 0 && tid >= 128 && tid < 256 && (tid & 31) < O) atomicAdd(a.gb3 + (tid & 31), sb3);
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -959,18 +954,23 @@ using namespace cb2;
 
 // ---------------------------------------------------------------------------
 // the network
+constexpr size_t kTailBytes = 16;
 struct cb2_mlp {
   int F = 0, H = 0, O = 0;
   size_t oW1 = 0, ob1 = 0, oW2 = 0, ob2 = 0, oW3 = 0, ob3 = 0, np = 0;
   float *master = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
   __nv_bfloat16 *w = nullptr;   // bfloat16 copy of every parameter (the products use W1, W2, W3)
   int t = 0;
-  size_t cap = 0;               // rows of the work buffers
+  float *work = nullptr;        // the work buffers below, one allocation
+  size_t cap = 0;               // their rows
   float *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr, *Yp = nullptr, *dY = nullptr;
   float *dH = nullptr, *dZ = nullptr;
   double *part = nullptr;       // loss partial sums
-  int *status = nullptr;        // device status word of the GEMMs (bit 2: a wait ran out)
-  double *loss = nullptr;       // loss of the last fused training pass
+  // behind the gradient in its allocation, read together: the loss of the
+  // last fused training pass and the status word of the products (bit 2: a
+  // wait ran out)
+  double *loss = nullptr;
+  int *status = nullptr;
   size_t ycap = 0;              // rows of Yp
   cudaStream_t stream = nullptr;
 };
@@ -985,30 +985,22 @@ bool fused_ok(const cb2_mlp *n) {
   return n->F <= 32 && n->H % 32 == 0 && n->H >= 64 && n->H <= 256 && n->O <= ML_O && n->oW2 % 8 == 0;
 }
 
-int grow(float **p, size_t count) {
-  if (*p) cudaFree(*p);
-  *p = nullptr;
-  CB2_CUDA(cudaMalloc(p, count * sizeof(float)));
-  return 0;
-}
-
-// Work buffers of `rows` rows.  The fused passes keep the activations on the
-// chip: inference needs none of these, training Z1, Z2 and the gradients dY,
-// dZ2 (in dZ) and dZ1 (in dH).
+// Work buffers of `rows` rows, one allocation.  The fused passes keep the
+// activations on the chip: inference needs none of these, training Z1, Z2 and
+// the gradients dY, dZ2 (in dZ) and dZ1 (in dH).
 int mlp_reserve(cb2_mlp *n, size_t rows, bool train) {
-  int rc = 0;
-  if (fused_ok(n) && !train) return 0;
-  if (rows <= n->cap) return 0;
-  n->cap = 0;
-  const size_t w = (size_t)n->H;
-  if ((rc = grow(&n->Z1, rows * w)) || (rc = grow(&n->Z2, rows * w)) || (rc = grow(&n->dH, rows * w)) ||
-      (rc = grow(&n->dZ, rows * w)) || (rc = grow(&n->dY, rows * n->O)))
-    return rc;
-  if (!fused_ok(n) && ((rc = grow(&n->H1, rows * w)) || (rc = grow(&n->H2, rows * w)))) return rc;
+  const bool fused = fused_ok(n);
+  if ((fused && !train) || rows <= n->cap) return 0;
+  const size_t w = (rows * n->H + 63) / 64 * 64, wy = (rows * n->O + 63) / 64 * 64;
   const size_t pc = std::max((size_t)blocks(rows * n->O), 4 * ((rows + 127) / 128)) + 1;
-  if (n->part) cudaFree(n->part);
-  n->part = nullptr;
-  CB2_CUDA(cudaMalloc(&n->part, pc * sizeof(double)));
+  n->cap = 0;
+  if (n->work) cudaFree(n->work);
+  n->work = nullptr;
+  CB2_CUDA(cudaMalloc(&n->work, ((fused ? 4 : 6) * w + wy) * sizeof(float) + pc * sizeof(double)));
+  n->Z1 = n->work; n->Z2 = n->Z1 + w; n->dH = n->Z2 + w; n->dZ = n->dH + w;
+  n->H1 = n->dZ + w; n->H2 = n->H1 + w;   // the general passes only
+  n->dY = n->dZ + (fused ? 1 : 3) * w;
+  n->part = reinterpret_cast<double *>(n->dY + wy);
   n->cap = rows;
   return 0;
 }
@@ -1017,7 +1009,9 @@ int mlp_reserve(cb2_mlp *n, size_t rows, bool train) {
 int mlp_reserve_y(cb2_mlp *n, size_t rows) {
   if (rows <= n->ycap) return 0;
   n->ycap = 0;
-  if (int rc = grow(&n->Yp, rows * n->O)) return rc;
+  if (n->Yp) cudaFree(n->Yp);
+  n->Yp = nullptr;
+  CB2_CUDA(cudaMalloc(&n->Yp, rows * n->O * sizeof(float)));
   n->ycap = rows;
   return 0;
 }
@@ -1129,15 +1123,13 @@ int mlp_backward_fused(cb2_mlp *nt, const float *X, const float *T, size_t n) {
   return 0;
 }
 
-// loss and gradients of the mean squared error over n rows (grad <- dL/dparams)
-int mlp_backward(cb2_mlp *nt, const float *X, const float *T, size_t n, double *loss) {
+// loss (nt->loss) and gradients (grad <- dL/dparams) of the mean squared error over n rows
+int mlp_backward(cb2_mlp *nt, const float *X, const float *T, size_t n) {
   cudaStream_t st = nt->stream;
   int rc = mlp_reserve(nt, n, true);
   if (rc) return rc;
   if (fused_ok(nt)) {
     if ((rc = mlp_backward_fused(nt, X, T, n))) return rc;
-    // the caller waits for the stream (mlp_status) before it reads the loss
-    if (loss) CB2_CUDA(cudaMemcpyAsync(loss, nt->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
     return 0;
   }
   if ((rc = mlp_reserve_y(nt, n)) || (rc = mlp_forward(nt, X, n, nt->Yp, st))) return rc;
@@ -1158,14 +1150,8 @@ int mlp_backward(cb2_mlp *nt, const float *X, const float *T, size_t n, double *
   gemm<float, float, true, false>(st, nt->status, H, F, (int)n, nt->dZ, H, X, F, nt->grad + nt->oW1, F, true);
   k_colsum<<<H, 256, 0, st>>>(n, H, nt->dZ, nt->grad + nt->ob1);
   CB2_CUDA(cudaGetLastError());
-  if (loss) {
-    std::vector<double> hp(nb);
-    CB2_CUDA(cudaMemcpyAsync(hp.data(), nt->part, nb * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CB2_CUDA(cudaStreamSynchronize(st));
-    double s = 0.0;
-    for (double x : hp) s += x;
-    *loss = s / ((double)n * O);
-  }
+  k_loss_sum<<<1, 256, 0, st>>>(nb, nt->part, 1.0 / ((double)n * O), nt->loss);
+  CB2_CUDA(cudaGetLastError());
   return 0;
 }
 
@@ -1236,19 +1222,20 @@ int cb2_mlp_create(int nin, int nhid, int nout, unsigned seed, cb2_mlp **out) {
   fill(n->oW2, (size_t)nhid * nhid, nhid);
   fill(n->oW3, (size_t)nout * nhid, nhid);
   auto fail = [&](int rc) { cb2_mlp_destroy(n); return rc; };
+  const size_t gtail = (n->np + 3) / 4 * 4;
   if (cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&n->master, n->np * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&n->grad, n->np * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&n->grad, gtail * sizeof(float) + kTailBytes) != cudaSuccess ||
       cudaMalloc(&n->m, n->np * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&n->v, n->np * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&n->w, n->np * sizeof(__nv_bfloat16)) != cudaSuccess ||
-      cudaMalloc(&n->loss, sizeof(double)) != cudaSuccess || cudaMalloc(&n->status, sizeof(int)) != cudaSuccess)
+      cudaMalloc(&n->w, n->np * sizeof(__nv_bfloat16)) != cudaSuccess)
     return fail(cuda_fail(cudaGetLastError(), "cb2_mlp_create"));
+  n->loss = reinterpret_cast<double *>(n->grad + gtail);
+  n->status = reinterpret_cast<int *>(n->loss + 1);
   cudaMemcpy(n->master, p.data(), n->np * sizeof(float), cudaMemcpyHostToDevice);
-  cudaMemset(n->grad, 0, n->np * sizeof(float));
+  cudaMemset(n->grad, 0, gtail * sizeof(float) + kTailBytes);
   cudaMemset(n->m, 0, n->np * sizeof(float));
   cudaMemset(n->v, 0, n->np * sizeof(float));
-  cudaMemset(n->status, 0, sizeof(int));
   k_to_bf16<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->w);
   if (cudaStreamSynchronize(n->stream) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "cb2_mlp_create"));
   *out = n;
@@ -1258,8 +1245,7 @@ int cb2_mlp_create(int nin, int nhid, int nout, unsigned seed, cb2_mlp **out) {
 int cb2_mlp_destroy(cb2_mlp *n) {
   if (!n) return 0;
   if (n->stream) cudaStreamSynchronize(n->stream);
-  void *ptrs[] = {n->master, n->grad, n->m, n->v, n->w, n->Z1, n->H1, n->Z2, n->H2, n->Yp, n->dY, n->dH, n->dZ,
-                  n->part, n->loss, n->status};
+  void *ptrs[] = {n->master, n->grad, n->m, n->v, n->w, n->work, n->Yp};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   if (n->stream) cudaStreamDestroy(n->stream);
@@ -1284,17 +1270,19 @@ int cb2_mlp_set_params(cb2_mlp *n, const float *host) {
   return 0;
 }
 
-// the GEMMs' status word after the stream has drained: a pipeline wait
-// that ran out is reported (and the word cleared)
-static int mlp_status(cb2_mlp *n) {
-  int st = 0;
-  CB2_CUDA(cudaMemcpyAsync(&st, n->status, sizeof(int), cudaMemcpyDeviceToHost, n->stream));
+// the status word (and the last loss) after the stream has drained: a
+// pipeline wait that ran out is reported (and the word cleared)
+static int mlp_status(cb2_mlp *n, double *loss = nullptr) {
+  struct { double loss; int st; int pad; } tail;
+  static_assert(sizeof(tail) == kTailBytes, "gradient tail");
+  CB2_CUDA(cudaMemcpyAsync(&tail, n->loss, sizeof(tail), cudaMemcpyDeviceToHost, n->stream));
   CB2_CUDA(cudaStreamSynchronize(n->stream));
-  if (st) {
+  if (tail.st) {
     CB2_CUDA(cudaMemsetAsync(n->status, 0, sizeof(int), n->stream));
     set_error("closure network: a tensor-core pipeline wait ran out");
     return CB2_ERR_TIMEOUT;
   }
+  if (loss) *loss = tail.loss;
   return 0;
 }
 
@@ -1310,8 +1298,8 @@ int cb2_mlp_loss_grad(cb2_mlp *n, const float *dev_x, const float *dev_t, long l
                       float *host_grad) {
   if (!n || !dev_x || !dev_t || rows <= 0) return CB2_ERR_ARG;
   double l = 0.0;
-  int rc = mlp_backward(n, dev_x, dev_t, (size_t)rows, &l);
-  if (rc || (rc = mlp_status(n))) return rc;
+  int rc = mlp_backward(n, dev_x, dev_t, (size_t)rows);
+  if (rc || (rc = mlp_status(n, &l))) return rc;
   if (loss) *loss = l;
   if (host_grad) CB2_CUDA(cudaMemcpy(host_grad, n->grad, n->np * sizeof(float), cudaMemcpyDeviceToHost));
   return 0;
