@@ -242,6 +242,19 @@ __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring
   for (int t = 0; t < NL; t++) yh[t] = 0.0;
 #pragma unroll
   for (int t = 0; t <= PD; t++) pend[t] = 0.0;
+  // the factors of the next row, loaded a row ahead: read where the
+  // recurrence needs them, each row waited on L1 or L2 twice (the interchange,
+  // then the multipliers).  L255 / Nr129 803 -> 733 us (56 -> 62 % of HBM);
+  // the step at L31 / Nr129, where the rows' chain is all, 334 -> 278.
+  double fn[NL];
+  int dn = 0;
+  auto factors = [&](int i) {
+    if (i >= n) return;
+    if constexpr (PD >= 1) dn = fac.piv(i);
+#pragma unroll
+    for (int t = 0; t < NL; t++) fn[t] = fac.at(i, NE, t);
+  };
+  factors(0);
   int sl = 0;
   for (int k = 0; k < n + PD; k++) {
     double b = 0.0;
@@ -261,15 +274,19 @@ __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring
     pend[PD] = b;
     const int i = k - PD;
     if (i >= 0 && i < n) {
+      double fc[NL];
+#pragma unroll
+      for (int t = 0; t < NL; t++) fc[t] = fn[t];
+      const int d = dn;
+      factors(i + 1);
       if constexpr (PD >= 1) {
-        const int d = fac.piv(i);
         if (d == 1) { const double t = pend[0]; pend[0] = pend[1]; pend[1] = t; }
         if constexpr (PD >= 2)
           if (d == 2) { const double t = pend[0]; pend[0] = pend[2]; pend[2] = t; }
       }
       double y = pend[0];
 #pragma unroll
-      for (int t = NL - 1; t >= 0; t--) y = y - fac.at(i, NE, t) * yh[t];
+      for (int t = NL - 1; t >= 0; t--) y = y - fc[t] * yh[t];
       S.stkeep(i, st, y, keep);
 #pragma unroll
       for (int t = NL - 1; t > 0; t--) yh[t] = yh[t - 1];
@@ -305,13 +322,24 @@ __device__ __forceinline__ void cn_backward(const CnCtx &q, FacCol fac, Ring rin
   double xh[NL];   // x(k + 1 + t)
 #pragma unroll
   for (int t = 0; t < NL; t++) xh[t] = 0.0;
+  double fn[NL + 1];   // the next row's factors, a row ahead as in cn_forward
+  auto factors = [&](int k) {
+    if (k < 0) return;
+#pragma unroll
+    for (int t = 0; t <= NL; t++) fn[t] = fac.at(k, NE, NL + t);
+  };
+  factors(n - 1);
   int sl = 0;
   for (int k = n - 1; k >= 0; k--) {
     cp_wait<CN_RING - 1>();
+    double fc[NL + 1];
+#pragma unroll
+    for (int t = 0; t <= NL; t++) fc[t] = fn[t];
+    factors(k - 1);
     double v = *ring.at(sl, 0);
 #pragma unroll
-    for (int t = 0; t < NL; t++) v = v - fac.at(k, NE, NL + t) * xh[t];
-    const double x = v * fac.at(k, NE, 2 * NL);
+    for (int t = 0; t < NL; t++) v = v - fc[t] * xh[t];
+    const double x = v * fc[NL];
 #pragma unroll
     for (int t = NL - 1; t > 0; t--) xh[t] = xh[t - 1];
     xh[0] = x;
