@@ -704,6 +704,12 @@ int cn_setup(Ctx &c) {
   c.cn_pack = new CnPack(pk);
   c.cn_smem = smem;
   c.cn_ready = true;
+  // The one kernel is the default wherever it takes the context.  Mixed steps,
+  // one kernel against the separate ones, us: L7 / Nr9 53 / 60, L15 / Nr17
+  // 74 / 85, L31 / Nr33 93 / 101, L31 / Nr129 278 / 317, L63 / Nr65 302 / 299,
+  // L127 / Nr25 326 / 354, L127 / Nr97 1129 / 1230, L191 / Nr65 3747 / 3853,
+  // L255 / Nr129 5075 / 5524.
+  c.tune[TUNE_CN] = 1;
   return 0;
 }
 

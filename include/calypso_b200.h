@@ -278,8 +278,8 @@ int cb2_free_pinned(void *p);
  * on the float64 tensor cores), mixed pack radial tile, FFT kernel of either
  * precision (384: the four-step kernel, used where nphi = 3 (ltr + 1);
  * 128, 256, 512: the Stockham kernel, float64 always with 512 threads), and
- * 1 to run the explicit update, the radial solves and the derived fields
- * of the step as one kernel, 0 (the default) as separate kernels; -1
+ * 1 (the default) to run the explicit update, the radial solves and the
+ * derived fields of the step as one kernel, 0 as separate kernels; -1
  * (fixed) where the one kernel cannot take the context (cb2_tuning_note
  * says why). */
 int cb2_autotune(cb2_ctx *ctx);
