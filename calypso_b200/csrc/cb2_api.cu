@@ -193,11 +193,12 @@ static int nonlinear(Ctx &c) {
   int rc = nl_head(c);
   if (rc) return rc;
   if (c.prec == CB2_PREC_FP64) {
-    leg_bwd_f64(c, 4, 1, kBwdSlots, (double *)c.d_four);
+    const MLayout64 fin = mlayout64(c, c.d_four, 4, 1), fout = mlayout64(c, c.d_four2, 4, 0);
+    leg_bwd_f64(c, kBwdSlots, fin);
     if (c.timers) cudaEventRecord(c.ev[12], c.stream);
-    fft_products<double>(c, (const double *)c.d_four, (double *)c.d_four2);
+    fft_products64(c, fin, fout);
     if (c.timers) cudaEventRecord(c.ev[13], c.stream);
-    leg_fwd_f64(c, 4, 0, (const double *)c.d_four2, kFwdSlots);
+    leg_fwd_f64(c, fout, kFwdSlots);
   } else {
     if ((rc = leg_bwd_gemm(c, mlayout(c, c.d_four, 4, 1)))) return rc;
     if ((rc = nl_grid(c))) return rc;
@@ -346,8 +347,7 @@ int cb2_create(const cb2_params *p, int precision, int device, cb2_ctx **out) {
     return fail(cuda_fail(cudaGetLastError(), "cudaMalloc(fields)"));
   cudaMemsetAsync(c->d_f, 0, (size_t)NSLOT * fs * sizeof(double), c->stream);
   size_t rows = (size_t)c->nth * c->nr * c->NS;
-  // float64 rows [theta][k][c][s] (13 and 12 components), or the padded
-  // order-major float32 layout of the mixed path
+  // order-major Fourier rows of 13 and 12 components, float64 or (padded) float32
   const size_t b1 = (precision == CB2_PREC_FP64) ? rows * 13 * sizeof(double) : mlayout_floats(*c) * sizeof(float);
   const size_t b2 = (precision == CB2_PREC_FP64) ? rows * 12 * sizeof(double) : mlayout_floats(*c) * sizeof(float);
   if (cudaMalloc(&c->d_four, b1) != cudaSuccess ||
@@ -765,12 +765,13 @@ int cb2_sht_backward(cb2_ctx *c, int nvec, int nscal, const double *spec, double
   double *dgrid = nullptr;
   CB2_CUDA(cudaMalloc(&dgrid, gsz * sizeof(double)));
   if (c->prec == CB2_PREC_FP64) {
-    leg_bwd_f64(*c, nvec, nscal, slots, (double *)c->d_four);
-    fft_backward_grid<double>(*c, nc, (const double *)c->d_four, dgrid);
+    const MLayout64 l = mlayout64(*c, c->d_four, nvec, nscal);
+    leg_bwd_f64(*c, slots, l);
+    fft_backward_grid<double>(*c, l, dgrid);
   } else {
     const MLayout l = mlayout(*c, c->d_four, nvec, nscal);
     if ((rc = leg_bwd_mixed(*c, slots, l))) { cudaFree(dgrid); return rc; }
-    fft_backward_grid_m(*c, l, dgrid);
+    fft_backward_grid<float>(*c, l, dgrid);
   }
   CB2_CUDA(cudaGetLastError());
   CB2_CUDA(cudaMemcpyAsync(grid, dgrid, gsz * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -791,11 +792,12 @@ int cb2_sht_forward(cb2_ctx *c, int nvec, int nscal, const double *grid, double 
   CB2_CUDA(cudaMalloc(&dgrid, gsz * sizeof(double)));
   CB2_CUDA(cudaMemcpyAsync(dgrid, grid, gsz * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   if (c->prec == CB2_PREC_FP64) {
-    fft_forward_grid<double>(*c, nc, dgrid, (double *)c->d_four);
-    leg_fwd_f64(*c, nvec, nscal, (const double *)c->d_four, slots);
+    const MLayout64 l = mlayout64(*c, c->d_four, nvec, nscal);
+    fft_forward_grid<double>(*c, dgrid, l);
+    leg_fwd_f64(*c, l, slots);
   } else {
     const MLayout l = mlayout(*c, c->d_four, nvec, nscal);
-    fft_forward_grid_m(*c, dgrid, l);
+    fft_forward_grid<float>(*c, dgrid, l);
     if ((rc = leg_fwd_mixed(*c, l, slots))) { cudaFree(dgrid); return rc; }
   }
   CB2_CUDA(cudaGetLastError());

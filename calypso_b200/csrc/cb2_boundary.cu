@@ -261,13 +261,6 @@ std::vector<Chunk> chunks(int prec, int nvec, int nscal) {
 
 constexpr int kBnd = 256;
 
-// e / n for 0 <= e < 2^16 and 1 <= n <= 2^15: (e * ceil(2^32 / n)) >> 32
-struct FastDiv {
-  unsigned n, mul;
-  explicit FastDiv(int d) : n((unsigned)d), mul((unsigned)((0x100000000ull + d - 1) / d)) {}
-  __device__ __forceinline__ int div(int e) const { return n == 1 ? e : (int)__umulhi((unsigned)e, mul); }
-};
-
 // rlm buffer <-> work slots (device order).  The slots run along jj, the
 // rlm buffer along the nq components of a mode (a run of 8 nq bytes): a block
 // takes JT modes of consecutive jj at one radial level and turns them round
@@ -330,7 +323,8 @@ k_rlm_slots(int nj, int nr, int ncomp, int is0, int is1, int comp0, FastDiv nq, 
 // components in a loop (k_four_to_rtm / k_rtm_to_four, which stay for the
 // other stride orders) wrote 8 bytes of every line at a time: 1112 us
 // outwards at L255 / Nr65 / 11 components, now 295 us (5.6 TB/s); 323 us
-// inwards at L170 / Nr49 / 12, now 140 us.  Bound by HBM.
+// inwards at L170 / Nr49 / 12, now 140 us; float64 at L106 / Nr41 / 11 inwards
+// 264 us, now 54.  Bound by HBM.
 struct CompOff {
   int off[13];     // element offset of component c (s = 0) within its block's radial level
   int inD;         // bit c: component c sits in the D block
@@ -338,28 +332,29 @@ struct CompOff {
 
 constexpr int RTH = 8;   // colatitudes a block: that many independent loads a thread
 
+template <typename T>
 __global__ void __launch_bounds__(kBnd)
-k_rows_to_rtm(MLayout ml, CompOff co, FastDiv nc, int ncomp, int is0, int is1, int is2, int comp0,
+k_rows_to_rtm(MLayoutT<T> ml, CompOff co, FastDiv nc, int ncomp, int is0, int is1, int is2, int comp0,
               const int4 *__restrict__ mo, double *__restrict__ WS) {
   __shared__ int off[13];
   const int4 me = mo[blockIdx.x];   // mp, |m|, s
   const int th0 = blockIdx.y * RTH, nt = min(RTH, ml.nth - th0), n = (int)nc.n;
   if (threadIdx.x < 13) off[threadIdx.x] = co.off[threadIdx.x];
   __syncthreads();
-  const float *P = ml.P + ((size_t)me.y * ml.nth + th0) * ml.sP() + me.z;
-  const float *D = ml.D + ((size_t)me.y * ml.nth + th0) * ml.sD() + me.z;
+  const T *P = ml.P + ((size_t)me.y * ml.nth + th0) * ml.sP() + me.z;
+  const T *D = ml.D + ((size_t)me.y * ml.nth + th0) * ml.sD() + me.z;
   const int rP = ml.rpP(), rD = ml.rpD();
   double *w = WS + (size_t)ncomp * ((size_t)th0 * is1 + (size_t)me.x * is2) + comp0;
   const size_t wt = (size_t)ncomp * is1;
   for (int e = threadIdx.x; e < ml.nr * n; e += kBnd) {
     const int k = nc.div(e), c = e - k * n;
     const bool d = co.inD >> c & 1;
-    const float *src = d ? D + k * rD + off[c] : P + k * rP + off[c];
+    const T *src = d ? D + k * rD + off[c] : P + k * rP + off[c];
     const size_t st = d ? ml.sD() : ml.sP();
     double *o = w + (size_t)ncomp * k * is0 + c;
-    float v[RTH];
+    T v[RTH];
 #pragma unroll
-    for (int i = 0; i < RTH; i++) v[i] = (i < nt) ? __ldg(src + i * st) : 0.0f;
+    for (int i = 0; i < RTH; i++) v[i] = (i < nt) ? __ldg(src + i * st) : (T)0;
 #pragma unroll
     for (int i = 0; i < RTH; i++)
       if (i < nt) o[i * wt] = (double)v[i];
@@ -368,45 +363,46 @@ k_rows_to_rtm(MLayout ml, CompOff co, FastDiv nc, int ncomp, int is0, int is1, i
 
 // every element of the order's rows, both signs: an order the table does not
 // list is zero, as are the sine part of m = 0 and the padding
+template <typename T>
 __global__ void __launch_bounds__(kBnd)
-k_rtm_to_rows(MLayout ml, int ncomp, int is0, int is1, int is2, int comp0, FastDiv rP, FastDiv rD,
+k_rtm_to_rows(MLayoutT<T> ml, int ncomp, int is0, int is1, int is2, int comp0, FastDiv rP, FastDiv rD,
               const int *__restrict__ mpos, const double *__restrict__ WR) {
   const int m = blockIdx.x, th = blockIdx.y, nr = ml.nr, nv = ml.nvec;
   const int mp0 = mpos[2 * m], mp1 = (m > 0) ? mpos[2 * m + 1] : -1;
   const double *w0 = WR + (size_t)ncomp * ((size_t)th * is1 + (size_t)max(mp0, 0) * is2) + comp0;
   const double *w1 = WR + (size_t)ncomp * ((size_t)th * is1 + (size_t)max(mp1, 0) * is2) + comp0;
   const size_t ks = (size_t)ncomp * is0;
-  float *P = ml.P + ((size_t)m * ml.nth + th) * ml.sP();
+  T *P = ml.P + ((size_t)m * ml.nth + th) * ml.sP();
   const int eP = nr * (int)rP.n, eP4 = (int)ml.sP(), eD = nr * (int)rD.n, eD4 = (int)ml.sD();
   for (int e = threadIdx.x; e < eP4; e += kBnd) {
     const int k = rP.div(e), x = e - k * (int)rP.n, fl = x >> 1, c = (fl < nv) ? 3 * fl : 2 * nv + fl;
-    float v = 0.0f;
-    if (e < eP && ((x & 1) ? mp1 : mp0) >= 0) v = (float)__ldg(((x & 1) ? w1 : w0) + k * ks + c);
+    T v = (T)0;
+    if (e < eP && ((x & 1) ? mp1 : mp0) >= 0) v = (T)__ldg(((x & 1) ? w1 : w0) + k * ks + c);
     P[e] = v;
   }
   if (nv == 0) return;
-  float *D = ml.D + ((size_t)m * ml.nth + th) * ml.sD();
+  T *D = ml.D + ((size_t)m * ml.nth + th) * ml.sD();
   for (int e = threadIdx.x; e < eD4; e += kBnd) {
     const int k = rD.div(e), x = e - k * (int)rD.n, c = 3 * (x >> 2) + 1 + ((x & 3) >> 1);
-    float v = 0.0f;
-    if (e < eD && ((x & 1) ? mp1 : mp0) >= 0) v = (float)__ldg(((x & 1) ? w1 : w0) + k * ks + c);
+    T v = (T)0;
+    if (e < eD && ((x & 1) ? mp1 : mp0) >= 0) v = (T)__ldg(((x & 1) ? w1 : w0) + k * ks + c);
     D[e] = v;
   }
 }
 
-// Fourier rows of the context (float64 [theta][k][c][slot] with nc
-// components, or the mixed float32 layout) <-> rtm buffer; one thread per
-// (theta, k), blockIdx.y = mp
+// Fourier rows of the context, in its precision: one thread per (theta, k) and
+// order with the components in a loop, for the stride orders the row kernels
+// above do not take
 struct FourView {
-  double *f64 = nullptr;   // float64 rows, nc components, NS slots
-  int nc = 0, NS = 0, nr = 0;
-  MLayout ml;              // mixed rows when f64 is null
+  int nc = 0;
+  bool f64 = false;
+  MLayout ml;
+  MLayout64 md;
   __device__ double get(int m, int th, int k, int c, int s) const {
-    if (f64) return f64[(((size_t)th * nr + k) * nc + c) * NS + 2 * m + s];
-    return (double)*ml.at(m, th, k, c, s);
+    return f64 ? *md.at(m, th, k, c, s) : (double)*ml.at(m, th, k, c, s);
   }
   __device__ void put(int m, int th, int k, int c, int s, double v) const {
-    if (f64) f64[(((size_t)th * nr + k) * nc + c) * NS + 2 * m + s] = v;
+    if (f64) *md.at(m, th, k, c, s) = v;
     else *ml.at(m, th, k, c, s) = (float)v;
   }
 };
@@ -460,10 +456,9 @@ __global__ void k_rtp_to_grid(int nc, int nr, int nth, int nph, int is0, int is1
 FourView four_view(Ctx &c, int nv, int ns, void *buf = nullptr) {
   if (!buf) buf = c.d_four;
   FourView fv;
-  fv.nr = c.nr;
-  fv.NS = c.NS;
   fv.nc = 3 * nv + ns;
-  if (c.prec == CB2_PREC_FP64) fv.f64 = (double *)buf;
+  fv.f64 = c.prec == CB2_PREC_FP64;
+  if (fv.f64) fv.md = mlayout64(c, buf, nv, ns);
   else fv.ml = mlayout(c, buf, nv, ns);
   return fv;
 }
@@ -473,39 +468,52 @@ size_t four_bytes(const Ctx &c) {
                                    : mlayout_floats(c) * sizeof(float);
 }
 
+// the row kernels of one chunk, where the radius runs faster than the order;
+// false: the strides are another kind, nothing done
+template <typename T>
+bool rows_out_k(Ctx &c, const cb2_sph_tables *t, const DevTab &dt, const MLayoutT<T> &ml, int ncomp, int comp0,
+                double *dWS) {
+  const int *is = t->istep_rtm, nm = t->nidx_rtm[2], nc = 3 * ml.nvec + ml.nscal;
+  if (is[0] > is[2] || c.nr * nc >= (1 << 16) || c.nth >= (1 << 16)) return false;
+  CompOff co{};
+  for (int q = 0; q < nc; q++) {
+    const int v = q / 3, cc = q - 3 * v;
+    if (q >= 3 * ml.nvec) co.off[q] = 2 * (ml.nvec + q - 3 * ml.nvec);
+    else if (cc == 0) co.off[q] = 2 * v;
+    else { co.off[q] = 4 * v + 2 * (cc - 1); co.inD |= 1 << q; }
+  }
+  k_rows_to_rtm<T><<<dim3(nm, cdiv(c.nth, RTH)), kBnd, 0, c.stream>>>(ml, co, FastDiv(nc), ncomp, is[0], is[1], is[2],
+                                                                      comp0, dt.mo, dWS);
+  return true;
+}
+
+template <typename T>
+bool rows_in_k(Ctx &c, const cb2_sph_tables *t, const DevTab &dt, const MLayoutT<T> &ml, int ncomp, int comp0,
+               const double *dWR) {
+  const int *is = t->istep_rtm;
+  if (is[0] > is[2] || ml.sP() >= (1u << 16) || ml.sD() >= (1u << 16) || c.nth >= (1 << 16)) return false;
+  k_rtm_to_rows<T><<<dim3(c.L + 1, c.nth), kBnd, 0, c.stream>>>(ml, ncomp, is[0], is[1], is[2], comp0,
+                                                                FastDiv(ml.rpP()), FastDiv(std::max(1, ml.rpD())),
+                                                                dt.mpos, dWR);
+  return true;
+}
+
 // Fourier rows -> rtm buffer of one chunk
 void rows_out(Ctx &c, const cb2_sph_tables *t, const DevTab &dt, const FourView &fv, int ncomp, int comp0, double *dWS) {
-  const int *is = t->istep_rtm, nm = t->nidx_rtm[2];
-  if (!fv.f64 && is[0] <= is[2] && c.nr * fv.nc < (1 << 16) && c.nth < (1 << 16)) {
-    CompOff co{};
-    const MLayout &ml = fv.ml;
-    for (int q = 0; q < fv.nc; q++) {
-      const int v = q / 3, cc = q - 3 * v;
-      if (q >= 3 * ml.nvec) co.off[q] = 2 * (ml.nvec + q - 3 * ml.nvec);
-      else if (cc == 0) co.off[q] = 2 * v;
-      else { co.off[q] = 4 * v + 2 * (cc - 1); co.inD |= 1 << q; }
-    }
-    k_rows_to_rtm<<<dim3(nm, cdiv(c.nth, RTH)), kBnd, 0, c.stream>>>(ml, co, FastDiv(fv.nc), ncomp, is[0], is[1], is[2], comp0,
-                                                          dt.mo, dWS);
-    return;
-  }
-  k_four_to_rtm<<<dim3(cdiv((long)c.nth * c.nr, kBnd), nm), kBnd, 0, c.stream>>>(fv, c.nth, c.nr, ncomp, is[0], is[1],
-                                                                                 is[2], comp0, dt.mq, dWS);
+  if (fv.f64 ? rows_out_k(c, t, dt, fv.md, ncomp, comp0, dWS) : rows_out_k(c, t, dt, fv.ml, ncomp, comp0, dWS)) return;
+  const int *is = t->istep_rtm;
+  k_four_to_rtm<<<dim3(cdiv((long)c.nth * c.nr, kBnd), t->nidx_rtm[2]), kBnd, 0, c.stream>>>(
+      fv, c.nth, c.nr, ncomp, is[0], is[1], is[2], comp0, dt.mq, dWS);
 }
 
 // rtm buffer -> every element of the Fourier rows of one chunk
 int rows_in(Ctx &c, const cb2_sph_tables *t, const DevTab &dt, const FourView &fv, int ncomp, int comp0,
             const double *dWR) {
-  const int *is = t->istep_rtm, nm = t->nidx_rtm[2];
-  if (!fv.f64 && is[0] <= is[2] && fv.ml.sP() < (1u << 16) && fv.ml.sD() < (1u << 16) && c.nth < (1 << 16)) {
-    const MLayout &ml = fv.ml;
-    k_rtm_to_rows<<<dim3(c.L + 1, c.nth), kBnd, 0, c.stream>>>(ml, ncomp, is[0], is[1], is[2], comp0, FastDiv(ml.rpP()),
-                                                               FastDiv(std::max(1, ml.rpD())), dt.mpos, dWR);
-    return 0;
-  }
-  CB2_CUDA(cudaMemsetAsync(fv.f64 ? (void *)fv.f64 : (void *)fv.ml.P, 0, four_bytes(c), c.stream));
-  k_rtm_to_four<<<dim3(cdiv((long)c.nth * c.nr, kBnd), nm), kBnd, 0, c.stream>>>(fv, c.nth, c.nr, ncomp, is[0], is[1],
-                                                                                 is[2], comp0, dt.mq, dWR);
+  if (fv.f64 ? rows_in_k(c, t, dt, fv.md, ncomp, comp0, dWR) : rows_in_k(c, t, dt, fv.ml, ncomp, comp0, dWR)) return 0;
+  const int *is = t->istep_rtm;
+  CB2_CUDA(cudaMemsetAsync(fv.f64 ? (void *)fv.md.P : (void *)fv.ml.P, 0, four_bytes(c), c.stream));
+  k_rtm_to_four<<<dim3(cdiv((long)c.nth * c.nr, kBnd), t->nidx_rtm[2]), kBnd, 0, c.stream>>>(
+      fv, c.nth, c.nr, ncomp, is[0], is[1], is[2], comp0, dt.mq, dWR);
   return 0;
 }
 
@@ -577,7 +585,7 @@ int cb2_leg_bwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, int nvector, int
         nj, c->nr, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, FastDiv(nc), MADV, dt.jo, const_cast<double *>(dWR),
         c->d_f, c->fsize(), c->jmax);
     if (c->prec == CB2_PREC_FP64) {
-      leg_bwd_f64(*c, ch.nv, ch.ns, slots, (double *)c->d_four);
+      leg_bwd_f64(*c, slots, mlayout64(*c, c->d_four, ch.nv, ch.ns));
     } else {
       const MLayout l = mlayout(*c, c->d_four, ch.nv, ch.ns);
       if ((rc = leg_bwd_mixed(*c, slots, l))) return rc;
@@ -614,7 +622,7 @@ int cb2_leg_fwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, int nvector, int
     for (int s = 0; s < ch.ns; s++) slots[ch.nv + s] = MADV + 3 * ch.nv + s;
     if ((rc = rows_in(*c, t, dt, four_view(*c, ch.nv, ch.ns), ncomp, ch.comp0, dWR))) return rc;
     if (c->prec == CB2_PREC_FP64) {
-      leg_fwd_f64(*c, ch.nv, ch.ns, (const double *)c->d_four, slots);
+      leg_fwd_f64(*c, mlayout64(*c, c->d_four, ch.nv, ch.ns), slots);
     } else {
       const MLayout l = mlayout(*c, c->d_four, ch.nv, ch.ns);
       if ((rc = leg_fwd_mixed(*c, l, slots))) return rc;
@@ -645,8 +653,8 @@ int cb2_fft_bwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, size_t n_WR, con
     const int nc = std::min(13, ncomp - c0);
     FourView fv = four_view(*c, 0, nc);
     if ((rc = rows_in(*c, t, dt, fv, ncomp, c0, dWR))) return rc;
-    if (c->prec == CB2_PREC_FP64) fft_backward_grid<double>(*c, nc, (const double *)c->d_four, c->d_bnd_grid);
-    else fft_backward_grid_m(*c, fv.ml, c->d_bnd_grid);
+    if (fv.f64) fft_backward_grid<double>(*c, fv.md, c->d_bnd_grid);
+    else fft_backward_grid<float>(*c, fv.ml, c->d_bnd_grid);
     k_grid_to_rtp<<<cdiv((long)nnod, kBnd), kBnd, 0, c->stream>>>(nc, c->nr, c->nth, c->nph, t->istep_rtp[0],
                                                                   t->istep_rtp[1], t->istep_rtp[2], c0, nnod,
                                                                   c->d_bnd_grid, dF);
@@ -673,7 +681,7 @@ int cb2_fft_products(cb2_ctx *c, const cb2_sph_tables *t, size_t n_WR, const dou
   if ((rc = clear_rtm(*c, t, 12, 12, n_WS, dWS))) return rc;
   const FourView fin = four_view(*c, 4, 1), fout = four_view(*c, 4, 0, c->d_four2);
   if ((rc = rows_in(*c, t, dt, fin, 13, 0, dWR))) return rc;
-  if (c->prec == CB2_PREC_FP64) fft_products<double>(*c, (const double *)c->d_four, (double *)c->d_four2);
+  if (fin.f64) fft_products64(*c, fin.md, fout.md);
   else fft_products_m(*c, fin.ml, fout.ml);
   rows_out(*c, t, dt, fout, 12, 0, dWS);
   CB2_CUDA(cudaGetLastError());
@@ -700,8 +708,8 @@ int cb2_fft_fwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, const double *fr
                                                                   t->istep_rtp[1], t->istep_rtp[2], c0, nnod, dF,
                                                                   c->d_bnd_grid);
     FourView fv = four_view(*c, 0, nc);
-    if (c->prec == CB2_PREC_FP64) fft_forward_grid<double>(*c, nc, c->d_bnd_grid, (double *)c->d_four);
-    else fft_forward_grid_m(*c, c->d_bnd_grid, fv.ml);
+    if (fv.f64) fft_forward_grid<double>(*c, c->d_bnd_grid, fv.md);
+    else fft_forward_grid<float>(*c, c->d_bnd_grid, fv.ml);
     rows_out(*c, t, dt, fv, ncomp, c0, dWS);
   }
   CB2_CUDA(cudaGetLastError());

@@ -143,44 +143,6 @@ __device__ T2 *block_fft(T2 *x, T2 *y, const FFTPlan &pl, const T2 *tw, int sign
   return x;
 }
 
-// spectrum of two real rows -> z = x + i y (Z = X + i Y, X Hermitian)
-template <typename T, typename T2>
-__device__ void load_pair(T2 *Z, int N, int L, const T *f0, const T *f1) {
-  for (int q = threadIdx.x; q < N; q += blockDim.x) Z[q] = T2{0, 0};
-  __syncthreads();
-  int mmax = min(L, (N + 1) / 2 - 1);
-  for (int m = threadIdx.x; m <= mmax; m += blockDim.x) {
-    T a0 = f0[2 * m], b0 = (m > 0) ? f0[2 * m + 1] : (T)0;
-    T a1 = f1 ? f1[2 * m] : (T)0, b1 = (f1 && m > 0) ? f1[2 * m + 1] : (T)0;
-    if (m == 0) {
-      Z[0] = T2{a0, a1};
-    } else {
-      T xr = (T)0.5 * a0, xi = (T)-0.5 * b0, yr = (T)0.5 * a1, yi = (T)-0.5 * b1;
-      Z[m] = T2{xr - yi, xi + yr};
-      Z[N - m] = T2{xr + yi, -xi + yr};
-    }
-  }
-  __syncthreads();
-}
-
-// FFT of z = x + i y -> (a_m, b_m) of both rows, m = 0..L
-template <typename T, typename T2>
-__device__ void store_pair(const T2 *Z, int N, int L, T *f0, T *f1) {
-  T an = (T)(1.0 / (double)N);
-  for (int m = threadIdx.x; m <= L; m += blockDim.x) {
-    if (m == 0) {
-      f0[0] = an * Z[0].x; f0[1] = 0;
-      if (f1) { f1[0] = an * Z[0].y; f1[1] = 0; }
-    } else if (m < N) {
-      T2 zk = Z[m % N], zn = Z[(N - m) % N];
-      T xr = (T)0.5 * (zk.x + zn.x), xi = (T)0.5 * (zk.y - zn.y);
-      T yr = (T)0.5 * (zk.y + zn.y), yi = (T)-0.5 * (zk.x - zn.x);
-      f0[2 * m] = (T)2 * an * xr; f0[2 * m + 1] = (T)-2 * an * xi;
-      if (f1) { f1[2 * m] = (T)2 * an * yr; f1[2 * m + 1] = (T)-2 * an * yi; }
-    }
-  }
-}
-
 struct ProdCoef {
   double cv, cl, ci, ct;
 };
@@ -250,164 +212,9 @@ __device__ T2 *batch_fft(T2 *x, T2 *y, int nf, const FFTPlan &pl, const T2 *__re
   return x;
 }
 
-// one block per (theta, r) row: 13 components -> grid -> 12 products -> spectra
-template <typename T>
-__global__ void __launch_bounds__(512)
-k_fft_products(FFTPlan pl, int L, int NS, const T *__restrict__ four, T *__restrict__ four2,
-               const typename C2<T>::t *__restrict__ tw, ProdCoef pc) {
-  using T2 = typename C2<T>::t;
-  using U = typename PairBits<T>::U;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int N = pl.n;
-  T2 *A = reinterpret_cast<T2 *>(smraw);    // 7 x N
-  T2 *B = A + 7 * N;                         // 7 x N
-  U *cmx = reinterpret_cast<U *>(B + 7 * N); // [13] input maxima, [13..24] product maxima (bits)
-  const size_t row = blockIdx.x;
-  const T *fin = four + row * 13 * NS;
-  T *fout = four2 + row * 12 * NS;
-  const int mmax = min(L, (N + 1) / 2 - 1);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  if (threadIdx.x < 25) cmx[threadIdx.x] = 0;
-  __syncthreads();
-  // pair scaling (pair_exp): the largest coefficient of each component
-  for (int c = warp; c < 13; c += nwarp) {
-    U mx = 0;
-    for (int q = lane; q < 2 * (mmax + 1); q += 32) mx = max(mx, PairBits<T>::abs_bits(fin[(size_t)c * NS + q]));
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, (U)__shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) cmx[c] = mx;
-  }
-  __syncthreads();
-  // Hermitian spectra of the 7 pairs (z = x + i y), the second row scaled
-  for (int idx = threadIdx.x; idx < 7 * N; idx += blockDim.x) {
-    int p = idx / N, n = idx - p * N;
-    const T *f0 = fin + (size_t)(2 * p) * NS;
-    const T *f1 = (2 * p + 1 < 13) ? fin + (size_t)(2 * p + 1) * NS : nullptr;
-    const T sy = f1 ? PairBits<T>::factor(cmx[2 * p], cmx[2 * p + 1], false) : (T)1;
-    T2 z = T2{0, 0};
-    if (n == 0) {
-      z = T2{f0[0], f1 ? f1[0] * sy : (T)0};
-    } else {
-      int m = (n <= mmax) ? n : ((N - n <= mmax) ? N - n : -1);
-      if (m > 0) {
-        T a0 = f0[2 * m], b0 = f0[2 * m + 1];
-        T a1 = f1 ? f1[2 * m] * sy : (T)0, b1 = f1 ? f1[2 * m + 1] * sy : (T)0;
-        T xr = (T)0.5 * a0, xi = (T)-0.5 * b0, yr = (T)0.5 * a1, yi = (T)-0.5 * b1;
-        z = (m == n) ? T2{xr - yi, xi + yr} : T2{xr + yi, -xi + yr};
-      }
-    }
-    A[idx] = z;
-  }
-  __syncthreads();
-  T2 *g = batch_fft<T, T2>(A, B, 7, pl, tw, +1);
-  T2 *h = (g == A) ? B : A;
-  const T cv = (T)pc.cv, cl = (T)pc.cl, ci = (T)pc.ci, ct = (T)pc.ct;
-  T iy[6];
-#pragma unroll
-  for (int p = 0; p < 6; p++) iy[p] = PairBits<T>::factor(cmx[2 * p], cmx[2 * p + 1], true);
-  U hm[12];
-#pragma unroll
-  for (int c = 0; c < 12; c++) hm[c] = 0;
-  for (int q = threadIdx.x; q < N; q += blockDim.x) {
-    T2 p0 = g[0 * N + q], p1 = g[1 * N + q], p2 = g[2 * N + q], p3 = g[3 * N + q];
-    T2 p4 = g[4 * N + q], p5 = g[5 * N + q], p6 = g[6 * N + q];
-    T ur = p0.x, ut = p0.y * iy[0], up = p1.x, wr = p1.y * iy[1], wt = p2.x, wp = p2.y * iy[2];
-    T br = p3.x, bt = p3.y * iy[3], bp = p4.x, jr = p4.y * iy[4], jt = p5.x, jp = p5.y * iy[5], tt = p6.x;
-    const T2 hv[6] = {T2{(wt * up - wp * ut) * cv, (wp * ur - wr * up) * cv},
-                      T2{(wr * ut - wt * ur) * cv, (jt * bp - jp * bt) * cl},
-                      T2{(jp * br - jr * bp) * cl, (jr * bt - jt * br) * cl},
-                      T2{(ut * bp - up * bt) * ci, (up * br - ur * bp) * ci},
-                      T2{(ur * bt - ut * br) * ci, ur * tt * ct},
-                      T2{ut * tt * ct, up * tt * ct}};
-#pragma unroll
-    for (int p = 0; p < 6; p++) {
-      h[p * N + q] = hv[p];
-      hm[2 * p] = max(hm[2 * p], PairBits<T>::abs_bits(hv[p].x));
-      hm[2 * p + 1] = max(hm[2 * p + 1], PairBits<T>::abs_bits(hv[p].y));
-    }
-  }
-  // row maxima of the 12 product rows: every lane of every warp takes part
-#pragma unroll
-  for (int c = 0; c < 12; c++) {
-    U v = hm[c];
-    for (int o = 16; o > 0; o >>= 1) v = max(v, (U)__shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) atomicMax(cmx + 13 + c, v);
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < 6 * N; idx += blockDim.x) {
-    const int p = idx / N;
-    h[idx].y *= PairBits<T>::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], false);
-  }
-  __syncthreads();
-  T2 *zf = batch_fft<T, T2>(h, g, 6, pl, tw, -1);
-  const T an = (T)(1.0 / (double)N);
-  for (int idx = threadIdx.x; idx < 6 * (L + 1); idx += blockDim.x) {
-    int p = idx / (L + 1), m = idx - p * (L + 1);
-    T *f0 = fout + (size_t)(2 * p) * NS, *f1 = fout + (size_t)(2 * p + 1) * NS;
-    const T2 *Z = zf + p * N;
-    const T ay = an * PairBits<T>::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], true);
-    if (m == 0) {
-      f0[0] = an * Z[0].x; f0[1] = 0;
-      f1[0] = ay * Z[0].y; f1[1] = 0;
-    } else {
-      T2 zk = Z[m % N], zn = Z[(N - m) % N];
-      T xr = (T)0.5 * (zk.x + zn.x), xi = (T)0.5 * (zk.y - zn.y);
-      T yr = (T)0.5 * (zk.y + zn.y), yi = (T)-0.5 * (zk.x - zn.x);
-      f0[2 * m] = (T)2 * an * xr; f0[2 * m + 1] = (T)-2 * an * xi;
-      f1[2 * m] = (T)2 * ay * yr; f1[2 * m + 1] = (T)-2 * ay * yi;
-    }
-  }
-}
-
-// Fourier rows -> grid (float64), for the standalone transform API
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_fft_to_grid(FFTPlan pl, int L, int NS, int nc, int nr, int nth, const T *four, double *grid,
-              const typename C2<T>::t *tw) {
-  using T2 = typename C2<T>::t;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int N = pl.n;
-  T2 *Z0 = reinterpret_cast<T2 *>(smraw), *Z1 = Z0 + N;
-  const size_t row = blockIdx.x;
-  const int th = (int)(row / nr), k = (int)(row % nr);
-  const T *fin = four + row * nc * NS;
-  for (int c = 0; c < nc; c += 2) {
-    load_pair<T, T2>(Z0, N, L, fin + (size_t)c * NS, (c + 1 < nc) ? fin + (size_t)(c + 1) * NS : nullptr);
-    T2 *z = block_fft<T, T2>(Z0, Z1, pl, tw, +1);
-    for (int q = threadIdx.x; q < N; q += blockDim.x) {
-      grid[(((size_t)c * nr + k) * nth + th) * N + q] = (double)z[q].x;
-      if (c + 1 < nc) grid[(((size_t)(c + 1) * nr + k) * nth + th) * N + q] = (double)z[q].y;
-    }
-    __syncthreads();
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_grid_to_fft(FFTPlan pl, int L, int NS, int nc, int nr, int nth, const double *grid, T *four,
-              const typename C2<T>::t *tw) {
-  using T2 = typename C2<T>::t;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int N = pl.n;
-  T2 *Z0 = reinterpret_cast<T2 *>(smraw), *Z1 = Z0 + N;
-  const size_t row = blockIdx.x;
-  const int th = (int)(row / nr), k = (int)(row % nr);
-  T *fout = four + row * nc * NS;
-  for (int c = 0; c < nc; c += 2) {
-    for (int q = threadIdx.x; q < N; q += blockDim.x) {
-      T x = (T)grid[(((size_t)c * nr + k) * nth + th) * N + q];
-      T y = (c + 1 < nc) ? (T)grid[(((size_t)(c + 1) * nr + k) * nth + th) * N + q] : (T)0;
-      Z0[q] = T2{x, y};
-    }
-    __syncthreads();
-    T2 *z = block_fft<T, T2>(Z0, Z1, pl, tw, -1);
-    store_pair<T, T2>(z, N, L, fout + (size_t)c * NS, (c + 1 < nc) ? fout + (size_t)(c + 1) * NS : nullptr);
-    __syncthreads();
-  }
-}
-
 // ---------------------------------------------------------------------------
-// Mixed-precision path: the same fused transform over the order-major
-// Fourier layout (MLayout).  Input 4 vectors (u, w, B, J) + 1 scalar (T),
+// The general float32 kernel over the order-major Fourier layout (MLayout).
+// Input 4 vectors (u, w, B, J) + 1 scalar (T),
 // output 4 vectors (w x u, J x B, u x B, u T).  At one (theta, k) the 26
 // input floats of an order m are one run of 10 (P block) and one of 16
 // (D block); threads take consecutive elements of a run, the values are
@@ -671,6 +478,27 @@ __host__ __device__ __forceinline__ void dftr(T2 (&v)[R]) {
     v[1] = cadd(e1, o1); v[5] = csub(e1, o1);
     v[2] = cadd(e2, o2); v[6] = csub(e2, o2);
     v[3] = cadd(e3, o3); v[7] = csub(e3, o3);
+  } else if constexpr (R == 9) {
+    // 3 x 3: n = 3 n1 + n2, k = k1 + 3 k2; W9^q = exp(SIGN 2 pi i q / 9)
+    constexpr T c1 = (T)0.76604444311897803520, s1 = (T)0.64278760968653932632;   // 40 degrees
+    constexpr T c2 = (T)0.17364817766693034885, s2 = (T)0.98480775301220805937;   // 80 degrees
+    constexpr T c4 = (T)-0.93969262078590838405, s4 = (T)0.34202014332566873304;  // 160 degrees
+    constexpr T sg = (SIGN < 0) ? (T)-1 : (T)1;
+    const T2 w1 = T2{c1, sg * s1}, w2 = T2{c2, sg * s2}, w4 = T2{c4, sg * s4};
+    T2 a[3][3];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; n2++) {
+      a[n2][0] = v[n2]; a[n2][1] = v[3 + n2]; a[n2][2] = v[6 + n2];
+      dftr<3, SIGN>(a[n2]);
+    }
+    a[1][1] = cmulf(a[1][1], w1); a[1][2] = cmulf(a[1][2], w2);
+    a[2][1] = cmulf(a[2][1], w2); a[2][2] = cmulf(a[2][2], w4);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; k1++) {
+      T2 b[3] = {a[0][k1], a[1][k1], a[2][k1]};
+      dftr<3, SIGN>(b);
+      v[k1] = b[0]; v[k1 + 3] = b[1]; v[k1 + 6] = b[2];
+    }
   } else {
     static_assert(R == 16, "radix");
     // 4 x 4: n = 4 n1 + n2, k = k1 + 4 k2
@@ -1116,9 +944,8 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
 
 // ---------------------------------------------------------------------------
 // The float64 four-step products kernel (the plain path's step): the data
-// flow of k_fft_products_4s on the float64 Fourier rows
-// four[(theta, k)][c][2 m + s] (a_m at 2 m, b_m at 2 m + 1), with the pair
-// scaling of k_fft_products (the second row of each pair, inputs and
+// flow of k_fft_products_4s on the float64 Fourier rows, with the pair
+// scaling of k_fft_products_g64 (the second row of each pair, inputs and
 // products, brought to the size of the first), so every row keeps float64
 // precision whatever the sizes of the fields.  One CTA per (theta, k), 384
 // threads, one CTA per SM (166 KB of shared memory at M = 256).
@@ -1137,8 +964,7 @@ struct F4Plan64 {
 
 template <int R1, int R2>
 __global__ void __launch_bounds__(f4_threads<R2>(), R2 == 16 ? 1 : R1 == 16 ? 2 : R2 == 8 ? 4 : 8)
-k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2, int NS,
-                    const double2 *__restrict__ tables, ProdCoef pc) {
+k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ tables, ProdCoef pc) {
   using P = F4Plan64<R1, R2>;
   using PB = PairBits<double>;
   using U = PB::U;
@@ -1150,17 +976,35 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
   double2 *TW3 = X + P::X;                             // [3][M]
   double2 *TWM = TW3 + 3 * M;                          // [R2][WP]
   U *cmx = reinterpret_cast<U *>(TWM + R2 * WP);      // [0, 13) input maxima, [13, 25) products
-  const size_t row = blockIdx.x;
-  const double *fin = four + row * 13 * (size_t)NS;
-  double *fout = four2 + row * 12 * (size_t)NS;
+  const int th = blockIdx.x / fin.nr, k = blockIdx.x % fin.nr;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = NT / 32;
   const int grp = tid / R2, lt = tid % R2;
-  for (int e = tid; e < P::NTW; e += NT) TW3[e] = tables[e];
   for (int e = tid; e < 14; e += NT) S2[e * MP2 + M] = double2{0.0, 0.0};
   for (int e = tid; e < M; e += NT) S2[13 * MP2 + e] = double2{0.0, 0.0};
-  for (int e = tid; e < 13 * M; e += NT) {
-    const int c = e / M, m = e - c * M;
-    S2[c * MP2 + m] = __ldg(reinterpret_cast<const double2 *>(fin + (size_t)c * NS) + m);
+  // input and tables by asynchronous 16-byte copies, as in k_fft_products_4s
+  auto cp16 = [](double2 *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+  };
+  for (int e = tid; e < P::NTW; e += NT) cp16(TW3 + e, tables + e);
+  {
+    const int j = lane & 15, hw = lane >> 4;
+    int c = 0;
+    const double *src = fin.P;
+    size_t mst = 0;
+    if (j < 5) {
+      c = (j < 4) ? 3 * j : 12;
+      src = fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + 2 * j;
+      mst = (size_t)fin.nth * fin.sP();
+    } else if (j < 13) {
+      const int jd = j - 5;
+      c = 3 * (jd >> 1) + 1 + (jd & 1);
+      src = fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + 2 * jd;
+      mst = (size_t)fin.nth * fin.sD();
+    }
+    if (j < 13)
+      for (int m = 2 * warp + hw; m < M; m += 2 * nwarp) cp16(S2 + c * MP2 + m, src + m * mst);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   }
   if (tid < 12) cmx[13 + tid] = 0;
   __syncthreads();
@@ -1330,54 +1174,301 @@ k_fft_products_4s64(const double *__restrict__ four, double *__restrict__ four2,
     }
   }
   __syncthreads();
-  for (int e = tid; e < 12 * M; e += NT) {
-    const int c = e / M, m = e - c * M;
-    reinterpret_cast<double2 *>(fout + (size_t)c * NS)[m] = S2[c * MP2 + m];
+  {
+    const int j = lane & 15, hw = lane >> 4;
+    int c = 0;
+    double *dst = fout.P;
+    size_t mst = 0;
+    if (j < 4) {
+      c = 3 * j;
+      dst = fout.P + (size_t)th * fout.sP() + (size_t)k * 8 + 2 * j;
+      mst = (size_t)fout.nth * fout.sP();
+    } else if (j < 12) {
+      const int jd = j - 4;
+      c = 3 * (jd >> 1) + 1 + (jd & 1);
+      dst = fout.D + (size_t)th * fout.sD() + (size_t)k * 16 + 2 * jd;
+      mst = (size_t)fout.nth * fout.sD();
+    }
+    if (j < 12)
+      for (int m = 2 * warp + hw; m < M; m += 2 * nwarp)
+        *reinterpret_cast<double2 *>(dst + m * mst) = S2[c * MP2 + m];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The general float64 products kernel, any N = 2^a 3^b (the grids that are not
+// nphi = 3 (L + 1) with L + 1 = 32 .. 256): Stockham passes of radix 16 and 9
+// while they divide, then 8, 4, 2 or 3, each butterfly a register DFT, the
+// index divisions by multiplication; rows in shared memory padded as in
+// k_fft_products_t.  Radix 4, 3 and 2 passes with run-time radices and
+// divisions took 1056 us at nphi = 256 / L85 / Nr65 (8320 rows).
+struct G64Stage {
+  int R, nb, Ns, tstride;   // radix, butterflies a row, product of the radices before, N / (Ns R)
+  FastDiv dnb, dNs;
+};
+struct G64Plan {
+  int n, np, nst;           // points, padded row length, stages
+  int psh;                  // index i lies at i + (i >> psh)
+  int mp;                   // pitch of a staging row of L + 1 orders
+  G64Stage st[12];
+  __device__ __forceinline__ int pad(int i) const { return i + (i >> psh); }
+};
+
+static size_t g64_bytes(int np) { return 14 * (size_t)np * sizeof(double2) + 32 * sizeof(double); }
+
+static G64Plan make_plan64(int n, int L) {
+  G64Plan p{};
+  p.n = n;
+  // the largest grids fit without the padding only, the smallest with an even
+  // staging pitch only
+  p.psh = g64_bytes(n + n / 16 + 1) <= 227 * 1024 ? 4 : 31;
+  p.np = p.psh == 4 ? n + n / 16 + 1 : n;
+  p.mp = 26 * (size_t)((L + 1) | 1) * sizeof(double) <= 7 * (size_t)p.np * sizeof(double2) ? (L + 1) | 1 : L + 1;
+  int m = n, Ns = 1;
+  auto add = [&](int R) {
+    p.st[p.nst++] = G64Stage{R, n / R, Ns, n / (Ns * R), FastDiv(n / R), FastDiv(Ns)};
+    Ns *= R;
+    m /= R;
+  };
+  while (m % 16 == 0) add(16);
+  for (int R : {8, 4, 2})
+    if (m % R == 0) add(R);
+  while (m % 9 == 0) add(9);
+  while (m % 3 == 0) add(3);
+  return p;
+}
+
+template <int R, int SIGN>
+__device__ __forceinline__ void g64_pass(const double2 *x, double2 *y, int nf, const G64Plan &pl, const G64Stage &st,
+                                         const double2 *__restrict__ tw) {
+  const int np = pl.np;
+  for (int idx = threadIdx.x; idx < nf * st.nb; idx += blockDim.x) {
+    const int f = st.dnb.div(idx), j = idx - f * st.nb, q = st.dNs.div(j), k = j - q * st.Ns;
+    const double2 *xf = x + f * np;
+    double2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      v[r] = xf[pl.pad(j + r * st.nb)];
+      if (r > 0 && k > 0) {
+        double2 w = __ldg(tw + r * k * st.tstride);
+        if (SIGN > 0) w.y = -w.y;
+        v[r] = cmulf(v[r], w);
+      }
+    }
+    dftr<R, SIGN>(v);
+    double2 *yf = y + f * np;
+    const int d = q * st.Ns * R + k;
+#pragma unroll
+    for (int r = 0; r < R; r++) yf[pl.pad(d + r * st.Ns)] = v[r];
+  }
+  __syncthreads();
+}
+
+template <int SIGN>
+__device__ __forceinline__ double2 *g64_fft(double2 *x, double2 *y, int nf, const G64Plan &pl,
+                                            const double2 *__restrict__ tw) {
+  for (int s = 0; s < pl.nst; s++) {
+    const G64Stage &st = pl.st[s];
+    switch (st.R) {
+      case 16: g64_pass<16, SIGN>(x, y, nf, pl, st, tw); break;
+      case 9: g64_pass<9, SIGN>(x, y, nf, pl, st, tw); break;
+      case 8: g64_pass<8, SIGN>(x, y, nf, pl, st, tw); break;
+      case 4: g64_pass<4, SIGN>(x, y, nf, pl, st, tw); break;
+      case 3: g64_pass<3, SIGN>(x, y, nf, pl, st, tw); break;
+      default: g64_pass<2, SIGN>(x, y, nf, pl, st, tw); break;
+    }
+    double2 *t = x; x = y; y = t;
+  }
+  return x;
+}
+
+__global__ void __launch_bounds__(512)
+k_fft_products_g64(const __grid_constant__ G64Plan pl, int L, MLayout64 fin, MLayout64 fout,
+                   const double2 *__restrict__ tw, ProdCoef pc) {
+  using PB = PairBits<double>;
+  using U = PB::U;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int N = pl.n, NP = pl.np, MP = pl.mp;
+  double2 *A = reinterpret_cast<double2 *>(smraw);   // 7 rows
+  double2 *B = A + 7 * NP;                            // 7 rows; first the input, last the output staging
+  U *cmx = reinterpret_cast<U *>(B + 7 * NP);         // [0, 13) input maxima, [13, 25) products
+  double *S = reinterpret_cast<double *>(B);          // [c * 2 + s][MP]
+  const int th = blockIdx.x / fin.nr, k = blockIdx.x % fin.nr;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  if (tid < 12) cmx[13 + tid] = 0;
+  // input: one warp per order, lane j < 26 element j of the 10 + 16 run
+  {
+    int cs = 0;
+    if (lane < 26) { int c, sg; m_comp_of_in(lane, c, sg); cs = c * 2 + sg; }
+    const double *src = (lane < 10) ? fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + lane
+                                    : fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + (lane - 10);
+    const size_t mst = (size_t)fin.nth * ((lane < 10) ? fin.sP() : fin.sD());
+    if (lane < 26) {
+      int m = warp;
+      for (; m + 3 * nwarp <= L; m += 4 * nwarp) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = __ldg(src + (size_t)(m + u * nwarp) * mst);
+#pragma unroll
+        for (int u = 0; u < 4; u++) S[cs * MP + m + u * nwarp] = v[u];
+      }
+      for (; m <= L; m += nwarp) S[cs * MP + m] = __ldg(src + (size_t)m * mst);
+    }
+  }
+  __syncthreads();
+  // pair scaling (pair_exp): the largest coefficient of each component
+  for (int c = warp; c < 13; c += nwarp) {
+    U mx = 0;
+    for (int m = lane; m <= L; m += 32) {
+      mx = max(mx, PB::abs_bits(S[(2 * c) * MP + m]));
+      if (m > 0) mx = max(mx, PB::abs_bits(S[(2 * c + 1) * MP + m]));
+    }
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, (U)__shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) cmx[c] = mx;
+  }
+  __syncthreads();
+  // Hermitian rows z = x + i y of the 7 pairs, the second row scaled
+  const int mmax = min(L, (N + 1) / 2 - 1);
+  for (int p = 0; p < 7; p++) {
+    const bool has1 = p < 6;
+    const double sy = has1 ? PB::factor(cmx[2 * p], cmx[2 * p + 1], false) : 0.0;
+    const double *a0 = S + (size_t)(4 * p) * MP, *b0 = a0 + MP, *a1 = has1 ? b0 + MP : a0, *b1 = has1 ? a1 + MP : a0;
+    double2 *Z = A + p * NP;
+    for (int m = tid; m <= mmax; m += blockDim.x) {
+      if (m == 0) {
+        Z[0] = double2{a0[0], a1[0] * sy};
+      } else {
+        const double xr = 0.5 * a0[m], xi = -0.5 * b0[m], yr = 0.5 * (a1[m] * sy), yi = -0.5 * (b1[m] * sy);
+        Z[pl.pad(m)] = double2{xr - yi, xi + yr};
+        Z[pl.pad(N - m)] = double2{xr + yi, -xi + yr};
+      }
+    }
+    for (int n = mmax + 1 + tid; n < N - mmax; n += blockDim.x) Z[pl.pad(n)] = double2{0.0, 0.0};
+  }
+  __syncthreads();
+  double2 *g = g64_fft<+1>(A, B, 7, pl, tw);
+  double2 *h = (g == A) ? B : A;
+  {
+    double iy[6];
+#pragma unroll
+    for (int p = 0; p < 6; p++) iy[p] = PB::factor(cmx[2 * p], cmx[2 * p + 1], true);
+    U hm[12];
+#pragma unroll
+    for (int c = 0; c < 12; c++) hm[c] = 0;
+    for (int qq = tid; qq < N; qq += blockDim.x) {
+      const int q = pl.pad(qq);
+      const double2 p0 = g[0 * NP + q], p1 = g[1 * NP + q], p2 = g[2 * NP + q], p3 = g[3 * NP + q];
+      const double2 p4 = g[4 * NP + q], p5 = g[5 * NP + q], p6 = g[6 * NP + q];
+      const double ur = p0.x, ut = p0.y * iy[0], up = p1.x, wr = p1.y * iy[1], wt = p2.x, wp = p2.y * iy[2];
+      const double br = p3.x, bt = p3.y * iy[3], bp = p4.x, jr = p4.y * iy[4], jt = p5.x, jp = p5.y * iy[5];
+      const double tt = p6.x, cv = pc.cv, cl = pc.cl, ci = pc.ci, ct = pc.ct;
+      const double2 hv[6] = {double2{(wt * up - wp * ut) * cv, (wp * ur - wr * up) * cv},
+                             double2{(wr * ut - wt * ur) * cv, (jt * bp - jp * bt) * cl},
+                             double2{(jp * br - jr * bp) * cl, (jr * bt - jt * br) * cl},
+                             double2{(ut * bp - up * bt) * ci, (up * br - ur * bp) * ci},
+                             double2{(ur * bt - ut * br) * ci, ur * tt * ct},
+                             double2{ut * tt * ct, up * tt * ct}};
+#pragma unroll
+      for (int p = 0; p < 6; p++) {
+        h[p * NP + q] = hv[p];
+        hm[2 * p] = max(hm[2 * p], PB::abs_bits(hv[p].x));
+        hm[2 * p + 1] = max(hm[2 * p + 1], PB::abs_bits(hv[p].y));
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 12; c++) {
+      U v = hm[c];
+      for (int o = 16; o > 0; o >>= 1) v = max(v, (U)__shfl_xor_sync(0xffffffffu, v, o));
+      if (lane == 0) atomicMax(cmx + 13 + c, v);
+    }
+  }
+  __syncthreads();
+  for (int p = 0; p < 6; p++) {
+    const double f = PB::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], false);
+    for (int q = tid; q < N; q += blockDim.x) h[p * NP + pl.pad(q)].y *= f;
+  }
+  __syncthreads();
+  const double2 *zf = g64_fft<-1>(h, g, 6, pl, tw);
+  double *O = reinterpret_cast<double *>((zf == A) ? B : A);   // [c * 2 + s][MP]
+  const double an = 1.0 / (double)N;
+  for (int p = 0; p < 6; p++) {
+    const double2 *Z = zf + p * NP;
+    double *o0 = O + (size_t)(4 * p) * MP, *o1 = o0 + 2 * MP;
+    const double ay = an * PB::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], true);
+    for (int m = tid; m <= L; m += blockDim.x) {
+      if (m == 0) {
+        o0[0] = an * Z[0].x; o0[MP] = 0.0; o1[0] = ay * Z[0].y; o1[MP] = 0.0;
+      } else {
+        const double2 zk = Z[pl.pad(m % N)], zn = Z[pl.pad((N - m) % N)];
+        o0[m] = an * (zk.x + zn.x); o0[MP + m] = -an * (zk.y - zn.y);
+        o1[m] = ay * (zk.y + zn.y); o1[MP + m] = ay * (zk.x - zn.x);
+      }
+    }
+  }
+  __syncthreads();
+  {
+    int cs = 0;
+    if (lane < 24) { int c, sg; m_comp_of_out(lane, c, sg); cs = c * 2 + sg; }
+    double *dst = (lane < 8) ? fout.P + (size_t)th * fout.sP() + (size_t)k * 8 + lane
+                             : fout.D + (size_t)th * fout.sD() + (size_t)k * 16 + (lane - 8);
+    const size_t mst = (size_t)fout.nth * ((lane < 8) ? fout.sP() : fout.sD());
+    if (lane < 24)
+      for (int m = warp; m <= L; m += nwarp) dst[(size_t)m * mst] = O[cs * MP + m];
   }
 }
 
 // order-major Fourier rows -> grid (float64), for the standalone transform API
+template <typename U>
+__device__ __forceinline__ U warp_max(U v) {
+  for (int o = 16; o > 0; o >>= 1) v = max(v, (U)__shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+template <typename T>
 __global__ void __launch_bounds__(256)
-k_fft_to_grid_m(FFTPlan pl, int L, MLayout fin, double *grid, const float2 *tw) {
+k_fft_to_grid_m(FFTPlan pl, int L, MLayoutT<T> fin, double *grid, const typename C2<T>::t *tw) {
+  using T2 = typename C2<T>::t;
+  using PB = PairBits<T>;
+  using U = typename PB::U;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int N = pl.n, nc = 3 * fin.nvec + fin.nscal, nr = fin.nr, nth = fin.nth;
-  float2 *Z0 = reinterpret_cast<float2 *>(smraw), *Z1 = Z0 + N;
+  T2 *Z0 = reinterpret_cast<T2 *>(smraw), *Z1 = Z0 + N;
   const int th = blockIdx.x / nr, k = blockIdx.x % nr;
   const int mmax = min(L, (N + 1) / 2 - 1);
-  __shared__ unsigned pmx[2];
+  __shared__ U pmx[2];
   for (int c = 0; c < nc; c += 2) {
     const bool has1 = c + 1 < nc;
-    if (threadIdx.x < 2) pmx[threadIdx.x] = 0u;
-    for (int q = threadIdx.x; q < N; q += blockDim.x) Z0[q] = float2{0, 0};
+    if (threadIdx.x < 2) pmx[threadIdx.x] = 0;
+    for (int q = threadIdx.x; q < N; q += blockDim.x) Z0[q] = T2{0, 0};
     __syncthreads();
     // pair scaling (pair_exp): the second row brought to the size of the first
     {
-      unsigned mx = 0u, my = 0u;
+      U mx = 0, my = 0;
       for (int m = threadIdx.x; m <= mmax; m += blockDim.x) {
-        mx = max(mx, max(abs_bits(*fin.at(m, th, k, c, 0)), abs_bits(*fin.at(m, th, k, c, 1))));
-        if (has1) my = max(my, max(abs_bits(*fin.at(m, th, k, c + 1, 0)), abs_bits(*fin.at(m, th, k, c + 1, 1))));
+        mx = max(mx, max(PB::abs_bits(*fin.at(m, th, k, c, 0)), PB::abs_bits(*fin.at(m, th, k, c, 1))));
+        if (has1)
+          my = max(my, max(PB::abs_bits(*fin.at(m, th, k, c + 1, 0)), PB::abs_bits(*fin.at(m, th, k, c + 1, 1))));
       }
-      mx = __reduce_max_sync(0xffffffffu, mx);
-      my = __reduce_max_sync(0xffffffffu, my);
+      mx = warp_max(mx);
+      my = warp_max(my);
       if ((threadIdx.x & 31) == 0) { atomicMax(pmx, mx); atomicMax(pmx + 1, my); }
     }
     __syncthreads();
-    const int ep = pair_exp(pmx[0], pmx[1]);
-    const float sy = pow2i(ep), iy = pow2i(-ep);
+    const T sy = PB::factor(pmx[0], pmx[1], false), iy = PB::factor(pmx[0], pmx[1], true);
     for (int m = threadIdx.x; m <= mmax; m += blockDim.x) {
-      const float a0 = *fin.at(m, th, k, c, 0), b0 = (m > 0) ? *fin.at(m, th, k, c, 1) : 0.0f;
-      const float a1 = has1 ? *fin.at(m, th, k, c + 1, 0) * sy : 0.0f;
-      const float b1 = (has1 && m > 0) ? *fin.at(m, th, k, c + 1, 1) * sy : 0.0f;
+      const T a0 = *fin.at(m, th, k, c, 0), b0 = (m > 0) ? *fin.at(m, th, k, c, 1) : (T)0;
+      const T a1 = has1 ? *fin.at(m, th, k, c + 1, 0) * sy : (T)0;
+      const T b1 = (has1 && m > 0) ? *fin.at(m, th, k, c + 1, 1) * sy : (T)0;
       if (m == 0) {
-        Z0[0] = float2{a0, a1};
+        Z0[0] = T2{a0, a1};
       } else {
-        const float xr = 0.5f * a0, xi = -0.5f * b0, yr = 0.5f * a1, yi = -0.5f * b1;
-        Z0[m] = float2{xr - yi, xi + yr};
-        Z0[N - m] = float2{xr + yi, -xi + yr};
+        const T xr = (T)0.5 * a0, xi = (T)-0.5 * b0, yr = (T)0.5 * a1, yi = (T)-0.5 * b1;
+        Z0[m] = T2{xr - yi, xi + yr};
+        Z0[N - m] = T2{xr + yi, -xi + yr};
       }
     }
     __syncthreads();
-    float2 *z = block_fft<float, float2>(Z0, Z1, pl, tw, +1);
+    T2 *z = block_fft<T, T2>(Z0, Z1, pl, tw, +1);
     for (int q = threadIdx.x; q < N; q += blockDim.x) {
       grid[(((size_t)c * nr + k) * nth + th) * N + q] = (double)z[q].x;
       if (has1) grid[(((size_t)(c + 1) * nr + k) * nth + th) * N + q] = (double)(z[q].y * iy);
@@ -1387,48 +1478,51 @@ k_fft_to_grid_m(FFTPlan pl, int L, MLayout fin, double *grid, const float2 *tw) 
 }
 
 // grid (float64) -> order-major Fourier rows
+template <typename T>
 __global__ void __launch_bounds__(256)
-k_grid_to_fft_m(FFTPlan pl, int L, const double *grid, MLayout fout, const float2 *tw) {
+k_grid_to_fft_m(FFTPlan pl, int L, const double *grid, MLayoutT<T> fout, const typename C2<T>::t *tw) {
+  using T2 = typename C2<T>::t;
+  using PB = PairBits<T>;
+  using U = typename PB::U;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int N = pl.n, nc = 3 * fout.nvec + fout.nscal, nr = fout.nr, nth = fout.nth;
-  float2 *Z0 = reinterpret_cast<float2 *>(smraw), *Z1 = Z0 + N;
+  T2 *Z0 = reinterpret_cast<T2 *>(smraw), *Z1 = Z0 + N;
   const int th = blockIdx.x / nr, k = blockIdx.x % nr;
-  const float an = (float)(1.0 / (double)N);
-  __shared__ unsigned pmx[2];
+  const T an = (T)(1.0 / (double)N);
+  __shared__ U pmx[2];
   for (int c = 0; c < nc; c += 2) {
     const bool has1 = c + 1 < nc;
-    if (threadIdx.x < 2) pmx[threadIdx.x] = 0u;
+    if (threadIdx.x < 2) pmx[threadIdx.x] = 0;
     __syncthreads();
-    unsigned mx = 0u, my = 0u;
+    U mx = 0, my = 0;
     for (int q = threadIdx.x; q < N; q += blockDim.x) {
-      const float x = (float)grid[(((size_t)c * nr + k) * nth + th) * N + q];
-      const float y = has1 ? (float)grid[(((size_t)(c + 1) * nr + k) * nth + th) * N + q] : 0.0f;
-      Z0[q] = float2{x, y};
-      mx = max(mx, abs_bits(x));
-      my = max(my, abs_bits(y));
+      const T x = (T)grid[(((size_t)c * nr + k) * nth + th) * N + q];
+      const T y = has1 ? (T)grid[(((size_t)(c + 1) * nr + k) * nth + th) * N + q] : (T)0;
+      Z0[q] = T2{x, y};
+      mx = max(mx, PB::abs_bits(x));
+      my = max(my, PB::abs_bits(y));
     }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    my = __reduce_max_sync(0xffffffffu, my);
+    mx = warp_max(mx);
+    my = warp_max(my);
     if ((threadIdx.x & 31) == 0) { atomicMax(pmx, mx); atomicMax(pmx + 1, my); }
     __syncthreads();
     // pair scaling (pair_exp): the second row brought to the size of the first
-    const int ep = pair_exp(pmx[0], pmx[1]);
-    if (ep != 0) {
-      const float sy = pow2i(ep);
+    const T sy = PB::factor(pmx[0], pmx[1], false);
+    if (sy != (T)1) {
       for (int q = threadIdx.x; q < N; q += blockDim.x) Z0[q].y *= sy;
       __syncthreads();
     }
-    const float ay = an * pow2i(-ep);
-    const float2 *z = block_fft<float, float2>(Z0, Z1, pl, tw, -1);
+    const T ay = an * PB::factor(pmx[0], pmx[1], true);
+    const T2 *z = block_fft<T, T2>(Z0, Z1, pl, tw, -1);
     for (int m = threadIdx.x; m <= L; m += blockDim.x) {
-      float a0, b0, a1, b1;
+      T a0, b0, a1, b1;
       if (m == 0) {
-        a0 = an * z[0].x; b0 = 0.0f; a1 = ay * z[0].y; b1 = 0.0f;
+        a0 = an * z[0].x; b0 = (T)0; a1 = ay * z[0].y; b1 = (T)0;
       } else {
-        const float2 zk = z[m % N], zn = z[(N - m) % N];
-        const float xr = 0.5f * (zk.x + zn.x), xi = 0.5f * (zk.y - zn.y);
-        const float yr = 0.5f * (zk.y + zn.y), yi = -0.5f * (zk.x - zn.x);
-        a0 = 2.0f * an * xr; b0 = -2.0f * an * xi; a1 = 2.0f * ay * yr; b1 = -2.0f * ay * yi;
+        const T2 zk = z[m % N], zn = z[(N - m) % N];
+        const T xr = (T)0.5 * (zk.x + zn.x), xi = (T)0.5 * (zk.y - zn.y);
+        const T yr = (T)0.5 * (zk.y + zn.y), yi = (T)-0.5 * (zk.x - zn.x);
+        a0 = (T)2 * an * xr; b0 = (T)-2 * an * xi; a1 = (T)2 * ay * yr; b1 = (T)-2 * ay * yi;
       }
       *fout.at(m, th, k, c, 0) = a0;
       *fout.at(m, th, k, c, 1) = b0;
@@ -1539,13 +1633,11 @@ int fft_setup(Ctx &c) {
   k_twiddles<<<cdiv(c.nph, 256), 256, 0, c.stream>>>(c.nph, (double2 *)c.d_tw_fft,
                                                      (float2 *)c.d_tw_fft32);
   CB2_CUDA(cudaGetLastError());
-  size_t big = 14 * (size_t)c.nph * sizeof(double2) + 32 * sizeof(double);
-  if (big > 227 * 1024) {
+  if (14 * (size_t)c.nph * sizeof(double2) + 32 * sizeof(double) > 227 * 1024) {
     set_error("ngrid_zonal_ctl too large for the fused FFT kernel");
     return CB2_ERR_ARG;
   }
-  CB2_CUDA(raise_smem_limit(k_fft_products<double>, (int)big));
-  CB2_CUDA(raise_smem_limit(k_fft_products<float>, (int)big));
+  if (c.prec == CB2_PREC_FP64) CB2_CUDA(raise_smem_limit(k_fft_products_g64, g64_bytes(make_plan64(c.nph, c.L).np)));
   CB2_CUDA(raise_smem_limit(k_fft_products_m, (int)(14 * (size_t)c.nph * sizeof(float2) + 32 * sizeof(float))));
   {
     int rc = 0;
@@ -1590,50 +1682,40 @@ static const typename C2<T>::t *twid(Ctx &c) {
 }
 
 template <int R1, int R2>
-static void launch_fft_4s64(Ctx &c, const double *four, double *four2, const ProdCoef &pc) {
+static void launch_fft_4s64(Ctx &c, const MLayout64 &in, const MLayout64 &out, const ProdCoef &pc) {
   k_fft_products_4s64<R1, R2><<<(unsigned)(c.nth * c.nr), f4_threads<R2>(), F4Plan64<R1, R2>::smem(), c.stream>>>(
-      four, four2, c.NS, (const double2 *)c.d_twf4_64, pc);
+      in, out, (const double2 *)c.d_twf4_64, pc);
 }
 
-template <typename T>
-void fft_products(Ctx &c, const T *four, T *four2) {
-  using T2 = typename C2<T>::t;
-  if constexpr (sizeof(T) == 8) {
-    // tuning value F4_THREADS selects the four-step kernel where it applies
-    if (c.d_twf4_64 && c.tune[TUNE_FFT_THREADS] == F4_THREADS) {
-      ProdCoef pc{c.p.coef_velo, c.p.coef_lor, c.p.coef_induct, c.p.coef_temp};
-      switch (c.nph) {
-        case 768: launch_fft_4s64<16, 16>(c, four, four2, pc); return;
-        case 384: launch_fft_4s64<16, 8>(c, four, four2, pc); return;
-        case 192: launch_fft_4s64<8, 8>(c, four, four2, pc); return;
-        case 96: launch_fft_4s64<8, 4>(c, four, four2, pc); return;
-        default: break;
-      }
+void fft_products64(Ctx &c, const MLayout64 &in, const MLayout64 &out) {
+  const ProdCoef pc{c.p.coef_velo, c.p.coef_lor, c.p.coef_induct, c.p.coef_temp};
+  // tuning value F4_THREADS selects the four-step kernel where it applies
+  if (c.d_twf4_64 && c.tune[TUNE_FFT_THREADS] == F4_THREADS) {
+    switch (c.nph) {
+      case 768: launch_fft_4s64<16, 16>(c, in, out, pc); return;
+      case 384: launch_fft_4s64<16, 8>(c, in, out, pc); return;
+      case 192: launch_fft_4s64<8, 8>(c, in, out, pc); return;
+      case 96: launch_fft_4s64<8, 4>(c, in, out, pc); return;
+      default: break;
     }
   }
-  FFTPlan p = make_plan(c.nph);
-  size_t sm = 14 * (size_t)c.nph * sizeof(T2) + 32 * sizeof(double);
-  ProdCoef pc{c.p.coef_velo, c.p.coef_lor, c.p.coef_induct, c.p.coef_temp};
-  k_fft_products<T><<<(unsigned)(c.nth * c.nr), 512, sm, c.stream>>>(p, c.L, c.NS, four, four2,
-                                                                     twid<T>(c), pc);
+  // about a thread per radix-16 butterfly of the seven rows
+  const int threads = std::min(512, std::max(96, 32 * cdiv(7 * c.nph, 16 * 32)));
+  const G64Plan pl = make_plan64(c.nph, c.L);
+  k_fft_products_g64<<<(unsigned)(c.nth * c.nr), threads, g64_bytes(pl.np), c.stream>>>(
+      pl, c.L, in, out, (const double2 *)c.d_tw_fft, pc);
 }
 
 template <typename T>
-void fft_backward_grid(Ctx &c, int ncomp, const T *four, double *grid) {
-  using T2 = typename C2<T>::t;
-  FFTPlan p = make_plan(c.nph);
-  size_t sm = 2 * (size_t)c.nph * sizeof(T2);
-  k_fft_to_grid<T><<<(unsigned)(c.nth * c.nr), 256, sm, c.stream>>>(p, c.L, c.NS, ncomp, c.nr, c.nth,
-                                                                    four, grid, twid<T>(c));
+void fft_backward_grid(Ctx &c, const MLayoutT<T> &in, double *grid) {
+  const size_t sm = 2 * (size_t)c.nph * sizeof(typename C2<T>::t);
+  k_fft_to_grid_m<T><<<(unsigned)(c.nth * c.nr), 256, sm, c.stream>>>(make_plan(c.nph), c.L, in, grid, twid<T>(c));
 }
 
 template <typename T>
-void fft_forward_grid(Ctx &c, int ncomp, const double *grid, T *four) {
-  using T2 = typename C2<T>::t;
-  FFTPlan p = make_plan(c.nph);
-  size_t sm = 2 * (size_t)c.nph * sizeof(T2);
-  k_grid_to_fft<T><<<(unsigned)(c.nth * c.nr), 256, sm, c.stream>>>(p, c.L, c.NS, ncomp, c.nr, c.nth,
-                                                                    grid, four, twid<T>(c));
+void fft_forward_grid(Ctx &c, const double *grid, const MLayoutT<T> &out) {
+  const size_t sm = 2 * (size_t)c.nph * sizeof(typename C2<T>::t);
+  k_grid_to_fft_m<T><<<(unsigned)(c.nth * c.nr), 256, sm, c.stream>>>(make_plan(c.nph), c.L, grid, out, twid<T>(c));
 }
 
 template <int N>
@@ -1678,23 +1760,9 @@ bool fft_products_m(Ctx &c, const MLayout &in, const MLayout &out, float *pmax) 
   return false;
 }
 
-void fft_backward_grid_m(Ctx &c, const MLayout &in, double *grid) {
-  FFTPlan p = make_plan(c.nph);
-  size_t sm = 2 * (size_t)c.nph * sizeof(float2);
-  k_fft_to_grid_m<<<(unsigned)(c.nth * c.nr), 256, sm, c.stream>>>(p, c.L, in, grid, (const float2 *)c.d_tw_fft32);
-}
-
-void fft_forward_grid_m(Ctx &c, const double *grid, const MLayout &out) {
-  FFTPlan p = make_plan(c.nph);
-  size_t sm = 2 * (size_t)c.nph * sizeof(float2);
-  k_grid_to_fft_m<<<(unsigned)(c.nth * c.nr), 256, sm, c.stream>>>(p, c.L, grid, out, (const float2 *)c.d_tw_fft32);
-}
-
-template void fft_products<double>(Ctx &, const double *, double *);
-template void fft_products<float>(Ctx &, const float *, float *);
-template void fft_backward_grid<double>(Ctx &, int, const double *, double *);
-template void fft_backward_grid<float>(Ctx &, int, const float *, double *);
-template void fft_forward_grid<double>(Ctx &, int, const double *, double *);
-template void fft_forward_grid<float>(Ctx &, int, const double *, float *);
+template void fft_backward_grid<double>(Ctx &, const MLayout64 &, double *);
+template void fft_backward_grid<float>(Ctx &, const MLayout &, double *);
+template void fft_forward_grid<double>(Ctx &, const double *, const MLayout64 &);
+template void fft_forward_grid<float>(Ctx &, const double *, const MLayout &);
 
 }  // namespace cb2

@@ -5,13 +5,14 @@
 //                   m = 0..L the block of l = m..L of order +m, then (m>0)
 //                   the block of l = m..L of order -m.  All rj operators
 //                   are elementwise in jj and 3-point stencils in k.
-//   Fourier data    F[theta][k][c][s] with s = 2m (cos, order +m) and
-//                   s = 2m+1 (sin, order -m), NS = 2(L+1) slots per row:
-//                   one (theta, k) row of all components is contiguous for
-//                   the fused FFT + product kernel.
+//   Fourier data    order-major rows [m][theta][(k, element)] of either
+//                   precision (MLayoutT): a Legendre tile of one order is a
+//                   dense box, and the FFT kernels, which work per (theta, k),
+//                   read and write runs of 10 and 16 (8 and 16) values per
+//                   order.
 //   Legendre tables per order m:  P_lt[m][l-m][i], i over the nh = nth/2
 //                   Gauss nodes nearest the south pole (the other half
-//                   follows from the parity of P_l^m), and P_tl[m][i][l-m].
+//                   follows from the parity of P_l^m).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -77,7 +78,7 @@ struct Ctx {
   double *d_reft0 = nullptr, *d_reft1 = nullptr, *d_om = nullptr;
   double *d_colat = nullptr, *d_wgt = nullptr, *d_asin = nullptr;
   size_t *d_poff = nullptr;
-  double *d_Plt = nullptr, *d_dPlt = nullptr, *d_Ptl = nullptr, *d_dPtl = nullptr;
+  double *d_Plt = nullptr, *d_dPlt = nullptr;
   int *d_jgi1 = nullptr, *d_jgi2 = nullptr, *d_jei1 = nullptr;
   double *d_sw = nullptr, *d_tw = nullptr;       // [6][jmax], [8][jmax]
   double *d_lu_vp = nullptr, *d_lu_vt = nullptr, *d_lu_bs = nullptr, *d_lu_bt = nullptr, *d_lu_t = nullptr;
@@ -108,8 +109,8 @@ struct Ctx {
   void *d_twf4_64 = nullptr;             // the same in float64 (float64 four-step kernel)
   // state
   double *d_f = nullptr;                 // NSLOT * nr * jmax
-  void *d_four = nullptr;                // F: nth*nr*13*NS (double or float)
-  void *d_four2 = nullptr;               // G: nth*nr*12*NS
+  void *d_four = nullptr;                // Fourier rows of up to 13 components (double or float)
+  void *d_four2 = nullptr;               // of the 12 product components
   double *d_ene = nullptr;               // energy partial sums
   double *h_stage = nullptr;             // pinned staging buffer
   size_t h_stage_bytes = 0;
@@ -175,17 +176,61 @@ inline cudaError_t raise_smem_limit(K *kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Fourier coefficients, order-major so that one Legendre GEMM row is one
+// contiguous element; T = float on the mixed path, double on the plain one.  For nvec vectors + nscal
+// scalars, at each (m, theta):
+//   P block: nr * 2 (nvec + nscal) values ordered (k, field, s): the r
+//            component of each vector, then each scalar;
+//   D block: nr * 4 nvec values ordered (k, vector, {theta s=0, theta s=1,
+//            phi s=0, phi s=1});
+// s = 0 is the cos (order +m) coefficient, s = 1 the sin (order -m) one.
+// P[m][theta][...] sits at `P`, D[m][theta][...] at `D`.
+template <typename T>
+struct MLayoutT {
+  static constexpr size_t kPad = 16 / sizeof(T);
+  T *P = nullptr, *D = nullptr;
+  int nvec = 0, nscal = 0, nr = 0, nth = 0;
+  __host__ __device__ int rpP() const { return 2 * (nvec + nscal); }
+  __host__ __device__ int rpD() const { return 4 * nvec; }
+  // per-(m, theta) block strides, rounded up to 16 bytes so TMA boxes and
+  // 16-byte copies can start on any block
+  __host__ __device__ size_t sP() const { return (((size_t)nr * rpP() + kPad - 1) / kPad) * kPad; }
+  __host__ __device__ size_t sD() const { return (((size_t)nr * rpD() + kPad - 1) / kPad) * kPad; }
+  // element of component c (vector v: 3v r, 3v+1 theta, 3v+2 phi; scalars
+  // after the vectors) at (m, theta, k), order sign s
+  __host__ __device__ T *at(int m, int th, int k, int c, int s) const {
+    if (c < 3 * nvec) {
+      const int v = c / 3, cc = c - 3 * v;
+      if (cc == 0) return P + ((size_t)m * nth + th) * sP() + (size_t)k * rpP() + 2 * v + s;
+      return D + ((size_t)m * nth + th) * sD() + (size_t)k * rpD() + 4 * v + 2 * (cc - 1) + s;
+    }
+    return P + ((size_t)m * nth + th) * sP() + (size_t)k * rpP() + 2 * (nvec + (c - 3 * nvec)) + s;
+  }
+};
+using MLayout = MLayoutT<float>;
+using MLayout64 = MLayoutT<double>;
+
+// e / n for 0 <= e < 2^16 and 1 <= n <= 2^15: (e * ceil(2^32 / n)) >> 32
+struct FastDiv {
+  unsigned n = 1, mul = 0;
+  FastDiv() = default;
+  explicit FastDiv(int d) : n((unsigned)d), mul((unsigned)((0x100000000ull + d - 1) / d)) {}
+  __device__ __forceinline__ int div(int e) const { return n == 1 ? e : (int)__umulhi((unsigned)e, mul); }
+};
+
 // set-up (cb2_tables.cu)
 int setup_tables(Ctx &c);
 void free_tables(Ctx &c);
 // Legendre fp64 (cb2_legendre_f64.cu)
-void leg_bwd_f64(Ctx &c, int nvec, int nscal, const int *slots, double *four);
-void leg_fwd_f64(Ctx &c, int nvec, int nscal, const double *four, const int *slots);
+MLayout64 mlayout64(const Ctx &c, void *buf, int nvec, int nscal);
+// slots: first rj slot of each vector, then of each scalar (nvec + nscal <= 13)
+void leg_bwd_f64(Ctx &c, const int *slots, const MLayout64 &out);
+void leg_fwd_f64(Ctx &c, const MLayout64 &in, const int *slots);
 // FFT and grid products (cb2_fft.cu)
 int fft_setup(Ctx &c);
-template <typename T> void fft_products(Ctx &c, const T *four, T *four2);
-template <typename T> void fft_backward_grid(Ctx &c, int ncomp, const T *four, double *grid);
-template <typename T> void fft_forward_grid(Ctx &c, int ncomp, const double *grid, T *four);
+void fft_products64(Ctx &c, const MLayout64 &in, const MLayout64 &out);
+template <typename T> void fft_backward_grid(Ctx &c, const MLayoutT<T> &in, double *grid);
+template <typename T> void fft_forward_grid(Ctx &c, const double *grid, const MLayoutT<T> &out);
 // rj operators and solves (cb2_rj.cu)
 void rj_explicit(Ctx &c, bool euler);
 void rj_implicit(Ctx &c);
@@ -206,35 +251,6 @@ void cn_free(Ctx &c);
 // the Crank-Nicolson stage as the tuning selects it: cn_step, or
 // rj_explicit + rj_implicit
 void cn_stage(Ctx &c, bool euler);
-// Fourier coefficients of the mixed-precision path, order-major so that one
-// Legendre GEMM row is one contiguous element.  For nvec vectors + nscal
-// scalars, at each (m, theta):
-//   P block: nr * 2 (nvec + nscal) floats ordered (k, field, s): the r
-//            component of each vector, then each scalar;
-//   D block: nr * 4 nvec floats ordered (k, vector, {theta s=0, theta s=1,
-//            phi s=0, phi s=1});
-// s = 0 is the cos (order +m) coefficient, s = 1 the sin (order -m) one.
-// P[m][theta][...] sits at `P`, D[m][theta][...] at `D`.
-struct MLayout {
-  float *P = nullptr, *D = nullptr;
-  int nvec = 0, nscal = 0, nr = 0, nth = 0;
-  __host__ __device__ int rpP() const { return 2 * (nvec + nscal); }
-  __host__ __device__ int rpD() const { return 4 * nvec; }
-  // per-(m, theta) block strides, rounded up to 4 floats (16 bytes) so TMA
-  // boxes can start on any block
-  __host__ __device__ size_t sP() const { return (((size_t)nr * rpP() + 3) / 4) * 4; }
-  __host__ __device__ size_t sD() const { return (((size_t)nr * rpD() + 3) / 4) * 4; }
-  // element of component c (vector v: 3v r, 3v+1 theta, 3v+2 phi; scalars
-  // after the vectors) at (m, theta, k), order sign s
-  __host__ __device__ float *at(int m, int th, int k, int c, int s) const {
-    if (c < 3 * nvec) {
-      const int v = c / 3, cc = c - 3 * v;
-      if (cc == 0) return P + ((size_t)m * nth + th) * sP() + (size_t)k * rpP() + 2 * v + s;
-      return D + ((size_t)m * nth + th) * sD() + (size_t)k * rpD() + 4 * v + 2 * (cc - 1) + s;
-    }
-    return P + ((size_t)m * nth + th) * sP() + (size_t)k * rpP() + 2 * (nvec + (c - 3 * nvec)) + s;
-  }
-};
 // layout over a float buffer of at least mlayout_floats(c) floats (any
 // nvec, nscal with 3 nvec + nscal <= 13)
 MLayout mlayout(const Ctx &c, void *buf, int nvec, int nscal);
@@ -273,13 +289,11 @@ const float *mixed_weights32(Ctx &c);
 // returns true when it wrote the partial row maxima into pmax (the
 // four-step kernel; pmax may be nullptr)
 bool fft_products_m(Ctx &c, const MLayout &in, const MLayout &out, float *pmax = nullptr);
-void fft_backward_grid_m(Ctx &c, const MLayout &in, double *grid);
-void fft_forward_grid_m(Ctx &c, const double *grid, const MLayout &out);
 
 // autotuned kernel variants (Ctx::tune)
 enum Tune {
-  TUNE_BWD_KT = 0,       // float64 backward Legendre: 1 tensor cores (mma f64); CUDA cores with 2 or 4 radial levels per block
-  TUNE_FWD_KT = 1,       // float64 forward Legendre: CUDA cores with 1 or 2 radial levels per block; 3 tensor cores (mma f64)
+  TUNE_BWD_KT = 0,       // float64 backward Legendre: kept, one kernel (float64 tensor cores) serves every value
+  TUNE_FWD_KT = 1,       // float64 forward Legendre: the same
   TUNE_PACK_KC = 2,      // mixed backward pack: radial levels per block (1, 2, 4)
   TUNE_FFT_THREADS = 3,  // mixed FFT + products: threads per row block; 384 = the four-step kernel
                          // (nphi = 3 (L + 1)), 128 / 256 / 512 = the Stockham kernel

@@ -158,7 +158,7 @@ __device__ static void d_schmidt_m(int ltr, int m, double th, double *p, double 
 
 // one thread per (m, node i < nh); scratch rows in global memory
 __global__ void k_plm(int L, int nh, const double *colat, const size_t *poff,
-                      double *scratch, double *Plt, double *dPlt, double *Ptl, double *dPtl) {
+                      double *scratch, double *Plt, double *dPlt) {
   int m = blockIdx.y;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (m > L || i >= nh) return;
@@ -168,7 +168,6 @@ __global__ void k_plm(int L, int nh, const double *colat, const size_t *poff,
   d_schmidt_m(L, m - 1, th, pn, df);
   d_schmidt_m(L, m + 1, th, pp, df);
   d_schmidt_m(L, m, th, p, df);
-  int nl = L + 1 - m;
   size_t o = poff[m];
   for (int l = m; l <= L; l++) {
     double dp;
@@ -185,8 +184,6 @@ __global__ void k_plm(int L, int nh, const double *colat, const size_t *poff,
     }
     Plt[o + (size_t)(l - m) * nh + i] = p[l];
     dPlt[o + (size_t)(l - m) * nh + i] = dp;
-    Ptl[o + (size_t)i * nl + (l - m)] = p[l];
-    dPtl[o + (size_t)i * nl + (l - m)] = dp;
   }
 }
 
@@ -391,14 +388,11 @@ int setup_tables(Ctx &c) {
   // Schmidt tables on the device
   CB2_CUDA(cudaMalloc(&c.d_Plt, po * sizeof(double)));
   CB2_CUDA(cudaMalloc(&c.d_dPlt, po * sizeof(double)));
-  CB2_CUDA(cudaMalloc(&c.d_Ptl, po * sizeof(double)));
-  CB2_CUDA(cudaMalloc(&c.d_dPtl, po * sizeof(double)));
   size_t sbytes = (size_t)(L + 1) * c.nh * 4 * (L + 4) * sizeof(double);
   double *scratch = nullptr;
   CB2_CUDA(cudaMalloc(&scratch, sbytes));
   dim3 grid(cdiv(c.nh, 64), L + 1);
-  k_plm<<<grid, 64, 0, c.stream>>>(L, c.nh, c.d_colat, c.d_poff, scratch, c.d_Plt, c.d_dPlt,
-                                   c.d_Ptl, c.d_dPtl);
+  k_plm<<<grid, 64, 0, c.stream>>>(L, c.nh, c.d_colat, c.d_poff, scratch, c.d_Plt, c.d_dPlt);
   CB2_CUDA(cudaGetLastError());
   CB2_CUDA(cudaStreamSynchronize(c.stream));
   CB2_CUDA(cudaFree(scratch));
@@ -408,8 +402,8 @@ int setup_tables(Ctx &c) {
 void free_tables(Ctx &c) {
   void *ptrs[] = {c.d_jl, c.d_jm, c.d_moff, c.d_g3, c.d_g3rlm, c.d_gl, c.d_g6, c.d_g7,
                   c.d_g11, c.d_g12, c.d_r, c.d_ar1, c.d_ar2, c.d_d1, c.d_d2, c.d_reft0, c.d_reft1,
-                  c.d_om, c.d_colat, c.d_wgt, c.d_asin, c.d_poff, c.d_Plt, c.d_dPlt, c.d_Ptl,
-                  c.d_dPtl, c.d_jgi1, c.d_jgi2, c.d_jei1, c.d_sw, c.d_tw};
+                  c.d_om, c.d_colat, c.d_wgt, c.d_asin, c.d_poff, c.d_Plt, c.d_dPlt,
+                  c.d_jgi1, c.d_jgi2, c.d_jei1, c.d_sw, c.d_tw};
   for (void *q : ptrs)
     if (q) cudaFree(q);
 }

@@ -46,20 +46,9 @@ static int time_stage(Ctx &c, int (*stage)(Ctx &), float *best_ms) {
 }
 
 static const int kBwdSlots[5] = {VELO, VORT, MAGNE, CURRENT, TEMP};
-static const int kFwdSlots[4] = {MADV, LOR, VPIND, HFLUX};
 
-static int stage_bwd_f64(Ctx &c) {
-  leg_bwd_f64(c, 4, 1, kBwdSlots, (double *)c.d_four);
-  CB2_CUDA(cudaGetLastError());
-  return 0;
-}
-static int stage_fwd_f64(Ctx &c) {
-  leg_fwd_f64(c, 4, 0, (const double *)c.d_four2, kFwdSlots);
-  CB2_CUDA(cudaGetLastError());
-  return 0;
-}
 static int stage_fft_f64(Ctx &c) {
-  fft_products<double>(c, (const double *)c.d_four, (double *)c.d_four2);
+  fft_products64(c, mlayout64(c, c.d_four, 4, 1), mlayout64(c, c.d_four2, 4, 0));
   CB2_CUDA(cudaGetLastError());
   return 0;
 }
@@ -89,9 +78,7 @@ int autotune(Ctx &c) {
   };
   std::vector<Item> items;
   if (c.prec == CB2_PREC_FP64) {
-    items.push_back({TUNE_BWD_KT, {1, 2, 4}, stage_bwd_f64});
-    items.push_back({TUNE_FWD_KT, {1, 2, 3}, stage_fwd_f64});
-    // 384: the float64 four-step kernel (where nphi = 3 (L + 1)), 512: Stockham
+    // 384: the float64 four-step kernel (where nphi = 3 (L + 1)), 512: the general one
     items.push_back({TUNE_FFT_THREADS, {384, 512}, stage_fft_f64});
   } else {
     items.push_back({TUNE_PACK_KC, {1, 2, 4}, stage_bwd_mixed});
