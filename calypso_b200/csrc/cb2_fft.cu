@@ -68,14 +68,16 @@ template <> struct PairBits<float> {
     return pow2i(inv ? -e : e);
   }
 };
+// (float64: the high words, which order the exponents; 32-bit maxima reduce
+// over a warp in one instruction)
 template <> struct PairBits<double> {
-  using U = unsigned long long;
-  __device__ static U abs_bits(double x) { return (U)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull; }
+  using U = unsigned;
+  __device__ static U abs_bits(double x) { return (U)__double2hiint(x) & 0x7FFFFFFFu; }
   __device__ static double factor(U mx, U my, bool inv) {
-    const int ex = (int)(mx >> 52), ey = (int)(my >> 52);
+    const int ex = (int)(mx >> 20), ey = (int)(my >> 20);
     if (ex == 0 || ey == 0) return 1.0;
     const int e = max(-1000, min(1000, ex - ey));
-    return __longlong_as_double((long long)(1023 + (inv ? -e : e)) << 52);
+    return __hiloint2double((1023 + (inv ? -e : e)) << 20, 0);
   }
 };
 
@@ -1015,7 +1017,7 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
       const double2 v = S2[c * MP2 + m];
       mx = max(mx, max(PB::abs_bits(v.x), PB::abs_bits(v.y)));
     }
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, (U)__shfl_xor_sync(0xffffffffu, mx, o));
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) cmx[c] = mx;
   }
   __syncthreads();
@@ -1099,24 +1101,23 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
     }
 #pragma unroll
     for (int c = 0; c < 12; c++) {
-      U v = hm[c];
-      for (int o = 16; o > 0; o >>= 1) v = max(v, (U)__shfl_xor_sync(0xffffffffu, v, o));
+      const U v = __reduce_max_sync(0xffffffffu, hm[c]);
       if (lane == 0) atomicMax(cmx + 13 + c, v);
     }
   }
   __syncthreads();
-  for (int idx = tid; idx < 6 * N; idx += NT) {
-    const int p = idx / N;
-    X[idx].y *= PB::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], false);
-  }
-  __syncthreads();
-  // ---- forward, step 1: column n2 = lt of the samples j = 3 (n1 R2 + n2) + r
+  // ---- forward, step 1: column n2 = lt of the samples j = 3 (n1 R2 + n2) + r,
+  // the second row of the pair scaled on the way in
   {
     double2 v[R1];
     if (grp < 18) {
       const double2 *G = X + gp * N + 3 * lt + gr;
+      const double sy = PB::factor(cmx[13 + 2 * gp], cmx[14 + 2 * gp], false);
 #pragma unroll
-      for (int n1 = 0; n1 < R1; n1++) v[n1] = G[3 * R2 * n1];
+      for (int n1 = 0; n1 < R1; n1++) {
+        v[n1] = G[3 * R2 * n1];
+        v[n1].y *= sy;
+      }
       dftr<R1, -1>(v);
 #pragma unroll
       for (int k1 = 1; k1 < R1; k1++) v[k1] = cmulc(v[k1], TWM[lt * WP + k1]);
@@ -1195,6 +1196,239 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
   }
 }
 
+// The same transform one residue after another, for M = 256: the grid samples
+// of the three residues do not meet until the orders are combined, so a CTA
+// needs the transposes and grid rows of one (30 KB instead of 91) and two CTAs
+// share an SM, one computing while the other moves data through shared memory;
+// the (a_m, b_m) of the 12 products add up in registers.  The product rows are
+// scaled pair by pair within each residue.  The three residues side by side in
+// one CTA of 384 threads and 166 KB took 5.7 ms at L255 / Nr129 (49536 rows).
+template <int R1, int R2>
+struct F4Plan64R {
+  static constexpr int M = R1 * R2, N = 3 * M, NT = 8 * R2;
+  static constexpr int TP = R2 + 1, TG = R1 * TP, X = 7 * TG;   // transposes / 7 M grid samples / 6 M orders
+  static constexpr int MP2 = M + 1, WP = R1 + 1, NTW = 3 * M + R2 * WP, SC = 14 * MP2;
+  static constexpr int MH = 6 * M / NT;                          // (pair, order) sums of a thread
+  static constexpr size_t smem() { return ((size_t)SC + X + NTW) * sizeof(double2) + 56 * sizeof(unsigned); }
+};
+
+template <int R1, int R2>
+__global__ void __launch_bounds__(F4Plan64R<R1, R2>::NT, 2)
+k_fft_products_4s64r(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ tables, ProdCoef pc) {
+  using P = F4Plan64R<R1, R2>;
+  using PB = PairBits<double>;
+  using U = PB::U;
+  static_assert(R1 == R2, "one row of the second step a thread");
+  constexpr int M = P::M, N = P::N, NT = P::NT, TP = P::TP, TG = P::TG, MP2 = P::MP2, WP = P::WP, MH = P::MH;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2 *S2 = reinterpret_cast<double2 *>(smraw);   // [14][MP2] (a_m, b_m); last [12][MP2] out
+  double2 *X = S2 + P::SC;
+  double2 *TW3 = X + P::X;                             // [3][M]
+  double2 *TWM = TW3 + 3 * M;                          // [R2][WP]
+  U *cmx = reinterpret_cast<U *>(TWM + R2 * WP);      // [0, 13) input maxima, 16 + 12 r: products of residue r
+  const int th = blockIdx.x / fin.nr, k = blockIdx.x % fin.nr;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = NT / 32;
+  const int gp = tid / R2, lt = tid % R2;              // pair (7: idle), column / row
+  for (int e = tid; e < 14; e += NT) S2[e * MP2 + M] = double2{0.0, 0.0};
+  for (int e = tid; e < M; e += NT) S2[13 * MP2 + e] = double2{0.0, 0.0};
+  for (int e = tid; e < 52; e += NT) cmx[e] = 0;
+  auto cp16 = [](double2 *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+  };
+  for (int e = tid; e < P::NTW; e += NT) cp16(TW3 + e, tables + e);
+  {
+    const int j = lane & 15, hw = lane >> 4;
+    int c = 0;
+    const double *src = fin.P;
+    size_t mst = 0;
+    if (j < 5) {
+      c = (j < 4) ? 3 * j : 12;
+      src = fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + 2 * j;
+      mst = (size_t)fin.nth * fin.sP();
+    } else if (j < 13) {
+      const int jd = j - 5;
+      c = 3 * (jd >> 1) + 1 + (jd & 1);
+      src = fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + 2 * jd;
+      mst = (size_t)fin.nth * fin.sD();
+    }
+    if (j < 13)
+      for (int m = 2 * warp + hw; m < M; m += 2 * nwarp) cp16(S2 + c * MP2 + m, src + m * mst);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  }
+  __syncthreads();
+  for (int c = warp; c < 13; c += nwarp) {
+    U mx = 0;
+    for (int m = lane; m < M; m += 32) {
+      const double2 v = S2[c * MP2 + m];
+      mx = max(mx, max(PB::abs_bits(v.x), PB::abs_bits(v.y)));
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) cmx[c] = mx;
+  }
+  __syncthreads();
+  // (a_m, b_m) of the two components of pair p, (p, m) = tid + i NT
+  double2 o0[MH], o1[MH];
+#pragma unroll
+  for (int i = 0; i < MH; i++) o0[i] = o1[i] = double2{0.0, 0.0};
+#pragma unroll 1
+  for (int r = 0; r < 3; r++) {
+    const double2 *tw = TW3 + r * M;
+    double2 v[R1];
+    // ---- backward, step 1: column n2 = lt, pair rows from the staging
+    if (gp < 7) {
+      const double2 *x0 = S2 + (2 * gp) * MP2, *y0 = S2 + (2 * gp + 1) * MP2;
+      const double sy = (gp < 6) ? PB::factor(cmx[2 * gp], cmx[2 * gp + 1], false) : 1.0;
+      const double2 om = (r == 0) ? double2{1.0, 0.0}
+                       : double2{-0.5, (r == 1) ? -0.86602540378443864676 : 0.86602540378443864676};
+#pragma unroll
+      for (int n1 = 0; n1 < R1; n1++) {
+        const int m = n1 * R2 + lt, mq = M - m;
+        const double2 a = x0[m], c = x0[mq];
+        const double2 b = double2{y0[m].x * sy, y0[m].y * sy}, d = double2{y0[mq].x * sy, y0[mq].y * sy};
+        double2 zm = double2{a.x + b.y, b.x - a.y};           // 2 Z[m]
+        const double2 zp = double2{c.x - d.y, c.y + d.x};     // 2 Z[N - (M - m)] (zero at m = 0)
+        if (n1 == 0 && lt == 0) zm = double2{2.0 * a.x, 2.0 * b.x};
+        v[n1] = cmulf(cadd(zm, cmulf(om, zp)), tw[m]);
+      }
+      dftr<R1, +1>(v);
+      double2 *T = X + gp * TG;
+#pragma unroll
+      for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = (k1 == 0) ? v[0] : cmulf(v[k1], TWM[lt * WP + k1]);
+    }
+    __syncwarp();   // the group's own transpose block
+    // ---- step 2: row k1 = lt -> samples j' = k1 + R1 k2
+    if (gp < 7) {
+      const double2 *T = X + gp * TG + lt * TP;
+#pragma unroll
+      for (int n2 = 0; n2 < R2; n2++) v[n2] = T[n2];
+      dftr<R2, +1>(v);
+    }
+    __syncthreads();
+    if (gp < 7) {
+      double2 *G = X + gp * M + lt;
+#pragma unroll
+      for (int k2 = 0; k2 < R2; k2++) G[R1 * k2] = v[k2];
+    }
+    __syncthreads();
+    // ---- products at the residue's samples, in place
+    {
+      const double cv = 0.25 * pc.cv, cl = 0.25 * pc.cl, ci = 0.25 * pc.ci, ct = 0.25 * pc.ct;
+      double iy[6];
+#pragma unroll
+      for (int p = 0; p < 6; p++) iy[p] = PB::factor(cmx[2 * p], cmx[2 * p + 1], true);
+      U hm[12];
+#pragma unroll
+      for (int c = 0; c < 12; c++) hm[c] = 0;
+#pragma unroll 1
+      for (int q = tid; q < M; q += NT) {
+        const double2 p0 = X[0 * M + q], p1 = X[1 * M + q], p2 = X[2 * M + q], p3 = X[3 * M + q];
+        const double2 p4 = X[4 * M + q], p5 = X[5 * M + q], p6 = X[6 * M + q];
+        const double ur = p0.x, ut = p0.y * iy[0], up = p1.x, wr = p1.y * iy[1], wt = p2.x, wp = p2.y * iy[2];
+        const double br = p3.x, bt = p3.y * iy[3], bp = p4.x, jr = p4.y * iy[4], jt = p5.x, jp = p5.y * iy[5];
+        const double tt = p6.x;
+        const double2 hv[6] = {double2{(wt * up - wp * ut) * cv, (wp * ur - wr * up) * cv},
+                               double2{(wr * ut - wt * ur) * cv, (jt * bp - jp * bt) * cl},
+                               double2{(jp * br - jr * bp) * cl, (jr * bt - jt * br) * cl},
+                               double2{(ut * bp - up * bt) * ci, (up * br - ur * bp) * ci},
+                               double2{(ur * bt - ut * br) * ci, ur * tt * ct},
+                               double2{ut * tt * ct, up * tt * ct}};
+#pragma unroll
+        for (int p = 0; p < 6; p++) {
+          X[p * M + q] = hv[p];
+          hm[2 * p] = max(hm[2 * p], PB::abs_bits(hv[p].x));
+          hm[2 * p + 1] = max(hm[2 * p + 1], PB::abs_bits(hv[p].y));
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 12; c++) {
+        const U u = __reduce_max_sync(0xffffffffu, hm[c]);
+        if (lane == 0) atomicMax(cmx + 16 + 12 * r + c, u);
+      }
+    }
+    __syncthreads();
+    // ---- forward, step 1: column n2 = lt of the samples n1 R2 + n2
+    const U *pmx = cmx + 16 + 12 * r;
+    if (gp < 6) {
+      const double2 *G = X + gp * M + lt;
+      const double sy = PB::factor(pmx[2 * gp], pmx[2 * gp + 1], false);
+#pragma unroll
+      for (int n1 = 0; n1 < R1; n1++) {
+        v[n1] = G[R2 * n1];
+        v[n1].y *= sy;
+      }
+      dftr<R1, -1>(v);
+#pragma unroll
+      for (int k1 = 1; k1 < R1; k1++) v[k1] = cmulc(v[k1], TWM[lt * WP + k1]);
+    }
+    __syncthreads();
+    if (gp < 6) {
+      double2 *T = X + gp * TG;
+#pragma unroll
+      for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = v[k1];
+    }
+    __syncwarp();
+    // ---- step 2: row k1 = lt -> F_r[k1 + R1 k2]
+    if (gp < 6) {
+      const double2 *T = X + gp * TG + lt * TP;
+#pragma unroll
+      for (int n2 = 0; n2 < R2; n2++) v[n2] = T[n2];
+      dftr<R2, -1>(v);
+    }
+    __syncthreads();
+    if (gp < 6) {
+      double2 *F = X + gp * M + lt;
+#pragma unroll
+      for (int k2 = 0; k2 < R2; k2++) F[R1 * k2] = v[k2];
+    }
+    __syncthreads();
+    // ---- this residue's part of Z[m], Z[N - m], taken apart into the
+    // (a_m, b_m) of both rows of each pair (the second unscaled)
+#pragma unroll
+    for (int i = 0; i < MH; i++) {
+      const int idx = tid + i * NT, p = idx / M, m = idx % M, mm = (M - m) & (M - 1);
+      const double2 t = tw[m];
+      const double2 zk = cmulc(X[p * M + m], t), zn = cmulf(X[p * M + mm], t);
+      const double ay = PB::factor(pmx[2 * p], pmx[2 * p + 1], true);
+      if (m == 0) {
+        o0[i].x += zk.x;
+        o1[i].x += ay * zk.y;
+      } else {
+        o0[i].x += zk.x + zn.x; o0[i].y -= zk.y - zn.y;
+        o1[i].x += ay * (zk.y + zn.y); o1[i].y += ay * (zk.x - zn.x);
+      }
+    }
+    __syncthreads();   // X holds the next residue's transposes
+  }
+  const double an = 1.0 / (double)N;
+#pragma unroll
+  for (int i = 0; i < MH; i++) {
+    const int idx = tid + i * NT, p = idx / M, m = idx % M;
+    S2[(2 * p) * MP2 + m] = double2{an * o0[i].x, an * o0[i].y};
+    S2[(2 * p + 1) * MP2 + m] = double2{an * o1[i].x, an * o1[i].y};
+  }
+  __syncthreads();
+  {
+    const int j = lane & 15, hw = lane >> 4;
+    int c = 0;
+    double *dst = fout.P;
+    size_t mst = 0;
+    if (j < 4) {
+      c = 3 * j;
+      dst = fout.P + (size_t)th * fout.sP() + (size_t)k * 8 + 2 * j;
+      mst = (size_t)fout.nth * fout.sP();
+    } else if (j < 12) {
+      const int jd = j - 4;
+      c = 3 * (jd >> 1) + 1 + (jd & 1);
+      dst = fout.D + (size_t)th * fout.sD() + (size_t)k * 16 + 2 * jd;
+      mst = (size_t)fout.nth * fout.sD();
+    }
+    if (j < 12)
+      for (int m = 2 * warp + hw; m < M; m += 2 * nwarp)
+        *reinterpret_cast<double2 *>(dst + m * mst) = S2[c * MP2 + m];
+  }
+}
+
 // ---------------------------------------------------------------------------
 // The general float64 products kernel, any N = 2^a 3^b (the grids that are not
 // nphi = 3 (L + 1) with L + 1 = 32 .. 256): Stockham passes of radix 16 and 9
@@ -1238,17 +1472,21 @@ static G64Plan make_plan64(int n, int L) {
   return p;
 }
 
+// mx (first pass of the forward transform): maxima of the rows, the second
+// row of each pair scaled to the first on the way in
 template <int R, int SIGN>
 __device__ __forceinline__ void g64_pass(const double2 *x, double2 *y, int nf, const G64Plan &pl, const G64Stage &st,
-                                         const double2 *__restrict__ tw) {
+                                         const double2 *__restrict__ tw, const unsigned *mx) {
   const int np = pl.np;
   for (int idx = threadIdx.x; idx < nf * st.nb; idx += blockDim.x) {
     const int f = st.dnb.div(idx), j = idx - f * st.nb, q = st.dNs.div(j), k = j - q * st.Ns;
     const double2 *xf = x + f * np;
+    const double sy = (SIGN < 0 && mx) ? PairBits<double>::factor(mx[2 * f], mx[2 * f + 1], false) : 1.0;
     double2 v[R];
 #pragma unroll
     for (int r = 0; r < R; r++) {
       v[r] = xf[pl.pad(j + r * st.nb)];
+      if (SIGN < 0 && mx) v[r].y *= sy;
       if (r > 0 && k > 0) {
         double2 w = __ldg(tw + r * k * st.tstride);
         if (SIGN > 0) w.y = -w.y;
@@ -1266,16 +1504,17 @@ __device__ __forceinline__ void g64_pass(const double2 *x, double2 *y, int nf, c
 
 template <int SIGN>
 __device__ __forceinline__ double2 *g64_fft(double2 *x, double2 *y, int nf, const G64Plan &pl,
-                                            const double2 *__restrict__ tw) {
+                                            const double2 *__restrict__ tw, const unsigned *mx = nullptr) {
   for (int s = 0; s < pl.nst; s++) {
     const G64Stage &st = pl.st[s];
+    const unsigned *m0 = (s == 0) ? mx : nullptr;
     switch (st.R) {
-      case 16: g64_pass<16, SIGN>(x, y, nf, pl, st, tw); break;
-      case 9: g64_pass<9, SIGN>(x, y, nf, pl, st, tw); break;
-      case 8: g64_pass<8, SIGN>(x, y, nf, pl, st, tw); break;
-      case 4: g64_pass<4, SIGN>(x, y, nf, pl, st, tw); break;
-      case 3: g64_pass<3, SIGN>(x, y, nf, pl, st, tw); break;
-      default: g64_pass<2, SIGN>(x, y, nf, pl, st, tw); break;
+      case 16: g64_pass<16, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 9: g64_pass<9, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 8: g64_pass<8, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 4: g64_pass<4, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 3: g64_pass<3, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      default: g64_pass<2, SIGN>(x, y, nf, pl, st, tw, m0); break;
     }
     double2 *t = x; x = y; y = t;
   }
@@ -1323,7 +1562,7 @@ k_fft_products_g64(const __grid_constant__ G64Plan pl, int L, MLayout64 fin, MLa
       mx = max(mx, PB::abs_bits(S[(2 * c) * MP + m]));
       if (m > 0) mx = max(mx, PB::abs_bits(S[(2 * c + 1) * MP + m]));
     }
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, (U)__shfl_xor_sync(0xffffffffu, mx, o));
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) cmx[c] = mx;
   }
   __syncthreads();
@@ -1377,18 +1616,12 @@ k_fft_products_g64(const __grid_constant__ G64Plan pl, int L, MLayout64 fin, MLa
     }
 #pragma unroll
     for (int c = 0; c < 12; c++) {
-      U v = hm[c];
-      for (int o = 16; o > 0; o >>= 1) v = max(v, (U)__shfl_xor_sync(0xffffffffu, v, o));
+      const U v = __reduce_max_sync(0xffffffffu, hm[c]);
       if (lane == 0) atomicMax(cmx + 13 + c, v);
     }
   }
   __syncthreads();
-  for (int p = 0; p < 6; p++) {
-    const double f = PB::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], false);
-    for (int q = tid; q < N; q += blockDim.x) h[p * NP + pl.pad(q)].y *= f;
-  }
-  __syncthreads();
-  const double2 *zf = g64_fft<-1>(h, g, 6, pl, tw);
+  const double2 *zf = g64_fft<-1>(h, g, 6, pl, tw, cmx + 13);
   double *O = reinterpret_cast<double *>((zf == A) ? B : A);   // [c * 2 + s][MP]
   const double an = 1.0 / (double)N;
   for (int p = 0; p < 6; p++) {
@@ -1418,12 +1651,6 @@ k_fft_products_g64(const __grid_constant__ G64Plan pl, int L, MLayout64 fin, MLa
 }
 
 // order-major Fourier rows -> grid (float64), for the standalone transform API
-template <typename U>
-__device__ __forceinline__ U warp_max(U v) {
-  for (int o = 16; o > 0; o >>= 1) v = max(v, (U)__shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_fft_to_grid_m(FFTPlan pl, int L, MLayoutT<T> fin, double *grid, const typename C2<T>::t *tw) {
@@ -1449,8 +1676,8 @@ k_fft_to_grid_m(FFTPlan pl, int L, MLayoutT<T> fin, double *grid, const typename
         if (has1)
           my = max(my, max(PB::abs_bits(*fin.at(m, th, k, c + 1, 0)), PB::abs_bits(*fin.at(m, th, k, c + 1, 1))));
       }
-      mx = warp_max(mx);
-      my = warp_max(my);
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      my = __reduce_max_sync(0xffffffffu, my);
       if ((threadIdx.x & 31) == 0) { atomicMax(pmx, mx); atomicMax(pmx + 1, my); }
     }
     __syncthreads();
@@ -1502,8 +1729,8 @@ k_grid_to_fft_m(FFTPlan pl, int L, const double *grid, MLayoutT<T> fout, const t
       mx = max(mx, PB::abs_bits(x));
       my = max(my, PB::abs_bits(y));
     }
-    mx = warp_max(mx);
-    my = warp_max(my);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    my = __reduce_max_sync(0xffffffffu, my);
     if ((threadIdx.x & 31) == 0) { atomicMax(pmx, mx); atomicMax(pmx + 1, my); }
     __syncthreads();
     // pair scaling (pair_exp): the second row brought to the size of the first
@@ -1604,7 +1831,8 @@ static int attr_fft_4s(Ctx &c) {
 template <int R1, int R2>
 static int attr_fft_4s64(Ctx &c) {
   using P = F4Plan64<R1, R2>;
-  CB2_CUDA(raise_smem_limit(k_fft_products_4s64<R1, R2>, (int)P::smem()));
+  if constexpr (R2 == 16) CB2_CUDA(raise_smem_limit(k_fft_products_4s64r<R1, R2>, F4Plan64R<R1, R2>::smem()));
+  else CB2_CUDA(raise_smem_limit(k_fft_products_4s64<R1, R2>, P::smem()));
   std::vector<double2> t(P::NTW, double2{0.0, 0.0});
   const double pi = 3.14159265358979323846;
   for (int r = 0; r < 3; r++)
@@ -1683,7 +1911,10 @@ static const typename C2<T>::t *twid(Ctx &c) {
 
 template <int R1, int R2>
 static void launch_fft_4s64(Ctx &c, const MLayout64 &in, const MLayout64 &out, const ProdCoef &pc) {
-  k_fft_products_4s64<R1, R2><<<(unsigned)(c.nth * c.nr), f4_threads<R2>(), F4Plan64<R1, R2>::smem(), c.stream>>>(
+  if constexpr (R2 == 16)
+    k_fft_products_4s64r<R1, R2><<<(unsigned)(c.nth * c.nr), F4Plan64R<R1, R2>::NT, F4Plan64R<R1, R2>::smem(),
+                                   c.stream>>>(in, out, (const double2 *)c.d_twf4_64, pc);
+  else k_fft_products_4s64<R1, R2><<<(unsigned)(c.nth * c.nr), f4_threads<R2>(), F4Plan64<R1, R2>::smem(), c.stream>>>(
       in, out, (const double2 *)c.d_twf4_64, pc);
 }
 
