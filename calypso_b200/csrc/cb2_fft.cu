@@ -149,79 +149,12 @@ struct ProdCoef {
   double cv, cl, ci, ct;
 };
 
-// Stockham stages over nf independent FFTs held in x[f*N + n]; all FFTs of
-// the row advance together so each stage costs one barrier
-template <typename T, typename T2>
-__device__ T2 *batch_fft(T2 *x, T2 *y, int nf, const FFTPlan &pl, const T2 *__restrict__ tw, int sign) {
-  const int N = pl.n;
-  int Ns = 1;
-  const T s32 = (T)(0.5 * sqrt(3.0));
-  for (int st = 0; st < pl.nst; st++) {
-    const int R = pl.rad[st];
-    const int nb = N / R, tstride = N / (Ns * R);
-    for (int idx = threadIdx.x; idx < nf * nb; idx += blockDim.x) {
-      int f = idx / nb, j = idx - f * nb;
-      int k = j % Ns;
-      const T2 *xf = x + f * N;
-      T2 v[4];
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        if (r < R) {
-          T2 a = xf[j + r * nb];
-          if (r > 0 && k > 0) {
-            T2 w = tw[r * k * tstride];
-            if (sign > 0) w.y = -w.y;
-            a = cmul(a, w);
-          }
-          v[r] = a;
-        }
-      }
-      T2 o[4];
-      if (R == 4) {
-        T2 a0, a1, a2, a3;
-        a0.x = v[0].x + v[2].x; a0.y = v[0].y + v[2].y;
-        a1.x = v[0].x - v[2].x; a1.y = v[0].y - v[2].y;
-        a2.x = v[1].x + v[3].x; a2.y = v[1].y + v[3].y;
-        T dx = v[1].x - v[3].x, dy = v[1].y - v[3].y;
-        if (sign < 0) { a3.x = dy; a3.y = -dx; } else { a3.x = -dy; a3.y = dx; }
-        o[0].x = a0.x + a2.x; o[0].y = a0.y + a2.y;
-        o[1].x = a1.x + a3.x; o[1].y = a1.y + a3.y;
-        o[2].x = a0.x - a2.x; o[2].y = a0.y - a2.y;
-        o[3].x = a1.x - a3.x; o[3].y = a1.y - a3.y;
-      } else if (R == 2) {
-        o[0].x = v[0].x + v[1].x; o[0].y = v[0].y + v[1].y;
-        o[1].x = v[0].x - v[1].x; o[1].y = v[0].y - v[1].y;
-      } else {
-        T2 t1, t2, t3;
-        t1.x = v[1].x + v[2].x; t1.y = v[1].y + v[2].y;
-        t2.x = v[0].x - (T)0.5 * t1.x; t2.y = v[0].y - (T)0.5 * t1.y;
-        T dx = v[1].x - v[2].x, dy = v[1].y - v[2].y;
-        if (sign < 0) { t3.x = s32 * dy; t3.y = -s32 * dx; } else { t3.x = -s32 * dy; t3.y = s32 * dx; }
-        o[0].x = v[0].x + t1.x; o[0].y = v[0].y + t1.y;
-        o[1].x = t2.x + t3.x; o[1].y = t2.y + t3.y;
-        o[2].x = t2.x - t3.x; o[2].y = t2.y - t3.y;
-      }
-      T2 *yf = y + f * N;
-      int d = (j / Ns) * Ns * R + k;
-#pragma unroll
-      for (int r = 0; r < 4; r++)
-        if (r < R) yf[d + r * Ns] = o[r];
-    }
-    __syncthreads();
-    T2 *t = x; x = y; y = t;
-    Ns *= R;
-  }
-  return x;
-}
-
 // ---------------------------------------------------------------------------
-// The general float32 kernel over the order-major Fourier layout (MLayout).
-// Input 4 vectors (u, w, B, J) + 1 scalar (T),
-// output 4 vectors (w x u, J x B, u x B, u T).  At one (theta, k) the 26
-// input floats of an order m are one run of 10 (P block) and one of 16
-// (D block); threads take consecutive elements of a run, the values are
-// staged in shared memory [component][s][m], and the Hermitian rows are
-// built from there.  Output is written the same way, one run per m.
+// The fused products kernels over the order-major Fourier layout (MLayoutT).
+// Input 4 vectors (u, w, B, J) + 1 scalar (T), output 4 vectors (w x u, J x B,
+// u x B, u T).  At one (theta, k) the 26 input values of an order m are one run
+// of 10 (P block) and one of 16 (D block), the 24 output values one of 8 and
+// one of 16; element j of a run:
 __device__ inline void m_comp_of_in(int j, int &c, int &s) {
   // P block (k, field, s): fields 0..3 = r of u, w, B, J; 4 = T
   if (j < 10) { const int f = j >> 1; s = j & 1; c = (f < 4) ? 3 * f : 12; return; }
@@ -234,130 +167,6 @@ __device__ inline void m_comp_of_out(int j, int &c, int &s) {
   if (j < 8) { s = j & 1; c = 3 * (j >> 1); return; }
   const int jd = j - 8, v = jd >> 2, q = jd & 3;
   c = 3 * v + 1 + (q >> 1); s = q & 1;
-}
-
-__global__ void __launch_bounds__(512)
-k_fft_products_m(FFTPlan pl, int L, MLayout fin, MLayout fout, const float2 *__restrict__ tw, ProdCoef pc) {
-  using T = float;
-  using T2 = float2;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int N = pl.n;
-  T2 *A = reinterpret_cast<T2 *>(smraw);    // 7 x N
-  T2 *B = A + 7 * N;                         // 7 x N (first used as the staging buffer)
-  T *S = reinterpret_cast<T *>(B);           // [c * 2 + s][m], 26 x (L+1)
-  float *SC = reinterpret_cast<float *>(B + 7 * N);        // pair factors [7], inverses [8..14]
-  unsigned *FMX = reinterpret_cast<unsigned *>(SC + 16);   // forward row maxima [12]
-  const int th = blockIdx.x / fin.nr, k = blockIdx.x % fin.nr;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int M1 = L + 1;
-  if (threadIdx.x < 12) FMX[threadIdx.x] = 0u;
-  const float *Pin = fin.P + (size_t)th * fin.sP() + (size_t)k * 10;
-  const float *Din = fin.D + (size_t)th * fin.sD() + (size_t)k * 16;
-  const size_t mstP = (size_t)fin.nth * fin.sP(), mstD = (size_t)fin.nth * fin.sD();
-  for (int idx = threadIdx.x; idx < 26 * M1; idx += blockDim.x) {
-    const int m = idx / 26, j = idx - 26 * m;
-    int c, s;
-    m_comp_of_in(j, c, s);
-    S[(c * 2 + s) * M1 + m] = (j < 10) ? Pin[m * mstP + j] : Din[m * mstD + (j - 10)];
-  }
-  __syncthreads();
-  // pair scaling (pair_exp) of the 6 full pairs; pair 6 (T alone) keeps 1
-  for (int p = warp; p < 7; p += nwarp) {
-    unsigned mx = 0u, my = 0u;
-    if (p < 6)
-      for (int m = lane; m < M1; m += 32) {
-        mx = max(mx, max(abs_bits(S[(4 * p) * M1 + m]), abs_bits(S[(4 * p + 1) * M1 + m])));
-        my = max(my, max(abs_bits(S[(4 * p + 2) * M1 + m]), abs_bits(S[(4 * p + 3) * M1 + m])));
-      }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    my = __reduce_max_sync(0xffffffffu, my);
-    const int e = pair_exp(mx, my);
-    if (lane == 0) { SC[p] = pow2i(e); SC[8 + p] = pow2i(-e); }
-  }
-  __syncthreads();
-  const int mmax = min(L, (N + 1) / 2 - 1);
-  for (int idx = threadIdx.x; idx < 7 * N; idx += blockDim.x) {
-    const int p = idx / N, n = idx - p * N;
-    const int c0 = 2 * p, c1 = 2 * p + 1;
-    const bool has1 = c1 < 13;
-    const T sy = SC[p];
-    T2 z = T2{0, 0};
-    if (n == 0) {
-      z = T2{S[(c0 * 2) * M1], has1 ? S[(c1 * 2) * M1] * sy : (T)0};
-    } else {
-      const int m = (n <= mmax) ? n : ((N - n <= mmax) ? N - n : -1);
-      if (m > 0) {
-        const T a0 = S[(c0 * 2) * M1 + m], b0 = S[(c0 * 2 + 1) * M1 + m];
-        const T a1 = has1 ? S[(c1 * 2) * M1 + m] * sy : (T)0, b1 = has1 ? S[(c1 * 2 + 1) * M1 + m] * sy : (T)0;
-        const T xr = (T)0.5 * a0, xi = (T)-0.5 * b0, yr = (T)0.5 * a1, yi = (T)-0.5 * b1;
-        z = (m == n) ? T2{xr - yi, xi + yr} : T2{xr + yi, -xi + yr};
-      }
-    }
-    A[idx] = z;
-  }
-  __syncthreads();
-  T2 *g = batch_fft<T, T2>(A, B, 7, pl, tw, +1);
-  T2 *hb = (g == A) ? B : A;
-  const T cv = (T)pc.cv, cl = (T)pc.cl, ci = (T)pc.ci, ct = (T)pc.ct;
-  {
-    const T i0 = SC[8], i1 = SC[9], i2 = SC[10], i3 = SC[11], i4 = SC[12], i5 = SC[13];
-    unsigned hm[12];
-#pragma unroll
-    for (int c = 0; c < 12; c++) hm[c] = 0u;
-    for (int q = threadIdx.x; q < N; q += blockDim.x) {
-      T2 p0 = g[0 * N + q], p1 = g[1 * N + q], p2 = g[2 * N + q], p3 = g[3 * N + q];
-      T2 p4 = g[4 * N + q], p5 = g[5 * N + q], p6 = g[6 * N + q];
-      T ur = p0.x, ut = p0.y * i0, up = p1.x, wr = p1.y * i1, wt = p2.x, wp = p2.y * i2;
-      T br = p3.x, bt = p3.y * i3, bp = p4.x, jr = p4.y * i4, jt = p5.x, jp = p5.y * i5, tt = p6.x;
-      const T2 h[6] = {T2{(wt * up - wp * ut) * cv, (wp * ur - wr * up) * cv},
-                       T2{(wr * ut - wt * ur) * cv, (jt * bp - jp * bt) * cl},
-                       T2{(jp * br - jr * bp) * cl, (jr * bt - jt * br) * cl},
-                       T2{(ut * bp - up * bt) * ci, (up * br - ur * bp) * ci},
-                       T2{(ur * bt - ut * br) * ci, ur * tt * ct},
-                       T2{ut * tt * ct, up * tt * ct}};
-#pragma unroll
-      for (int p = 0; p < 6; p++) {
-        hb[p * N + q] = h[p];
-        hm[2 * p] = max(hm[2 * p], abs_bits(h[p].x));
-        hm[2 * p + 1] = max(hm[2 * p + 1], abs_bits(h[p].y));
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 12; c++) {
-      const unsigned r = __reduce_max_sync(0xffffffffu, hm[c]);
-      if (lane == 0) atomicMax(FMX + c, r);
-    }
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < 6 * N; idx += blockDim.x) {
-    const int p = idx / N;
-    const int e = pair_exp(FMX[2 * p], FMX[2 * p + 1]);
-    if (e != 0) hb[idx].y *= pow2i(e);
-  }
-  __syncthreads();
-  const T2 *zf = batch_fft<T, T2>(hb, g, 6, pl, tw, -1);
-  const T an = (T)(1.0 / (double)N);
-  float *Pout = fout.P + (size_t)th * fout.sP() + (size_t)k * 8;
-  float *Dout = fout.D + (size_t)th * fout.sD() + (size_t)k * 16;
-  const size_t oP = (size_t)fout.nth * fout.sP(), oD = (size_t)fout.nth * fout.sD();
-  for (int idx = threadIdx.x; idx < 24 * M1; idx += blockDim.x) {
-    const int m = idx / 24, j = idx - 24 * m;
-    int c, s;
-    m_comp_of_out(j, c, s);
-    const T2 *Z = zf + (c >> 1) * N;
-    const bool isy = c & 1;
-    const T a = isy ? an * pow2i(-pair_exp(FMX[c - 1], FMX[c])) : an;
-    T v;
-    if (m == 0) {
-      v = (s == 0) ? a * (isy ? Z[0].y : Z[0].x) : (T)0;
-    } else {
-      const T2 zk = Z[m % N], zn = Z[(N - m) % N];
-      if (!isy) v = (s == 0) ? (T)2 * a * (T)0.5 * (zk.x + zn.x) : (T)-2 * a * (T)0.5 * (zk.y - zn.y);
-      else v = (s == 0) ? (T)2 * a * (T)0.5 * (zk.y + zn.y) : (T)2 * a * (T)0.5 * (zk.x - zn.x);
-    }
-    if (j < 8) Pout[m * oP + j] = v;
-    else Dout[m * oD + (j - 8)] = v;
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -480,27 +289,6 @@ __host__ __device__ __forceinline__ void dftr(T2 (&v)[R]) {
     v[1] = cadd(e1, o1); v[5] = csub(e1, o1);
     v[2] = cadd(e2, o2); v[6] = csub(e2, o2);
     v[3] = cadd(e3, o3); v[7] = csub(e3, o3);
-  } else if constexpr (R == 9) {
-    // 3 x 3: n = 3 n1 + n2, k = k1 + 3 k2; W9^q = exp(SIGN 2 pi i q / 9)
-    constexpr T c1 = (T)0.76604444311897803520, s1 = (T)0.64278760968653932632;   // 40 degrees
-    constexpr T c2 = (T)0.17364817766693034885, s2 = (T)0.98480775301220805937;   // 80 degrees
-    constexpr T c4 = (T)-0.93969262078590838405, s4 = (T)0.34202014332566873304;  // 160 degrees
-    constexpr T sg = (SIGN < 0) ? (T)-1 : (T)1;
-    const T2 w1 = T2{c1, sg * s1}, w2 = T2{c2, sg * s2}, w4 = T2{c4, sg * s4};
-    T2 a[3][3];
-#pragma unroll
-    for (int n2 = 0; n2 < 3; n2++) {
-      a[n2][0] = v[n2]; a[n2][1] = v[3 + n2]; a[n2][2] = v[6 + n2];
-      dftr<3, SIGN>(a[n2]);
-    }
-    a[1][1] = cmulf(a[1][1], w1); a[1][2] = cmulf(a[1][2], w2);
-    a[2][1] = cmulf(a[2][1], w2); a[2][2] = cmulf(a[2][2], w4);
-#pragma unroll
-    for (int k1 = 0; k1 < 3; k1++) {
-      T2 b[3] = {a[0][k1], a[1][k1], a[2][k1]};
-      dftr<3, SIGN>(b);
-      v[k1] = b[0]; v[k1 + 3] = b[1]; v[k1 + 6] = b[2];
-    }
   } else {
     static_assert(R == 16, "radix");
     // 4 x 4: n = 4 n1 + n2, k = k1 + 4 k2
@@ -563,7 +351,7 @@ __device__ __forceinline__ float2 *fft_passes(float2 *x, float2 *y, const float2
   }
 }
 
-// The fused row kernel for N = 3 * 2^b (see k_fft_products_m for the data
+// The fused row kernel for N = 3 * 2^b (see k_fft_products_g for the data
 // flow).  Staging rows are padded to an odd stride so the transposes between
 // the (m, element) order of HBM and the (element, m) order of the FFT rows
 // are free of bank conflicts.
@@ -947,7 +735,7 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
 // ---------------------------------------------------------------------------
 // The float64 four-step products kernel (the plain path's step): the data
 // flow of k_fft_products_4s on the float64 Fourier rows, with the pair
-// scaling of k_fft_products_g64 (the second row of each pair, inputs and
+// scaling of k_fft_products_g (the second row of each pair, inputs and
 // products, brought to the size of the first), so every row keeps float64
 // precision whatever the sizes of the fields.  One CTA per (theta, k), 384
 // threads, one CTA per SM (166 KB of shared memory at M = 256).
@@ -1430,137 +1218,229 @@ k_fft_products_4s64r(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// The general float64 products kernel, any N = 2^a 3^b (the grids that are not
-// nphi = 3 (L + 1) with L + 1 = 32 .. 256): Stockham passes of radix 16 and 9
-// while they divide, then 8, 4, 2 or 3, each butterfly a register DFT, the
-// index divisions by multiplication; rows in shared memory padded as in
-// k_fft_products_t.  Radix 4, 3 and 2 passes with run-time radices and
-// divisions took 1056 us at nphi = 256 / L85 / Nr65 (8320 rows).
-struct G64Stage {
-  int R, nb, Ns, tstride;   // radix, butterflies a row, product of the radices before, N / (Ns R)
-  FastDiv dnb, dNs;
+// The general products kernel, either precision and any N = 2^a 3^b (the grids
+// that are not nphi = 3 (L + 1) with L + 1 = 32 .. 256).  Stockham stages of
+// radix 3, 4 and 2 over the seven (six) rows of a (theta, k), two stages a pass
+// through shared memory: the R2 butterflies of the first stage whose outputs a
+// second-stage butterfly reads are R2 rows of a thread's registers, so fusing
+// changes no operation and no result.  Index divisions are multiplications,
+// rows carry one pad element per 16, the input comes by cp.async, and the
+// scaling of the product rows is applied where the first forward pass reads
+// them.  Bound by latency: a few hundred butterflies a pass and barrier.  With
+// a stage a pass, run-time radices and divisions -> now: float64 nphi = 256 /
+// L85 / Nr65 (8320 rows) 1056 -> 334 us; single 614 -> 194 us there, 2600 ->
+// 1107 us at nphi = 576 / L191 / Nr65 (18720 rows), 252 -> 76 us at nphi = 216 /
+// L63 / Nr33.
+struct GStage {
+  int R1, R2, Ns;           // radices of the two stages (R2 = 1: one stage), product of the radices before
+  int n12, nb1, ts1, ts2;   // N / (R1 R2), N / R1, N / (Ns R1), N / (Ns R1 R2)
+  FastDiv d12, dNs;
 };
-struct G64Plan {
-  int n, np, nst;           // points, padded row length, stages
+struct GPlan {
+  int n, np, nst;           // points, padded row length, passes
   int psh;                  // index i lies at i + (i >> psh)
   int mp;                   // pitch of a staging row of L + 1 orders
-  G64Stage st[12];
+  GStage st[12];
   __device__ __forceinline__ int pad(int i) const { return i + (i >> psh); }
 };
 
-static size_t g64_bytes(int np) { return 14 * (size_t)np * sizeof(double2) + 32 * sizeof(double); }
+template <typename T>
+static size_t gplan_bytes(int np) { return 14 * (size_t)np * 2 * sizeof(T) + 32 * sizeof(double); }
 
-static G64Plan make_plan64(int n, int L) {
-  G64Plan p{};
+template <typename T>
+static GPlan make_gplan(int n, int L) {
+  GPlan p{};
   p.n = n;
-  // the largest grids fit without the padding only, the smallest with an even
-  // staging pitch only
-  p.psh = g64_bytes(n + n / 16 + 1) <= 227 * 1024 ? 4 : 31;
+  // the largest float64 grids fit without the padding only, the smallest grids
+  // with an even staging pitch only
+  p.psh = gplan_bytes<T>(n + n / 16 + 1) <= 227 * 1024 ? 4 : 31;
   p.np = p.psh == 4 ? n + n / 16 + 1 : n;
-  p.mp = 26 * (size_t)((L + 1) | 1) * sizeof(double) <= 7 * (size_t)p.np * sizeof(double2) ? (L + 1) | 1 : L + 1;
-  int m = n, Ns = 1;
-  auto add = [&](int R) {
-    p.st[p.nst++] = G64Stage{R, n / R, Ns, n / (Ns * R), FastDiv(n / R), FastDiv(Ns)};
-    Ns *= R;
-    m /= R;
-  };
-  while (m % 16 == 0) add(16);
-  for (int R : {8, 4, 2})
-    if (m % R == 0) add(R);
-  while (m % 9 == 0) add(9);
-  while (m % 3 == 0) add(3);
+  p.mp = 13 * ((L + 1) | 1) <= 7 * p.np ? (L + 1) | 1 : L + 1;
+  int rad[24], nr = 0, m = n, Ns = 1;
+  while (m % 3 == 0) { rad[nr++] = 3; m /= 3; }
+  while (m % 4 == 0) { rad[nr++] = 4; m /= 4; }
+  if (m % 2 == 0) rad[nr++] = 2;
+  for (int i = 0; i < nr; i += 2) {
+    const int R1 = rad[i], R2 = (i + 1 < nr) ? rad[i + 1] : 1;
+    p.st[p.nst++] = GStage{R1, R2, Ns, n / (R1 * R2), n / R1, n / (Ns * R1), n / (Ns * R1 * R2), FastDiv(n / (R1 * R2)),
+                           FastDiv(Ns)};
+    Ns *= R1 * R2;
+  }
   return p;
 }
 
-// mx (first pass of the forward transform): maxima of the rows, the second
-// row of each pair scaled to the first on the way in
-template <int R, int SIGN>
-__device__ __forceinline__ void g64_pass(const double2 *x, double2 *y, int nf, const G64Plan &pl, const G64Stage &st,
-                                         const double2 *__restrict__ tw, const unsigned *mx) {
-  const int np = pl.np;
-  for (int idx = threadIdx.x; idx < nf * st.nb; idx += blockDim.x) {
-    const int f = st.dnb.div(idx), j = idx - f * st.nb, q = st.dNs.div(j), k = j - q * st.Ns;
-    const double2 *xf = x + f * np;
-    const double sy = (SIGN < 0 && mx) ? PairBits<double>::factor(mx[2 * f], mx[2 * f + 1], false) : 1.0;
-    double2 v[R];
+// Products and sums of two products, in single precision with the rounding
+// written out: the results do not depend on how the compiler contracts them
+// where the passes are inlined (they are those of one stage a pass, bit for bit).
+__device__ __forceinline__ float2 gmul(float2 a, float2 b) {
+  return float2{__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y))};
+}
+__device__ __forceinline__ double2 gmul(double2 a, double2 b) { return cmul(a, b); }
+__device__ __forceinline__ float gdet(float a, float b, float c, float d) {   // a b - c d
+  return __fmaf_rn(a, b, -__fmul_rn(c, d));
+}
+__device__ __forceinline__ double gdet(double a, double b, double c, double d) { return a * b - c * d; }
+__device__ __forceinline__ float gfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double gfma(double a, double b, double c) { return fma(a, b, c); }
+
+// butterfly of R points, natural order in and out
+template <int R, int SIGN, typename T2>
+__device__ __forceinline__ void gbf(T2 (&v)[R]) {
+  using T = typename ScalarOf<T2>::t;
+  T2 o[R];
+  if constexpr (R == 4) {
+    T2 a0, a1, a2, a3;
+    a0.x = v[0].x + v[2].x; a0.y = v[0].y + v[2].y;
+    a1.x = v[0].x - v[2].x; a1.y = v[0].y - v[2].y;
+    a2.x = v[1].x + v[3].x; a2.y = v[1].y + v[3].y;
+    T dx = v[1].x - v[3].x, dy = v[1].y - v[3].y;
+    if (SIGN < 0) { a3.x = dy; a3.y = -dx; } else { a3.x = -dy; a3.y = dx; }
+    o[0].x = a0.x + a2.x; o[0].y = a0.y + a2.y;
+    o[1].x = a1.x + a3.x; o[1].y = a1.y + a3.y;
+    o[2].x = a0.x - a2.x; o[2].y = a0.y - a2.y;
+    o[3].x = a1.x - a3.x; o[3].y = a1.y - a3.y;
+  } else if constexpr (R == 2) {
+    o[0].x = v[0].x + v[1].x; o[0].y = v[0].y + v[1].y;
+    o[1].x = v[0].x - v[1].x; o[1].y = v[0].y - v[1].y;
+  } else if constexpr (R == 3) {
+    const T s32 = (T)(0.5 * sqrt(3.0));
+    T2 t1, t2;
+    t1.x = v[1].x + v[2].x; t1.y = v[1].y + v[2].y;
+    t2.x = v[0].x - (T)0.5 * t1.x; t2.y = v[0].y - (T)0.5 * t1.y;
+    const T dx = v[1].x - v[2].x, dy = v[1].y - v[2].y, sx = SIGN < 0 ? s32 : -s32;
+    o[0].x = v[0].x + t1.x; o[0].y = v[0].y + t1.y;
+    o[1].x = gfma(sx, dy, t2.x); o[1].y = gfma(-sx, dx, t2.y);
+    o[2].x = gfma(-sx, dy, t2.x); o[2].y = gfma(sx, dx, t2.y);
+  } else {
+    o[0] = v[0];
+  }
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      v[r] = xf[pl.pad(j + r * st.nb)];
-      if (SIGN < 0 && mx) v[r].y *= sy;
-      if (r > 0 && k > 0) {
-        double2 w = __ldg(tw + r * k * st.tstride);
-        if (SIGN > 0) w.y = -w.y;
-        v[r] = cmulf(v[r], w);
-      }
+  for (int r = 0; r < R; r++) v[r] = o[r];
+}
+
+// one pass.  The butterflies j0 + r' n12 (r' < R2) of the first stage have one
+// k = j0 mod Ns and feed the second stage's butterflies k + r Ns (r < R1) of
+// the same block.  mx (first pass of the forward transform): maxima of the
+// rows, the second row of each pair scaled to the first on the way in.
+template <int R1, int R2, int SIGN, typename T2>
+__device__ __forceinline__ void g_pass(const T2 *x, T2 *y, int nf, const GPlan &pl, const GStage &st,
+                                       const T2 *__restrict__ tw, const unsigned *mx) {
+  using T = typename ScalarOf<T2>::t;
+  const int Ns = st.Ns;
+  for (int idx = threadIdx.x; idx < nf * st.n12; idx += blockDim.x) {
+    const int f = st.d12.div(idx), j0 = idx - f * st.n12, J = st.dNs.div(j0), k = j0 - J * Ns;
+    const T2 *xf = x + f * pl.np;
+    T2 v[R2][R1], w[R1];
+#pragma unroll
+    for (int r = 1; r < R1; r++) {
+      w[r] = __ldg(tw + r * k * st.ts1);
+      if (SIGN > 0) w[r].y = -w[r].y;
     }
-    dftr<R, SIGN>(v);
-    double2 *yf = y + f * np;
-    const int d = q * st.Ns * R + k;
+    T sy = (T)1;
+    if (SIGN < 0 && mx) sy = PairBits<T>::factor(mx[2 * f], mx[2 * f + 1], false);
 #pragma unroll
-    for (int r = 0; r < R; r++) yf[pl.pad(d + r * st.Ns)] = v[r];
+    for (int q = 0; q < R2; q++) {
+#pragma unroll
+      for (int r = 0; r < R1; r++) {
+        T2 a = xf[pl.pad(j0 + q * st.n12 + r * st.nb1)];
+        if (SIGN < 0 && mx) a.y *= sy;
+        if (r > 0 && k > 0) a = gmul(a, w[r]);
+        v[q][r] = a;
+      }
+      gbf<R1, SIGN>(v[q]);
+    }
+    T2 *yf = y + f * pl.np;
+    const int d = J * Ns * (R1 * R2);
+#pragma unroll
+    for (int r = 0; r < R1; r++) {
+      const int kk = k + r * Ns;
+      T2 u[R2];
+#pragma unroll
+      for (int q = 0; q < R2; q++) {
+        T2 a = v[q][r];
+        if (q > 0 && kk > 0) {
+          T2 z = __ldg(tw + q * kk * st.ts2);
+          if (SIGN > 0) z.y = -z.y;
+          a = gmul(a, z);
+        }
+        u[q] = a;
+      }
+      gbf<R2, SIGN>(u);
+#pragma unroll
+      for (int q = 0; q < R2; q++) yf[pl.pad(d + kk + q * Ns * R1)] = u[q];
+    }
   }
   __syncthreads();
 }
 
-template <int SIGN>
-__device__ __forceinline__ double2 *g64_fft(double2 *x, double2 *y, int nf, const G64Plan &pl,
-                                            const double2 *__restrict__ tw, const unsigned *mx = nullptr) {
+template <int SIGN, typename T2>
+__device__ __forceinline__ T2 *g_fft(T2 *x, T2 *y, int nf, const GPlan &pl, const T2 *__restrict__ tw,
+                                     const unsigned *mx = nullptr) {
   for (int s = 0; s < pl.nst; s++) {
-    const G64Stage &st = pl.st[s];
+    const GStage &st = pl.st[s];
     const unsigned *m0 = (s == 0) ? mx : nullptr;
-    switch (st.R) {
-      case 16: g64_pass<16, SIGN>(x, y, nf, pl, st, tw, m0); break;
-      case 9: g64_pass<9, SIGN>(x, y, nf, pl, st, tw, m0); break;
-      case 8: g64_pass<8, SIGN>(x, y, nf, pl, st, tw, m0); break;
-      case 4: g64_pass<4, SIGN>(x, y, nf, pl, st, tw, m0); break;
-      case 3: g64_pass<3, SIGN>(x, y, nf, pl, st, tw, m0); break;
-      default: g64_pass<2, SIGN>(x, y, nf, pl, st, tw, m0); break;
+    switch (st.R1 * 8 + st.R2) {
+      case 3 * 8 + 3: g_pass<3, 3, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 3 * 8 + 4: g_pass<3, 4, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 3 * 8 + 2: g_pass<3, 2, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 3 * 8 + 1: g_pass<3, 1, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 4 * 8 + 4: g_pass<4, 4, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 4 * 8 + 2: g_pass<4, 2, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      case 4 * 8 + 1: g_pass<4, 1, SIGN>(x, y, nf, pl, st, tw, m0); break;
+      default: g_pass<2, 1, SIGN>(x, y, nf, pl, st, tw, m0); break;
     }
-    double2 *t = x; x = y; y = t;
+    T2 *t = x; x = y; y = t;
   }
   return x;
 }
 
+template <typename T>
 __global__ void __launch_bounds__(512)
-k_fft_products_g64(const __grid_constant__ G64Plan pl, int L, MLayout64 fin, MLayout64 fout,
-                   const double2 *__restrict__ tw, ProdCoef pc) {
-  using PB = PairBits<double>;
-  using U = PB::U;
+k_fft_products_g(const __grid_constant__ GPlan pl, int L, MLayoutT<T> fin, MLayoutT<T> fout,
+                 const typename C2<T>::t *__restrict__ tw, ProdCoef pc) {
+  using T2 = typename C2<T>::t;
+  using PB = PairBits<T>;
+  using U = unsigned;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int N = pl.n, NP = pl.np, MP = pl.mp;
-  double2 *A = reinterpret_cast<double2 *>(smraw);   // 7 rows
-  double2 *B = A + 7 * NP;                            // 7 rows; first the input, last the output staging
-  U *cmx = reinterpret_cast<U *>(B + 7 * NP);         // [0, 13) input maxima, [13, 25) products
-  double *S = reinterpret_cast<double *>(B);          // [c * 2 + s][MP]
+  T2 *A = reinterpret_cast<T2 *>(smraw);      // 7 rows
+  T2 *B = A + 7 * NP;                          // 7 rows; first the input, last the output staging
+  U *cmx = reinterpret_cast<U *>(B + 7 * NP);  // [0, 13) input maxima, [13, 25) products
+  T2 *S = B;                                   // [c][MP] (a_m, b_m)
   const int th = blockIdx.x / fin.nr, k = blockIdx.x % fin.nr;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
   if (tid < 12) cmx[13 + tid] = 0;
-  // input: one warp per order, lane j < 26 element j of the 10 + 16 run
+  // input: an order's 13 (cos, sin) pairs, a run of 5 in the P block and one of
+  // 8 in the D block; half-warp h of warp w copies the orders 2 (w + nwarp i) + h
   {
-    int cs = 0;
-    if (lane < 26) { int c, sg; m_comp_of_in(lane, c, sg); cs = c * 2 + sg; }
-    const double *src = (lane < 10) ? fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + lane
-                                    : fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + (lane - 10);
-    const size_t mst = (size_t)fin.nth * ((lane < 10) ? fin.sP() : fin.sD());
-    if (lane < 26) {
-      int m = warp;
-      for (; m + 3 * nwarp <= L; m += 4 * nwarp) {
-        double v[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) v[u] = __ldg(src + (size_t)(m + u * nwarp) * mst);
-#pragma unroll
-        for (int u = 0; u < 4; u++) S[cs * MP + m + u * nwarp] = v[u];
-      }
-      for (; m <= L; m += nwarp) S[cs * MP + m] = __ldg(src + (size_t)m * mst);
+    const int j = lane & 15, hw = lane >> 4;
+    int c = 0;
+    const T *src = fin.P;
+    size_t mst = 0;
+    if (j < 5) {
+      c = (j < 4) ? 3 * j : 12;
+      src = fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + 2 * j;
+      mst = (size_t)fin.nth * fin.sP();
+    } else if (j < 13) {
+      const int jd = j - 5;
+      c = 3 * (jd >> 1) + 1 + (jd & 1);
+      src = fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + 2 * jd;
+      mst = (size_t)fin.nth * fin.sD();
     }
+    if (j < 13)
+      for (int m = 2 * warp + hw; m <= L; m += 2 * nwarp)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(S + c * MP + m)),
+                     "l"(src + m * mst), "n"(sizeof(T2))
+                     : "memory");
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   }
   __syncthreads();
   // pair scaling (pair_exp): the largest coefficient of each component
   for (int c = warp; c < 13; c += nwarp) {
     U mx = 0;
     for (int m = lane; m <= L; m += 32) {
-      mx = max(mx, PB::abs_bits(S[(2 * c) * MP + m]));
-      if (m > 0) mx = max(mx, PB::abs_bits(S[(2 * c + 1) * MP + m]));
+      const T2 v = S[c * MP + m];
+      mx = max(mx, max(PB::abs_bits(v.x), PB::abs_bits(v.y)));
     }
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) cmx[c] = mx;
@@ -1570,25 +1450,28 @@ k_fft_products_g64(const __grid_constant__ G64Plan pl, int L, MLayout64 fin, MLa
   const int mmax = min(L, (N + 1) / 2 - 1);
   for (int p = 0; p < 7; p++) {
     const bool has1 = p < 6;
-    const double sy = has1 ? PB::factor(cmx[2 * p], cmx[2 * p + 1], false) : 0.0;
-    const double *a0 = S + (size_t)(4 * p) * MP, *b0 = a0 + MP, *a1 = has1 ? b0 + MP : a0, *b1 = has1 ? a1 + MP : a0;
-    double2 *Z = A + p * NP;
+    const T sy = has1 ? PB::factor(cmx[2 * p], cmx[2 * p + 1], false) : (T)1;
+    const T2 *x0 = S + (2 * p) * MP, *y0 = has1 ? x0 + MP : x0;
+    T2 *Z = A + p * NP;
     for (int m = tid; m <= mmax; m += blockDim.x) {
+      const T2 ab = x0[m], cd = y0[m];
+      const T a1 = has1 ? cd.x * sy : (T)0, b1 = has1 ? cd.y * sy : (T)0;
       if (m == 0) {
-        Z[0] = double2{a0[0], a1[0] * sy};
+        Z[0] = T2{ab.x, a1};
       } else {
-        const double xr = 0.5 * a0[m], xi = -0.5 * b0[m], yr = 0.5 * (a1[m] * sy), yi = -0.5 * (b1[m] * sy);
-        Z[pl.pad(m)] = double2{xr - yi, xi + yr};
-        Z[pl.pad(N - m)] = double2{xr + yi, -xi + yr};
+        const T xr = (T)0.5 * ab.x, xi = (T)-0.5 * ab.y, yr = (T)0.5 * a1, yi = (T)-0.5 * b1;
+        Z[pl.pad(m)] = T2{xr - yi, xi + yr};
+        Z[pl.pad(N - m)] = T2{xr + yi, -xi + yr};
       }
     }
-    for (int n = mmax + 1 + tid; n < N - mmax; n += blockDim.x) Z[pl.pad(n)] = double2{0.0, 0.0};
+    for (int n = mmax + 1 + tid; n < N - mmax; n += blockDim.x) Z[pl.pad(n)] = T2{0, 0};
   }
   __syncthreads();
-  double2 *g = g64_fft<+1>(A, B, 7, pl, tw);
-  double2 *h = (g == A) ? B : A;
+  T2 *g = g_fft<+1>(A, B, 7, pl, tw);
+  T2 *h = (g == A) ? B : A;
   {
-    double iy[6];
+    const T cv = (T)pc.cv, cl = (T)pc.cl, ci = (T)pc.ci, ct = (T)pc.ct;
+    T iy[6];
 #pragma unroll
     for (int p = 0; p < 6; p++) iy[p] = PB::factor(cmx[2 * p], cmx[2 * p + 1], true);
     U hm[12];
@@ -1596,17 +1479,16 @@ k_fft_products_g64(const __grid_constant__ G64Plan pl, int L, MLayout64 fin, MLa
     for (int c = 0; c < 12; c++) hm[c] = 0;
     for (int qq = tid; qq < N; qq += blockDim.x) {
       const int q = pl.pad(qq);
-      const double2 p0 = g[0 * NP + q], p1 = g[1 * NP + q], p2 = g[2 * NP + q], p3 = g[3 * NP + q];
-      const double2 p4 = g[4 * NP + q], p5 = g[5 * NP + q], p6 = g[6 * NP + q];
-      const double ur = p0.x, ut = p0.y * iy[0], up = p1.x, wr = p1.y * iy[1], wt = p2.x, wp = p2.y * iy[2];
-      const double br = p3.x, bt = p3.y * iy[3], bp = p4.x, jr = p4.y * iy[4], jt = p5.x, jp = p5.y * iy[5];
-      const double tt = p6.x, cv = pc.cv, cl = pc.cl, ci = pc.ci, ct = pc.ct;
-      const double2 hv[6] = {double2{(wt * up - wp * ut) * cv, (wp * ur - wr * up) * cv},
-                             double2{(wr * ut - wt * ur) * cv, (jt * bp - jp * bt) * cl},
-                             double2{(jp * br - jr * bp) * cl, (jr * bt - jt * br) * cl},
-                             double2{(ut * bp - up * bt) * ci, (up * br - ur * bp) * ci},
-                             double2{(ur * bt - ut * br) * ci, ur * tt * ct},
-                             double2{ut * tt * ct, up * tt * ct}};
+      const T2 p0 = g[0 * NP + q], p1 = g[1 * NP + q], p2 = g[2 * NP + q], p3 = g[3 * NP + q];
+      const T2 p4 = g[4 * NP + q], p5 = g[5 * NP + q], p6 = g[6 * NP + q];
+      const T ur = p0.x, ut = p0.y * iy[0], up = p1.x, wr = p1.y * iy[1], wt = p2.x, wp = p2.y * iy[2];
+      const T br = p3.x, bt = p3.y * iy[3], bp = p4.x, jr = p4.y * iy[4], jt = p5.x, jp = p5.y * iy[5], tt = p6.x;
+      const T2 hv[6] = {T2{gdet(wt, up, wp, ut) * cv, gdet(wp, ur, wr, up) * cv},
+                        T2{gdet(wr, ut, wt, ur) * cv, gdet(jt, bp, jp, bt) * cl},
+                        T2{gdet(jp, br, jr, bp) * cl, gdet(jr, bt, jt, br) * cl},
+                        T2{gdet(ut, bp, up, bt) * ci, gdet(up, br, ur, bp) * ci},
+                        T2{gdet(ur, bt, ut, br) * ci, ur * tt * ct},
+                        T2{ut * tt * ct, up * tt * ct}};
 #pragma unroll
       for (int p = 0; p < 6; p++) {
         h[p * NP + q] = hv[p];
@@ -1621,32 +1503,43 @@ k_fft_products_g64(const __grid_constant__ G64Plan pl, int L, MLayout64 fin, MLa
     }
   }
   __syncthreads();
-  const double2 *zf = g64_fft<-1>(h, g, 6, pl, tw, cmx + 13);
-  double *O = reinterpret_cast<double *>((zf == A) ? B : A);   // [c * 2 + s][MP]
-  const double an = 1.0 / (double)N;
+  const T2 *zf = g_fft<-1>(h, g, 6, pl, tw, cmx + 13);
+  T2 *O = (zf == A) ? B : A;   // [c][MP] (a_m, b_m)
+  const T an = (T)(1.0 / (double)N);
   for (int p = 0; p < 6; p++) {
-    const double2 *Z = zf + p * NP;
-    double *o0 = O + (size_t)(4 * p) * MP, *o1 = o0 + 2 * MP;
-    const double ay = an * PB::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], true);
+    const T2 *Z = zf + p * NP;
+    T2 *o0 = O + (2 * p) * MP, *o1 = o0 + MP;
+    const T ay = an * PB::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], true);
     for (int m = tid; m <= L; m += blockDim.x) {
       if (m == 0) {
-        o0[0] = an * Z[0].x; o0[MP] = 0.0; o1[0] = ay * Z[0].y; o1[MP] = 0.0;
+        o0[0] = T2{an * Z[0].x, (T)0};
+        o1[0] = T2{ay * Z[0].y, (T)0};
       } else {
-        const double2 zk = Z[pl.pad(m % N)], zn = Z[pl.pad((N - m) % N)];
-        o0[m] = an * (zk.x + zn.x); o0[MP + m] = -an * (zk.y - zn.y);
-        o1[m] = ay * (zk.y + zn.y); o1[MP + m] = ay * (zk.x - zn.x);
+        const T2 zk = Z[pl.pad(m % N)], zn = Z[pl.pad((N - m) % N)];
+        o0[m] = T2{an * (zk.x + zn.x), -an * (zk.y - zn.y)};
+        o1[m] = T2{ay * (zk.y + zn.y), ay * (zk.x - zn.x)};
       }
     }
   }
   __syncthreads();
+  // output: 12 pairs an order, a run of 4 in the P block and one of 8 in the D block
   {
-    int cs = 0;
-    if (lane < 24) { int c, sg; m_comp_of_out(lane, c, sg); cs = c * 2 + sg; }
-    double *dst = (lane < 8) ? fout.P + (size_t)th * fout.sP() + (size_t)k * 8 + lane
-                             : fout.D + (size_t)th * fout.sD() + (size_t)k * 16 + (lane - 8);
-    const size_t mst = (size_t)fout.nth * ((lane < 8) ? fout.sP() : fout.sD());
-    if (lane < 24)
-      for (int m = warp; m <= L; m += nwarp) dst[(size_t)m * mst] = O[cs * MP + m];
+    const int j = lane & 15, hw = lane >> 4;
+    int c = 0;
+    T *dst = fout.P;
+    size_t mst = 0;
+    if (j < 4) {
+      c = 3 * j;
+      dst = fout.P + (size_t)th * fout.sP() + (size_t)k * 8 + 2 * j;
+      mst = (size_t)fout.nth * fout.sP();
+    } else if (j < 12) {
+      const int jd = j - 4;
+      c = 3 * (jd >> 1) + 1 + (jd & 1);
+      dst = fout.D + (size_t)th * fout.sD() + (size_t)k * 16 + 2 * jd;
+      mst = (size_t)fout.nth * fout.sD();
+    }
+    if (j < 12)
+      for (int m = 2 * warp + hw; m <= L; m += 2 * nwarp) *reinterpret_cast<T2 *>(dst + m * mst) = O[c * MP + m];
   }
 }
 
@@ -1865,8 +1758,8 @@ int fft_setup(Ctx &c) {
     set_error("ngrid_zonal_ctl too large for the fused FFT kernel");
     return CB2_ERR_ARG;
   }
-  if (c.prec == CB2_PREC_FP64) CB2_CUDA(raise_smem_limit(k_fft_products_g64, g64_bytes(make_plan64(c.nph, c.L).np)));
-  CB2_CUDA(raise_smem_limit(k_fft_products_m, (int)(14 * (size_t)c.nph * sizeof(float2) + 32 * sizeof(float))));
+  if (c.prec == CB2_PREC_FP64) CB2_CUDA(raise_smem_limit(k_fft_products_g<double>, gplan_bytes<double>(make_gplan<double>(c.nph, c.L).np)));
+  else CB2_CUDA(raise_smem_limit(k_fft_products_g<float>, gplan_bytes<float>(make_gplan<float>(c.nph, c.L).np)));
   {
     int rc = 0;
     switch (c.nph) {
@@ -1909,6 +1802,15 @@ static const typename C2<T>::t *twid(Ctx &c) {
   return (const typename C2<T>::t *)c.d_tw_fft32;
 }
 
+template <typename T>
+static void launch_fft_g(Ctx &c, const MLayoutT<T> &in, const MLayoutT<T> &out, const ProdCoef &pc) {
+  const GPlan pl = make_gplan<T>(c.nph, c.L);
+  // about a thread per pair-stage butterfly of the seven rows
+  const int threads = std::min(512, std::max(96, 32 * cdiv(7 * c.nph, 16 * 32)));
+  k_fft_products_g<T><<<(unsigned)(c.nth * c.nr), threads, gplan_bytes<T>(pl.np), c.stream>>>(pl, c.L, in, out,
+                                                                                               twid<T>(c), pc);
+}
+
 template <int R1, int R2>
 static void launch_fft_4s64(Ctx &c, const MLayout64 &in, const MLayout64 &out, const ProdCoef &pc) {
   if constexpr (R2 == 16)
@@ -1930,11 +1832,7 @@ void fft_products64(Ctx &c, const MLayout64 &in, const MLayout64 &out) {
       default: break;
     }
   }
-  // about a thread per radix-16 butterfly of the seven rows
-  const int threads = std::min(512, std::max(96, 32 * cdiv(7 * c.nph, 16 * 32)));
-  const G64Plan pl = make_plan64(c.nph, c.L);
-  k_fft_products_g64<<<(unsigned)(c.nth * c.nr), threads, g64_bytes(pl.np), c.stream>>>(
-      pl, c.L, in, out, (const double2 *)c.d_tw_fft, pc);
+  launch_fft_g<double>(c, in, out, pc);
 }
 
 template <typename T>
@@ -1984,10 +1882,7 @@ bool fft_products_m(Ctx &c, const MLayout &in, const MLayout &out, float *pmax) 
     case 96: launch_fft_t<96>(c, in, out, pc); return false;
     default: break;
   }
-  FFTPlan p = make_plan(c.nph);
-  size_t sm = 14 * (size_t)c.nph * sizeof(float2) + 32 * sizeof(float);
-  k_fft_products_m<<<(unsigned)(c.nth * c.nr), 512, sm, c.stream>>>(p, c.L, in, out, (const float2 *)c.d_tw_fft32,
-                                                                   pc);
+  launch_fft_g<float>(c, in, out, pc);
   return false;
 }
 

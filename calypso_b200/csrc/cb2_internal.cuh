@@ -214,7 +214,7 @@ using MLayout64 = MLayoutT<double>;
 struct FastDiv {
   unsigned n = 1, mul = 0;
   FastDiv() = default;
-  explicit FastDiv(int d) : n((unsigned)d), mul((unsigned)((0x100000000ull + d - 1) / d)) {}
+  __host__ __device__ explicit FastDiv(int d) : n((unsigned)d), mul((unsigned)((0x100000000ull + d - 1) / d)) {}
   __device__ __forceinline__ int div(int e) const { return n == 1 ? e : (int)__umulhi((unsigned)e, mul); }
 };
 
