@@ -164,6 +164,7 @@ constexpr int FAB = 2;   // A/B stages
 // overlap the main loop of the next; with one set, the tiles narrow enough
 // for half of tensor memory alternate between the halves (AccSched).
 constexpr int FW_CONV = 256, FW_EPI = 256, FW_THREADS = FW_CONV + FW_EPI + 64;
+constexpr int FW_CV = FKB * TM / FW_CONV;   // K values a converter thread and block
 constexpr int FW_PROD_WARP = (FW_CONV + FW_EPI) / 32, FW_MMA_WARP = FW_PROD_WARP + 1;
 
 // epilogue staging of one warp: 16 rows x 16 degrees (+1 pad) floats, then
@@ -503,6 +504,9 @@ k_leg_fwd_ws(const __grid_constant__ FwdShell one, const FwdShell *__restrict__ 
       const float sc = fwd_row_scale(a, q, row);
       // Gauss weight of node i: staged in shared memory for one shell
       auto wt = [&](int i) { return MULTI ? __ldg(a.wgt + i) : w[i]; };
+      auto wt4 = [&](int i) {
+        return MULTI ? __ldg(reinterpret_cast<const float4 *>(a.wgt + i)) : *reinterpret_cast<const float4 *>(w + i);
+      };
       for (int b = 0; b < q.NB; b++) {
         const int tb = q.g ? (b >> 1) : b, part = q.g ? (b & 1) : 0;
         const uint32_t rs = nraw % FRS, s = nab % FAB;
@@ -521,14 +525,33 @@ k_leg_fwd_ws(const __grid_constant__ FwdShell one, const FwdShell *__restrict__ 
           if (part == 0) { sg = (q4 < 2) ? sc : -sc; swap = true; }
           else { src = r - q4 + 3 - q4; sg = (q4 & 1) ? sc : -sc; }
         }
-        float x2[2][16];
+        // the weights of this thread's nodes and their mirrors, 16 bytes a load
+        // (nth is a multiple of 8): one at a time they were half of the
+        // converters' shared-memory reads
+        float ws[FW_CV], wn[FW_CV];
+        const int i0 = tb * FKB + h * FW_CV;
+        if (i0 < a.nh && i0 + FW_CV <= a.nth) {
 #pragma unroll
-        for (int e = 0; e < 16; e++) {
-          const int kk = h * 16 + e, i = tb * FKB + kk;
+          for (int e = 0; e < FW_CV; e += 4) {
+            const float4 u = wt4(i0 + e), v = wt4(a.nth - 4 - i0 - e);
+            ws[e] = u.x; ws[e + 1] = u.y; ws[e + 2] = u.z; ws[e + 3] = u.w;
+            wn[e] = v.w; wn[e + 1] = v.z; wn[e + 2] = v.y; wn[e + 3] = v.x;
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < FW_CV; e++) {
+            ws[e] = (i0 + e < a.nh) ? wt(i0 + e) : 0.0f;
+            wn[e] = (i0 + e < a.nh) ? wt(a.nth - 1 - i0 - e) : 0.0f;
+          }
+        }
+        float x2[2][FW_CV];
+#pragma unroll
+        for (int e = 0; e < FW_CV; e++) {
+          const int kk = h * FW_CV + e, i = tb * FKB + kk;
           float vs = 0.0f, va = 0.0f;
           if (i < a.nh) {
-            const float fa = rs_s[kk * TM + src] * wt(i);
-            const float fb = rs_n[(FKB - 1 - kk) * TM + src] * wt(a.nth - 1 - i);
+            const float fa = rs_s[kk * TM + src] * ws[e];
+            const float fb = rs_n[(FKB - 1 - kk) * TM + src] * wn[e];
             vs = (fa + fb) * sg;
             va = (fa - fb) * sg;
           }
@@ -540,14 +563,14 @@ k_leg_fwd_ws(const __grid_constant__ FwdShell one, const FwdShell *__restrict__ 
         for (int p = 0; p < 2; p++) {
           unsigned char *ahi = at + (2 * p) * FA_BYTES, *alo = ahi + FA_BYTES;
 #pragma unroll
-          for (int c = 0; c < 2; c++) {
+          for (int c = 0; c < FW_CV / 8; c++) {
             uint32_t hh[4], ll[4];
 #pragma unroll
             for (int e = 0; e < 8; e += 2) {
               if (split) split_pair_q(x2[p][c * 8 + e], x2[p][c * 8 + e + 1], hh[e >> 1], ll[e >> 1]);
               else split_pair(x2[p][c * 8 + e], x2[p][c * 8 + e + 1], hh[e >> 1], ll[e >> 1]);
             }
-            const uint32_t off = sw64_chunk(r, 2 * h + c);
+            const uint32_t off = sw64_chunk(r, (FW_CV / 8) * h + c);
             *reinterpret_cast<uint4 *>(ahi + off) = make_uint4(hh[0], hh[1], hh[2], hh[3]);
             *reinterpret_cast<uint4 *>(alo + off) = make_uint4(ll[0], ll[1], ll[2], ll[3]);
           }
@@ -840,10 +863,11 @@ struct BwdShell {
 // at TMEM column p nhp; two sets (epilogue of one tile overlapping the main
 // loop of the next) when 4 nhp columns fit, else one.
 constexpr int BW_ST = 3;
-// roles: converters warps 0-7, epilogue warps 8-15 (two per TMEM lane
-// quarter, one per half of the colatitude columns), producer 16, MMA 17
-constexpr int BW_CONV = 256, BW_EPI = 256, BW_THREADS = 576;
-constexpr int BW_PROD_WARP = 16, BW_MMA_WARP = 17;
+// roles: converters warps 0-7, epilogue warps 8-23 (four per TMEM lane
+// quarter, one per quarter of the colatitude columns), producer 24, MMA 25
+constexpr int BW_CONV = 256, BW_EPI = 512, BW_THREADS = BW_CONV + BW_EPI + 64;
+constexpr int BW_PROD_WARP = (BW_CONV + BW_EPI) / 32, BW_MMA_WARP = BW_PROD_WARP + 1;
+constexpr int BW_EC = 16;   // colatitude columns an epilogue thread reads at a time
 
 struct BwdWsBars {
   uint64_t full[BW_ST], afull[BW_ST], empty[BW_ST];
@@ -914,7 +938,7 @@ k_leg_bwd_ws(const __grid_constant__ BwdShell one, const BwdShell *__restrict__ 
   const uint32_t B_BYTES = (uint32_t)nhp_max * FKB * 2;     // one of hi / lo
   const uint32_t ST_BYTES = BRAW_BYTES + 2 * FA_BYTES + 2 * B_BYTES;
   BwdWsBars *sb = reinterpret_cast<BwdWsBars *>(base + BW_ST * ST_BYTES);
-  float *buntab = reinterpret_cast<float *>(base + BW_ST * ST_BYTES + 256);   // [8 epilogue warps][nhp_max]
+  float *buntab = reinterpret_cast<float *>(base + BW_ST * ST_BYTES + 256);   // [epilogue warps][nhp_max]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t accw = tmem_cols / (uint32_t)nacc;         // columns of one accumulator set
   auto shell = [&](int t) -> const BwdShell & { return MULTI ? shell_of(tab, nsh, t) : one; };
@@ -1106,11 +1130,11 @@ k_leg_bwd_ws(const __grid_constant__ BwdShell one, const BwdShell *__restrict__ 
     }
     if (bad) sb->abort = 1;
   } else {
-    // epilogue warps 8-15: TMEM lanes 32 (warp % 4) .. + 31, one row per
-    // thread, warps 8-11 the first half of the 32-column chunks and 12-15
-    // the rest; south (acc0 + acc1) and north (acc0 - acc1) colatitudes,
-    // each store 32 consecutive rows.  Each warp keeps its own copy of the
-    // tile's column unscale (no barrier between the epilogue warps).
+    // epilogue warps 8-23: TMEM lanes 32 (warp % 4) .. + 31, one row per
+    // thread, each group of four warps a quarter of the 16-column chunks;
+    // south (acc0 + acc1) and north (acc0 - acc1) colatitudes, each store 32
+    // consecutive rows.  Each warp keeps its own copy of the tile's column
+    // unscale (no barrier between the epilogue warps).
     // Decisions that guard the warp-collective TMEM loads are warp-uniform.
     const int ew = warp - BW_CONV / 32, er = (ew & 3) * 32 + lane, hc = ew >> 2;
     float *bw = buntab + ew * nhp_max;
@@ -1137,21 +1161,22 @@ k_leg_bwd_ws(const __grid_constant__ BwdShell one, const BwdShell *__restrict__ 
       if (!__all_sync(0xffffffffu, ok)) { sb->abort = 1; break; }
       tc_fence_after();
       const uint32_t tl = tmem + (uint32_t)ab * accw + ((uint32_t)((ew & 3) * 32) << 16);
-      const int nch = (a.nh + 31) / 32, ch = (nch + 1) / 2;
-      const int c0 = hc ? ch : 0, c1 = hc ? nch : ch;
+      const int nch = (a.nh + BW_EC - 1) / BW_EC, ng = BW_EPI / 128;
+      const int c0 = nch * hc / ng, c1 = nch * (hc + 1) / ng;
       if (c0 == c1) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sb->accempty[ab]);
       }
       for (int c = c0; c < c1; c++) {
-        float e[32], o[32];
+        float e[BW_EC], o[BW_EC];
+        const uint32_t col = tl + (uint32_t)(c * BW_EC);
         if (has1) {
-          tmem_ld32x2(tl + (uint32_t)(c * 32), tl + acc1 + (uint32_t)(c * 32), e, o);
+          tmem_ld16x2(col, col + acc1, e, o);
         } else {
-          tmem_ld32x2(tl + (uint32_t)(c * 32), tl + (uint32_t)(c * 32), e, o);
+          tmem_ld16x2(col, col, e, o);
 #pragma unroll
-          for (int u = 0; u < 32; u++) o[u] = 0.0f;
+          for (int u = 0; u < BW_EC; u++) o[u] = 0.0f;
         }
         if (c == c1 - 1) {
           tc_fence_before();
@@ -1160,8 +1185,8 @@ k_leg_bwd_ws(const __grid_constant__ BwdShell one, const BwdShell *__restrict__ 
         }
         if (valid) {
 #pragma unroll
-          for (int u = 0; u < 32; u++) {
-            const int th = c * 32 + u;
+          for (int u = 0; u < BW_EC; u++) {
+            const int th = c * BW_EC + u;
             if (th < a.nh) {
               const float us = ua * bw[th];
               ob[(size_t)th * so] = (e[u] + o[u]) * us;
