@@ -741,7 +741,7 @@ struct PackArgs {
   int L, nr, jmax, nvec, ng, kc;
   int slot[8];
   const int *moff;
-  const double *g3rlm, *ar1, *f;
+  const double *ar1, *f;
   size_t fs;
   float *rlmP, *rlmD;
   int pitchP, pitchD;      // row pitch (floats) of the two blocks
@@ -749,66 +749,89 @@ struct PackArgs {
   float *maxP, *maxD;      // [m][pitch] row maxima
 };
 
+// Bound by HBM once enough loads are in flight: a warp takes PK_U segments of
+// 64 degrees, of whatever rows, at a time.  A warp per row, 256 degrees a pass,
+// left most of its eight loads beyond the truncation at the higher orders and
+// took 406 us at L255 / Nr129 (1.3 GB) and 128 us at L127 / Nr97; segments of
+// 32 degrees took 457 and 113 us (the bookkeeping of a segment).
+constexpr int PK_U = 8, PK_W = 2;   // segments in flight a warp, loads of a segment
+constexpr int PK_ROWS = 4 * 26;  // rows of a block at most (4 radial levels)
+
 __global__ void __launch_bounds__(256)
 k_pack_bwd(const __grid_constant__ PackArgs a) {
   extern __shared__ float T[];   // [kc * RK][NLP]
+  __shared__ long long rsrc[PK_ROWS];   // offset of the row's degree m in the fields, -1: zero
+  __shared__ double rfac[PK_ROWS];
+  __shared__ unsigned rmax[PK_ROWS];
+  __shared__ int rvec[PK_ROWS];         // poloidal part of a vector
   const int m = blockIdx.x, k0 = blockIdx.y * a.kc, nk = min(a.kc, a.nr - k0);
   const int nl = a.L + 1 - m, NLP = nl | 1;
   const int RP = 2 * a.ng, RD = 4 * a.nvec, RK = RP + RD;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int jm = a.moff[m];
-  // rows in: one warp per (radial level, row), lanes along l (coalesced
-  // float64 reads, 256 degrees per pass with all loads in flight together),
-  // the row maximum on the way
-  for (int rl = warp; rl < nk * RK; rl += nw) {
+  const int jm = a.moff[m], nrow = nk * RK;
+  for (int rl = threadIdx.x; rl < nrow; rl += blockDim.x) {
     const int kq = rl / RK, j = rl - kq * RK, k = k0 + kq;
-    const double *src;
-    double rowf;
-    bool vec;
-    int s;
+    int slot, s;
+    double f = a.ar1[k];
     if (j < RP) {
       const int fl = j >> 1;
       s = j & 1;
-      src = a.f + (size_t)a.slot[fl] * a.fs + (size_t)k * a.jmax + jm + s * nl;
-      vec = fl < a.nvec;
-      const double ar = a.ar1[k];
-      rowf = vec ? ar * ar : 1.0;
+      slot = a.slot[fl];
+      f = (fl < a.nvec) ? f * f : 1.0;
     } else {
-      const int jd = j - RP, vv = jd >> 2, comp = (jd & 3) >> 1;
+      const int jd = j - RP;
       s = jd & 1;
-      src = a.f + (size_t)(a.slot[vv] + 1 + comp) * a.fs + (size_t)k * a.jmax + jm + s * nl;
-      vec = false;
-      rowf = a.ar1[k];
+      slot = a.slot[jd >> 2] + 1 + ((jd & 3) >> 1);
     }
-    const bool zero = (m == 0 && s == 1);
-    const double *g3 = a.g3rlm + jm + s * nl;
-    float mx = 0.0f;
-    for (int l0 = 0; l0 < nl; l0 += 256) {
-      double x[8], gg[8];
+    rsrc[rl] = (m == 0 && s == 1) ? -1
+                                  : (long long)slot * (long long)a.fs + (long long)k * a.jmax + jm + s * nl;
+    rfac[rl] = f;
+    rvec[rl] = j < RP && (j >> 1) < a.nvec;
+    rmax[rl] = 0u;
+  }
+  __syncthreads();
+  // rows in: (row, 32 PK_W degrees) items, coalesced float64 reads, l(l+1) for
+  // the poloidal parts, the row maxima on the way
+  const int nseg = (nl + 32 * PK_W - 1) / (32 * PK_W), nitem = nrow * nseg;
+  const FastDiv dseg(nseg);
+  for (int i0 = warp; i0 < nitem; i0 += PK_U * nw) {
+    double x[PK_U][PK_W];
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int lm = l0 + u * 32 + lane;
-        const bool ok = !zero && lm < nl;
-        x[u] = ok ? __ldg(src + lm) : 0.0;
-        gg[u] = (ok && vec) ? __ldg(g3 + lm) : 1.0;
-      }
+    for (int u = 0; u < PK_U; u++) {
+      const int it = i0 + u * nw, rl = dseg.div(it), lm = (it - rl * nseg) * (32 * PK_W) + lane;
+      const long long so = (it < nitem) ? rsrc[rl] : -1;
+      const double *src = a.f + (so >= 0 ? so : 0);
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int lm = l0 + u * 32 + lane;
-        if (lm < nl) {
-          const float v = (float)(vec ? x[u] * (rowf * gg[u]) : x[u] * rowf);
-          T[rl * NLP + lm] = v;
+      for (int w = 0; w < PK_W; w++) x[u][w] = (so >= 0 && lm + 32 * w < nl) ? __ldg(src + lm + 32 * w) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < PK_U; u++) {
+      const int it = i0 + u * nw, rl = dseg.div(it), lm = (it - rl * nseg) * (32 * PK_W) + lane;
+      if (it >= nitem) break;
+      const double rowf = rfac[rl];
+      const bool vec = rvec[rl] != 0;
+      float mx = 0.0f;
+#pragma unroll
+      for (int w = 0; w < PK_W; w++) {
+        const int l = m + lm + 32 * w;
+        const double gg = (l == 0) ? 0.5 : (double)(l * (l + 1));
+        const float v = (float)(vec ? x[u][w] * (rowf * gg) : x[u][w] * rowf);
+        if (lm + 32 * w < nl) {
+          T[rl * NLP + lm + 32 * w] = v;
           mx = fmaxf(mx, fabsf(v));
         }
       }
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) {
-      if (j < RP) a.maxP[(size_t)m * a.pitchP + k * RP + j] = mx;
-      else a.maxD[(size_t)m * a.pitchD + k * RD + (j - RP)] = mx;
+      const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+      if (lane == 0) atomicMax(rmax + rl, mb);
     }
   }
   __syncthreads();
+  for (int rl = threadIdx.x; rl < nrow; rl += blockDim.x) {
+    const int kq = rl / RK, j = rl - kq * RK, k = k0 + kq;
+    const float mx = __uint_as_float(rmax[rl]);
+    if (j < RP) a.maxP[(size_t)m * a.pitchP + k * RP + j] = mx;
+    else a.maxD[(size_t)m * a.pitchD + k * RD + (j - RP)] = mx;
+  }
   // rows out: per (parity, kk) one contiguous run of nk RP (P block) and
   // nk RD (D block) values; a lane keeps its (level, row) for every kk
   const int wP = nk * RP, wD = nk * RD;
@@ -1621,7 +1644,7 @@ int leg_bwd_pack(Ctx &c, const int *slots, const MLayout &out) {
   pk.L = c.L; pk.nr = c.nr; pk.jmax = c.jmax; pk.nvec = nvec; pk.ng = ng;
   pk.kc = (c.tune[TUNE_PACK_KC] == 1 || c.tune[TUNE_PACK_KC] == 4) ? c.tune[TUNE_PACK_KC] : 2;
   for (int q = 0; q < ng; q++) pk.slot[q] = slots[q];
-  pk.moff = c.d_moff; pk.g3rlm = c.d_g3rlm; pk.ar1 = c.d_ar1; pk.f = c.d_f; pk.fs = c.fsize();
+  pk.moff = c.d_moff; pk.ar1 = c.d_ar1; pk.f = c.d_f; pk.fs = c.fsize();
   pk.rlmP = t->rlmP; pk.rlmD = t->rlmD; pk.pitchP = pitchP; pk.pitchD = pitchD;
   pk.kbase = t->kbase; pk.maxP = t->maxP; pk.maxD = t->maxD;
   const size_t smp = (size_t)pk.kc * (2 * ng + 4 * nvec) * ((c.L + 1) | 1) * sizeof(float);
