@@ -39,7 +39,10 @@
 namespace cb2 {
 
 constexpr int CN_THREADS = 256;   // a block: 8 warps, each 32 consecutive degrees of one (m, sign)
-constexpr int CN_RING = 4;        // rows each thread keeps in flight (cp.async ring)
+// rows each thread keeps in flight (cp.async ring): 4 leaves room for four
+// blocks an SM; shells of at most CN_DEEP_TILES blocks, whose time is the
+// latency of the rows, take 8
+constexpr int CN_RING = 4, CN_RING_DEEP = 8, CN_DEEP_TILES = 2 * 148;
 constexpr int CN_RV = 4;          // values per ring slot (forward: X, D, F, P; backward: y)
 
 // Forms of one field's factors.  Per row i: NL multipliers L(i,i-1) ..
@@ -53,8 +56,8 @@ __host__ __device__ constexpr int cn_entries(int f) { return 2 * cn_nl(f) + 1; }
 
 // shared memory of a block: the radial coefficients, then the per-thread rings
 __host__ __device__ inline size_t cn_ring_offset(int n) { return 9 * (size_t)n * sizeof(double); }
-static size_t cn_smem(int n) {
-  return cn_ring_offset(n) + (size_t)CN_RING * CN_RV * CN_THREADS * sizeof(double);
+static size_t cn_smem(int n, int ring) {
+  return cn_ring_offset(n) + (size_t)ring * CN_RV * CN_THREADS * sizeof(double);
 }
 
 struct LuSet {
@@ -213,7 +216,7 @@ struct FacCol {
 // 4 toroidal magnetic field.  fac: the column's factors.  The
 // inputs of row k + CN_RING are copied into the thread's ring while row k
 // is computed, so a thread keeps CN_RING rows of loads in flight.
-template <int FLD, int FORM>
+template <int RING, int FLD, int FORM>
 __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring,
                                            Col X, Col D, Col F, Col P, Col S, int euler) {
   constexpr int NL = cn_nl(FORM), PD = cn_pd(FORM), NE = cn_entries(FORM);
@@ -235,7 +238,7 @@ __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring
     cp_commit();
   };
 #pragma unroll
-  for (int r = 0; r < CN_RING; r++) fetch(r, r);
+  for (int r = 0; r < RING; r++) fetch(r, r);
   double yh[NL];       // y(i - 1 - t)
   double pend[PD + 1]; // right-hand side of rows i .. i + PD, interchanges of rows < i applied
 #pragma unroll
@@ -249,66 +252,85 @@ __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring
   double fn[NL];
   int dn = 0;
   auto factors = [&](int i) {
-    if (i >= n) return;
     if constexpr (PD >= 1) dn = fac.piv(i);
 #pragma unroll
     for (int t = 0; t < NL; t++) fn[t] = fac.at(i, NE, t);
   };
   factors(0);
   int sl = 0;
-  for (int k = 0; k < n + PD; k++) {
-    double b = 0.0;
-    if (k < n) {
-      cp_wait<CN_RING - 1>();   // row k has landed
-      const double xv = *ring.at(sl, 0), dv = *ring.at(sl, 1), fv = *ring.at(sl, 2);
-      const double pw = euler ? 0.0 : *ring.at(sl, 3);
-      // the temperature's force is minus the heat advection (pH = -H)
-      const double f = (FLD == 2) ? -fv : fv;
-      const double rhs = euler ? xv + dt * (ce * dv + f) : xv + dt * (ce * dv + adam_0 * f + adam_1 * pw);
-      P.stcs(k, st, f);
-      const bool wall = (k == 0 || k == n - 1);
-      if (FLD == 0 || FLD == 1 || FLD == 4) b = (q.jj != 0 && !wall) ? rhs : 0.0;
-      else if (FLD == 2) b = (k == 0) ? fbi : (k == n - 1) ? fbo : rhs;
-      else b = (q.jj != 0) ? rhs : 0.0;
+  // explicit right-hand side of row k
+  auto explicit_row = [&](int k) {
+    cp_wait<RING - 1>();   // row k has landed
+    const double xv = *ring.at(sl, 0), dv = *ring.at(sl, 1), fv = *ring.at(sl, 2);
+    const double pw = euler ? 0.0 : *ring.at(sl, 3);
+    // the temperature's force is minus the heat advection (pH = -H)
+    const double f = (FLD == 2) ? -fv : fv;
+    const double rhs = euler ? xv + dt * (ce * dv + f) : xv + dt * (ce * dv + adam_0 * f + adam_1 * pw);
+    P.stcs(k, st, f);
+    const bool wall = (k == 0 || k == n - 1);
+    double b;
+    if (FLD == 0 || FLD == 1 || FLD == 4) b = (q.jj != 0 && !wall) ? rhs : 0.0;
+    else if (FLD == 2) b = (k == 0) ? fbi : (k == n - 1) ? fbo : rhs;
+    else b = (q.jj != 0) ? rhs : 0.0;
+    return b;
+  };
+  // refill the slot of row k (its values are used by then)
+  auto refill = [&](int k) {
+    fetch(sl, k + RING);
+    sl = (sl + 1 == RING) ? 0 : sl + 1;
+  };
+  // y of row i from the window of right-hand sides
+  auto eliminate = [&](int i, bool more) {
+    double fc[NL];
+#pragma unroll
+    for (int t = 0; t < NL; t++) fc[t] = fn[t];
+    const int d = dn;
+    if (more) factors(i + 1);
+    if constexpr (PD >= 1) {
+      if (d == 1) { const double t = pend[0]; pend[0] = pend[1]; pend[1] = t; }
+      if constexpr (PD >= 2)
+        if (d == 2) { const double t = pend[0]; pend[0] = pend[2]; pend[2] = t; }
     }
-    pend[PD] = b;
-    const int i = k - PD;
-    if (i >= 0 && i < n) {
-      double fc[NL];
+    double y = pend[0];
 #pragma unroll
-      for (int t = 0; t < NL; t++) fc[t] = fn[t];
-      const int d = dn;
-      factors(i + 1);
-      if constexpr (PD >= 1) {
-        if (d == 1) { const double t = pend[0]; pend[0] = pend[1]; pend[1] = t; }
-        if constexpr (PD >= 2)
-          if (d == 2) { const double t = pend[0]; pend[0] = pend[2]; pend[2] = t; }
-      }
-      double y = pend[0];
+    for (int t = NL - 1; t >= 0; t--) y = y - fc[t] * yh[t];
+    S.stkeep(i, st, y, keep);
 #pragma unroll
-      for (int t = NL - 1; t >= 0; t--) y = y - fc[t] * yh[t];
-      S.stkeep(i, st, y, keep);
-#pragma unroll
-      for (int t = NL - 1; t > 0; t--) yh[t] = yh[t - 1];
-      yh[0] = y;
-    }
+    for (int t = NL - 1; t > 0; t--) yh[t] = yh[t - 1];
+    yh[0] = y;
+  };
+  auto shift = [&](double b) {
 #pragma unroll
     for (int t = 0; t < PD; t++) pend[t] = pend[t + 1];
-    if (k < n) {
-      // refill the slot just read (its values are used above)
-      fetch(sl, k + CN_RING);
-      sl = (sl + 1 == CN_RING) ? 0 : sl + 1;
-    }
+    pend[PD] = b;
+  };
+  // the window runs a row behind the right-hand sides, so the two chains of a
+  // row (its right-hand side, and the elimination PD + 1 rows back) do not wait
+  // on each other
+  for (int k = 0; k <= PD; k++) {
+    shift(explicit_row(k));
+    refill(k);
+  }
+  for (int k = PD + 1; k < n; k++) {
+    const double b = explicit_row(k);
+    eliminate(k - PD - 1, true);
+    shift(b);
+    refill(k);
+  }
+  for (int i = n - PD - 1; i < n; i++) {
+    eliminate(i, i + 1 < n);
+    shift(0.0);
   }
   cp_wait<0>();   // the ring is free for the backward sweep
 }
 
 // backward sweep: U x = y, rows n-1 .. 0, handing each x to the emitter:
 // em.point(k, x) for the row itself, then em.top() once rows n-1 .. n-3
-// are known, em.interior(r) for rows r = n-2 .. 1 as soon as row r - 1 is
-// known, and em.bottom() at the end.  y of row k - CN_RING is copied into
-// the ring while row k is computed.
-template <int FORM, class Em>
+// are known, em.interior(r) for rows r = n-2 .. 1 a row after row r - 1 is
+// known (so that it does not wait on the row being solved), and em.bottom()
+// at the end.  y of row k - RING is copied into the ring while row k is
+// computed.
+template <int RING, int FORM, class Em>
 __device__ __forceinline__ void cn_backward(const CnCtx &q, FacCol fac, Ring ring, Col S, Em &em) {
   constexpr int NL = cn_nl(FORM), NE = cn_entries(FORM);
   const int n = q.n;
@@ -318,7 +340,7 @@ __device__ __forceinline__ void cn_backward(const CnCtx &q, FacCol fac, Ring rin
     cp_commit();
   };
 #pragma unroll
-  for (int r = 0; r < CN_RING; r++) fetch(r, n - 1 - r);
+  for (int r = 0; r < RING; r++) fetch(r, n - 1 - r);
   double xh[NL];   // x(k + 1 + t)
 #pragma unroll
   for (int t = 0; t < NL; t++) xh[t] = 0.0;
@@ -330,8 +352,8 @@ __device__ __forceinline__ void cn_backward(const CnCtx &q, FacCol fac, Ring rin
   };
   factors(n - 1);
   int sl = 0;
-  for (int k = n - 1; k >= 0; k--) {
-    cp_wait<CN_RING - 1>();
+  auto solve = [&](int k) {
+    cp_wait<RING - 1>();
     double fc[NL + 1];
 #pragma unroll
     for (int t = 0; t <= NL; t++) fc[t] = fn[t];
@@ -343,17 +365,25 @@ __device__ __forceinline__ void cn_backward(const CnCtx &q, FacCol fac, Ring rin
 #pragma unroll
     for (int t = NL - 1; t > 0; t--) xh[t] = xh[t - 1];
     xh[0] = x;
-    em.point(k, x);
-    // refill the slot just read (its value is stored above, through x)
-    fetch(sl, k - CN_RING);
-    sl = (sl + 1 == CN_RING) ? 0 : sl + 1;
-    if (k == n - 3) {
-      em.top();
-      em.interior(n - 2);
-    } else if (k < n - 3) {
-      em.interior(k + 1);
-    }
+    return x;
+  };
+  // refill the slot of row k (its value is stored by then, through x)
+  auto refill = [&](int k) {
+    fetch(sl, k - RING);
+    sl = (sl + 1 == RING) ? 0 : sl + 1;
+  };
+  for (int k = n - 1; k >= n - 3; k--) {
+    em.point(k, solve(k));
+    refill(k);
   }
+  em.top();
+  for (int k = n - 4; k >= 0; k--) {
+    const double x = solve(k);
+    em.interior(k + 2);
+    em.point(k, x);
+    refill(k);
+  }
+  em.interior(1);
   em.bottom();
   cp_wait<0>();
 }
@@ -539,32 +569,32 @@ struct EmMagTor {
 
 // ---------------------------------------------------------------------------
 // one (field, column) thread: the sweeps with the field's slots and emitter
-template <int FLD, int FORM>
+template <int RING, int FLD, int FORM>
 __device__ __forceinline__ void cn_column(const CnCtx &q, double *col, size_t fs, FacCol fac, Ring ring,
                                           int euler) {
   auto C = [&](int slot) { return Col{col + (size_t)slot * fs}; };
   if constexpr (FLD == 0) {
-    cn_forward<0, FORM>(q, fac, ring, C(VORT + 2), C(WDIFF + 2), C(FORCES + 2), C(PREMOM + 2), C(VELO), euler);
+    cn_forward<RING, 0, FORM>(q, fac, ring, C(VORT + 2), C(WDIFF + 2), C(FORCES + 2), C(PREMOM + 2), C(VELO), euler);
     EmVelPol em{q, C(VELO), C(VELO + 1), C(VORT + 2), C(WDIFF + 2)};
-    cn_backward<FORM>(q, fac, ring, C(VELO), em);
+    cn_backward<RING, FORM>(q, fac, ring, C(VELO), em);
   } else if constexpr (FLD == 1) {
-    cn_forward<1, FORM>(q, fac, ring, C(VORT), C(WDIFF), C(FORCES), C(PREMOM), C(VELO + 2), euler);
+    cn_forward<RING, 1, FORM>(q, fac, ring, C(VORT), C(WDIFF), C(FORCES), C(PREMOM), C(VELO + 2), euler);
     EmVelTor em{q, C(VELO + 2), C(VORT), C(VORT + 1), C(WDIFF)};
-    cn_backward<FORM>(q, fac, ring, C(VELO + 2), em);
+    cn_backward<RING, FORM>(q, fac, ring, C(VELO + 2), em);
   } else if constexpr (FLD == 2) {
-    cn_forward<2, FORM>(q, fac, ring, C(TEMP), C(TDIFF), C(HADV), C(PREHEAT), C(TEMP), euler);
+    cn_forward<RING, 2, FORM>(q, fac, ring, C(TEMP), C(TDIFF), C(HADV), C(PREHEAT), C(TEMP), euler);
     EmTemp em{q, C(TEMP), C(ROTBUO + 2), C(TDIFF), (q.jj == 0) ? q.a.temp_icb_fld : 0.0,
               (q.jj == 0) ? q.a.temp_cmb_fld : 0.0};
-    cn_backward<FORM>(q, fac, ring, C(TEMP), em);
+    cn_backward<RING, FORM>(q, fac, ring, C(TEMP), em);
   } else if constexpr (FLD == 3) {
-    cn_forward<3, FORM>(q, fac, ring, C(MAGNE), C(BDIFF), C(INDUCT), C(PREUXB), C(MAGNE), euler);
+    cn_forward<RING, 3, FORM>(q, fac, ring, C(MAGNE), C(BDIFF), C(INDUCT), C(PREUXB), C(MAGNE), euler);
     EmMagPol em{q, C(MAGNE), C(MAGNE + 1), C(CURRENT + 2), C(BDIFF)};
-    cn_backward<FORM>(q, fac, ring, C(MAGNE), em);
+    cn_backward<RING, FORM>(q, fac, ring, C(MAGNE), em);
   } else {
-    cn_forward<4, FORM>(q, fac, ring, C(MAGNE + 2), C(BDIFF + 2), C(INDUCT + 2), C(PREUXB + 2), C(MAGNE + 2),
+    cn_forward<RING, 4, FORM>(q, fac, ring, C(MAGNE + 2), C(BDIFF + 2), C(INDUCT + 2), C(PREUXB + 2), C(MAGNE + 2),
                         euler);
     EmMagTor em{q, C(MAGNE + 2), C(CURRENT), C(CURRENT + 1), C(BDIFF + 2)};
-    cn_backward<FORM>(q, fac, ring, C(MAGNE + 2), em);
+    cn_backward<RING, FORM>(q, fac, ring, C(MAGNE + 2), em);
   }
 }
 
@@ -590,7 +620,8 @@ __device__ __forceinline__ CnField cn_field(const CnPack &pk, int fld) {
 // the degree l0 + lane, so every access of a warp to a slot row is 32
 // consecutive doubles.  The block stages the radial coefficients in shared
 // memory; each thread then runs its column.
-__global__ void __launch_bounds__(CN_THREADS, 4)
+template <int RING>
+__global__ void __launch_bounds__(CN_THREADS, RING == CN_RING ? 4 : 2)
 k_cn_step(RJArgs a, double *f, size_t fs, CnPack pk, const int *moff, const int4 *tiles, int euler) {
   extern __shared__ double cn_sm[];
   const int n = a.nr, nl = a.L + 1, tid = threadIdx.x;
@@ -618,16 +649,16 @@ k_cn_step(RJArgs a, double *f, size_t fs, CnPack pk, const int *moff, const int4
   const FacCol fac{fd.fac + l, fd.piv ? fd.piv + l : nullptr, nl};
   const Ring ring{reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(cn_sm) + cn_ring_offset(n)) + tid};
   switch (fld * 4 + form) {
-    case 0 * 4 + CN_N5: cn_column<0, CN_N5>(q, col, fs, fac, ring, euler); break;
-    case 0 * 4 + CN_W5: cn_column<0, CN_W5>(q, col, fs, fac, ring, euler); break;
-    case 1 * 4 + CN_N3: cn_column<1, CN_N3>(q, col, fs, fac, ring, euler); break;
-    case 1 * 4 + CN_W3: cn_column<1, CN_W3>(q, col, fs, fac, ring, euler); break;
-    case 2 * 4 + CN_N3: cn_column<2, CN_N3>(q, col, fs, fac, ring, euler); break;
-    case 2 * 4 + CN_W3: cn_column<2, CN_W3>(q, col, fs, fac, ring, euler); break;
-    case 3 * 4 + CN_N3: cn_column<3, CN_N3>(q, col, fs, fac, ring, euler); break;
-    case 3 * 4 + CN_W3: cn_column<3, CN_W3>(q, col, fs, fac, ring, euler); break;
-    case 4 * 4 + CN_N3: cn_column<4, CN_N3>(q, col, fs, fac, ring, euler); break;
-    case 4 * 4 + CN_W3: cn_column<4, CN_W3>(q, col, fs, fac, ring, euler); break;
+    case 0 * 4 + CN_N5: cn_column<RING, 0, CN_N5>(q, col, fs, fac, ring, euler); break;
+    case 0 * 4 + CN_W5: cn_column<RING, 0, CN_W5>(q, col, fs, fac, ring, euler); break;
+    case 1 * 4 + CN_N3: cn_column<RING, 1, CN_N3>(q, col, fs, fac, ring, euler); break;
+    case 1 * 4 + CN_W3: cn_column<RING, 1, CN_W3>(q, col, fs, fac, ring, euler); break;
+    case 2 * 4 + CN_N3: cn_column<RING, 2, CN_N3>(q, col, fs, fac, ring, euler); break;
+    case 2 * 4 + CN_W3: cn_column<RING, 2, CN_W3>(q, col, fs, fac, ring, euler); break;
+    case 3 * 4 + CN_N3: cn_column<RING, 3, CN_N3>(q, col, fs, fac, ring, euler); break;
+    case 3 * 4 + CN_W3: cn_column<RING, 3, CN_W3>(q, col, fs, fac, ring, euler); break;
+    case 4 * 4 + CN_N3: cn_column<RING, 4, CN_N3>(q, col, fs, fac, ring, euler); break;
+    case 4 * 4 + CN_W3: cn_column<RING, 4, CN_W3>(q, col, fs, fac, ring, euler); break;
     default: break;
   }
 }
@@ -670,7 +701,7 @@ int cn_setup(Ctx &c) {
     dbl += (size_t)n * cn_entries(pk.form[q]) * nl;
     if (cn_pd(pk.form[q])) byt += (size_t)n * nl;
   }
-  smem = cn_smem(n);
+  smem = cn_smem(n, CN_RING);
   if (smem > 227 * 1024) {
     c.tune[TUNE_CN] = -1;
     c.cn_off_reason = "the per-thread input rings need more than 227 KB of shared memory";
@@ -699,16 +730,23 @@ int cn_setup(Ctx &c) {
   c.cn_tiles = (int)tl.size();
   CB2_CUDA(cudaMalloc(&c.d_cn_tiles, tl.size() * sizeof(int4)));
   CB2_CUDA(cudaMemcpyAsync(c.d_cn_tiles, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream));
-  CB2_CUDA(raise_smem_limit(k_cn_step, smem));
+  c.cn_ring = CN_RING;
+  if (c.cn_tiles <= CN_DEEP_TILES && cn_smem(n, CN_RING_DEEP) <= 227 * 1024) {
+    c.cn_ring = CN_RING_DEEP;
+    smem = cn_smem(n, CN_RING_DEEP);
+    CB2_CUDA(raise_smem_limit(k_cn_step<CN_RING_DEEP>, smem));
+  } else {
+    CB2_CUDA(raise_smem_limit(k_cn_step<CN_RING>, smem));
+  }
   CB2_CUDA(cudaStreamSynchronize(c.stream));
   c.cn_pack = new CnPack(pk);
   c.cn_smem = smem;
   c.cn_ready = true;
   // The one kernel is the default wherever it takes the context.  Mixed steps,
-  // one kernel against the separate ones, us: L7 / Nr9 53 / 60, L15 / Nr17
-  // 74 / 85, L31 / Nr33 93 / 101, L31 / Nr129 278 / 317, L63 / Nr65 302 / 299,
-  // L127 / Nr25 326 / 354, L127 / Nr97 1129 / 1230, L191 / Nr65 3747 / 3853,
-  // L255 / Nr129 5075 / 5524.
+  // one kernel against the separate ones, us: L7 / Nr9 49 / 58, L15 / Nr17
+  // 57 / 70, L31 / Nr33 79 / 94, L31 / Nr129 246 / 297, L63 / Nr65 271 / 283,
+  // L127 / Nr25 320 / 347, L127 / Nr97 1097 / 1206, L191 / Nr65 2221 / 2335,
+  // L255 / Nr129 5106 / 5552.
   c.tune[TUNE_CN] = 1;
   return 0;
 }
@@ -729,9 +767,13 @@ void cn_stage(Ctx &c, bool euler) {
 
 // one launch for the five fields (the 5-band field's blocks first)
 void cn_step(Ctx &c, bool euler) {
-  k_cn_step<<<c.cn_tiles, CN_THREADS, c.cn_smem, c.stream>>>(c.rj_args(), c.d_f, c.fsize(),
-                                                              *static_cast<const CnPack *>(c.cn_pack), c.d_moff,
-                                                              c.d_cn_tiles, euler ? 1 : 0);
+  const CnPack &pk = *static_cast<const CnPack *>(c.cn_pack);
+  if (c.cn_ring == CN_RING_DEEP)
+    k_cn_step<CN_RING_DEEP><<<c.cn_tiles, CN_THREADS, c.cn_smem, c.stream>>>(
+        c.rj_args(), c.d_f, c.fsize(), pk, c.d_moff, c.d_cn_tiles, euler ? 1 : 0);
+  else
+    k_cn_step<CN_RING><<<c.cn_tiles, CN_THREADS, c.cn_smem, c.stream>>>(
+        c.rj_args(), c.d_f, c.fsize(), pk, c.d_moff, c.d_cn_tiles, euler ? 1 : 0);
 }
 
 }  // namespace cb2
