@@ -284,14 +284,22 @@ k_tc_gemm(int M, int N, int NT, int K, const TAT *__restrict__ A, int lda, const
 // pass of 16384 rows: 35 + 45 + 51 us of kernels, before 500 us.
 //
 // A CTA keeps the bfloat16 weights in shared memory and walks tiles of 128
-// rows.  Warps 0-7 are the epilogue: warp w reads tensor-memory lanes
-// 32 (w & 3) .. + 31, one row a thread, the warps 0-3 (group 0) the even and
-// 4-7 (group 1) the odd chunks of 32 columns.  A chunk of an activation is
+// rows.  Warps 0-11 are the epilogue: warp w reads tensor-memory lanes
+// 32 (w & 3) .. + 31, one row a thread, the four warps of group w >> 2 every
+// third chunk of 32 columns (with two groups the SiLU chains left the
+// schedulers idle: 189 us for 266240 rows).  A chunk of an activation is
 // split into bfloat16 hi + lo and written as the next product's A operand
-// into one of ML_ST stages; warp 8 issues the MMAs of a chunk as soon as it
-// is there, so the second product runs behind the first one's epilogue.  The
-// last layer (O <= 8 columns) is float32 FMAs on the thread's row.
-constexpr int ML_EPI = 256, ML_THREADS = ML_EPI + 32, ML_ST = 3, ML_O = 8;
+// into one of ML_ST stages; the last warp issues the MMAs of a chunk as soon as
+// it is there, so the second product runs behind the first one's epilogue.  The
+// last layer (OC = 5 or 8 columns) is float32 FMAs on the thread's row.
+//
+// The stages' empty barriers are waited on by phase parity, so whoever fills
+// use q of a stage must know that use q - 2 ML_ST has been released.  A group
+// fills every ML_G-th use and has seen its own last use's predecessor released,
+// q - ML_G - ML_ST: hence ML_G <= ML_ST.  (The first uses of a tile follow a
+// barrier that every release of the last tile precedes.)
+constexpr int ML_G = 3, ML_EPI = 128 * ML_G, ML_THREADS = ML_EPI + 32, ML_ST = 3, ML_O = 8;
+static_assert(ML_G <= ML_ST, "a group may not run two phases ahead of a stage");
 constexpr uint32_t ML_STAGE = 2 * GA_BYTES;   // hi and lo of 128 rows x 32 columns
 
 struct MlpArgs {
@@ -328,7 +336,7 @@ __host__ __device__ inline MlpLayout mlp_layout(int H) {
   o.b1 = p; p += (uint32_t)H * 4;
   o.b2 = p; p += (uint32_t)H * 4;
   o.w3 = p; p += (uint32_t)H * ML_O * 4;
-  o.yp = p; p += 128 * ML_O * 4;
+  o.yp = p; p += (ML_G - 1) * 128 * ML_O * 4;
   o.bar = p; p += 128;
   o.total = p;
   return o;
@@ -340,16 +348,16 @@ __device__ inline float dsilu(float z) {
   return s * (1.0f + z * (1.0f - s));
 }
 
-// barrier of the 256 epilogue threads; true when any of them passes true
+// barrier of the epilogue threads; true when any of them passes true
 __device__ inline bool epi_any(bool v) {
   int r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.s32 p, %1, 0;\n\t"
-      "barrier.cta.red.or.pred q, 1, 256, p;\n\t"
+      "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
       "selp.s32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
-      : "r"((int)v)
+      : "r"((int)v), "n"(ML_EPI)
       : "memory");
   return r != 0;
 }
@@ -426,7 +434,7 @@ __device__ inline void mlp_finish(const MlpArgs &a, MlpBars *sb, uint32_t tmem, 
   if (threadIdx.x >> 5 == 0) tc::tmem_dealloc(tmem, 512);
 }
 
-template <bool TRAIN>
+template <bool TRAIN, int OC>
 __global__ void __launch_bounds__(ML_THREADS, 1)
 k_mlp_fwd(const __grid_constant__ MlpArgs a) {
   extern __shared__ unsigned char g_smem_raw[];
@@ -518,11 +526,14 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
       if (!bad && !tc::mbar_wait(&sb->d1, i & 1, a.wait_ns)) bad = true;
       bad = __any_sync(0xffffffffu, bad);
       tc::tc_fence_after();
-      for (int c = g; c < nch; c += 2) {
+      for (int c = g; c < nch; c += ML_G) {
         float z[32];
         tmem_ld32(tl + c * 32, z);
 #pragma unroll
-        for (int j = 0; j < 32; j++) z[j] += b1[c * 32 + j];
+        for (int j = 0; j < 32; j += 4) {
+          const float4 bv = *reinterpret_cast<const float4 *>(b1 + c * 32 + j);
+          z[j] += bv.x; z[j + 1] += bv.y; z[j + 2] += bv.z; z[j + 3] += bv.w;
+        }
         if (TRAIN && in) store32(a.Z1 + row * H + c * 32, z);
 #pragma unroll
         for (int j = 0; j < 32; j++) z[j] = silu(z[j]);
@@ -536,40 +547,48 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
       if (!bad && !tc::mbar_wait(&sb->d2, i & 1, a.wait_ns)) bad = true;
       bad = __any_sync(0xffffffffu, bad);
       tc::tc_fence_after();
-      float y[ML_O];
+      float y[OC];
 #pragma unroll
-      for (int o = 0; o < ML_O; o++) y[o] = 0.0f;
-      for (int c = g; c < nch; c += 2) {
+      for (int o = 0; o < OC; o++) y[o] = 0.0f;
+      for (int c = g; c < nch; c += ML_G) {
         float z[32];
         tmem_ld32(tl + 256 + c * 32, z);
 #pragma unroll
-        for (int j = 0; j < 32; j++) z[j] += b2[c * 32 + j];
+        for (int j = 0; j < 32; j += 4) {
+          const float4 bv = *reinterpret_cast<const float4 *>(b2 + c * 32 + j);
+          z[j] += bv.x; z[j + 1] += bv.y; z[j + 2] += bv.z; z[j + 3] += bv.w;
+        }
         if (TRAIN && in) store32(a.Z2 + row * H + c * 32, z);
 #pragma unroll
         for (int j = 0; j < 32; j++) {
           const float h = silu(z[j]);
           const float4 wa = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O);
           y[0] += h * wa.x; y[1] += h * wa.y; y[2] += h * wa.z; y[3] += h * wa.w;
-          if (a.O > 4) {
+          if constexpr (OC == 5) {
+            y[4] += h * w3[(c * 32 + j) * ML_O + 4];
+          } else {
             const float4 wb = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O + 4);
             y[4] += h * wb.x; y[5] += h * wb.y; y[6] += h * wb.z; y[7] += h * wb.w;
           }
         }
       }
-      if (g == 1) {
+      if (g > 0) {
 #pragma unroll
-        for (int o = 0; o < ML_O; o++) yp[r * ML_O + o] = y[o];
+        for (int o = 0; o < OC; o++) yp[((g - 1) * 128 + r) * ML_O + o] = y[o];
       }
-      // both groups have read the accumulators: the next tile may refill them
+      // every group has read the accumulators: the next tile may refill them
       tc::tc_fence_before();
       bad = epi_any(bad);
       if (bad) break;
       if (g == 0) {
         double e = 0.0;
 #pragma unroll
-        for (int o = 0; o < ML_O; o++)
+        for (int o = 0; o < OC; o++)
           if (in && o < a.O) {
-            const float v = y[o] + yp[r * ML_O + o] + a.b3[o];
+            float v = y[o];
+#pragma unroll
+            for (int u = 0; u < ML_G - 1; u++) v += yp[(u * 128 + r) * ML_O + o];
+            v += a.b3[o];
             if (!TRAIN) {
               a.Y[row * a.O + o] = v;
             } else {
@@ -647,7 +666,7 @@ k_mlp_bwd(const __grid_constant__ MlpArgs a) {
       float dy[ML_O];
 #pragma unroll
       for (int o = 0; o < ML_O; o++) dy[o] = (in && o < a.O) ? a.dY[row * a.O + o] : 0.0f;
-      for (int c = g; c < nch; c += 2) {
+      for (int c = g; c < nch; c += ML_G) {
         float z[32];
         if (in) load32(a.Z2 + row * H + c * 32, z);
 #pragma unroll
@@ -672,7 +691,7 @@ k_mlp_bwd(const __grid_constant__ MlpArgs a) {
       if (!bad && !tc::mbar_wait(&sb->d1, i & 1, a.wait_ns)) bad = true;
       bad = __any_sync(0xffffffffu, bad);
       tc::tc_fence_after();
-      for (int c = g; c < nch; c += 2) {
+      for (int c = g; c < nch; c += ML_G) {
         float d[32], z[32];
         tmem_ld32(tl + c * 32, d);
         if (in) {
@@ -682,7 +701,7 @@ k_mlp_bwd(const __grid_constant__ MlpArgs a) {
           store32(a.dZ1 + row * H + c * 32, d);
         }
       }
-      // both groups have read this half before the tile after next refills it
+      // every group has read this half before the tile after next refills it
       tc::tc_fence_before();
       bad = epi_any(bad);
       if (bad) break;
@@ -1079,7 +1098,7 @@ int mlp_forward(cb2_mlp *nt, const float *X, size_t n, float *Y, cudaStream_t st
   if (fused_ok(nt)) {
     MlpArgs a = mlp_args(nt, X, n, status);
     a.Y = Y;
-    return launch_rows(k_mlp_fwd<false>, a, st);
+    return nt->O <= 5 ? launch_rows(k_mlp_fwd<false, 5>, a, st) : launch_rows(k_mlp_fwd<false, 8>, a, st);
   }
   int rc = mlp_reserve(nt, n, false);
   if (rc) return rc;
@@ -1102,7 +1121,7 @@ int mlp_backward_fused(cb2_mlp *nt, const float *X, const float *T, size_t n) {
   MlpArgs a = mlp_args(nt, X, n, nt->status);
   a.T = T; a.Z1 = nt->Z1; a.Z2 = nt->Z2; a.dY = nt->dY; a.dZ2 = nt->dZ; a.dZ1 = nt->dH; a.part = nt->part;
   CB2_CUDA(cudaMemsetAsync(nt->grad, 0, nt->np * sizeof(float), st));
-  int rc = launch_rows(k_mlp_fwd<true>, a, st);
+  int rc = nt->O <= 5 ? launch_rows(k_mlp_fwd<true, 5>, a, st) : launch_rows(k_mlp_fwd<true, 8>, a, st);
   if (rc) return rc;
   k_loss_sum<<<1, 256, 0, st>>>(4 * ((a.n + 127) / 128), nt->part, 1.0 / ((double)n * nt->O), nt->loss);
   if ((rc = launch_rows(k_mlp_bwd, a, st))) return rc;
