@@ -805,7 +805,7 @@ __device__ inline void coriolis_terms(const RJArgs &a, const Fields &F, const Co
 // curl / divergence of the transformed forces and the force sum
 // (const_sph_force_rot2, const_sph_rotation_uxb, const_sph_scalar_advect,
 //  add_reftemp_advect_sph_MHD, set_MHD_terms_to_force)
-__global__ void k_after_transform(RJArgs a, Fields F, CorTables ct, int roundtrip) {
+__global__ void k_after_transform(RJArgs a, Fields F, CorTables ct) {
   // grid (jj blocks, radial level k): no division to find k and jj
   const int jj = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
   if (jj >= a.jmax) return;
@@ -874,13 +874,6 @@ __global__ void k_after_transform(RJArgs a, Fields F, CorTables ct, int roundtri
   coriolis_terms(a, F, ct, jj, k, rc0, rc2);
   F(FORCES)[idx] = -rot[0][0] + rc0 + rot[1][0];
   F(FORCES + 2)[idx] = -rot[0][2] + rc2 + rot[1][2] + F(ROTBUO + 2)[idx];
-  // the temperature round trip of a step's end (nothing above reads the
-  // temperature): its own launch was 2 us of a 115 us step at L31
-  if (roundtrip && jj == 0) {
-    double *T = F(TEMP);
-    const double v = T[idx] + a.reft0[k];
-    T[idx] = v - a.reft0[k];
-  }
 }
 
 __global__ void k_temp_total(RJArgs a, Fields F, double sign) {
@@ -961,10 +954,9 @@ void rj_start_derived(Ctx &c) {
   k_derived_b<<<dim3(cdiv(c.jmax, kThreads), c.nr), kThreads, 0, c.stream>>>(a, fields(c));
 }
 
-void rj_after_transform(Ctx &c, bool roundtrip) {
+void rj_after_transform(Ctx &c) {
   const CorTables ct{c.d_jgi1, c.d_jgi2, c.d_jei1, c.d_sw, c.d_tw};
-  k_after_transform<<<dim3(cdiv(c.jmax, kThreads), c.nr), kThreads, 0, c.stream>>>(c.rj_args(), fields(c), ct,
-                                                                                          roundtrip ? 1 : 0);
+  k_after_transform<<<dim3(cdiv(c.jmax, kThreads), c.nr), kThreads, 0, c.stream>>>(c.rj_args(), fields(c), ct);
 }
 
 void rj_temp_total(Ctx &c, double sign) {
