@@ -480,12 +480,19 @@ template <int R1, int R2>
 struct F4Plan {
   static constexpr int M = R1 * R2, N = 3 * M;
   static constexpr int TP = R2 + 1;            // transpose row pitch (complex)
-  static constexpr int TG = R1 * TP;           // transpose block of one group
-  static constexpr int X = (21 * TG > 7 * N) ? 21 * TG : 7 * N;   // work buffer (complex)
-  static constexpr int MP2 = M + 1;            // staging row pitch (complex), slot M stays zero
+  // the block of a group (complex): its transposes, then its grid samples,
+  // then its F_r.  Half a warp is 16 / R2 groups, whose blocks start R2
+  // elements apart modulo 16, so that the groups' accesses fall on different
+  // banks.
+  static constexpr int T0 = (R1 * TP > M) ? R1 * TP : M;
+  static constexpr int TG = T0 + (R2 == 16 ? 0 : (R2 + 16 - T0 % 16) % 16);
+  static constexpr int X = 21 * TG;            // work buffer (complex)
+  static constexpr int MP2 = M + 1;            // staging row pitch (complex)
   static constexpr int WP = R1 + 1;            // twiddle row pitch (complex)
-  static constexpr int NTW = 3 * M + R2 * WP;  // tables: [3][M] e^{2 pi i m r/N}, [R2][WP] e^{2 pi i n2 k1/M}
-  // staging (floats): 14 rows x MP2 complex in, later 12 rows x MP2 complex out
+  // tables: [2][TWP] e^{2 pi i m r/N} of r = 1, 2, then [R2][WP] e^{2 pi i n2 k1/M}
+  static constexpr int TWP = M + 8, NTW = 2 * TWP + R2 * WP;
+  // staging (floats): 7 rows x MP2 (Z[m], Z[N - (M - m)]) in, later 12 rows x
+  // MP2 complex out
   static constexpr int SF = 28 * MP2;
   static constexpr size_t smem() { return (size_t)SF * 4 + ((size_t)X + NTW) * 8; }
 };
@@ -509,93 +516,114 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
   static_assert(R1 % R2 == 0, "rows of the second step");
   constexpr int M = P::M, N = P::N, TP = P::TP, TG = P::TG, MP2 = P::MP2, WP = P::WP;
   extern __shared__ __align__(16) unsigned char smraw[];
-  // input staging [7 pairs][MP2][2]: the (a_m, b_m) of components 2p and
-  // 2p + 1 side by side (component 13 zero), so one 16-byte load reads both
+  // input staging [7 pairs][MP2] of (2 Z[m], 2 Z[N - (M - m)])
   float2 *S2 = reinterpret_cast<float2 *>(smraw);
-  float2 *X = reinterpret_cast<float2 *>(smraw + (size_t)P::SF * 4);   // transposes / grid rows / F_r
-  float2 *TW3 = X + P::X;                                          // [3][M]
-  float2 *TWM = TW3 + 3 * M;                                       // [R2][WP]
+  float2 *X = reinterpret_cast<float2 *>(smraw + (size_t)P::SF * 4);   // [21 groups][TG]
+  float2 *TW3 = X + P::X;                                          // [2][TWP]: r = 1, 2
+  float2 *TWM = TW3 + 2 * P::TWP;                                  // [R2][WP]
   const int th = blockIdx.x / fin.nr, k = blockIdx.x % fin.nr;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = NT / 32;
   const int grp = tid / R2, lt = tid % R2;
-  for (int e = tid; e < 14; e += NT) S2[((e >> 1) * MP2 + M) * 2 + (e & 1)] = float2{0.0f, 0.0f};
-  for (int e = tid; e < M; e += NT) S2[(6 * MP2 + e) * 2 + 1] = float2{0.0f, 0.0f};
-  // input and tables by asynchronous 8-byte copies, all in flight at once.
-  // At one (theta, k) an order m has 13 (cos, sin) pairs: a run of 5 in the
-  // P block and one of 8 in the D block; half-warp h of warp w copies the
-  // orders 2 (w + nwarp i) + h, lane j < 13 of the half pair j into the
-  // staging row of its component
-  for (int e = tid; e < P::NTW; e += NT) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(TW3 + e);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(tables + e) : "memory");
+  // tables by asynchronous 16-byte copies
+  for (int e = 2 * tid; e < 2 * M + R2 * WP; e += 2 * NT) {
+    const int to = (e < M) ? e : (e < 2 * M) ? P::TWP + e - M : 2 * P::TWP + e - 2 * M;
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(TW3 + to);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(tables + M + e) : "memory");
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  // input: at one (theta, k) an order m has 13 (cos, sin) pairs, a run of 5
+  // in the P block and one of 8 in the D block.  A thread takes a pair of
+  // components at the orders m and M - m, which make both rows' entries of
+  // the complex transform there, once for the three residues.
   {
-    const int j = lane & 15, hw = lane >> 4;
-    int c = 0;
-    const float *src = fin.P;
-    size_t mst = 0;
-    if (j < 5) {
-      c = (j < 4) ? 3 * j : 12;
-      src = fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + 2 * j;
-      mst = (size_t)fin.nth * fin.sP();
-    } else if (j < 13) {
-      const int jd = j - 5;
-      c = 3 * (jd >> 1) + 1 + (jd & 1);
-      src = fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + 2 * jd;
-      mst = (size_t)fin.nth * fin.sD();
-    }
-    if (j < 13)
-      for (int m = 2 * warp + hw; m < M; m += 2 * nwarp) {
-        const uint32_t d = (uint32_t)__cvta_generic_to_shared(S2 + ((c >> 1) * MP2 + m) * 2 + (c & 1));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src + m * mst) : "memory");
+    constexpr int IT = (4 * M + NT - 1) / NT;
+    const int p = tid & 7;
+    auto comp = [&](int c, const float *&src, size_t &mst) {
+      const int v = c / 3, s = c - 3 * v;
+      if (s == 0) {
+        src = fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + 2 * v;
+        mst = (size_t)fin.nth * fin.sP();
+      } else {
+        src = fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + 2 * (2 * v + s - 1);
+        mst = (size_t)fin.nth * fin.sD();
       }
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    };
+    const float *s0, *s1;
+    size_t t0, t1;
+    comp(min(2 * p, 12), s0, t0);
+    comp(min(2 * p + 1, 12), s1, t1);
+    float2 a[IT], b[IT], c[IT], d[IT];
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+      const int mi = (tid + i * NT) >> 3, mj = mi ? M - mi : M / 2;
+      const bool on = p < 7 && mi < M / 2;
+      const float2 z{0.0f, 0.0f};
+      a[i] = on ? __ldg(reinterpret_cast<const float2 *>(s0 + mi * t0)) : z;
+      c[i] = on ? __ldg(reinterpret_cast<const float2 *>(s0 + mj * t0)) : z;
+      b[i] = (on && p < 6) ? __ldg(reinterpret_cast<const float2 *>(s1 + mi * t1)) : z;
+      d[i] = (on && p < 6) ? __ldg(reinterpret_cast<const float2 *>(s1 + mj * t1)) : z;
+    }
+    float4 *row = reinterpret_cast<float4 *>(S2) + p * MP2;
+#pragma unroll
+    for (int i = 0; i < IT; i++) {
+      const int mi = (tid + i * NT) >> 3, mj = mi ? M - mi : M / 2;
+      if (p < 7 && mi < M / 2) {
+        const float4 za{a[i].x + b[i].y, b[i].x - a[i].y, c[i].x - d[i].y, c[i].y + d[i].x};
+        const float4 zc{c[i].x + d[i].y, d[i].x - c[i].y, a[i].x - b[i].y, a[i].y + b[i].x};
+        // m = 0: 2 Z[0] = 2 (a_0, a'_0) and no partner; m = M / 2 is its own
+        row[mi] = mi ? za : float4{2.0f * a[i].x, 2.0f * b[i].x, 0.0f, 0.0f};
+        row[mj] = mi ? zc : float4{zc.x, zc.y, za.z, za.w};
+      }
+    }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   const int gp = grp / 3, gr = grp - 3 * gp;   // pair, residue of this group
+  float2 *W = X + grp * TG;                    // its block
   // ---- backward, step 1: column n2 = lt, pair rows built from the staging
   if (grp < 21) {
-    const float4 *xy = reinterpret_cast<const float4 *>(S2) + gp * MP2;   // (x_m, y_m) of the pair
+    const float4 *xy = reinterpret_cast<const float4 *>(S2) + gp * MP2;
     const float2 om = (gr == 0) ? float2{1.0f, 0.0f}
                     : float2{-0.5f, (gr == 1) ? -0.86602540378443864676f : 0.86602540378443864676f};
-    const float2 *tw = TW3 + gr * M;
+    const float2 *tw = TW3 + (gr == 2 ? P::TWP : 0);
     float2 v[R1];
 #pragma unroll
     for (int n1 = 0; n1 < R1; n1++) {
-      const int m = n1 * R2 + lt, mq = M - m;
-      const float4 ab = xy[m], cd = xy[mq];
-      const float2 a = float2{ab.x, ab.y}, b = float2{ab.z, ab.w}, c = float2{cd.x, cd.y}, d = float2{cd.z, cd.w};
-      float2 zm = float2{a.x + b.y, b.x - a.y};           // 2 Z[m]
-      const float2 zp = float2{c.x - d.y, c.y + d.x};     // 2 Z[N - (M - m)] (zero at m = 0)
-      if (n1 == 0 && lt == 0) zm = float2{2.0f * a.x, 2.0f * b.x};   // 2 Z[0] = 2 (a_0, a'_0)
-      v[n1] = cmulf(cadd(zm, cmulf(om, zp)), tw[m]);
+      const int m = n1 * R2 + lt;
+      const float4 z = xy[m];
+      const float2 zm{z.x, z.y}, zp{z.z, z.w};
+      float2 t{1.0f, 0.0f};
+      if (gr) t = tw[m];
+      // (zm + om zp) t with the rounding written out: it does not hang on how
+      // the compiler contracts it here
+      const float2 q{__fadd_rn(zm.x, __fmaf_rn(om.x, zp.x, -__fmul_rn(om.y, zp.y))),
+                     __fadd_rn(zm.y, __fmaf_rn(om.x, zp.y, __fmul_rn(om.y, zp.x)))};
+      v[n1] = float2{__fmaf_rn(q.x, t.x, -__fmul_rn(q.y, t.y)), __fmaf_rn(q.x, t.y, __fmul_rn(q.y, t.x))};
     }
     dftr<R1, +1>(v);
-    float2 *T = X + grp * TG;
 #pragma unroll
-    for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = (k1 == 0) ? v[0] : cmulf(v[k1], TWM[lt * WP + k1]);
+    for (int k1 = 0; k1 < R1; k1++) W[k1 * TP + lt] = (k1 == 0) ? v[0] : cmulf(v[k1], TWM[lt * WP + k1]);
   }
-  // the transpose block T of a group is written and read by the group's own
-  // R2 threads, which sit in one warp
+  // the block W of a group is written and read by the group's own R2 threads,
+  // which sit in one warp
   __syncwarp();
   // ---- backward, step 2: row k1 = lt -> grid samples j = 3 (k1 + R1 k2) + r
   float2 w[RU][R2];
   if (grp < 21) {
 #pragma unroll
     for (int u = 0; u < RU; u++) {
-      const float2 *T = X + grp * TG + (lt + R2 * u) * TP;
+      const float2 *T = W + (lt + R2 * u) * TP;
 #pragma unroll
       for (int n2 = 0; n2 < R2; n2++) w[u][n2] = T[n2];
       dftr<R2, +1>(w[u]);
     }
   }
-  __syncthreads();
+  __syncwarp();
   if (grp < 21) {
 #pragma unroll
     for (int u = 0; u < RU; u++) {
-      float2 *G = X + gp * N + 3 * (lt + R2 * u) + gr;
 #pragma unroll
-      for (int k2 = 0; k2 < R2; k2++) G[3 * R1 * k2] = w[u][k2];
+      for (int k2 = 0; k2 < R2; k2++) W[lt + R2 * u + R1 * k2] = w[u][k2];
     }
   }
   __syncthreads();
@@ -604,53 +632,52 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
     const float cv = 0.25f * (float)pc.cv, cl = 0.25f * (float)pc.cl, ci = 0.25f * (float)pc.ci,
                 ct = 0.25f * (float)pc.ct;
     for (int q = tid; q < N; q += NT) {
-      const float2 p0 = X[0 * N + q], p1 = X[1 * N + q], p2 = X[2 * N + q], p3 = X[3 * N + q];
-      const float2 p4 = X[4 * N + q], p5 = X[5 * N + q], p6 = X[6 * N + q];
+      float2 *G = X + (q / M) * TG + q % M;
+      constexpr int PT = 3 * TG;
+      const float2 p0 = G[0 * PT], p1 = G[1 * PT], p2 = G[2 * PT], p3 = G[3 * PT];
+      const float2 p4 = G[4 * PT], p5 = G[5 * PT], p6 = G[6 * PT];
       const float ur = p0.x, ut = p0.y, up = p1.x, wr = p1.y, wt = p2.x, wp = p2.y;
       const float br = p3.x, bt = p3.y, bp = p4.x, jr = p4.y, jt = p5.x, jp = p5.y, tt = p6.x;
-      X[0 * N + q] = float2{(wt * up - wp * ut) * cv, (wp * ur - wr * up) * cv};
-      X[1 * N + q] = float2{(wr * ut - wt * ur) * cv, (jt * bp - jp * bt) * cl};
-      X[2 * N + q] = float2{(jp * br - jr * bp) * cl, (jr * bt - jt * br) * cl};
-      X[3 * N + q] = float2{(ut * bp - up * bt) * ci, (up * br - ur * bp) * ci};
-      X[4 * N + q] = float2{(ur * bt - ut * br) * ci, ur * tt * ct};
-      X[5 * N + q] = float2{ut * tt * ct, up * tt * ct};
+      G[0 * PT] = float2{(wt * up - wp * ut) * cv, (wp * ur - wr * up) * cv};
+      G[1 * PT] = float2{(wr * ut - wt * ur) * cv, (jt * bp - jp * bt) * cl};
+      G[2 * PT] = float2{(jp * br - jr * bp) * cl, (jr * bt - jt * br) * cl};
+      G[3 * PT] = float2{(ut * bp - up * bt) * ci, (up * br - ur * bp) * ci};
+      G[4 * PT] = float2{(ur * bt - ut * br) * ci, ur * tt * ct};
+      G[5 * PT] = float2{ut * tt * ct, up * tt * ct};
     }
   }
   __syncthreads();
   // ---- forward, step 1: column n2 = lt of the samples j = 3 (n1 R2 + n2) + r
   float2 v[R1];
   if (grp < 18) {
-    const float2 *G = X + gp * N + 3 * lt + gr;
 #pragma unroll
-    for (int n1 = 0; n1 < R1; n1++) v[n1] = G[3 * R2 * n1];
+    for (int n1 = 0; n1 < R1; n1++) v[n1] = W[n1 * R2 + lt];
     dftr<R1, -1>(v);
 #pragma unroll
     for (int k1 = 1; k1 < R1; k1++) v[k1] = cmulc(v[k1], TWM[lt * WP + k1]);
   }
-  __syncthreads();
+  __syncwarp();
   if (grp < 18) {
-    float2 *T = X + grp * TG;
 #pragma unroll
-    for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = v[k1];
+    for (int k1 = 0; k1 < R1; k1++) W[k1 * TP + lt] = v[k1];
   }
-  __syncwarp();   // the group's own transpose block, as in the backward steps
+  __syncwarp();
   // ---- forward, step 2: row k1 = lt -> F_r[k1 + R1 k2]
   if (grp < 18) {
 #pragma unroll
     for (int u = 0; u < RU; u++) {
-      const float2 *T = X + grp * TG + (lt + R2 * u) * TP;
+      const float2 *T = W + (lt + R2 * u) * TP;
 #pragma unroll
       for (int n2 = 0; n2 < R2; n2++) w[u][n2] = T[n2];
       dftr<R2, -1>(w[u]);
     }
   }
-  __syncthreads();
+  __syncwarp();
   if (grp < 18) {
 #pragma unroll
     for (int u = 0; u < RU; u++) {
-      float2 *F = X + grp * M + lt + R2 * u;   // [pair][r][M]: grp = 3 p + r
 #pragma unroll
-      for (int k2 = 0; k2 < R2; k2++) F[R1 * k2] = w[u][k2];
+      for (int k2 = 0; k2 < R2; k2++) W[lt + R2 * u + R1 * k2] = w[u][k2];
     }
   }
   __syncthreads();
@@ -672,18 +699,18 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
     };
     for (int idx = tid; idx < 6 * MH; idx += NT) {
       const int p = idx / MH, m = idx - p * MH, mm = (M - m) & (M - 1);
-      const float2 *F = X + p * 3 * M;
+      const float2 *F = X + p * 3 * TG;
       float2 *o0 = O2 + (2 * p) * MP2, *o1 = o0 + MP2;
-      const float2 f0 = F[m], f1 = F[M + m], f2 = F[2 * M + m];
-      const float2 g0 = F[mm], g1 = F[M + mm], g2 = F[2 * M + mm];
+      const float2 f0 = F[m], f1 = F[TG + m], f2 = F[2 * TG + m];
+      const float2 g0 = F[mm], g1 = F[TG + mm], g2 = F[2 * TG + mm];
       {
-        const float2 t1 = TW3[M + m], t2 = TW3[2 * M + m];
+        const float2 t1 = TW3[m], t2 = TW3[P::TWP + m];
         const float2 zk = cadd(f0, cadd(cmulc(f1, t1), cmulc(f2, t2)));
         const float2 zn = cadd(g0, cadd(cmulf(g1, t1), cmulf(g2, t2)));
         out(o0, o1, m, zk, zn);
       }
       if (m > 0 && mm != m) {   // the partner order M - m
-        const float2 t1 = TW3[M + mm], t2 = TW3[2 * M + mm];
+        const float2 t1 = TW3[mm], t2 = TW3[P::TWP + mm];
         const float2 zk = cadd(g0, cadd(cmulc(g1, t1), cmulc(g2, t2)));
         const float2 zn = cadd(f0, cadd(cmulf(f1, t1), cmulf(f2, t2)));
         out(o0, o1, mm, zk, zn);
@@ -718,37 +745,114 @@ k_fft_products_4s(MLayout fin, MLayout fout, const float2 *__restrict__ tables, 
     const float wt = __ldg(wgt + th);
     const size_t E = fout.sP() + fout.sD();
     float *pm = pmax + (size_t)th * MB * E;
-    for (int t = tid; t < 24 * MB; t += NT) {
-      const int j = t % 24, mb = t / 24;
-      int c, sg;
-      m_comp_of_out(j, c, sg);
-      const float *row = reinterpret_cast<const float *>(O2 + c * MP2 + mb * 16) + sg;
-      float mx = 0.0f;
+    for (int t = tid; t < 12 * MB; t += NT) {
+      const int c = t % 12, mb = t / 12, v = c / 3, s = c - 3 * v;
+      const float2 *row = O2 + c * MP2 + mb * 16;
+      float ma = 0.0f, mc = 0.0f;
 #pragma unroll
-      for (int u = 0; u < 16; u++) mx = fmaxf(mx, fabsf(row[2 * u]));
-      const size_t e = (j < 8) ? (size_t)k * 8 + j : fout.sP() + (size_t)k * 16 + (j - 8);
-      pm[(size_t)mb * E + e] = mx * wt;
+      for (int u = 0; u < 16; u++) {
+        const float2 x = row[u];
+        ma = fmaxf(ma, fabsf(x.x));
+        mc = fmaxf(mc, fabsf(x.y));
+      }
+      const size_t e = (s == 0) ? (size_t)k * 8 + 2 * v : fout.sP() + (size_t)k * 16 + 2 * (2 * v + s - 1);
+      *reinterpret_cast<float2 *>(pm + (size_t)mb * E + e) = float2{ma * wt, mc * wt};
     }
   }
 }
 
 // ---------------------------------------------------------------------------
+// Input of the float64 four-step kernels, as in k_fft_products_4s: a thread
+// takes a pair of components at the orders m and M - m.  rows: [7][M + 1]
+// 2 Z[m], then [7][M + 1] 2 Z[N - (M - m)] of the pairs, the second component
+// scaled to the first; cmx: [0, 14) the components' maxima, the rest of its
+// ncmx entries zero.  Ends with the rows written, not yet a barrier.
+template <int M, int NT>
+__device__ __forceinline__ void stage_pairs64(const MLayout64 &fin, int th, int k, double2 *S2, PairBits<double>::U *cmx,
+                                              int ncmx) {
+  using PB = PairBits<double>;
+  using U = PB::U;
+  constexpr int MP2 = M + 1;
+  const int tid = threadIdx.x, lane = tid & 31;
+  constexpr int IT = (4 * M + NT - 1) / NT;
+  const int p = tid & 7;
+  auto comp = [&](int c, const double *&src, size_t &mst) {
+    const int v = c / 3, s = c - 3 * v;
+    if (s == 0) {
+      src = fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + 2 * v;
+      mst = (size_t)fin.nth * fin.sP();
+    } else {
+      src = fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + 2 * (2 * v + s - 1);
+      mst = (size_t)fin.nth * fin.sD();
+    }
+  };
+  const double *s0, *s1;
+  size_t t0, t1;
+  comp(min(2 * p, 12), s0, t0);
+  comp(min(2 * p + 1, 12), s1, t1);
+  double2 a[IT], b[IT], c[IT], d[IT];
+#pragma unroll
+  for (int i = 0; i < IT; i++) {
+    const int mi = (tid + i * NT) >> 3, mj = mi ? M - mi : M / 2;
+    const bool on = p < 7 && mi < M / 2;
+    const double2 z{0.0, 0.0};
+    a[i] = on ? __ldg(reinterpret_cast<const double2 *>(s0 + mi * t0)) : z;
+    c[i] = on ? __ldg(reinterpret_cast<const double2 *>(s0 + mj * t0)) : z;
+    b[i] = (on && p < 6) ? __ldg(reinterpret_cast<const double2 *>(s1 + mi * t1)) : z;
+    d[i] = (on && p < 6) ? __ldg(reinterpret_cast<const double2 *>(s1 + mj * t1)) : z;
+  }
+  if (tid < ncmx) cmx[tid] = 0;
+  __syncthreads();
+  U m0 = 0, m1 = 0;
+#pragma unroll
+  for (int i = 0; i < IT; i++) {
+    m0 = max(max(m0, max(PB::abs_bits(a[i].x), PB::abs_bits(a[i].y))), max(PB::abs_bits(c[i].x), PB::abs_bits(c[i].y)));
+    m1 = max(max(m1, max(PB::abs_bits(b[i].x), PB::abs_bits(b[i].y))), max(PB::abs_bits(d[i].x), PB::abs_bits(d[i].y)));
+  }
+#pragma unroll
+  for (int o = 8; o <= 16; o *= 2) {
+    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+  if (lane < 7) {
+    atomicMax(cmx + 2 * p, m0);
+    atomicMax(cmx + 2 * p + 1, m1);
+  }
+  __syncthreads();
+  const double sy = (p < 6) ? PB::factor(cmx[2 * p], cmx[2 * p + 1], false) : 1.0;
+  double2 *rm = S2 + p * MP2, *rp = S2 + (7 + p) * MP2;
+#pragma unroll
+  for (int i = 0; i < IT; i++) {
+    const int mi = (tid + i * NT) >> 3, mj = mi ? M - mi : M / 2;
+    if (p < 7 && mi < M / 2) {
+      const double2 A = a[i], C = c[i], B{b[i].x * sy, b[i].y * sy}, D{d[i].x * sy, d[i].y * sy};
+      // m = 0: 2 Z[0] = 2 (a_0, a'_0) and no partner; m = M / 2 is its own
+      rm[mi] = mi ? double2{A.x + B.y, B.x - A.y} : double2{2.0 * A.x, 2.0 * B.x};
+      rp[mi] = mi ? double2{C.x - D.y, C.y + D.x} : double2{0.0, 0.0};
+      rm[mj] = double2{C.x + D.y, D.x - C.y};
+      rp[mj] = mi ? double2{A.x - B.y, A.y + B.x} : double2{C.x - D.y, C.y + D.x};
+    }
+  }
+}
+
 // The float64 four-step products kernel (the plain path's step): the data
 // flow of k_fft_products_4s on the float64 Fourier rows, with the pair
 // scaling of k_fft_products_g (the second row of each pair, inputs and
 // products, brought to the size of the first), so every row keeps float64
-// precision whatever the sizes of the fields.  One CTA per (theta, k), 384
-// threads, one CTA per SM (166 KB of shared memory at M = 256).
+// precision whatever the sizes of the fields.  One CTA per (theta, k).
 template <int R1, int R2>
 struct F4Plan64 {
   static constexpr int M = R1 * R2, N = 3 * M;
   static constexpr int TP = R2 + 1;
-  static constexpr int TG = R1 * TP;
-  static constexpr int X = (21 * TG > 7 * N) ? 21 * TG : 7 * N;
-  static constexpr int MP2 = M + 1;            // staging row pitch, slot M stays zero
+  // a group's block; 16-byte accesses go eight lanes at a time, two groups of
+  // four at R2 = 4, whose blocks then start four elements apart modulo 8
+  static constexpr int T0 = (R1 * TP > M) ? R1 * TP : M;
+  static constexpr int TG = T0 + (R2 >= 8 ? 0 : (R2 + 8 - T0 % 8) % 8);
+  static constexpr int X = 21 * TG;
+  static constexpr int MP2 = M + 1;            // staging row pitch
   static constexpr int WP = R1 + 1;
-  static constexpr int NTW = 3 * M + R2 * WP;
-  static constexpr int SC = 14 * MP2;          // staging: 14 rows in, then 12 rows out
+  static constexpr int TWP = M + 4, NTW = 2 * TWP + R2 * WP;
+  static constexpr int SC = 14 * MP2;          // staging: Z[m], Z[N - (M - m)] of 7 pairs in, then 12 rows out
   static constexpr size_t smem() { return ((size_t)SC + X + NTW) * sizeof(double2) + 32 * sizeof(double); }
 };
 
@@ -761,99 +865,63 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
   constexpr int NT = f4_threads<R2>(), RU = R1 / R2;
   constexpr int M = P::M, N = P::N, TP = P::TP, TG = P::TG, MP2 = P::MP2, WP = P::WP;
   extern __shared__ __align__(16) unsigned char smraw[];
-  double2 *S2 = reinterpret_cast<double2 *>(smraw);   // [14][MP2] (a_m, b_m); later [12][MP2] out
-  double2 *X = S2 + P::SC;                             // transposes / grid rows / F_r
-  double2 *TW3 = X + P::X;                             // [3][M]
-  double2 *TWM = TW3 + 3 * M;                          // [R2][WP]
-  U *cmx = reinterpret_cast<U *>(TWM + R2 * WP);      // [0, 13) input maxima, [13, 25) products
+  double2 *S2 = reinterpret_cast<double2 *>(smraw);   // [7][MP2] 2 Z[m], [7][MP2] 2 Z[N - (M - m)]; later [12][MP2] out
+  double2 *X = S2 + P::SC;                             // [21 groups][TG]
+  double2 *TW3 = X + P::X;                             // [2][TWP]: r = 1, 2
+  double2 *TWM = TW3 + 2 * P::TWP;                     // [R2][WP]
+  U *cmx = reinterpret_cast<U *>(TWM + R2 * WP);      // [0, 14) input maxima, [14, 26) products
   const int th = blockIdx.x / fin.nr, k = blockIdx.x % fin.nr;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = NT / 32;
   const int grp = tid / R2, lt = tid % R2;
-  for (int e = tid; e < 14; e += NT) S2[e * MP2 + M] = double2{0.0, 0.0};
-  for (int e = tid; e < M; e += NT) S2[13 * MP2 + e] = double2{0.0, 0.0};
-  // input and tables by asynchronous 16-byte copies, as in k_fft_products_4s
-  auto cp16 = [](double2 *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-  };
-  for (int e = tid; e < P::NTW; e += NT) cp16(TW3 + e, tables + e);
-  {
-    const int j = lane & 15, hw = lane >> 4;
-    int c = 0;
-    const double *src = fin.P;
-    size_t mst = 0;
-    if (j < 5) {
-      c = (j < 4) ? 3 * j : 12;
-      src = fin.P + (size_t)th * fin.sP() + (size_t)k * 10 + 2 * j;
-      mst = (size_t)fin.nth * fin.sP();
-    } else if (j < 13) {
-      const int jd = j - 5;
-      c = 3 * (jd >> 1) + 1 + (jd & 1);
-      src = fin.D + (size_t)th * fin.sD() + (size_t)k * 16 + 2 * jd;
-      mst = (size_t)fin.nth * fin.sD();
-    }
-    if (j < 13)
-      for (int m = 2 * warp + hw; m < M; m += 2 * nwarp) cp16(S2 + c * MP2 + m, src + m * mst);
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  // tables by asynchronous copies
+  for (int e = tid; e < 2 * M + R2 * WP; e += NT) {
+    const int to = (e < M) ? e : (e < 2 * M) ? P::TWP + e - M : 2 * P::TWP + e - 2 * M;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(TW3 + to)),
+                 "l"(tables + M + e) : "memory");
   }
-  if (tid < 12) cmx[13 + tid] = 0;
-  __syncthreads();
-  // largest magnitude of each input row (one warp per row)
-  for (int c = warp; c < 13; c += nwarp) {
-    U mx = 0;
-    for (int m = lane; m < M; m += 32) {
-      const double2 v = S2[c * MP2 + m];
-      mx = max(mx, max(PB::abs_bits(v.x), PB::abs_bits(v.y)));
-    }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (lane == 0) cmx[c] = mx;
-  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  stage_pairs64<M, NT>(fin, th, k, S2, cmx, 26);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   const int gp = grp / 3, gr = grp - 3 * gp;
-  // ---- backward, step 1: column n2 = lt, pair rows from the staging (the
-  // second row of the pair scaled by sy)
+  double2 *W = X + grp * TG;   // the group's block, written and read by its own threads (one warp)
+  // ---- backward, step 1: column n2 = lt
   if (grp < 21) {
-    const double2 *x0 = S2 + (2 * gp) * MP2, *y0 = S2 + (2 * gp + 1) * MP2;
-    const double sy = (2 * gp + 1 < 13) ? PB::factor(cmx[2 * gp], cmx[2 * gp + 1], false) : 1.0;
+    const double2 *rm = S2 + gp * MP2, *rp = S2 + (7 + gp) * MP2;
     const double2 om = (gr == 0) ? double2{1.0, 0.0}
                      : double2{-0.5, (gr == 1) ? -0.86602540378443864676 : 0.86602540378443864676};
-    const double2 *tw = TW3 + gr * M;
+    const double2 *tw = TW3 + (gr == 2 ? P::TWP : 0);
     double2 v[R1];
 #pragma unroll
     for (int n1 = 0; n1 < R1; n1++) {
-      const int m = n1 * R2 + lt, mq = M - m;
-      const double2 a = x0[m], c = x0[mq];
-      const double2 b = double2{y0[m].x * sy, y0[m].y * sy}, d = double2{y0[mq].x * sy, y0[mq].y * sy};
-      double2 zm = double2{a.x + b.y, b.x - a.y};           // 2 Z[m]
-      const double2 zp = double2{c.x - d.y, c.y + d.x};     // 2 Z[N - (M - m)] (zero at m = 0)
-      if (n1 == 0 && lt == 0) zm = double2{2.0 * a.x, 2.0 * b.x};
-      v[n1] = cmulf(cadd(zm, cmulf(om, zp)), tw[m]);
+      const int m = n1 * R2 + lt;
+      double2 t{1.0, 0.0};
+      if (gr) t = tw[m];
+      v[n1] = cmulf(cadd(rm[m], cmulf(om, rp[m])), t);
     }
     dftr<R1, +1>(v);
-    double2 *T = X + grp * TG;
 #pragma unroll
-    for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = (k1 == 0) ? v[0] : cmulf(v[k1], TWM[lt * WP + k1]);
+    for (int k1 = 0; k1 < R1; k1++) W[k1 * TP + lt] = (k1 == 0) ? v[0] : cmulf(v[k1], TWM[lt * WP + k1]);
   }
-  __syncwarp();   // the group's own transpose block
+  __syncwarp();
   // ---- backward, step 2: row k1 = lt -> grid samples j = 3 (k1 + R1 k2) + r
   {
     double2 w[RU][R2];
     if (grp < 21) {
 #pragma unroll
       for (int u = 0; u < RU; u++) {
-        const double2 *T = X + grp * TG + (lt + R2 * u) * TP;
+        const double2 *T = W + (lt + R2 * u) * TP;
 #pragma unroll
         for (int n2 = 0; n2 < R2; n2++) w[u][n2] = T[n2];
         dftr<R2, +1>(w[u]);
       }
     }
-    __syncthreads();
+    __syncwarp();
     if (grp < 21) {
 #pragma unroll
       for (int u = 0; u < RU; u++) {
-        double2 *G = X + gp * N + 3 * (lt + R2 * u) + gr;
 #pragma unroll
-        for (int k2 = 0; k2 < R2; k2++) G[3 * R1 * k2] = w[u][k2];
+        for (int k2 = 0; k2 < R2; k2++) W[lt + R2 * u + R1 * k2] = w[u][k2];
       }
     }
   }
@@ -869,8 +937,10 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
 #pragma unroll
     for (int c = 0; c < 12; c++) hm[c] = 0;
     for (int q = tid; q < N; q += NT) {
-      const double2 p0 = X[0 * N + q], p1 = X[1 * N + q], p2 = X[2 * N + q], p3 = X[3 * N + q];
-      const double2 p4 = X[4 * N + q], p5 = X[5 * N + q], p6 = X[6 * N + q];
+      double2 *G = X + (q / M) * TG + q % M;
+      constexpr int PT = 3 * TG;
+      const double2 p0 = G[0 * PT], p1 = G[1 * PT], p2 = G[2 * PT], p3 = G[3 * PT];
+      const double2 p4 = G[4 * PT], p5 = G[5 * PT], p6 = G[6 * PT];
       const double ur = p0.x, ut = p0.y * iy[0], up = p1.x, wr = p1.y * iy[1], wt = p2.x, wp = p2.y * iy[2];
       const double br = p3.x, bt = p3.y * iy[3], bp = p4.x, jr = p4.y * iy[4], jt = p5.x, jp = p5.y * iy[5];
       const double tt = p6.x;
@@ -882,7 +952,7 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
                              double2{ut * tt * ct, up * tt * ct}};
 #pragma unroll
       for (int p = 0; p < 6; p++) {
-        X[p * N + q] = hv[p];
+        G[p * PT] = hv[p];
         hm[2 * p] = max(hm[2 * p], PB::abs_bits(hv[p].x));
         hm[2 * p + 1] = max(hm[2 * p + 1], PB::abs_bits(hv[p].y));
       }
@@ -890,7 +960,7 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
 #pragma unroll
     for (int c = 0; c < 12; c++) {
       const U v = __reduce_max_sync(0xffffffffu, hm[c]);
-      if (lane == 0) atomicMax(cmx + 13 + c, v);
+      if (lane == 0) atomicMax(cmx + 14 + c, v);
     }
   }
   __syncthreads();
@@ -899,22 +969,20 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
   {
     double2 v[R1];
     if (grp < 18) {
-      const double2 *G = X + gp * N + 3 * lt + gr;
-      const double sy = PB::factor(cmx[13 + 2 * gp], cmx[14 + 2 * gp], false);
+      const double sy = PB::factor(cmx[14 + 2 * gp], cmx[15 + 2 * gp], false);
 #pragma unroll
       for (int n1 = 0; n1 < R1; n1++) {
-        v[n1] = G[3 * R2 * n1];
+        v[n1] = W[n1 * R2 + lt];
         v[n1].y *= sy;
       }
       dftr<R1, -1>(v);
 #pragma unroll
       for (int k1 = 1; k1 < R1; k1++) v[k1] = cmulc(v[k1], TWM[lt * WP + k1]);
     }
-    __syncthreads();
+    __syncwarp();
     if (grp < 18) {
-      double2 *T = X + grp * TG;
 #pragma unroll
-      for (int k1 = 0; k1 < R1; k1++) T[k1 * TP + lt] = v[k1];
+      for (int k1 = 0; k1 < R1; k1++) W[k1 * TP + lt] = v[k1];
     }
   }
   __syncwarp();
@@ -924,19 +992,18 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
     if (grp < 18) {
 #pragma unroll
       for (int u = 0; u < RU; u++) {
-        const double2 *T = X + grp * TG + (lt + R2 * u) * TP;
+        const double2 *T = W + (lt + R2 * u) * TP;
 #pragma unroll
         for (int n2 = 0; n2 < R2; n2++) w[u][n2] = T[n2];
         dftr<R2, -1>(w[u]);
       }
     }
-    __syncthreads();
+    __syncwarp();
     if (grp < 18) {
 #pragma unroll
       for (int u = 0; u < RU; u++) {
-        double2 *F = X + grp * M + lt + R2 * u;   // [pair][r][M]: grp = 3 p + r
 #pragma unroll
-        for (int k2 = 0; k2 < R2; k2++) F[R1 * k2] = w[u][k2];
+        for (int k2 = 0; k2 < R2; k2++) W[lt + R2 * u + R1 * k2] = w[u][k2];
       }
     }
   }
@@ -947,11 +1014,11 @@ k_fft_products_4s64(MLayout64 fin, MLayout64 fout, const double2 *__restrict__ t
     const double an = 1.0 / (double)N;
     for (int idx = tid; idx < 6 * M; idx += NT) {
       const int p = idx / M, m = idx - p * M, mm = (M - m) & (M - 1);
-      const double2 *F = X + p * 3 * M;
-      const double2 t1 = TW3[M + m], t2 = TW3[2 * M + m];
-      const double2 zk = cadd(F[m], cadd(cmulc(F[M + m], t1), cmulc(F[2 * M + m], t2)));
-      const double2 zn = cadd(F[mm], cadd(cmulf(F[M + mm], t1), cmulf(F[2 * M + mm], t2)));
-      const double ay = an * PB::factor(cmx[13 + 2 * p], cmx[14 + 2 * p], true);
+      const double2 *F = X + p * 3 * TG;
+      const double2 t1 = TW3[m], t2 = TW3[P::TWP + m];
+      const double2 zk = cadd(F[m], cadd(cmulc(F[TG + m], t1), cmulc(F[2 * TG + m], t2)));
+      const double2 zn = cadd(F[mm], cadd(cmulf(F[TG + mm], t1), cmulf(F[2 * TG + mm], t2)));
+      const double ay = an * PB::factor(cmx[14 + 2 * p], cmx[15 + 2 * p], true);
       double2 *o0 = S2 + (2 * p) * MP2, *o1 = S2 + (2 * p + 1) * MP2;
       if (m == 0) {
         o0[0] = double2{an * zk.x, 0.0};
@@ -1704,7 +1771,7 @@ template <int R1, int R2>
 static int attr_fft_4s(Ctx &c) {
   using P = F4Plan<R1, R2>;
   CB2_CUDA(raise_smem_limit(k_fft_products_4s<R1, R2>, (int)P::smem()));
-  std::vector<float2> t(P::NTW, float2{0.0f, 0.0f});
+  std::vector<float2> t(3 * P::M + R2 * P::WP, float2{0.0f, 0.0f});
   const double pi = 3.14159265358979323846;
   for (int r = 0; r < 3; r++)
     for (int m = 0; m < P::M; m++) {
@@ -1726,7 +1793,7 @@ static int attr_fft_4s64(Ctx &c) {
   using P = F4Plan64<R1, R2>;
   if constexpr (R2 == 16) CB2_CUDA(raise_smem_limit(k_fft_products_4s64r<R1, R2>, F4Plan64R<R1, R2>::smem()));
   else CB2_CUDA(raise_smem_limit(k_fft_products_4s64<R1, R2>, P::smem()));
-  std::vector<double2> t(P::NTW, double2{0.0, 0.0});
+  std::vector<double2> t(3 * P::M + R2 * P::WP, double2{0.0, 0.0});
   const double pi = 3.14159265358979323846;
   for (int r = 0; r < 3; r++)
     for (int m = 0; m < P::M; m++) {
