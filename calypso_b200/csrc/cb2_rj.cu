@@ -782,98 +782,131 @@ struct CorTables {
   const double *sw, *tw;   // [6][jmax], [8][jmax]
 };
 
-__device__ inline void coriolis_terms(const RJArgs &a, const Fields &F, const CorTables &ct, int jj, int k,
-                                      double &rc0, double &rc2) {
-  size_t base = (size_t)k * a.jmax, J = a.jmax;
-  const double *vS = F(VELO), *vdS = F(VELO + 1), *wS = F(VORT), *wdS = F(VORT + 1), *wT = F(VORT + 2);
-  const double *sw = ct.sw, *tw = ct.tw;
-  size_t i11 = base + ct.jgi1[jj], i21 = base + ct.jgi2[jj], i12 = base + ct.jei1[jj];
-  double a1 = a.ar1[k], o0 = a.om[k], o1 = a.om[a.nr + k], o2 = a.om[2 * a.nr + k];
-  double d2vp_l1 = a1 * a1 * a.g3rlm[jj] * vS[i12] - wT[i12];
-  double dwp1 = wdS[i11] - 2.0 * a1 * wS[i11];
-  double dwp2 = wdS[i21] - 2.0 * a1 * wS[i21];
-  double p = sw[0 * J + jj] * o0 * vdS[i11] + sw[1 * J + jj] * o0 * vdS[i21]
-           + sw[4 * J + jj] * o0 * wS[i12] + sw[2 * J + jj] * o1 * vS[i11]
-           + sw[3 * J + jj] * o1 * vS[i21];
-  double t = tw[0 * J + jj] * o0 * d2vp_l1 - tw[2 * J + jj] * o2 * vS[i12]
-           + tw[4 * J + jj] * o1 * wS[i11] + tw[5 * J + jj] * o1 * wS[i21]
-           + tw[6 * J + jj] * o0 * dwp1 + tw[7 * J + jj] * o0 * dwp2;
-  rc0 = -a.coef_cor * p * a1 * a1;
-  rc2 = -a.coef_cor * t * a1 * a1;
-}
+// the couplings of one (l, m): columns of the three neighbours and weights
+struct CorCol {
+  int j11, j21, j12;
+  double g3, sw[5], tw[6];
+  __device__ __forceinline__ CorCol(const RJArgs &a, const CorTables &ct, int jj)
+      : j11(ct.jgi1[jj]), j21(ct.jgi2[jj]), j12(ct.jei1[jj]), g3(a.g3rlm[jj]) {
+    const size_t J = a.jmax;
+#pragma unroll
+    for (int i = 0; i < 5; i++) sw[i] = ct.sw[i * J + jj];
+#pragma unroll
+    for (int i = 0; i < 6; i++) tw[i] = ct.tw[(i == 0 ? 0 : i == 1 ? 2 : i + 2) * J + jj];   // 0, 2, 4 .. 7
+  }
+};
 
 // curl / divergence of the transformed forces and the force sum
 // (const_sph_force_rot2, const_sph_rotation_uxb, const_sph_scalar_advect,
-//  add_reftemp_advect_sph_MHD, set_MHD_terms_to_force)
-__global__ void k_after_transform(RJArgs a, Fields F, CorTables ct) {
-  // grid (jj blocks, radial level k): no division to find k and jj
-  const int jj = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+//  add_reftemp_advect_sph_MHD, set_MHD_terms_to_force).
+// A thread takes kl radial levels of one (l, m): the rows k - 1, k, k + 1 of
+// the seven differentiated fields slide through registers and the Coriolis
+// weights are read once.  Bound by HBM and the latency of the rows.  A thread
+// per point read every row three times and the 16 table entries at each level
+// (L2 traffic three times that of DRAM): 432 -> 372 us at L255 / Nr129, 84 ->
+// 77 us at L127 / Nr97.
+constexpr int AT_THREADS = 128, AT_LEVELS = 8;
+
+__global__ void __launch_bounds__(AT_THREADS, 4) k_after_transform(RJArgs a, Fields F, CorTables ct, int kl) {
+  const int jj = blockIdx.x * AT_THREADS + threadIdx.x;
   if (jj >= a.jmax) return;
-  const size_t idx = (size_t)k * a.jmax + jj;
-  size_t s = a.jmax;
+  const size_t s = a.jmax;
   const BCW &b = a.bc;
-  double g3 = a.g3[jj], gl = a.gl[jj];
-  int ki = a.kin, ko = a.kout;
-  double rot[2][3];
-  const int src[2] = {MADV, LOR};
-  for (int q = 0; q < 2; q++) {
-    const double *fS = F(src[q]), *fdS = F(src[q] + 1), *fT = F(src[q] + 2);
-    if (k == ki) {
-      double d2s = b.fix_dr_icb[1][3] * fS[idx] + b.fix_dr_icb[2][3] * fS[idx + s];
-      double d1t = b.fix_fld_icb[0][2] * fT[idx] + b.fix_fld_icb[1][2] * fT[idx + s]
-                 + b.fix_fld_icb[2][2] * fT[idx + 2 * s];
-      rot[q][0] = fT[idx]; rot[q][1] = d1t; rot[q][2] = -(d2s - g3 * b.r_icb[2] * fS[idx]);
-    } else if (k == ko) {
-      double d2s = b.fix_dr_cmb[0][3] * fS[idx - s] + b.fix_dr_cmb[1][3] * fS[idx];
-      double d1t = b.fix_fld_cmb[2][2] * fT[idx - 2 * s] + b.fix_fld_cmb[1][2] * fT[idx - s]
-                 + b.fix_fld_cmb[0][2] * fT[idx];
-      rot[q][0] = fT[idx]; rot[q][1] = d1t; rot[q][2] = -(d2s - g3 * b.r_cmb[2] * fS[idx]);
-    } else if (k > ki && k < ko) {
-      rot[q][0] = fT[idx];
-      rot[q][1] = D1(a, fT, k, jj);
-      rot[q][2] = -D1(a, fdS, k, jj) + g3 * a.ar2[k] * fS[idx];
-    } else {
-      rot[q][0] = rot[q][1] = rot[q][2] = 0.0;
+  const double g3 = a.g3[jj], gl = a.gl[jj];
+  const int ki = a.kin, ko = a.kout, n = a.nr;
+  const int k0 = blockIdx.y * kl, k1 = min(k0 + kl, n);
+  const CorCol cc(a, ct, jj);
+  // poloidal derivative and toroidal part of the three forces, the heat flux
+  const int dif[7] = {MADV + 1, MADV + 2, LOR + 1, LOR + 2, VPIND + 1, VPIND + 2, HFLUX};
+  double w[7][3];
+#pragma unroll
+  for (int f = 0; f < 7; f++) {
+    w[f][1] = (k0 > 0) ? __ldg(F(dif[f]) + (k0 - 1) * s + jj) : 0.0;
+    w[f][2] = __ldg(F(dif[f]) + k0 * s + jj);
+  }
+  for (int k = k0; k < k1; k++) {
+    const size_t idx = k * s + jj;
+#pragma unroll
+    for (int f = 0; f < 7; f++) {
+      w[f][0] = w[f][1];
+      w[f][1] = w[f][2];
+      w[f][2] = (k + 1 < n) ? __ldg(F(dif[f]) + idx + s) : 0.0;
     }
-  }
-  for (int c = 0; c < 3; c++) {
-    F(ROTINERT + c)[idx] = rot[0][c];
-    F(ROTLOR + c)[idx] = rot[1][c];
-  }
-  // induction
-  {
-    const double *fS = F(VPIND), *fdS = F(VPIND + 1), *fT = F(VPIND + 2);
-    double r0, r1, r2;
-    if (k == ki) { r0 = fT[idx]; r1 = (gl + 1.0) * b.r_icb[1] * fT[idx]; r2 = 0.0; }
-    else if (k == ko) { r0 = fT[idx]; r1 = -gl * b.r_cmb[1] * fT[idx]; r2 = 0.0; }
-    else if (k > ki && k < ko) {
-      r0 = fT[idx]; r1 = D1(a, fT, k, jj); r2 = -D1(a, fdS, k, jj) + g3 * a.ar2[k] * fS[idx];
-    } else { r0 = r1 = r2 = 0.0; }
-    F(INDUCT)[idx] = r0; F(INDUCT + 1)[idx] = r1; F(INDUCT + 2)[idx] = r2;
-  }
-  // heat advection
-  {
-    const double *fS = F(HFLUX), *fdS = F(HFLUX + 1);
-    double gm = fmax(g3, 0.5), h = 0.0;
-    if (k == ki) {
-      double d1s = b.fix_fld_icb[0][2] * icb_fld(a, jj) + b.fix_fld_icb[1][2] * fS[idx + s]
-                 + b.fix_fld_icb[2][2] * fS[idx + 2 * s];
-      h = (d1s - fdS[idx]) * gm * b.r_icb[2];
-    } else if (k == ko) {
-      double d1s = b.fix_fld_cmb[2][2] * fS[idx - 2 * s] + b.fix_fld_cmb[1][2] * fS[idx - s]
-                 + b.fix_fld_cmb[0][2] * cmb_fld(a, jj);
-      h = (d1s - fdS[idx]) * gm * b.r_cmb[2];
-    } else if (k > ki && k < ko) {
-      h = (D1(a, fS, k, jj) - fdS[idx]) * gm * a.ar2[k];
+    const double pol[3] = {__ldg(F(MADV) + idx), __ldg(F(LOR) + idx), __ldg(F(VPIND) + idx)};
+    const double dhf = __ldg(F(HFLUX + 1) + idx), vel = __ldg(F(VELO) + idx), buo = __ldg(F(ROTBUO + 2) + idx);
+    const size_t i11 = k * s + cc.j11, i21 = k * s + cc.j21, i12 = k * s + cc.j12;
+    const double *vS = F(VELO), *vdS = F(VELO + 1), *wS = F(VORT), *wdS = F(VORT + 1), *wT = F(VORT + 2);
+    const double vS11 = __ldg(vS + i11), vS21 = __ldg(vS + i21), vS12 = __ldg(vS + i12);
+    const double vd11 = __ldg(vdS + i11), vd21 = __ldg(vdS + i21);
+    const double wS11 = __ldg(wS + i11), wS21 = __ldg(wS + i21), wS12 = __ldg(wS + i12);
+    const double wd11 = __ldg(wdS + i11), wd21 = __ldg(wdS + i21), wT12 = __ldg(wT + i12);
+    const double da = a.d1[k], db = a.d1[n + k], dc = a.d1[2 * n + k], r2 = a.ar2[k];
+    auto d1 = [&](int f) { return da * w[f][0] + db * w[f][1] + dc * w[f][2]; };
+    double rot[3][3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const double T = w[2 * q + 1][1];
+      rot[q][0] = T;
+      if (k > ki && k < ko) {
+        rot[q][1] = d1(2 * q + 1);
+        rot[q][2] = -d1(2 * q) + g3 * r2 * pol[q];
+      } else if (k == ki || k == ko) {
+        const double *fS = F(q == 0 ? MADV : q == 1 ? LOR : VPIND), *fT = fS + 2 * F.fs;
+        if (q == 2) {   // induction: potential field outside
+          rot[q][1] = (k == ki) ? (gl + 1.0) * b.r_icb[1] * T : -gl * b.r_cmb[1] * T;
+          rot[q][2] = 0.0;
+        } else if (k == ki) {
+          const double d2s = b.fix_dr_icb[1][3] * pol[q] + b.fix_dr_icb[2][3] * fS[idx + s];
+          rot[q][1] = b.fix_fld_icb[0][2] * T + b.fix_fld_icb[1][2] * fT[idx + s]
+                    + b.fix_fld_icb[2][2] * fT[idx + 2 * s];
+          rot[q][2] = -(d2s - g3 * b.r_icb[2] * pol[q]);
+        } else {
+          const double d2s = b.fix_dr_cmb[0][3] * fS[idx - s] + b.fix_dr_cmb[1][3] * pol[q];
+          rot[q][1] = b.fix_fld_cmb[2][2] * fT[idx - 2 * s] + b.fix_fld_cmb[1][2] * fT[idx - s]
+                    + b.fix_fld_cmb[0][2] * T;
+          rot[q][2] = -(d2s - g3 * b.r_cmb[2] * pol[q]);
+        }
+      } else {
+        rot[q][0] = rot[q][1] = rot[q][2] = 0.0;
+      }
     }
-    if (a.use_ref_temp && k >= ki && k <= ko)
-      h = h + a.coef_temp * g3 * a.ar2[k] * a.reft1[k] * F(VELO)[idx];
+    // heat advection
+    const double gm = fmax(g3, 0.5);
+    double h = 0.0;
+    if (k > ki && k < ko) {
+      h = (d1(6) - dhf) * gm * r2;
+    } else if (k == ki) {
+      const double *fS = F(HFLUX);
+      const double d1s = b.fix_fld_icb[0][2] * icb_fld(a, jj) + b.fix_fld_icb[1][2] * fS[idx + s]
+                       + b.fix_fld_icb[2][2] * fS[idx + 2 * s];
+      h = (d1s - dhf) * gm * b.r_icb[2];
+    } else if (k == ko) {
+      const double *fS = F(HFLUX);
+      const double d1s = b.fix_fld_cmb[2][2] * fS[idx - 2 * s] + b.fix_fld_cmb[1][2] * fS[idx - s]
+                       + b.fix_fld_cmb[0][2] * cmb_fld(a, jj);
+      h = (d1s - dhf) * gm * b.r_cmb[2];
+    }
+    if (a.use_ref_temp && k >= ki && k <= ko) h = h + a.coef_temp * g3 * r2 * a.reft1[k] * vel;
+    // Coriolis term
+    const double a1 = a.ar1[k], o0 = a.om[k], o1 = a.om[n + k], o2 = a.om[2 * n + k];
+    const double d2vp_l1 = a1 * a1 * cc.g3 * vS12 - wT12;
+    const double dwp1 = wd11 - 2.0 * a1 * wS11, dwp2 = wd21 - 2.0 * a1 * wS21;
+    const double cp = cc.sw[0] * o0 * vd11 + cc.sw[1] * o0 * vd21 + cc.sw[4] * o0 * wS12 + cc.sw[2] * o1 * vS11
+                    + cc.sw[3] * o1 * vS21;
+    const double tt = cc.tw[0] * o0 * d2vp_l1 - cc.tw[1] * o2 * vS12 + cc.tw[2] * o1 * wS11 + cc.tw[3] * o1 * wS21
+                    + cc.tw[4] * o0 * dwp1 + cc.tw[5] * o0 * dwp2;
+    const double rc0 = -a.coef_cor * cp * a1 * a1, rc2 = -a.coef_cor * tt * a1 * a1;
+    // the curls of inertia and Lorentz force are not read again in the step
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      __stcs(F(ROTINERT + c) + idx, rot[0][c]);
+      __stcs(F(ROTLOR + c) + idx, rot[1][c]);
+      F(INDUCT + c)[idx] = rot[2][c];
+    }
     F(HADV)[idx] = h;
+    F(FORCES)[idx] = -rot[0][0] + rc0 + rot[1][0];
+    F(FORCES + 2)[idx] = -rot[0][2] + rc2 + rot[1][2] + buo;
   }
-  double rc0, rc2;
-  coriolis_terms(a, F, ct, jj, k, rc0, rc2);
-  F(FORCES)[idx] = -rot[0][0] + rc0 + rot[1][0];
-  F(FORCES + 2)[idx] = -rot[0][2] + rc2 + rot[1][2] + F(ROTBUO + 2)[idx];
 }
 
 __global__ void k_temp_total(RJArgs a, Fields F, double sign) {
@@ -956,7 +989,14 @@ void rj_start_derived(Ctx &c) {
 
 void rj_after_transform(Ctx &c) {
   const CorTables ct{c.d_jgi1, c.d_jgi2, c.d_jei1, c.d_sw, c.d_tw};
-  k_after_transform<<<dim3(cdiv(c.jmax, kThreads), c.nr), kThreads, 0, c.stream>>>(c.rj_args(), fields(c), ct);
+  // levels a thread: eight where that leaves four waves of blocks (four
+  // blocks an SM), else as many up to four as leave one.  L255 / Nr129
+  // (14.7 waves of eight) 372 us with eight, 380 with four; L127 / Nr97
+  // (2.8 waves) 79 and 77; a 12-member ensemble 43 and 41 on average.
+  const int nb = cdiv(c.jmax, AT_THREADS), wave = 4 * 148;
+  int kl = (nb * cdiv(c.nr, AT_LEVELS) < 4 * wave) ? AT_LEVELS / 2 : AT_LEVELS;
+  while (kl > 1 && nb * cdiv(c.nr, kl) < wave) kl /= 2;
+  k_after_transform<<<dim3(nb, cdiv(c.nr, kl)), AT_THREADS, 0, c.stream>>>(c.rj_args(), fields(c), ct, kl);
 }
 
 void rj_temp_total(Ctx &c, double sign) {
