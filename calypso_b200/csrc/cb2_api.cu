@@ -24,6 +24,7 @@ int cuda_fail(cudaError_t e, const char *what) {
 
 // l = 0 part of the temperature: (T + T_ref) - T_ref each step, as the
 // reference's trans_per_temp_to_temp_sph / sync_temp_by_per_temp_sph pair
+// (a step without a closure does it in k_after_transform)
 __global__ void k_temp_roundtrip(int nr, size_t jmax, const double *reft0, double *T) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nr) return;
@@ -178,18 +179,23 @@ static int nl_grid(Ctx &c) {
   return 0;
 }
 
-static int nl_tail(Ctx &c) {
+// roundtrip: with the temperature round trip that ends a step (the closure's
+// features read the temperature before it)
+static int nl_tail(Ctx &c, bool roundtrip) {
   if (c.timers) cudaEventRecord(c.ev[14], c.stream);
-  rj_after_transform(c);
+  const bool rt = roundtrip && c.p.use_ref_temp;
+  rj_after_transform(c, rt && !c.closure);
   if (c.closure) {
     int rc = closure_apply(c);
     if (rc) return rc;
+    if (rt)
+      k_temp_roundtrip<<<cdiv(c.nr, 128), 128, 0, c.stream>>>(c.nr, (size_t)c.jmax, c.d_reft0, c.fld(TEMP));
   }
   if (c.timers) cudaEventRecord(c.ev[15], c.stream);
   return 0;
 }
 
-static int nonlinear(Ctx &c) {
+static int nonlinear(Ctx &c, bool roundtrip = false) {
   int rc = nl_head(c);
   if (rc) return rc;
   if (c.prec == CB2_PREC_FP64) {
@@ -204,12 +210,7 @@ static int nonlinear(Ctx &c) {
     if ((rc = nl_grid(c))) return rc;
     if ((rc = leg_fwd_gemm(c, mlayout(c, c.d_four2, 4, 0), kFwdSlots))) return rc;
   }
-  return nl_tail(c);
-}
-
-static void temp_roundtrip(Ctx &c) {
-  if (!c.p.use_ref_temp) return;
-  k_temp_roundtrip<<<cdiv(c.nr, 128), 128, 0, c.stream>>>(c.nr, (size_t)c.jmax, c.d_reft0, c.fld(TEMP));
+  return nl_tail(c, roundtrip);
 }
 
 // explicit update and radial solves of a step
@@ -230,8 +231,7 @@ static void solve(Ctx &c) {
 
 int step_once(Ctx &c) {
   solve(c);
-  int rc = nonlinear(c);
-  temp_roundtrip(c);
+  int rc = nonlinear(c, true);
   if (c.timers) cudaEventRecord(c.ev[3], c.stream);
   return rc;
 }
@@ -246,8 +246,7 @@ int step_phase(Ctx &c, int phase) {
     return nl_head(c);
   }
   if (phase == 1) return nl_grid(c);
-  const int rc = nl_tail(c);
-  temp_roundtrip(c);
+  const int rc = nl_tail(c, true);
   if (c.timers) cudaEventRecord(c.ev[3], c.stream);
   return rc;
 }
@@ -452,9 +451,8 @@ int cb2_start(cb2_ctx *c) {
 // the nonlinear terms of the current state, when the last call left them out
 static int fresh_terms(Ctx &c) {
   if (!c.terms_stale) return 0;
-  int rc = nonlinear(c);
+  int rc = nonlinear(c, true);
   if (rc) return rc;
-  temp_roundtrip(c);
   c.terms_stale = false;
   return 0;
 }

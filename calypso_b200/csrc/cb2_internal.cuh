@@ -234,7 +234,8 @@ template <typename T> void fft_forward_grid(Ctx &c, const double *grid, const ML
 // rj operators and solves (cb2_rj.cu)
 void rj_explicit(Ctx &c, bool euler);
 void rj_implicit(Ctx &c);
-void rj_after_transform(Ctx &c);
+// roundtrip: the l = 0 temperature through (T + T_ref) - T_ref as well
+void rj_after_transform(Ctx &c, bool roundtrip = false);
 void rj_start_derived(Ctx &c);
 void rj_temp_total(Ctx &c, double sign);
 int rj_energies(Ctx &c, double out[7]);

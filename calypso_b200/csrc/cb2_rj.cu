@@ -807,14 +807,25 @@ struct CorCol {
 // 77 us at L127 / Nr97.
 constexpr int AT_THREADS = 128, AT_LEVELS = 8;
 
-__global__ void __launch_bounds__(AT_THREADS, 4) k_after_transform(RJArgs a, Fields F, CorTables ct, int kl) {
+__global__ void __launch_bounds__(AT_THREADS, 4) k_after_transform(RJArgs a, Fields F, CorTables ct, int kl, int nb) {
+  const int k0 = blockIdx.y * kl, k1 = min(k0 + kl, a.nr);
+  if (blockIdx.x == nb) {
+    // a column of blocks beyond the (l, m): the temperature round trip of a
+    // step's end (no other block reads the temperature).  A launch of its own
+    // was 2 us of a 62 us step at L31.
+    for (int k = k0 + threadIdx.x; k < k1; k += AT_THREADS) {
+      double *T = F(TEMP) + (size_t)k * a.jmax;
+      const double v = *T + a.reft0[k];
+      *T = v - a.reft0[k];
+    }
+    return;
+  }
   const int jj = blockIdx.x * AT_THREADS + threadIdx.x;
   if (jj >= a.jmax) return;
   const size_t s = a.jmax;
   const BCW &b = a.bc;
   const double g3 = a.g3[jj], gl = a.gl[jj];
   const int ki = a.kin, ko = a.kout, n = a.nr;
-  const int k0 = blockIdx.y * kl, k1 = min(k0 + kl, n);
   const CorCol cc(a, ct, jj);
   // poloidal derivative and toroidal part of the three forces, the heat flux
   const int dif[7] = {MADV + 1, MADV + 2, LOR + 1, LOR + 2, VPIND + 1, VPIND + 2, HFLUX};
@@ -987,7 +998,7 @@ void rj_start_derived(Ctx &c) {
   k_derived_b<<<dim3(cdiv(c.jmax, kThreads), c.nr), kThreads, 0, c.stream>>>(a, fields(c));
 }
 
-void rj_after_transform(Ctx &c) {
+void rj_after_transform(Ctx &c, bool roundtrip) {
   const CorTables ct{c.d_jgi1, c.d_jgi2, c.d_jei1, c.d_sw, c.d_tw};
   // levels a thread: eight where that leaves four waves of blocks (four
   // blocks an SM), else as many up to four as leave one.  L255 / Nr129
@@ -996,7 +1007,8 @@ void rj_after_transform(Ctx &c) {
   const int nb = cdiv(c.jmax, AT_THREADS), wave = 4 * 148;
   int kl = (nb * cdiv(c.nr, AT_LEVELS) < 4 * wave) ? AT_LEVELS / 2 : AT_LEVELS;
   while (kl > 1 && nb * cdiv(c.nr, kl) < wave) kl /= 2;
-  k_after_transform<<<dim3(nb, cdiv(c.nr, kl)), AT_THREADS, 0, c.stream>>>(c.rj_args(), fields(c), ct, kl);
+  k_after_transform<<<dim3(nb + (roundtrip ? 1 : 0), cdiv(c.nr, kl)), AT_THREADS, 0, c.stream>>>(c.rj_args(), fields(c),
+                                                                                                  ct, kl, nb);
 }
 
 void rj_temp_total(Ctx &c, double sign) {
