@@ -38,11 +38,15 @@
 
 namespace cb2 {
 
-constexpr int CN_THREADS = 256;   // a block: 8 warps, each 32 consecutive degrees of one (m, sign)
-// rows each thread keeps in flight (cp.async ring): 4 leaves room for four
-// blocks an SM; shells of at most CN_DEEP_TILES blocks, whose time is the
-// latency of the rows, take 8
-constexpr int CN_RING = 4, CN_RING_DEEP = 8, CN_DEEP_TILES = 2 * 148;
+// Rows each thread keeps in flight (cp.async ring) and threads of a block.
+// Large shells: 4 rows, which leaves room for four blocks of 256 an SM (the
+// factors two rows ahead cost registers for three: L255 / Nr129 step 4980 us
+// for 4860).  Shells of at most CN_DEEP columns (two blocks of 256 an SM),
+// whose time is the latency of the rows: 8 rows, the factors two rows ahead,
+// and blocks of 64, to use every SM (step at L31 / Nr33 79 -> 76 -> 74 us).
+constexpr int CN_RING = 4, CN_RING_DEEP = 8, CN_DEEP = 2 * 148 * 256;
+__host__ __device__ constexpr int cn_threads(int ring) { return ring == CN_RING ? 256 : 64; }
+__host__ __device__ constexpr int cn_ahead(int ring) { return ring == CN_RING ? 1 : 2; }
 constexpr int CN_RV = 4;          // values per ring slot (forward: X, D, F, P; backward: y)
 
 // Forms of one field's factors.  Per row i: NL multipliers L(i,i-1) ..
@@ -57,7 +61,7 @@ __host__ __device__ constexpr int cn_entries(int f) { return 2 * cn_nl(f) + 1; }
 // shared memory of a block: the radial coefficients, then the per-thread rings
 __host__ __device__ inline size_t cn_ring_offset(int n) { return 9 * (size_t)n * sizeof(double); }
 static size_t cn_smem(int n, int ring) {
-  return cn_ring_offset(n) + (size_t)ring * CN_RV * CN_THREADS * sizeof(double);
+  return cn_ring_offset(n) + (size_t)ring * CN_RV * cn_threads(ring) * sizeof(double);
 }
 
 struct LuSet {
@@ -167,10 +171,11 @@ __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// this thread's ring: slot s, value v at base[(s * CN_RV + v) * CN_THREADS]
+// this thread's ring: slot s, value v
+template <int RING>
 struct Ring {
   double *base;
-  __device__ double *at(int s, int v) const { return base + (s * CN_RV + v) * CN_THREADS; }
+  __device__ double *at(int s, int v) const { return base + (s * CN_RV + v) * cn_threads(RING); }
 };
 
 __device__ __forceinline__ uint64_t l2_evict_last() {
@@ -196,9 +201,8 @@ struct CnCtx {
 };
 
 // one degree's factors in global memory (degree-interleaved, so the 32
-// lanes of a warp read 32 consecutive values; the block's 8 warps share
-// them through L1): entry e of row i at p[(i * NE + e) * nl], the
-// interchange offset of row i at pv[i * nl]
+// lanes of a warp read runs of consecutive values): entry e of row i at
+// p[(i * NE + e) * nl], the interchange offset of row i at pv[i * nl]
 struct FacCol {
   const double *p;
   const unsigned char *pv;
@@ -214,12 +218,12 @@ struct FacCol {
 // FLD: 0 poloidal velocity (from the toroidal vorticity), 1 toroidal
 // velocity (from the poloidal vorticity), 2 temperature, 3 poloidal and
 // 4 toroidal magnetic field.  fac: the column's factors.  The
-// inputs of row k + CN_RING are copied into the thread's ring while row k
-// is computed, so a thread keeps CN_RING rows of loads in flight.
+// inputs of row k + RING are copied into the thread's ring while row k
+// is computed, so a thread keeps RING rows of loads in flight.
 template <int RING, int FLD, int FORM>
-__device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring,
+__device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring<RING> ring,
                                            Col X, Col D, Col F, Col P, Col S, int euler) {
-  constexpr int NL = cn_nl(FORM), PD = cn_pd(FORM), NE = cn_entries(FORM);
+  constexpr int NL = cn_nl(FORM), PD = cn_pd(FORM), NE = cn_entries(FORM), FD = cn_ahead(RING);
   const RJArgs &a = q.a;
   const int n = q.n;
   const unsigned st = q.st;
@@ -249,14 +253,15 @@ __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring
   // recurrence needs them, each row waited on L1 or L2 twice (the interchange,
   // then the multipliers).  L255 / Nr129 803 -> 733 us (56 -> 62 % of HBM);
   // the step at L31 / Nr129, where the rows' chain is all, 334 -> 278.
-  double fn[NL];
-  int dn = 0;
-  auto factors = [&](int i) {
-    if constexpr (PD >= 1) dn = fac.piv(i);
+  double fn[FD][NL];
+  int dn[FD] = {};
+  auto factors = [&](int h, int i) {
+    if constexpr (PD >= 1) dn[h] = fac.piv(i);
 #pragma unroll
-    for (int t = 0; t < NL; t++) fn[t] = fac.at(i, NE, t);
+    for (int t = 0; t < NL; t++) fn[h][t] = fac.at(i, NE, t);
   };
-  factors(0);
+#pragma unroll
+  for (int h = 0; h < FD; h++) factors(h, h);
   int sl = 0;
   // explicit right-hand side of row k
   auto explicit_row = [&](int k) {
@@ -280,12 +285,18 @@ __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring
     sl = (sl + 1 == RING) ? 0 : sl + 1;
   };
   // y of row i from the window of right-hand sides
-  auto eliminate = [&](int i, bool more) {
+  auto eliminate = [&](int i) {
     double fc[NL];
 #pragma unroll
-    for (int t = 0; t < NL; t++) fc[t] = fn[t];
-    const int d = dn;
-    if (more) factors(i + 1);
+    for (int t = 0; t < NL; t++) fc[t] = fn[0][t];
+    const int d = dn[0];
+#pragma unroll
+    for (int h = 0; h + 1 < FD; h++) {
+      dn[h] = dn[h + 1];
+#pragma unroll
+      for (int t = 0; t < NL; t++) fn[h][t] = fn[h + 1][t];
+    }
+    if (i + FD < n) factors(FD - 1, i + FD);
     if constexpr (PD >= 1) {
       if (d == 1) { const double t = pend[0]; pend[0] = pend[1]; pend[1] = t; }
       if constexpr (PD >= 2)
@@ -313,12 +324,12 @@ __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring
   }
   for (int k = PD + 1; k < n; k++) {
     const double b = explicit_row(k);
-    eliminate(k - PD - 1, true);
+    eliminate(k - PD - 1);
     shift(b);
     refill(k);
   }
   for (int i = n - PD - 1; i < n; i++) {
-    eliminate(i, i + 1 < n);
+    eliminate(i);
     shift(0.0);
   }
   cp_wait<0>();   // the ring is free for the backward sweep
@@ -331,8 +342,8 @@ __device__ __forceinline__ void cn_forward(const CnCtx &q, FacCol fac, Ring ring
 // at the end.  y of row k - RING is copied into the ring while row k is
 // computed.
 template <int RING, int FORM, class Em>
-__device__ __forceinline__ void cn_backward(const CnCtx &q, FacCol fac, Ring ring, Col S, Em &em) {
-  constexpr int NL = cn_nl(FORM), NE = cn_entries(FORM);
+__device__ __forceinline__ void cn_backward(const CnCtx &q, FacCol fac, Ring<RING> ring, Col S, Em &em) {
+  constexpr int NL = cn_nl(FORM), NE = cn_entries(FORM), FD = cn_ahead(RING);
   const int n = q.n;
   const unsigned st = q.st;
   auto fetch = [&](int sl, int k) {
@@ -344,20 +355,25 @@ __device__ __forceinline__ void cn_backward(const CnCtx &q, FacCol fac, Ring rin
   double xh[NL];   // x(k + 1 + t)
 #pragma unroll
   for (int t = 0; t < NL; t++) xh[t] = 0.0;
-  double fn[NL + 1];   // the next row's factors, a row ahead as in cn_forward
-  auto factors = [&](int k) {
+  double fn[FD][NL + 1];   // the next rows' factors, as in cn_forward
+  auto factors = [&](int h, int k) {
     if (k < 0) return;
 #pragma unroll
-    for (int t = 0; t <= NL; t++) fn[t] = fac.at(k, NE, NL + t);
+    for (int t = 0; t <= NL; t++) fn[h][t] = fac.at(k, NE, NL + t);
   };
-  factors(n - 1);
+#pragma unroll
+  for (int h = 0; h < FD; h++) factors(h, n - 1 - h);
   int sl = 0;
   auto solve = [&](int k) {
     cp_wait<RING - 1>();
     double fc[NL + 1];
 #pragma unroll
-    for (int t = 0; t <= NL; t++) fc[t] = fn[t];
-    factors(k - 1);
+    for (int t = 0; t <= NL; t++) fc[t] = fn[0][t];
+#pragma unroll
+    for (int h = 0; h + 1 < FD; h++)
+#pragma unroll
+      for (int t = 0; t <= NL; t++) fn[h][t] = fn[h + 1][t];
+    factors(FD - 1, k - FD);
     double v = *ring.at(sl, 0);
 #pragma unroll
     for (int t = 0; t < NL; t++) v = v - fc[t] * xh[t];
@@ -570,7 +586,7 @@ struct EmMagTor {
 // ---------------------------------------------------------------------------
 // one (field, column) thread: the sweeps with the field's slots and emitter
 template <int RING, int FLD, int FORM>
-__device__ __forceinline__ void cn_column(const CnCtx &q, double *col, size_t fs, FacCol fac, Ring ring,
+__device__ __forceinline__ void cn_column(const CnCtx &q, double *col, size_t fs, FacCol fac, Ring<RING> ring,
                                           int euler) {
   auto C = [&](int slot) { return Col{col + (size_t)slot * fs}; };
   if constexpr (FLD == 0) {
@@ -615,39 +631,40 @@ __device__ __forceinline__ CnField cn_field(const CnPack &pk, int fld) {
   }
 }
 
-// One block: 8 warps of one field (the tile's x); warp w takes the (m, sign)
-// pair p0 + w (pair 0: m = 0; pair 2m - 1: (m, +); pair 2m: (m, -)), lane
-// the degree l0 + lane, so every access of a warp to a slot row is 32
-// consecutive doubles.  The block stages the radial coefficients in shared
-// memory; each thread then runs its column.
+// One block: consecutive columns jj of one field (the five-band field's
+// blocks first), so that a block's accesses to a row are one run of memory.
+// Blocks of 8 (m, sign) pairs x 32 degrees shared the factors between warps,
+// but read each row in eight unaligned pieces and left a fifth of the lanes
+// without a column: L255 / Nr129 721 -> 644 us, L31 / Nr33 23 -> 18 (with the
+// small blocks), L127 / Nr97 169 -> 168.  The block stages the radial
+// coefficients in shared memory; each thread then runs its column.
 template <int RING>
-__global__ void __launch_bounds__(CN_THREADS, RING == CN_RING ? 4 : 2)
-k_cn_step(RJArgs a, double *f, size_t fs, CnPack pk, const int *moff, const int4 *tiles, int euler) {
+__global__ void __launch_bounds__(cn_threads(RING), RING == CN_RING ? 4 : 8)
+k_cn_step(RJArgs a, double *f, size_t fs, CnPack pk, int nb, int euler) {
+  constexpr int NT = cn_threads(RING);
   extern __shared__ double cn_sm[];
   const int n = a.nr, nl = a.L + 1, tid = threadIdx.x;
-  const int4 tl = tiles[blockIdx.x];   // (field, p0, l0, -)
-  const int fld = tl.x;
+  const int fld = blockIdx.x / nb;
   const CnField fd = cn_field(pk, fld);
   const int form = fd.form;
   double *sco = cn_sm;                 // [9][n]
-  for (int e = tid; e < 3 * n; e += CN_THREADS) {
+  for (int e = tid; e < 3 * n; e += NT) {
     sco[e] = __ldg(a.d1 + e);
     sco[3 * n + e] = __ldg(a.d2 + e);
   }
-  for (int e = tid; e < n; e += CN_THREADS) {
+  for (int e = tid; e < n; e += NT) {
     sco[6 * n + e] = __ldg(a.ar1 + e);
     sco[7 * n + e] = __ldg(a.ar2 + e);
     sco[8 * n + e] = __ldg(a.r + e);
   }
   __syncthreads();
-  const int p = tl.y + tid / 32, l = tl.z + tid % 32;
-  const int m = (p + 1) >> 1, sgn = (p > 0 && (p & 1) == 0) ? 1 : 0;
-  if (l >= nl || m > l) return;
-  const int jj = moff[m] + sgn * (nl - m) + (l - m);
+  const int jj = (blockIdx.x - fld * nb) * NT + tid;
+  if (jj >= a.jmax) return;
   const CnCtx q{a, RadCo{sco, n}, n, (unsigned)a.jmax, jj, __ldg(a.g3 + jj), __ldg(a.gl + jj)};
+  const int l = (int)q.gl;
   double *col = f + jj;
   const FacCol fac{fd.fac + l, fd.piv ? fd.piv + l : nullptr, nl};
-  const Ring ring{reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(cn_sm) + cn_ring_offset(n)) + tid};
+  const Ring<RING> ring{reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(cn_sm) + cn_ring_offset(n)) + tid};
   switch (fld * 4 + form) {
     case 0 * 4 + CN_N5: cn_column<RING, 0, CN_N5>(q, col, fs, fac, ring, euler); break;
     case 0 * 4 + CN_W5: cn_column<RING, 0, CN_W5>(q, col, fs, fac, ring, euler); break;
@@ -719,19 +736,8 @@ int cn_setup(Ctx &c) {
   }
   k_cn_pack<<<cdiv(5 * nl, 128), 128, 0, c.stream>>>(n, nl, set, pk);
   CB2_CUDA(cudaGetLastError());
-  // blocks: (field, p0, l0) tiles of 8 (m, sign) pairs x 32 degrees
-  std::vector<int4> tl;
-  for (int q = 0; q < 5; q++) {
-    for (int l0 = 0; l0 <= c.L; l0 += 32) {
-      const int npair = 2 * std::min(l0 + 31, c.L) + 1;
-      for (int p0 = 0; p0 < npair; p0 += 8) tl.push_back(int4{q, p0, l0, 0});
-    }
-  }
-  c.cn_tiles = (int)tl.size();
-  CB2_CUDA(cudaMalloc(&c.d_cn_tiles, tl.size() * sizeof(int4)));
-  CB2_CUDA(cudaMemcpyAsync(c.d_cn_tiles, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream));
   c.cn_ring = CN_RING;
-  if (c.cn_tiles <= CN_DEEP_TILES && cn_smem(n, CN_RING_DEEP) <= 227 * 1024) {
+  if (5 * c.jmax <= CN_DEEP && cn_smem(n, CN_RING_DEEP) <= 227 * 1024) {
     c.cn_ring = CN_RING_DEEP;
     smem = cn_smem(n, CN_RING_DEEP);
     CB2_CUDA(raise_smem_limit(k_cn_step<CN_RING_DEEP>, smem));
@@ -743,10 +749,10 @@ int cn_setup(Ctx &c) {
   c.cn_smem = smem;
   c.cn_ready = true;
   // The one kernel is the default wherever it takes the context.  Mixed steps,
-  // one kernel against the separate ones, us: L7 / Nr9 49 / 58, L15 / Nr17
-  // 57 / 70, L31 / Nr33 79 / 94, L31 / Nr129 246 / 297, L63 / Nr65 271 / 283,
-  // L127 / Nr25 320 / 347, L127 / Nr97 1097 / 1206, L191 / Nr65 2221 / 2335,
-  // L255 / Nr129 5106 / 5552.
+  // one kernel against the separate ones, us: L7 / Nr9 47 / 56, L15 / Nr17
+  // 53 / 68, L31 / Nr33 76 / 96, L31 / Nr129 236 / 296, L63 / Nr65 260 / 275,
+  // L127 / Nr25 291 / 320, L127 / Nr97 987 / 1099, L191 / Nr65 2162 / 2299,
+  // L255 / Nr129 4770 / 5303.
   c.tune[TUNE_CN] = 1;
   return 0;
 }
@@ -768,12 +774,12 @@ void cn_stage(Ctx &c, bool euler) {
 // one launch for the five fields (the 5-band field's blocks first)
 void cn_step(Ctx &c, bool euler) {
   const CnPack &pk = *static_cast<const CnPack *>(c.cn_pack);
-  if (c.cn_ring == CN_RING_DEEP)
-    k_cn_step<CN_RING_DEEP><<<c.cn_tiles, CN_THREADS, c.cn_smem, c.stream>>>(
-        c.rj_args(), c.d_f, c.fsize(), pk, c.d_moff, c.d_cn_tiles, euler ? 1 : 0);
-  else
-    k_cn_step<CN_RING><<<c.cn_tiles, CN_THREADS, c.cn_smem, c.stream>>>(
-        c.rj_args(), c.d_f, c.fsize(), pk, c.d_moff, c.d_cn_tiles, euler ? 1 : 0);
+  auto launch = [&](auto kernel, int threads) {
+    const int nb = cdiv(c.jmax, threads);
+    kernel<<<5 * nb, threads, c.cn_smem, c.stream>>>(c.rj_args(), c.d_f, c.fsize(), pk, nb, euler ? 1 : 0);
+  };
+  if (c.cn_ring == CN_RING_DEEP) launch(k_cn_step<CN_RING_DEEP>, cn_threads(CN_RING_DEEP));
+  else launch(k_cn_step<CN_RING>, cn_threads(CN_RING));
 }
 
 }  // namespace cb2

@@ -91,8 +91,7 @@ struct Ctx {
   // allocation), int4 (field, m0, l0, -) block tiles, the kernel's view of
   // the factors (CnPack), its shared memory; cn_ready when usable
   double *d_cn_lu = nullptr;
-  int4 *d_cn_tiles = nullptr;
-  int cn_tiles = 0, cn_ring = 0;   // blocks; rows a thread keeps in flight
+  int cn_ring = 0;   // rows a thread keeps in flight
   void *cn_pack = nullptr;
   size_t cn_smem = 0;
   bool cn_ready = false;
