@@ -749,15 +749,65 @@ struct PackArgs {
   float *maxP, *maxD;      // [m][pitch] row maxima
 };
 
-// Bound by HBM once enough loads are in flight: a warp takes PK_U segments of
-// 64 degrees, of whatever rows, at a time.  A warp per row, 256 degrees a pass,
-// left most of its eight loads beyond the truncation at the higher orders and
-// took 406 us at L255 / Nr129 (1.3 GB) and 128 us at L127 / Nr97; segments of
-// 32 degrees took 457 and 113 us (the bookkeeping of a segment).
-constexpr int PK_U = 8, PK_W = 2;   // segments in flight a warp, loads of a segment
 constexpr int PK_ROWS = 4 * 26;  // rows of a block at most (4 radial levels)
 
-__global__ void __launch_bounds__(256)
+// Rows of a block in: (row, 32 W degrees) items, U of them in flight a warp;
+// coalesced float64 reads, l(l+1) for the poloidal parts, the row maxima on the
+// way.  Bound by the instructions of an item and, beyond them, HBM.  A warp per
+// row, 256 degrees a pass, left most of its eight loads beyond the truncation at
+// the higher orders.  L255 / Nr129 (1.3 GB) and L127 / Nr97: a row a warp 406 and
+// 128 us, items of 32 degrees 457 and 113, of 64 (eight in flight, three blocks
+// an SM) 395 and 102, of 128 (four, four blocks) 359 and 94; with items of 128
+// also where an order has at most 64 degrees the step at L47 / Nr92 was 1.6 %
+// slower.
+template <int U, int W>
+__device__ __forceinline__ void pack_rows(const double *__restrict__ f, float *T, const long long *rsrc,
+                                          const double *rfac, const int *rvec, unsigned *rmax, int m, int nl, int NLP,
+                                          int nrow) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int nseg = (nl + 32 * W - 1) / (32 * W), nitem = nrow * nseg;
+  const FastDiv dseg(nseg);
+  for (int i0 = warp; i0 < nitem; i0 += U * nw) {
+    double x[U][W];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int it = i0 + u * nw, rl = dseg.div(it), lm = (it - rl * nseg) * (32 * W) + lane;
+      const long long so = (it < nitem) ? rsrc[rl] : -1;
+      const double *src = f + (so >= 0 ? so : 0);
+#pragma unroll
+      for (int w = 0; w < W; w++) x[u][w] = (so >= 0 && lm + 32 * w < nl) ? __ldg(src + lm + 32 * w) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int it = i0 + u * nw, rl = dseg.div(it), lm = (it - rl * nseg) * (32 * W) + lane;
+      if (it >= nitem) break;
+      const double rowf = rfac[rl];
+      float mx = 0.0f;
+      if (rvec[rl]) {   // the same for the whole warp
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+          const int l = m + lm + 32 * w;
+          x[u][w] *= rowf * ((l == 0) ? 0.5 : (double)(l * (l + 1)));
+        }
+      } else {
+#pragma unroll
+        for (int w = 0; w < W; w++) x[u][w] *= rowf;
+      }
+#pragma unroll
+      for (int w = 0; w < W; w++) {
+        const float v = (float)x[u][w];
+        if (lm + 32 * w < nl) {
+          T[rl * NLP + lm + 32 * w] = v;
+          mx = fmaxf(mx, fabsf(v));
+        }
+      }
+      const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+      if (lane == 0) atomicMax(rmax + rl, mb);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256, 4)
 k_pack_bwd(const __grid_constant__ PackArgs a) {
   extern __shared__ float T[];   // [kc * RK][NLP]
   __shared__ long long rsrc[PK_ROWS];   // offset of the row's degree m in the fields, -1: zero
@@ -790,41 +840,10 @@ k_pack_bwd(const __grid_constant__ PackArgs a) {
     rmax[rl] = 0u;
   }
   __syncthreads();
-  // rows in: (row, 32 PK_W degrees) items, coalesced float64 reads, l(l+1) for
-  // the poloidal parts, the row maxima on the way
-  const int nseg = (nl + 32 * PK_W - 1) / (32 * PK_W), nitem = nrow * nseg;
-  const FastDiv dseg(nseg);
-  for (int i0 = warp; i0 < nitem; i0 += PK_U * nw) {
-    double x[PK_U][PK_W];
-#pragma unroll
-    for (int u = 0; u < PK_U; u++) {
-      const int it = i0 + u * nw, rl = dseg.div(it), lm = (it - rl * nseg) * (32 * PK_W) + lane;
-      const long long so = (it < nitem) ? rsrc[rl] : -1;
-      const double *src = a.f + (so >= 0 ? so : 0);
-#pragma unroll
-      for (int w = 0; w < PK_W; w++) x[u][w] = (so >= 0 && lm + 32 * w < nl) ? __ldg(src + lm + 32 * w) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < PK_U; u++) {
-      const int it = i0 + u * nw, rl = dseg.div(it), lm = (it - rl * nseg) * (32 * PK_W) + lane;
-      if (it >= nitem) break;
-      const double rowf = rfac[rl];
-      const bool vec = rvec[rl] != 0;
-      float mx = 0.0f;
-#pragma unroll
-      for (int w = 0; w < PK_W; w++) {
-        const int l = m + lm + 32 * w;
-        const double gg = (l == 0) ? 0.5 : (double)(l * (l + 1));
-        const float v = (float)(vec ? x[u][w] * (rowf * gg) : x[u][w] * rowf);
-        if (lm + 32 * w < nl) {
-          T[rl * NLP + lm + 32 * w] = v;
-          mx = fmaxf(mx, fabsf(v));
-        }
-      }
-      const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-      if (lane == 0) atomicMax(rmax + rl, mb);
-    }
-  }
+  // rows in: as long a segment as the order fills
+  if (nl > 64) pack_rows<4, 4>(a.f, T, rsrc, rfac, rvec, rmax, m, nl, NLP, nrow);
+  else if (nl > 32) pack_rows<8, 2>(a.f, T, rsrc, rfac, rvec, rmax, m, nl, NLP, nrow);
+  else pack_rows<8, 1>(a.f, T, rsrc, rfac, rvec, rmax, m, nl, NLP, nrow);
   __syncthreads();
   for (int rl = threadIdx.x; rl < nrow; rl += blockDim.x) {
     const int kq = rl / RK, j = rl - kq * RK, k = k0 + kq;
@@ -842,12 +861,14 @@ k_pack_bwd(const __grid_constant__ PackArgs a) {
       const int kq = rr / RP, j = rr - kq * RP;
       const float *tr = T + (kq * RK + j) * NLP + par;
       float *dst = a.rlmP + base * a.pitchP + (size_t)k0 * RP + rr;
+#pragma unroll 4
       for (int kk = warp; kk < cnt; kk += nw) dst[(size_t)kk * a.pitchP] = tr[2 * kk];
     }
     for (int rr = lane; rr < wD; rr += 32) {
       const int kq = rr / RD, j = rr - kq * RD;
       const float *tr = T + (kq * RK + RP + j) * NLP + par;
       float *dst = a.rlmD + base * a.pitchD + (size_t)k0 * RD + rr;
+#pragma unroll 4
       for (int kk = warp; kk < cnt; kk += nw) dst[(size_t)kk * a.pitchD] = tr[2 * kk];
     }
   }
