@@ -1283,26 +1283,37 @@ k_rowmax_four(MLayout in, const float *wgt, float *Mf) {
 
 // the same maxima from the four-step FFT kernel's partial maxima
 // pm[theta][mb][e] (largest |x| w over the 16 orders of block mb at one
-// colatitude): a row's scale then covers its block of 16 orders
+// colatitude): a row's scale then covers its block of 16 orders.  A block takes
+// 32 elements, its warps every eighth colatitude each: with a thread walking
+// all the colatitudes of an element (80 blocks at L127 / Nr97) it was latency,
+// 12 -> 5.8 us there, 27 -> 20 us at L255 / Nr129.
+constexpr int RM_U = 8;   // colatitudes in flight a thread
 __global__ void __launch_bounds__(256)
 k_rowmax_reduce(const float *__restrict__ pm, int nth, int MB, size_t E, int L, float *__restrict__ Mf) {
-  const int mb = blockIdx.y;
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  const float *x = pm + (size_t)mb * E + e;
-  const size_t st = (size_t)MB * E;
+  const int mb = blockIdx.y, g = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t e = (size_t)blockIdx.x * 32 + lane;
   float mx = 0.0f;
-  int th = 0;
-  for (; th + 16 <= nth; th += 16) {
-    float v[16];
+  if (e < E) {
+    const float *x = pm + (size_t)mb * E + e;
+    const size_t st = (size_t)MB * E;
+    int th = g;
+    for (; th + 8 * (RM_U - 1) < nth; th += 8 * RM_U) {
+      float v[RM_U];
 #pragma unroll
-    for (int u = 0; u < 16; u++) v[u] = __ldg(x + (size_t)(th + u) * st);
+      for (int u = 0; u < RM_U; u++) v[u] = __ldg(x + (size_t)(th + 8 * u) * st);
 #pragma unroll
-    for (int u = 0; u < 16; u++) mx = fmaxf(mx, v[u]);
+      for (int u = 0; u < RM_U; u++) mx = fmaxf(mx, v[u]);
+    }
+    for (; th < nth; th += 8) mx = fmaxf(mx, __ldg(x + (size_t)th * st));
   }
-  for (; th < nth; th++) mx = fmaxf(mx, __ldg(x + (size_t)th * st));
+  __shared__ float part[8][32];
+  part[g][lane] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; q++) mx = fmaxf(mx, part[q][lane]);
   const int m1 = min(L + 1, mb * 16 + 16);
-  for (int m = mb * 16; m < m1; m++) Mf[(size_t)m * E + e] = 2.0f * mx;
+  if (e < E)
+    for (int m = mb * 16 + g; m < m1; m += 8) Mf[(size_t)m * E + e] = 2.0f * mx;
 }
 
 // ---------------------------------------------------------------------------
@@ -1736,7 +1747,7 @@ void leg_fwd_rowmax(Ctx &c, const MLayout &in, bool rowmax_ready) {
   MixedTables *t = (MixedTables *)c.mixed;
   if (rowmax_ready && t->fwd_pmax && in.nvec == 4 && in.nscal == 0) {
     const size_t E = in.sP() + in.sD();
-    k_rowmax_reduce<<<dim3(cdiv((long)E, 256), t->pmax_mb), 256, 0, c.stream>>>(t->fwd_pmax, c.nth, t->pmax_mb, E,
+    k_rowmax_reduce<<<dim3(cdiv((long)E, 32), t->pmax_mb), 256, 0, c.stream>>>(t->fwd_pmax, c.nth, t->pmax_mb, E,
                                                                                c.L, t->rowmax_four);
   } else {
     k_rowmax_four<<<dim3(cdiv((long)(in.sP() + in.sD()), 256), c.L + 1), 256, 0, c.stream>>>(in, t->wgt32,
