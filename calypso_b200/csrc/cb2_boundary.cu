@@ -20,6 +20,7 @@
 // context's Fourier buffers.
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "cb2_internal.cuh"
@@ -135,22 +136,47 @@ int jj_host(const Ctx &c, int l, int m) {
   return c.h_moff[am] + ((m < 0) ? (c.L + 1 - am) : 0) + (l - am);
 }
 
+// both device tables, one allocation of the largest the checks let through
+int tables_alloc(Ctx &c) {
+  if (c.d_bnd_tab) return 0;
+  const size_t M1 = c.L + 1, rlm = (2 * (size_t)c.jmax + 3) / 4 * 4, rtm = 6 * (2 * M1 - 1) + 2 * M1;
+  CB2_CUDA(cudaMalloc(&c.d_bnd_tab, (rlm + rtm) * sizeof(int)));
+  c.d_bnd_mtab = c.d_bnd_tab + rlm;
+  return 0;
+}
+
 int upload_rlm(Ctx &c, const cb2_sph_tables *t) {
   const int nj = t->nidx_rlm[1];
   const int *lm = t->idx_gl_1d_rlm_j + nj;   // l of every j, then m
-  // entries of equal key keep the table's order (a table may list a mode twice)
-  std::vector<int> head(c.jmax, -1), next(nj), h;
-  for (int j = nj - 1; j >= 0; j--) {
-    const int jj = jj_host(c, lm[j], lm[nj + j]);
-    next[j] = head[jj];
-    head[jj] = j;
+  // Every mode once: the entry of jj is its place in the table.  A first call
+  // pays for this on the host, 0.1 - 0.5 ms at L255; the sort below, with its
+  // lists, takes 0.3 - 1.0 ms.
+  std::unique_ptr<int[]> pairs(new int[2 * (size_t)nj]);
+  bool once = nj == c.jmax;
+  if (once) {
+    std::memset(pairs.get(), 0xff, 2 * (size_t)nj * sizeof(int));
+    for (int j = 0; j < nj && once; j++) {
+      const int jj = jj_host(c, lm[j], lm[nj + j]);
+      once = pairs[2 * (size_t)jj] < 0;
+      pairs[2 * (size_t)jj] = j;
+      pairs[2 * (size_t)jj + 1] = jj;
+    }
   }
-  h.reserve(2 * (size_t)nj);
-  for (int jj = 0; jj < c.jmax; jj++)
-    for (int j = head[jj]; j >= 0; j = next[j]) { h.push_back(j); h.push_back(jj); }
+  if (!once) {
+    // entries of equal key keep the table's order (a table may list a mode twice)
+    std::vector<int> head(c.jmax, -1), next(nj);
+    for (int j = nj - 1; j >= 0; j--) {
+      const int jj = jj_host(c, lm[j], lm[nj + j]);
+      next[j] = head[jj];
+      head[jj] = j;
+    }
+    size_t at = 0;
+    for (int jj = 0; jj < c.jmax; jj++)
+      for (int j = head[jj]; j >= 0; j = next[j]) { pairs[at++] = j; pairs[at++] = jj; }
+  }
   c.bnd_rlm_key.clear();   // no key while the device table changes
-  if (int rc = grow((void **)&c.d_bnd_tab, &c.bnd_tab_bytes, h.size() * sizeof(int))) return rc;
-  CB2_CUDA(cudaMemcpyAsync(c.d_bnd_tab, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
+  if (int rc = tables_alloc(c)) return rc;
+  CB2_CUDA(cudaMemcpyAsync(c.d_bnd_tab, pairs.get(), 2 * (size_t)nj * sizeof(int), cudaMemcpyHostToDevice, c.stream));
   c.bnd_rlm_key.assign(lm, lm + 2 * (size_t)nj);
   return 0;
 }
@@ -174,7 +200,7 @@ int upload_rtm(Ctx &c, const cb2_sph_tables *t) {
   for (int mp = 0; mp < nm; mp++) { h.push_back(std::abs(om[mp])); h.push_back((om[mp] < 0) ? 1 : 0); }
   h.insert(h.end(), mpos.begin(), mpos.end());
   c.bnd_rtm_key.clear();
-  if (int rc = grow((void **)&c.d_bnd_mtab, &c.bnd_mtab_bytes, h.size() * sizeof(int))) return rc;
+  if (int rc = tables_alloc(c)) return rc;
   CB2_CUDA(cudaMemcpyAsync(c.d_bnd_mtab, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
   c.bnd_rtm_key.assign(om, om + nm);
   return 0;

@@ -128,8 +128,7 @@ struct Ctx {
   // caller's host buffers, a grid buffer and the index tables, grown on demand
   double *d_bnd_a = nullptr, *d_bnd_b = nullptr, *d_bnd_grid = nullptr;
   size_t bnd_a_bytes = 0, bnd_b_bytes = 0, bnd_grid_bytes = 0;
-  int *d_bnd_tab = nullptr, *d_bnd_mtab = nullptr;
-  size_t bnd_tab_bytes = 0, bnd_mtab_bytes = 0;
+  int *d_bnd_tab = nullptr, *d_bnd_mtab = nullptr;   // one allocation (d_bnd_tab)
   std::vector<int> bnd_rlm_key, bnd_rtm_key;   // the values the two device tables were made from
   int istep = 0;
   bool started = false;
