@@ -13,9 +13,11 @@
 //
 // Network: MLP nin -> nhid -> nhid -> nout, SiLU activations, weights kept
 // in bfloat16 for every product (float32 master copy for the optimiser),
-// float32 activations and accumulation.  Kernels: a tiled GEMM with either
-// operand transposed (split-K with float32 atomics for the weight
-// gradients), bias + activation, its derivative, column sums and Adam.
+// float32 activations and accumulation.  Kernels: for the widths of fused_ok
+// one each for the forward pass, the data gradients and the weight gradients;
+// for others a tiled GEMM with either operand transposed (split-K with float32
+// atomics for the weight gradients), bias + activation, its derivative and
+// column sums; and Adam.
 // Training runs on the GPU through these kernels; the oracle restates the
 // same forward and backward in float64 (numpy) to check the gradients.
 #include <cuda_bf16.h>

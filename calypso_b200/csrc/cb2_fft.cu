@@ -12,9 +12,9 @@
 // Normalisation (t_MHD_multi_FFTW.F90:220-355):
 //   f(phi_p) = a_0 + sum_{m=1..L} (a_m cos m phi_p + b_m sin m phi_p),
 //   a_0 = (1/N) sum f, a_m = (2/N) sum f cos, b_m = (2/N) sum f sin.
-// Two real rows share one complex FFT (x + i y).  The complex FFT is a
-// shared-memory Stockham autosort transform with radix 3, 4 and 2 stages,
-// N = 3^a 2^b.
+// Two real rows share one complex FFT (x + i y), N = 3^a 2^b: a four-step
+// transform where N = 3 (L + 1), L + 1 = 32 .. 256, else a shared-memory
+// Stockham autosort transform with radix 3, 4 and 2 stages.
 #include <algorithm>
 #include <cmath>
 #include <vector>
