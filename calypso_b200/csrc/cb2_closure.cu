@@ -976,6 +976,7 @@ using namespace cb2;
 // ---------------------------------------------------------------------------
 // the network
 constexpr size_t kTailBytes = 16;
+struct ClosureState;
 struct cb2_mlp {
   int F = 0, H = 0, O = 0;
   size_t oW1 = 0, ob1 = 0, oW2 = 0, ob2 = 0, oW3 = 0, ob3 = 0, np = 0;
@@ -994,6 +995,11 @@ struct cb2_mlp {
   int *status = nullptr;
   size_t ycap = 0;              // rows of Yp
   cudaStream_t stream = nullptr;
+  // the parameters are written on `stream` and read there and on the streams of
+  // the contexts the network is attached to: `written` follows their last
+  // change, and each user's `read` its last pass
+  cudaEvent_t written = nullptr;
+  std::vector<ClosureState *> users;
 };
 
 namespace cb2 {
@@ -1185,9 +1191,22 @@ struct ClosureState {
   float *norm = nullptr;     // [nr][16 mean], [nr][16 1/std], [nr][5 out scale]
   float *X = nullptr, *Xn = nullptr;
   size_t rows = 0;
+  cudaEvent_t read = nullptr;   // after the last pass that read the network's parameters
 };
 
 namespace cb2 {
+// An event between a context's stream and the network's.  Where the step is
+// being captured into a graph, the wait and the record become nodes of the
+// graph, which each launch runs anew.
+static int event_on(cudaStream_t st, cudaEvent_t e, bool wait) {
+  cudaStreamCaptureStatus cap;
+  CB2_CUDA(cudaStreamIsCapturing(st, &cap));
+  const bool graph = cap == cudaStreamCaptureStatusActive;
+  if (wait) CB2_CUDA(cudaStreamWaitEvent(st, e, graph ? cudaEventWaitExternal : cudaEventWaitDefault));
+  else CB2_CUDA(cudaEventRecordWithFlags(e, st, graph ? cudaEventRecordExternal : cudaEventRecordDefault));
+  return 0;
+}
+
 // called by the time step after the explicit nonlinear terms are formed
 int closure_apply(Ctx &c) {
   ClosureState *cs = static_cast<ClosureState *>(c.closure);
@@ -1197,8 +1216,9 @@ int closure_apply(Ctx &c) {
                                               c.h_r[c.kout], c.d_f, c.fsize(), feat_slots(), cs->X);
   const size_t nn = (size_t)c.nr * NF;
   k_normalise<<<blocks(n * NF), 256, 0, c.stream>>>(n, c.jmax, cs->X, cs->norm, cs->norm + nn, cs->Xn);
-  int rc = mlp_forward(cs->net, cs->Xn, n, cs->net->Yp, c.stream, c.d_status);
-  if (rc) return rc;
+  int rc = event_on(c.stream, cs->net->written, true);
+  if (rc || (rc = mlp_forward(cs->net, cs->Xn, n, cs->net->Yp, c.stream, c.d_status))) return rc;
+  if ((rc = event_on(c.stream, cs->read, false))) return rc;
   k_add_tendency<<<blocks(n), 256, 0, c.stream>>>(n, c.nr, c.jmax, cs->net->Yp, cs->norm + 2 * nn, c.d_f, c.fsize(),
                                                   out_slots());
   return 0;
@@ -1210,6 +1230,11 @@ void closure_free(Ctx &c) {
   if (cs->norm) cudaFree(cs->norm);
   if (cs->X) cudaFree(cs->X);
   if (cs->Xn) cudaFree(cs->Xn);
+  if (cs->read) cudaEventDestroy(cs->read);
+  if (cs->net) {
+    auto &u = cs->net->users;
+    u.erase(std::remove(u.begin(), u.end(), cs), u.end());
+  }
   delete cs;
   c.closure = nullptr;
 }
@@ -1245,6 +1270,7 @@ int cb2_mlp_create(int nin, int nhid, int nout, unsigned seed, cb2_mlp **out) {
   auto fail = [&](int rc) { cb2_mlp_destroy(n); return rc; };
   const size_t gtail = (n->np + 3) / 4 * 4;
   if (cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&n->written, cudaEventDisableTiming) != cudaSuccess ||
       cudaMalloc(&n->master, n->np * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&n->grad, gtail * sizeof(float) + kTailBytes) != cudaSuccess ||
       cudaMalloc(&n->m, n->np * sizeof(float)) != cudaSuccess ||
@@ -1253,11 +1279,13 @@ int cb2_mlp_create(int nin, int nhid, int nout, unsigned seed, cb2_mlp **out) {
     return fail(cuda_fail(cudaGetLastError(), "cb2_mlp_create"));
   n->loss = reinterpret_cast<double *>(n->grad + gtail);
   n->status = reinterpret_cast<int *>(n->loss + 1);
-  cudaMemcpy(n->master, p.data(), n->np * sizeof(float), cudaMemcpyHostToDevice);
-  cudaMemset(n->grad, 0, gtail * sizeof(float) + kTailBytes);
-  cudaMemset(n->m, 0, n->np * sizeof(float));
-  cudaMemset(n->v, 0, n->np * sizeof(float));
+  // all on the network's stream, which does not wait for the default one
+  cudaMemcpyAsync(n->master, p.data(), n->np * sizeof(float), cudaMemcpyHostToDevice, n->stream);
+  cudaMemsetAsync(n->grad, 0, gtail * sizeof(float) + kTailBytes, n->stream);
+  cudaMemsetAsync(n->m, 0, n->np * sizeof(float), n->stream);
+  cudaMemsetAsync(n->v, 0, n->np * sizeof(float), n->stream);
   k_to_bf16<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->w);
+  cudaEventRecord(n->written, n->stream);
   if (cudaStreamSynchronize(n->stream) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "cb2_mlp_create"));
   *out = n;
   return 0;
@@ -1266,9 +1294,11 @@ int cb2_mlp_create(int nin, int nhid, int nout, unsigned seed, cb2_mlp **out) {
 int cb2_mlp_destroy(cb2_mlp *n) {
   if (!n) return 0;
   if (n->stream) cudaStreamSynchronize(n->stream);
+  for (ClosureState *cs : n->users) cs->net = nullptr;
   void *ptrs[] = {n->master, n->grad, n->m, n->v, n->w, n->work, n->Yp};
   for (void *q : ptrs)
     if (q) cudaFree(q);
+  if (n->written) cudaEventDestroy(n->written);
   if (n->stream) cudaStreamDestroy(n->stream);
   delete n;
   return 0;
@@ -1279,14 +1309,25 @@ int cb2_mlp_num_params(const cb2_mlp *n) { return n ? (int)n->np : -1; }
 // float32 master parameters: W1 [H][F], b1 [H], W2 [H][H], b2 [H], W3 [O][H], b3 [O]
 int cb2_mlp_get_params(cb2_mlp *n, float *host) {
   if (!n || !host) return CB2_ERR_ARG;
-  CB2_CUDA(cudaMemcpy(host, n->master, n->np * sizeof(float), cudaMemcpyDeviceToHost));
+  // behind the updates queued on the network's stream
+  CB2_CUDA(cudaMemcpyAsync(host, n->master, n->np * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
+  CB2_CUDA(cudaStreamSynchronize(n->stream));
+  return 0;
+}
+
+// the network's stream behind every pass of an attached context that reads the
+// parameters, before they change
+static int params_begin(cb2_mlp *n) {
+  for (ClosureState *cs : n->users) CB2_CUDA(cudaStreamWaitEvent(n->stream, cs->read, cudaEventWaitDefault));
   return 0;
 }
 
 int cb2_mlp_set_params(cb2_mlp *n, const float *host) {
   if (!n || !host) return CB2_ERR_ARG;
-  CB2_CUDA(cudaMemcpy(n->master, host, n->np * sizeof(float), cudaMemcpyHostToDevice));
+  if (int rc = params_begin(n)) return rc;
+  CB2_CUDA(cudaMemcpyAsync(n->master, host, n->np * sizeof(float), cudaMemcpyHostToDevice, n->stream));
   k_to_bf16<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->w);
+  CB2_CUDA(cudaEventRecord(n->written, n->stream));
   CB2_CUDA(cudaStreamSynchronize(n->stream));
   return 0;
 }
@@ -1328,10 +1369,12 @@ int cb2_mlp_loss_grad(cb2_mlp *n, const float *dev_x, const float *dev_t, long l
 
 int cb2_mlp_adam_step(cb2_mlp *n, float lr, float beta1, float beta2, float eps) {
   if (!n) return CB2_ERR_ARG;
+  if (int rc = params_begin(n)) return rc;
   n->t += 1;
   const float c1 = 1.0f - std::pow(beta1, (float)n->t), c2 = 1.0f - std::pow(beta2, (float)n->t);
   k_adam<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->grad, n->m, n->v, lr, beta1, beta2, eps, c1, c2, n->w);
   CB2_CUDA(cudaGetLastError());
+  CB2_CUDA(cudaEventRecord(n->written, n->stream));
   return 0;
 }
 
@@ -1428,12 +1471,14 @@ int cb2_closure_attach(cb2_ctx *c, cb2_mlp *net, const float *norm) {
   ClosureState *cs = new ClosureState();
   c->closure = cs;
   cs->net = net;
+  net->users.push_back(cs);
+  CB2_CUDA(cudaEventCreateWithFlags(&cs->read, cudaEventDisableTiming));
   cs->rows = c->fsize();
   const size_t nn = (size_t)c->nr * NF;
   std::vector<float> hn(norm, norm + 2 * nn + (size_t)c->nr * NO);
   for (size_t q = 0; q < nn; q++) hn[nn + q] = hn[nn + q] > 0.0f ? 1.0f / hn[nn + q] : 1.0f;
   CB2_CUDA(cudaMalloc(&cs->norm, hn.size() * sizeof(float)));
-  CB2_CUDA(cudaMemcpy(cs->norm, hn.data(), hn.size() * sizeof(float), cudaMemcpyHostToDevice));
+  CB2_CUDA(cudaMemcpyAsync(cs->norm, hn.data(), hn.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   CB2_CUDA(cudaMalloc(&cs->X, cs->rows * NF * sizeof(float)));
   CB2_CUDA(cudaMalloc(&cs->Xn, cs->rows * NF * sizeof(float)));
   if (int rc = mlp_reserve(net, cs->rows, false)) return rc;
