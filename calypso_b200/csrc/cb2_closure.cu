@@ -281,28 +281,44 @@ k_tc_gemm(int M, int N, int NT, int K, const TAT *__restrict__ A, int lda, const
 // Three GEMMs with the activations between them in memory moved 1.6 GB for
 // 266240 rows (2031 us: the GEMMs, whose threads read a row each, 1510, bias
 // and SiLU 505); kept in tensor and shared memory the pass reads 64 and
-// writes 20 bytes a row and takes 189 us, bound by the SiLU epilogue (an
-// __expf and a divide per unit and layer) and the operand split.  A training
-// pass of 16384 rows: 35 + 45 + 51 us of kernels, before 500 us.
+// writes 20 bytes a row and takes 196 us, bound by the SiLU epilogue (an
+// __expf and a reciprocal per unit and layer) and the operand split.  A
+// training pass of 16384 rows: 29 + 39 + 52 us of kernels, before 500 us.
+//
+// A training pass forms every product and activation with the terms, the order
+// and the rounding of the general kernels (k_tc_gemm, k_bias_act, k_mse,
+// k_act_grad), so its loss and gradients do not depend on which of the two a
+// network's widths select: they are equal bit for bit but for the order of the
+// float32 atomics that add the weight gradients' row chunks.  That matters
+// because an optimiser carries a difference on: an Adam step is +- lr where a
+// gradient is far above eps, whatever its size, and one weight that rounds the
+// other way to bfloat16 moves the next gradient by 1e-5.
 //
 // A CTA keeps the bfloat16 weights in shared memory and walks tiles of 128
 // rows.  Warps 0-11 are the epilogue: warp w reads tensor-memory lanes
 // 32 (w & 3) .. + 31, one row a thread, the four warps of group w >> 2 every
-// third chunk of 32 columns (with two groups the SiLU chains left the
-// schedulers idle: 189 us for 266240 rows).  A chunk of an activation is
+// third chunk of 32 columns (with two groups the SiLU chains leave the
+// schedulers idle: a ninth longer at 266240 rows).  A chunk of an activation is
 // split into bfloat16 hi + lo and written as the next product's A operand
 // into one of ML_ST stages; the last warp issues the MMAs of a chunk as soon as
 // it is there, so the second product runs behind the first one's epilogue.  The
-// last layer (OC = 5 or 8 columns) is float32 FMAs on the thread's row.
+// last layer (OC = 5 or 8 columns) is float32 FMAs on the thread's row; in
+// training it is a third product over the same stages, whose 16 columns of sums
+// take the place of the first layer's.
 //
 // The stages' empty barriers are waited on by phase parity, so whoever fills
-// use q of a stage must know that use q - 2 ML_ST has been released.  A group
-// fills every ML_G-th use and has seen its own last use's predecessor released,
-// q - ML_G - ML_ST: hence ML_G <= ML_ST.  (The first uses of a tile follow a
-// barrier that every release of the last tile precedes.)
+// use q of a stage must know that use q - 2 ML_ST has been released.  Within a
+// layer a group fills every ML_G-th use and has seen its own last use's
+// predecessor released, q - ML_G - ML_ST: hence ML_G <= ML_ST.  The first uses
+// of a layer follow a wait for the accumulator before them (d1, d2, d3), which
+// the MMA thread commits once use q - ML_ST has been filled, and whoever filled
+// that one had seen use q - 2 ML_ST released; a next tile's input that goes in
+// front of the last epilogue follows its group's last chunk.
 constexpr int ML_G = 3, ML_EPI = 128 * ML_G, ML_THREADS = ML_EPI + 32, ML_ST = 3, ML_O = 8;
 static_assert(ML_G <= ML_ST, "a group may not run two phases ahead of a stage");
 constexpr uint32_t ML_STAGE = 2 * GA_BYTES;   // hi and lo of 128 rows x 32 columns
+constexpr uint32_t W3_TILE = 16 * 64;          // 16 outputs x 32 units of W3
+static_assert(W3_TILE == 32 * ML_O * 4, "the tile takes the place of the float weights");
 
 struct MlpArgs {
   long long n;
@@ -310,10 +326,10 @@ struct MlpArgs {
   const float *X, *b1, *b2, *b3;
   const __nv_bfloat16 *W1, *W2, *W3;
   float *Y;                      // forward output, n x O
-  // training: targets, 2 / (n O), pre-activations, dL/dY, loss partial sums
-  // (4 a tile), and the data gradients of the hidden layers
+  // training: targets, n O, pre-activations, dL/dY, loss partial sums (4 a
+  // tile), and the data gradients of the hidden layers
   const float *T;
-  float scale;
+  float count;
   float *Z1, *Z2, *dY, *dZ2, *dZ1;
   double *part;
   int *status;
@@ -321,13 +337,13 @@ struct MlpArgs {
 };
 
 struct MlpBars {
-  uint64_t full[ML_ST], empty[ML_ST], d1, d2, fin;
+  uint64_t full[ML_ST], empty[ML_ST], d1, d2, d3, fin;
   uint32_t tmem;
   int abort;
 };
 
 struct MlpLayout {
-  uint32_t w2, w1, st, b1, b2, w3, yp, bar, total;
+  uint32_t w2, w1, st, w3, b1, b2, yp, bar, total;
 };
 __host__ __device__ inline MlpLayout mlp_layout(int H) {
   MlpLayout o;
@@ -335,19 +351,60 @@ __host__ __device__ inline MlpLayout mlp_layout(int H) {
   o.w2 = p; p += (uint32_t)H * H * 2;
   o.w1 = p; p += (uint32_t)H * 64;
   o.st = p; p += ML_ST * ML_STAGE;
+  o.w3 = p; p += (uint32_t)H * ML_O * 4;   // float [H][ML_O], or the bfloat16 tile of 16 outputs (W3_TILE a chunk)
   o.b1 = p; p += (uint32_t)H * 4;
   o.b2 = p; p += (uint32_t)H * 4;
-  o.w3 = p; p += (uint32_t)H * ML_O * 4;
   o.yp = p; p += (ML_G - 1) * 128 * ML_O * 4;
   o.bar = p; p += 128;
   o.total = p;
   return o;
 }
 
-__device__ inline float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
-__device__ inline float dsilu(float z) {
-  const float s = __fdividef(1.0f, 1.0f + __expf(-z));
-  return s * (1.0f + z * (1.0f - s));
+// The sigmoid with an IEEE division.  The fused passes take it apart: for
+// z >= kSigmLow the divisor lies in [1, 2^126), where one step of Newton's
+// iteration from the approximate reciprocal rounds as 1.0f / x does (compared
+// for every float of that range), without the division's range check a value,
+// which kept the 32 chains of a thread apart (closure forward of 266240 rows:
+// 333 us with 1.0f / x, 196 so).
+__device__ inline float sigm(float z) { return 1.0f / (1.0f + __expf(-z)); }
+constexpr float kSigmLow = -87.0f;
+__device__ inline float sigm_mid(float z) {
+  const float x = 1.0f + __expf(-z);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+}
+template <int N>
+__device__ inline bool all_mid(const float *z) {
+  float lo = z[0];
+#pragma unroll
+  for (int j = 1; j < N; j++) lo = fminf(lo, z[j]);
+  return !(lo < kSigmLow);
+}
+// z = SiLU(z), and d = d SiLU'(z), of N values, rounded as in k_bias_act and
+// k_act_grad
+template <int N>
+__device__ inline void silu(float *z) {
+  if (all_mid<N>(z)) {
+#pragma unroll
+    for (int j = 0; j < N; j++) z[j] = __fmul_rn(z[j], sigm_mid(z[j]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; j++) z[j] = __fmul_rn(z[j], sigm(z[j]));
+  }
+}
+__device__ inline float act_grad(float d, float z, float s) {
+  return __fmul_rn(__fmul_rn(d, s), __fmaf_rn(z, 1.0f - s, 1.0f));
+}
+template <int N>
+__device__ inline void act_grad(float *d, const float *z) {
+  if (all_mid<N>(z)) {
+#pragma unroll
+    for (int j = 0; j < N; j++) d[j] = act_grad(d[j], z[j], sigm_mid(z[j]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; j++) d[j] = act_grad(d[j], z[j], sigm(z[j]));
+  }
 }
 
 // barrier of the epilogue threads; true when any of them passes true
@@ -386,12 +443,16 @@ __device__ inline void store32(float *dst, const float v[32]) {
 #pragma unroll
   for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
 }
-__device__ inline void load32(const float *src, float v[32]) {
+// d *= SiLU'(z) for 32 columns of a row, kept and stored
+__device__ inline void act_grad32(float d[32], const float *z, float *dst) {
 #pragma unroll
-  for (int j = 0; j < 32; j += 4) {
-    const float4 x = *reinterpret_cast<const float4 *>(src + j);
-    v[j] = x.x; v[j + 1] = x.y; v[j + 2] = x.z; v[j + 3] = x.w;
+  for (int j = 0; j < 32; j += 8) {
+    const float4 x = __ldg(reinterpret_cast<const float4 *>(z + j));
+    const float4 y = __ldg(reinterpret_cast<const float4 *>(z + j + 4));
+    const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    act_grad<8>(d + j, v);
   }
+  store32(dst, d);
 }
 
 // one thread: acc (+)= (hi + lo) of `stage` times the bfloat16 tile `b`, ks
@@ -406,23 +467,39 @@ __device__ inline void mma_chunk(uint32_t acc, const unsigned char *stage, const
   }
 }
 
-// shared set-up of the two row kernels: barriers, 512 tensor-memory columns,
-// biases and the last layer's weights
+// shared set-up of the two row kernels: barriers and, for the forward pass,
+// the biases and the last layer's weights (as floats, or as tiles of 16 outputs
+// x 32 units)
+enum MlpPass { ML_FORWARD, ML_TRAIN, ML_BACKWARD };
+template <MlpPass PASS>
 __device__ inline void mlp_setup(const MlpArgs &a, unsigned char *base, const MlpLayout &lay, MlpBars *sb) {
   const int tid = threadIdx.x;
   if (tid == 0) {
     for (int q = 0; q < ML_ST; q++) { tc::mbar_init(&sb->full[q], 4); tc::mbar_init(&sb->empty[q], 1); }
-    tc::mbar_init(&sb->d1, 1); tc::mbar_init(&sb->d2, 1); tc::mbar_init(&sb->fin, 1);
+    tc::mbar_init(&sb->d1, 1); tc::mbar_init(&sb->d2, 1); tc::mbar_init(&sb->d3, 1); tc::mbar_init(&sb->fin, 1);
     sb->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if constexpr (PASS == ML_BACKWARD) return;
   float *b1 = reinterpret_cast<float *>(base + lay.b1), *b2 = reinterpret_cast<float *>(base + lay.b2);
-  float *w3 = reinterpret_cast<float *>(base + lay.w3);
   for (int c = tid; c < a.H; c += ML_THREADS) {
     b1[c] = a.b1[c];
     b2[c] = a.b2[c];
+  }
+  if constexpr (PASS == ML_TRAIN) {
+    for (int e = tid; e < 16 * (a.H / 8); e += ML_THREADS) {
+      const int o = e & 15, c8 = e >> 4;   // 8 units from 8 c8
+      __nv_bfloat16 v[8];
 #pragma unroll
-    for (int o = 0; o < ML_O; o++) w3[c * ML_O + o] = (o < a.O) ? __bfloat162float(a.W3[(size_t)o * a.H + c]) : 0.0f;
+      for (int u = 0; u < 8; u++) v[u] = (o < a.O) ? a.W3[(size_t)o * a.H + c8 * 8 + u] : __float2bfloat16_rn(0.0f);
+      *reinterpret_cast<uint4 *>(base + lay.w3 + (c8 >> 2) * W3_TILE + tc::sw64_chunk(o, c8 & 3)) =
+          *reinterpret_cast<const uint4 *>(v);
+    }
+  } else {
+    float *w3 = reinterpret_cast<float *>(base + lay.w3);
+    for (int c = tid; c < a.H; c += ML_THREADS)
+#pragma unroll
+      for (int o = 0; o < ML_O; o++) w3[c * ML_O + o] = (o < a.O) ? __bfloat162float(a.W3[(size_t)o * a.H + c]) : 0.0f;
   }
 }
 
@@ -448,7 +525,8 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
   const float *w3 = reinterpret_cast<float *>(base + lay.w3);
   float *yp = reinterpret_cast<float *>(base + lay.yp);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = a.H, nch = H / 32;
-  mlp_setup(a, base, lay, sb);
+  const int seq = TRAIN ? 2 * nch + 1 : nch + 1;   // stage uses of a tile
+  mlp_setup<TRAIN ? ML_TRAIN : ML_FORWARD>(a, base, lay, sb);
   if (warp == 0) tc::tmem_alloc(&sb->tmem, 512);
   // W1 [n = unit][k = input] as one chunk, W2 [n][k] as H / 32 chunks
   for (int e = tid; e < H * 4; e += ML_THREADS) {
@@ -472,18 +550,21 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
   bool bad = false;
   if (warp == ML_EPI / 32) {
     if (lane == 0) {
-      const uint32_t idesc = tc::idesc_bf16_f32(128, H);
+      const uint32_t idesc = tc::idesc_bf16_f32(128, H), idesc3 = tc::idesc_bf16_f32(128, 16);
       uint32_t q = 0;
       for (long long t = blockIdx.x; t < ntile && !bad; t += gridDim.x)
-        for (int c = -1; c < nch; c++, q++) {   // c = -1: the input rows
+        for (int c = -1; c < seq - 1; c++, q++) {   // c = -1: the input rows; from nch on: the last layer
           const uint32_t s = q % ML_ST;
           if (!tc::mbar_wait(&sb->full[s], (q / ML_ST) & 1, a.wait_ns)) { bad = true; break; }
           tc::tc_fence_after();
-          if (c < 0) mma_chunk(tmem, st0 + s * ML_STAGE, W1s, idesc, (a.F + 15) / 16, true);
-          else mma_chunk(tmem + 256, st0 + s * ML_STAGE, W2s + (size_t)c * H * 64, idesc, 2, c == 0);
+          unsigned char *st = st0 + s * ML_STAGE;
+          if (c < 0) mma_chunk(tmem, st, W1s, idesc, (a.F + 15) / 16, true);
+          else if (c < nch) mma_chunk(tmem + 256, st, W2s + (size_t)c * H * 64, idesc, 2, c == 0);
+          else mma_chunk(tmem, st, base + lay.w3 + (c - nch) * W3_TILE, idesc3, 2, c == nch);
           tc::mma_commit(&sb->empty[s]);
           if (c < 0) tc::mma_commit(&sb->d1);
           else if (c == nch - 1) tc::mma_commit(&sb->d2);
+          else if (TRAIN && c == seq - 2) tc::mma_commit(&sb->d3);
         }
       tc::mma_commit(&sb->fin);
       if (!tc::mbar_wait(&sb->fin, 0)) bad = true;
@@ -522,7 +603,7 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
     uint32_t q0 = 0;
     if (g == 0) put_input(blockIdx.x, 0);
     int i = 0;
-    for (long long t = blockIdx.x; t < ntile; t += gridDim.x, i++, q0 += nch + 1) {
+    for (long long t = blockIdx.x; t < ntile; t += gridDim.x, i++, q0 += seq) {
       const long long row = t * 128 + r;
       const bool in = row < a.n;
       if (!bad && !tc::mbar_wait(&sb->d1, i & 1, a.wait_ns)) bad = true;
@@ -537,15 +618,15 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
           z[j] += bv.x; z[j + 1] += bv.y; z[j + 2] += bv.z; z[j + 3] += bv.w;
         }
         if (TRAIN && in) store32(a.Z1 + row * H + c * 32, z);
-#pragma unroll
-        for (int j = 0; j < 32; j++) z[j] = silu(z[j]);
+        silu<32>(z);
         unsigned char *s = stage(q0 + 1 + c);
         if (!bad) put_chunk(s, r, z);
         tc::tc_fence_before();
         publish(q0 + 1 + c);
       }
-      // the next tile's input goes in front of this tile's last epilogue
-      if (g == 0 && t + gridDim.x < ntile) put_input(t + gridDim.x, q0 + nch + 1);
+      // the next tile's input goes in front of this tile's last epilogue (in
+      // training its product would overwrite the last layer's sums: after them)
+      if (!TRAIN && g == 0 && t + gridDim.x < ntile) put_input(t + gridDim.x, q0 + seq);
       if (!bad && !tc::mbar_wait(&sb->d2, i & 1, a.wait_ns)) bad = true;
       bad = __any_sync(0xffffffffu, bad);
       tc::tc_fence_after();
@@ -561,22 +642,41 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
           z[j] += bv.x; z[j + 1] += bv.y; z[j + 2] += bv.z; z[j + 3] += bv.w;
         }
         if (TRAIN && in) store32(a.Z2 + row * H + c * 32, z);
+        silu<32>(z);
+        if constexpr (TRAIN) {
+          unsigned char *s = stage(q0 + 1 + nch + c);
+          if (!bad) put_chunk(s, r, z);
+          tc::tc_fence_before();
+          publish(q0 + 1 + nch + c);
+        } else {
 #pragma unroll
-        for (int j = 0; j < 32; j++) {
-          const float h = silu(z[j]);
-          const float4 wa = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O);
-          y[0] += h * wa.x; y[1] += h * wa.y; y[2] += h * wa.z; y[3] += h * wa.w;
-          if constexpr (OC == 5) {
-            y[4] += h * w3[(c * 32 + j) * ML_O + 4];
-          } else {
-            const float4 wb = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O + 4);
-            y[4] += h * wb.x; y[5] += h * wb.y; y[6] += h * wb.z; y[7] += h * wb.w;
+          for (int j = 0; j < 32; j++) {
+            const float h = z[j];
+            const float4 wa = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O);
+            y[0] += h * wa.x; y[1] += h * wa.y; y[2] += h * wa.z; y[3] += h * wa.w;
+            if constexpr (OC == 5) {
+              y[4] += h * w3[(c * 32 + j) * ML_O + 4];
+            } else {
+              const float4 wb = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O + 4);
+              y[4] += h * wb.x; y[5] += h * wb.y; y[6] += h * wb.z; y[7] += h * wb.w;
+            }
           }
         }
       }
-      if (g > 0) {
+      if (!TRAIN && g > 0) {
 #pragma unroll
         for (int o = 0; o < OC; o++) yp[((g - 1) * 128 + r) * ML_O + o] = y[o];
+      }
+      if (TRAIN && g == 0) {   // the sums of the last layer, over the first one's
+        if (!bad && !tc::mbar_wait(&sb->d3, i & 1, a.wait_ns)) bad = true;
+        bad = __any_sync(0xffffffffu, bad);
+        tc::tc_fence_after();
+        float z[32];
+        tmem_ld32(tl, z);
+#pragma unroll
+        for (int o = 0; o < OC; o++) y[o] = z[o];
+        tc::tc_fence_before();
+        if (t + gridDim.x < ntile) put_input(t + gridDim.x, q0 + seq);
       }
       // every group has read the accumulators: the next tile may refill them
       tc::tc_fence_before();
@@ -588,14 +688,13 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
         for (int o = 0; o < OC; o++)
           if (in && o < a.O) {
             float v = y[o];
-#pragma unroll
-            for (int u = 0; u < ML_G - 1; u++) v += yp[(u * 128 + r) * ML_O + o];
-            v += a.b3[o];
             if (!TRAIN) {
-              a.Y[row * a.O + o] = v;
+#pragma unroll
+              for (int u = 0; u < ML_G - 1; u++) v += yp[(u * 128 + r) * ML_O + o];
+              a.Y[row * a.O + o] = v + a.b3[o];
             } else {
-              const float d = v - a.T[row * a.O + o];
-              a.dY[row * a.O + o] = d * a.scale;
+              const float d = v + a.b3[o] - a.T[row * a.O + o];
+              a.dY[row * a.O + o] = 2.0f * d / a.count;
               e += (double)d * (double)d;
             }
           }
@@ -609,21 +708,21 @@ k_mlp_fwd(const __grid_constant__ MlpArgs a) {
   mlp_finish(a, sb, tmem, bad);
 }
 
-// Data gradients of the hidden layers: dZ2 = (dY W3) SiLU'(Z2), written out
-// and, a chunk of 32 columns at a time, the A operand of dH1 = dZ2 W2 (the
-// CTA holds W2 transposed: [n = input unit][k = output unit]); then
-// dZ1 = dH1 SiLU'(Z1).  The same roles as k_mlp_fwd; tile i accumulates in
-// half i & 1 of tensor memory.
+// Data gradients of the hidden layers: dH2 = dY W3, dZ2 = dH2 SiLU'(Z2),
+// written out and, a chunk of 32 columns at a time, the A operand of
+// dH1 = dZ2 W2; then dZ1 = dH1 SiLU'(Z1).  The CTA holds W2 and W3 transposed
+// ([n = input unit][k = output unit], K of W3 padded to 16); dY goes through a
+// stage as the input rows of k_mlp_fwd do.  The same roles and hand-overs as
+// there, dH2 in the first half of tensor memory and dH1 in the second.
 __global__ void __launch_bounds__(ML_THREADS, 1)
 k_mlp_bwd(const __grid_constant__ MlpArgs a) {
   extern __shared__ unsigned char g_smem_raw[];
   unsigned char *base = tc::smem_base_1024(g_smem_raw);
   const MlpLayout lay = mlp_layout(a.H);
   MlpBars *sb = reinterpret_cast<MlpBars *>(base + lay.bar);
-  unsigned char *W2s = base + lay.w2, *st0 = base + lay.st;
-  const float *w3 = reinterpret_cast<float *>(base + lay.w3);
+  unsigned char *W2s = base + lay.w2, *W3s = base + lay.w1, *st0 = base + lay.st;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = a.H, nch = H / 32;
-  mlp_setup(a, base, lay, sb);
+  mlp_setup<ML_BACKWARD>(a, base, lay, sb);
   if (warp == 0) tc::tmem_alloc(&sb->tmem, 512);
   for (int e = tid; e < H * (H / 8); e += ML_THREADS) {
     const int r = e % H, c8 = e / H;   // lanes along the input units: coalesced reads of W2's rows
@@ -632,6 +731,13 @@ k_mlp_bwd(const __grid_constant__ MlpArgs a) {
     for (int u = 0; u < 8; u++) v[u] = a.W2[(size_t)(c8 * 8 + u) * H + r];
     *reinterpret_cast<uint4 *>(W2s + (size_t)(c8 >> 2) * H * 64 + tc::sw64_chunk(r, c8 & 3)) =
         *reinterpret_cast<const uint4 *>(v);
+  }
+  for (int e = tid; e < 2 * H; e += ML_THREADS) {
+    const int r = e % H, c = e / H;
+    __nv_bfloat16 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = (c * 8 + u < a.O) ? a.W3[(size_t)(c * 8 + u) * H + r] : __float2bfloat16_rn(0.0f);
+    *reinterpret_cast<uint4 *>(W3s + tc::sw64_chunk(r, c)) = *reinterpret_cast<const uint4 *>(v);
   }
   tc::fence_proxy_async();
   tc::tc_fence_before();
@@ -644,66 +750,69 @@ k_mlp_bwd(const __grid_constant__ MlpArgs a) {
     if (lane == 0) {
       const uint32_t idesc = tc::idesc_bf16_f32(128, H);
       uint32_t q = 0;
-      int i = 0;
-      for (long long t = blockIdx.x; t < ntile && !bad; t += gridDim.x, i++)
-        for (int c = 0; c < nch; c++, q++) {
+      for (long long t = blockIdx.x; t < ntile && !bad; t += gridDim.x)
+        for (int c = -1; c < nch; c++, q++) {   // c = -1: the rows of dY
           const uint32_t s = q % ML_ST;
           if (!tc::mbar_wait(&sb->full[s], (q / ML_ST) & 1, a.wait_ns)) { bad = true; break; }
           tc::tc_fence_after();
-          mma_chunk(tmem + (i & 1) * 256, st0 + s * ML_STAGE, W2s + (size_t)c * H * 64, idesc, 2, c == 0);
+          if (c < 0) mma_chunk(tmem, st0 + s * ML_STAGE, W3s, idesc, 1, true);
+          else mma_chunk(tmem + 256, st0 + s * ML_STAGE, W2s + (size_t)c * H * 64, idesc, 2, c == 0);
           tc::mma_commit(&sb->empty[s]);
-          if (c == nch - 1) tc::mma_commit(&sb->d1);
+          if (c < 0) tc::mma_commit(&sb->d1);
+          else if (c == nch - 1) tc::mma_commit(&sb->d2);
         }
       tc::mma_commit(&sb->fin);
       if (!tc::mbar_wait(&sb->fin, 0)) bad = true;
     }
   } else {
     const int qd = warp & 3, g = warp >> 2, r = qd * 32 + lane;
+    const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
+    // v into the stage of sequence number q, once its last MMAs have read it
+    auto put = [&](uint32_t q, const float v[32]) {
+      if (q >= ML_ST && !bad && !tc::mbar_wait(&sb->empty[q % ML_ST], ((q / ML_ST) - 1) & 1, a.wait_ns)) bad = true;
+      bad = __any_sync(0xffffffffu, bad);
+      if (!bad) put_chunk(st0 + (q % ML_ST) * ML_STAGE, r, v);
+      tc::tc_fence_before();
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&sb->full[q % ML_ST]);
+    };
+    auto put_dy = [&](long long t, uint32_t q) {
+      const long long row = t * 128 + r;
+      float x[32];
+#pragma unroll
+      for (int o = 0; o < 32; o++) x[o] = (o < ML_O && o < a.O && row < a.n) ? a.dY[row * a.O + o] : 0.0f;
+      put(q, x);
+    };
     uint32_t q0 = 0;
+    if (g == 0) put_dy(blockIdx.x, 0);
     int i = 0;
-    for (long long t = blockIdx.x; t < ntile; t += gridDim.x, i++, q0 += nch) {
+    for (long long t = blockIdx.x; t < ntile; t += gridDim.x, i++, q0 += nch + 1) {
       const long long row = t * 128 + r;
       const bool in = row < a.n;
-      const uint32_t tl = tmem + (i & 1) * 256 + ((uint32_t)(qd * 32) << 16);
-      float dy[ML_O];
-#pragma unroll
-      for (int o = 0; o < ML_O; o++) dy[o] = (in && o < a.O) ? a.dY[row * a.O + o] : 0.0f;
-      for (int c = g; c < nch; c += ML_G) {
-        float z[32];
-        if (in) load32(a.Z2 + row * H + c * 32, z);
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-          const float4 wa = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O);
-          float d = dy[0] * wa.x + dy[1] * wa.y + dy[2] * wa.z + dy[3] * wa.w;
-          if (a.O > 4) {
-            const float4 wb = *reinterpret_cast<const float4 *>(w3 + (c * 32 + j) * ML_O + 4);
-            d += dy[4] * wb.x + dy[5] * wb.y + dy[6] * wb.z + dy[7] * wb.w;
-          }
-          z[j] = in ? d * dsilu(z[j]) : 0.0f;
-        }
-        if (in) store32(a.dZ2 + row * H + c * 32, z);
-        const uint32_t q = q0 + c;
-        if (q >= ML_ST && !bad && !tc::mbar_wait(&sb->empty[q % ML_ST], ((q / ML_ST) - 1) & 1, a.wait_ns)) bad = true;
-        bad = __any_sync(0xffffffffu, bad);
-        if (!bad) put_chunk(st0 + (q % ML_ST) * ML_STAGE, r, z);
-        tc::fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&sb->full[q % ML_ST]);
-      }
       if (!bad && !tc::mbar_wait(&sb->d1, i & 1, a.wait_ns)) bad = true;
       bad = __any_sync(0xffffffffu, bad);
       tc::tc_fence_after();
       for (int c = g; c < nch; c += ML_G) {
-        float d[32], z[32];
+        float d[32];
         tmem_ld32(tl + c * 32, d);
-        if (in) {
-          load32(a.Z1 + row * H + c * 32, z);
+        if (in) act_grad32(d, a.Z2 + row * H + c * 32, a.dZ2 + row * H + c * 32);
+        else
 #pragma unroll
-          for (int j = 0; j < 32; j++) d[j] *= dsilu(z[j]);
-          store32(a.dZ1 + row * H + c * 32, d);
-        }
+          for (int j = 0; j < 32; j++) d[j] = 0.0f;
+        put(q0 + 1 + c, d);
       }
-      // every group has read this half before the tile after next refills it
+      // the next tile's dY goes in front of this tile's last epilogue
+      if (g == 0 && t + gridDim.x < ntile) put_dy(t + gridDim.x, q0 + nch + 1);
+      if (!bad && !tc::mbar_wait(&sb->d2, i & 1, a.wait_ns)) bad = true;
+      bad = __any_sync(0xffffffffu, bad);
+      tc::tc_fence_after();
+      for (int c = g; c < nch; c += ML_G) {
+        float d[32];
+        tmem_ld32(tl + 256 + c * 32, d);
+        if (in) act_grad32(d, a.Z1 + row * H + c * 32, a.dZ1 + row * H + c * 32);
+      }
+      // every group has read the accumulators: the next tile may refill them
       tc::tc_fence_before();
       bad = epi_any(bad);
       if (bad) break;
@@ -781,7 +890,8 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
         hh[e] = in ? __ldg(a.Z2 + at) : 0.0f;
       }
 #pragma unroll
-      for (int e = 0; e < 8; e++) { sb2 += v2[e]; sb1 += v1[e]; hh[e] = silu(hh[e]); }
+      for (int e = 0; e < 8; e++) { sb2 += v2[e]; sb1 += v1[e]; }
+      silu<8>(hh);
       put_row8<2>(st, GA_BYTES, m, c, v2);
       put_row8<2>(st + 2 * GA_BYTES, GA_BYTES, m, c, v1);
       put_row8<2>(st + 4 * GA_BYTES, GA_BYTES, m, c, hh);
@@ -795,8 +905,7 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
         const long long k = kb + c * 8 + e;
         v[e] = (k < k1) ? __ldg(a.Z1 + (size_t)k * H + u) : 0.0f;
       }
-#pragma unroll
-      for (int e = 0; e < 8; e++) v[e] = silu(v[e]);
+      silu<8>(v);
       put_row8<2>(tB, bb, u, c, v);
     }
     // B tiles X and dY: thread = (chunk of 8 rows, column)
@@ -825,16 +934,19 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
       for (int ks = 0; ks < GK / 16; ks++) {
         const uint64_t o = (uint64_t)(ks * 2);
         const uint32_t first = (ib == 0 && ks == 0) ? 0u : 1u;
-        auto mul = [&](uint32_t acc, const unsigned char *A, const unsigned char *B, uint32_t lo, uint32_t idesc) {
+        // the cross terms in the order of k_tc_gemm's dZ^T H, dZ^T X and dY^T H (W3: A and B change places)
+        auto mul = [&](uint32_t acc, const unsigned char *A, const unsigned char *B, uint32_t lo, uint32_t idesc,
+                       bool swapped) {
           const uint64_t ah = tc::smem_desc_sw64(A) + o, al = tc::smem_desc_sw64(A + GA_BYTES) + o;
           const uint64_t bh = tc::smem_desc_sw64(B) + o, bl = tc::smem_desc_sw64(B + lo) + o;
           tc::mma_f16(acc, ah, bh, idesc, first);
+          if (swapped) tc::mma_f16(acc, al, bh, idesc, 1u);
           tc::mma_f16(acc, ah, bl, idesc, 1u);
-          tc::mma_f16(acc, al, bh, idesc, 1u);
+          if (!swapped) tc::mma_f16(acc, al, bh, idesc, 1u);
         };
-        mul(tmem, st, tB, bb, id2);
-        mul(tmem + 256, st + 2 * GA_BYTES, tX, 32 * 64, id1);
-        mul(tmem + 288, st + 4 * GA_BYTES, tY, 32 * 64, id3);
+        mul(tmem, st, tB, bb, id2, false);
+        mul(tmem + 256, st + 2 * GA_BYTES, tX, 32 * 64, id1, false);
+        mul(tmem + 288, st + 4 * GA_BYTES, tY, 32 * 64, id3, true);
       }
       tc::mma_commit(&bar[s]);
     }
@@ -893,8 +1005,6 @@ k_loss_sum(long long np, const double *part, double inv, double *out) {
   }
   if (threadIdx.x == 0) out[0] = sh[0] * inv;
 }
-
-__device__ inline float sigm(float z) { return 1.0f / (1.0f + __expf(-z)); }
 
 // Z += b (per column); H = SiLU(Z) (act != 0) or Z
 __global__ void k_bias_act(size_t n, int w, float *Z, const float *b, float *H, int act) {
@@ -1050,7 +1160,7 @@ MlpArgs mlp_args(const cb2_mlp *n, const float *X, size_t rows, int *status) {
   a.vec = n->F % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
   a.b1 = n->master + n->ob1; a.b2 = n->master + n->ob2; a.b3 = n->master + n->ob3;
   a.W1 = n->w + n->oW1; a.W2 = n->w + n->oW2; a.W3 = n->w + n->oW3;
-  a.scale = 2.0f / (float)(rows * (size_t)n->O);
+  a.count = (float)(rows * (size_t)n->O);
   a.status = status;
   a.wait_ns = kWaitNsGemm;
   return a;
@@ -1067,6 +1177,13 @@ int launch_rows(K *kernel, const MlpArgs &a, cudaStream_t st) {
   kernel<<<(unsigned)std::min<long long>(sms, (a.n + 127) / 128), ML_THREADS, smem, st>>>(a);
   CB2_CUDA(cudaGetLastError());
   return 0;
+}
+
+// rows of a chunk of a sum over n rows into `tiles` output tiles: at least 256,
+// and the chunks cover the SMs about twice
+int split_chunk(long long n, int tiles) {
+  const long long nz = std::max<long long>(1, std::min<long long>((n + 255) / 256, (2 * 148 + tiles - 1) / tiles));
+  return (int)(((n + nz - 1) / nz + GK - 1) / GK * GK);
 }
 
 // C = opA opB on the tensor cores (k_tc_gemm).  split_k: K is cut into
@@ -1090,8 +1207,7 @@ void gemm(cudaStream_t st, int *status, int M, int N, int K, const TAT *A, int l
   const int tiles = ((N + NT - 1) / NT) * ((M + 127) / 128);
   int kchunk = K, nz = 1;
   if (split_k) {
-    nz = std::max(1, std::min((K + 255) / 256, (2 * 148 + tiles - 1) / tiles));
-    kchunk = (((K + nz - 1) / nz) + GK - 1) / GK * GK;
+    kchunk = split_chunk(K, tiles);
     nz = (K + kchunk - 1) / kchunk;
     cudaMemsetAsync(C, 0, (size_t)M * ldc * sizeof(float), st);
   }
@@ -1139,10 +1255,8 @@ int mlp_backward_fused(cb2_mlp *nt, const float *X, const float *T, size_t n) {
   w.gW1 = nt->grad + nt->oW1; w.gb1 = nt->grad + nt->ob1; w.gW2 = nt->grad + nt->oW2; w.gb2 = nt->grad + nt->ob2;
   w.gW3 = nt->grad + nt->oW3; w.gb3 = nt->grad + nt->ob3;
   w.status = nt->status; w.wait_ns = kWaitNsGemm;
-  // about one CTA an SM: 74 row chunks x 2 halves of the units
   const int ny = (a.H + 127) / 128;
-  const long long want = std::max<long long>(1, 148 / ny);
-  w.kchunk = (int)(((a.n + want - 1) / want + GK - 1) / GK * GK);
+  w.kchunk = split_chunk(a.n, ny);
   const size_t smem = 2 * (size_t)wg_stage(a.H) + 64 + 1024;
   CB2_CUDA(raise_smem_limit(k_mlp_wgrad, smem));
   k_mlp_wgrad<<<dim3((unsigned)((a.n + w.kchunk - 1) / w.kchunk), ny), WG_THREADS, smem, st>>>(w);
