@@ -283,13 +283,14 @@ k_tc_gemm(int M, int N, int NT, int K, const TAT *__restrict__ A, int lda, const
 // and SiLU 505); kept in tensor and shared memory the pass reads 64 and
 // writes 20 bytes a row and takes 196 us, bound by the SiLU epilogue (an
 // __expf and a reciprocal per unit and layer) and the operand split.  A
-// training pass of 16384 rows: 29 + 39 + 52 us of kernels, before 500 us.
+// training pass of 16384 rows: 29 + 39 + 55 + 3 us of kernels, before 500 us.
 //
 // A training pass forms every product and activation with the terms, the order
 // and the rounding of the general kernels (k_tc_gemm, k_bias_act, k_mse,
 // k_act_grad), so its loss and gradients do not depend on which of the two a
 // network's widths select: they are equal bit for bit but for the order of the
-// float32 atomics that add the weight gradients' row chunks.  That matters
+// float32 atomics that add the weight gradients' row chunks and of the float64
+// sums of the bias gradients.  That matters
 // because an optimiser carries a difference on: an Adam step is +- lr where a
 // gradient is far above eps, whatever its size, and one weight that rounds the
 // other way to bfloat16 moves the next gradient by 1e-5.
@@ -828,6 +829,9 @@ k_mlp_bwd(const __grid_constant__ MlpArgs a) {
 // K-major tiles (the lanes along the columns, so every read is a whole line),
 // float32 values as bfloat16 hi + lo: products hi hi', hi lo', lo hi' as in
 // k_tc_gemm.  The partial sums are added with 16-byte float32 atomics.
+// The bias gradients, sums of up to a whole batch that cancel, are float64
+// throughout: per thread, per CTA into `bias`, and over the CTAs in a fixed
+// order (k_mlp_sums), so they are rounded once and the same in every run.
 // One launch for what three k_tc_gemm launches (96 us at 16384 rows) and
 // three column-sum launches (63 us, one block a column) did.
 constexpr int WG_THREADS = 512;
@@ -835,7 +839,8 @@ struct WgradArgs {
   long long n;
   int F, H, O, kchunk;
   const float *X, *Z1, *Z2, *dY, *dZ1, *dZ2;
-  float *gW1, *gb1, *gW2, *gb2, *gW3, *gb3;
+  float *gW1, *gW2, *gW3;
+  double *bias;              // [x][2 H + ML_O]: column sums of dZ1, dZ2 and dY
   int *status;
   unsigned long long wait_ns;
 };
@@ -866,7 +871,7 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
   const int nblk = (int)((k1 - k0 + GK - 1) / GK);
   const int NF = ((F + 15) / 16) * 16, NO16 = 16;
   const uint32_t id2 = tc::idesc_bf16_f32(128, H), id1 = tc::idesc_bf16_f32(128, NF), id3 = tc::idesc_bf16_f32(128, NO16);
-  float sb1 = 0.0f, sb2 = 0.0f, sb3 = 0.0f;   // column sums of dZ1, dZ2 (thread = unit m0 + tid) and dY
+  double sb1 = 0.0, sb2 = 0.0, sb3 = 0.0;   // column sums of dZ1, dZ2 (thread = unit m0 + (tid & 127)) and dY
   bool bad = false;
   for (int ib = 0; ib < nblk; ib++) {
     const int s = ib & 1;
@@ -890,7 +895,7 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
         hh[e] = in ? __ldg(a.Z2 + at) : 0.0f;
       }
 #pragma unroll
-      for (int e = 0; e < 8; e++) { sb2 += v2[e]; sb1 += v1[e]; }
+      for (int e = 0; e < 8; e++) { sb2 += (double)v2[e]; sb1 += (double)v1[e]; }
       silu<8>(hh);
       put_row8<2>(st, GA_BYTES, m, c, v2);
       put_row8<2>(st + 2 * GA_BYTES, GA_BYTES, m, c, v1);
@@ -922,7 +927,7 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
       }
       if (!isx) {
 #pragma unroll
-        for (int e = 0; e < 8; e++) sb3 += v[e];
+        for (int e = 0; e < 8; e++) sb3 += (double)v[e];
       }
       put_row8<2>(isx ? tX : tY, 32 * 64, u, c, v);
     }
@@ -980,21 +985,28 @@ k_mlp_wgrad(const __grid_constant__ WgradArgs a) {
       for (int j = 0; j < ML_O; j++)
         if (u < H && j < O) atomicAdd(a.gW3 + (size_t)j * H + u, v[j]);
     }
-    if (m0 + (tid & 127) < H) {
-      atomicAdd(a.gb1 + m0 + (tid & 127), sb1);
-      atomicAdd(a.gb2 + m0 + (tid & 127), sb2);
+    // the four threads of a unit (and of a column of dY), in the stages' memory
+    double *red = reinterpret_cast<double *>(base);
+    red[tid] = sb1;
+    red[WG_THREADS + tid] = sb2;
+    if (tid >= 128 && tid < 256) red[2 * WG_THREADS + tid - 128] = sb3;
+    __syncthreads();
+    double *out = a.bias + (size_t)blockIdx.x * (2 * H + ML_O);
+    auto sum4 = [](const double *x, int st) { return ((x[0] + x[st]) + x[2 * st]) + x[3 * st]; };
+    if (tid < 256) {
+      const int m = tid & 127, which = tid >> 7;
+      if (m0 + m < H) out[which * H + m0 + m] = sum4(red + which * WG_THREADS + m, 128);
+    } else if (blockIdx.y == 0 && tid < 256 + O) {
+      out[2 * H + tid - 256] = sum4(red + 2 * WG_THREADS + tid - 256, 32);
     }
-    if (blockIdx.y == 0 && tid >= 128 && tid < 256 && (tid & 31) < O) atomicAdd(a.gb3 + (tid & 31), sb3);
   }
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, 512);
 }
 
-// loss = sum of the partial sums / (n O) (one block, fixed order)
-__global__ void __launch_bounds__(256)
-k_loss_sum(long long np, const double *part, double inv, double *out) {
-  __shared__ double sh[256];
+// loss = sum of the partial sums / (n O) (one block of 256, fixed order)
+__device__ inline void loss_sum(double *sh, long long np, const double *part, double inv, double *out) {
   double s = 0.0;
   for (long long i = threadIdx.x; i < np; i += 256) s += part[i];
   sh[threadIdx.x] = s;
@@ -1004,6 +1016,33 @@ k_loss_sum(long long np, const double *part, double inv, double *out) {
     __syncthreads();
   }
   if (threadIdx.x == 0) out[0] = sh[0] * inv;
+}
+__global__ void __launch_bounds__(256)
+k_loss_sum(long long np, const double *part, double inv, double *out) {
+  __shared__ double sh[256];
+  loss_sum(sh, np, part, inv, out);
+}
+
+// after k_mlp_wgrad: a block adds 32 columns of its nx partial sums, eight
+// threads a column, into the bias gradients; the last block the loss
+__global__ void __launch_bounds__(256)
+k_mlp_sums(int nx, int H, int O, const double *bias, float *gb1, float *gb2, float *gb3, long long np,
+           const double *part, double inv, double *loss) {
+  __shared__ double sh[256];
+  if (blockIdx.x == gridDim.x - 1) {
+    loss_sum(sh, np, part, inv, loss);
+    return;
+  }
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31);
+  double s = 0.0;
+  if (c < 2 * H + O)
+    for (int x = threadIdx.x >> 5; x < nx; x += 8) s += bias[(size_t)x * (2 * H + ML_O) + c];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x >= 32 || c >= 2 * H + O) return;
+  for (int q = 1; q < 8; q++) s += sh[32 * q + threadIdx.x];
+  float *g = (c < H) ? gb1 + c : (c < 2 * H) ? gb2 + c - H : gb3 + c - 2 * H;
+  *g = (float)s;
 }
 
 // Z += b (per column); H = SiLU(Z) (act != 0) or Z
@@ -1098,6 +1137,7 @@ struct cb2_mlp {
   float *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr, *Yp = nullptr, *dY = nullptr;
   float *dH = nullptr, *dZ = nullptr;
   double *part = nullptr;       // loss partial sums
+  double *bias = nullptr;       // bias gradients' partial sums (fused passes)
   // behind the gradient in its allocation, read together: the loss of the
   // last fused training pass and the status word of the products (bit 2: a
   // wait ran out)
@@ -1122,6 +1162,16 @@ bool fused_ok(const cb2_mlp *n) {
   return n->F <= 32 && n->H % 32 == 0 && n->H >= 64 && n->H <= 256 && n->O <= ML_O && n->oW2 % 8 == 0;
 }
 
+// chunks (at most) and rows of a chunk of a sum over n rows into `tiles` output tiles: at
+// least 256 rows, and the chunks cover the SMs about twice
+long long split_chunks(long long n, int tiles) {
+  return std::max<long long>(1, std::min<long long>((n + 255) / 256, (2 * 148 + tiles - 1) / tiles));
+}
+int split_chunk(long long n, int tiles) {
+  const long long nz = split_chunks(n, tiles);
+  return (int)(((n + nz - 1) / nz + GK - 1) / GK * GK);
+}
+
 // Work buffers of `rows` rows, one allocation.  The fused passes keep the
 // activations on the chip: inference needs none of these, training Z1, Z2 and
 // the gradients dY, dZ2 (in dZ) and dZ1 (in dH).
@@ -1130,14 +1180,16 @@ int mlp_reserve(cb2_mlp *n, size_t rows, bool train) {
   if ((fused && !train) || rows <= n->cap) return 0;
   const size_t w = (rows * n->H + 63) / 64 * 64, wy = (rows * n->O + 63) / 64 * 64;
   const size_t pc = std::max((size_t)blocks(rows * n->O), 4 * ((rows + 127) / 128)) + 1;
+  const size_t bc = fused ? (size_t)split_chunks(rows, (n->H + 127) / 128) * (2 * n->H + ML_O) : 0;
   n->cap = 0;
   if (n->work) cudaFree(n->work);
   n->work = nullptr;
-  CB2_CUDA(cudaMalloc(&n->work, ((fused ? 4 : 6) * w + wy) * sizeof(float) + pc * sizeof(double)));
+  CB2_CUDA(cudaMalloc(&n->work, ((fused ? 4 : 6) * w + wy) * sizeof(float) + (pc + bc) * sizeof(double)));
   n->Z1 = n->work; n->Z2 = n->Z1 + w; n->dH = n->Z2 + w; n->dZ = n->dH + w;
   n->H1 = n->dZ + w; n->H2 = n->H1 + w;   // the general passes only
   n->dY = n->dZ + (fused ? 1 : 3) * w;
   n->part = reinterpret_cast<double *>(n->dY + wy);
+  n->bias = n->part + pc;
   n->cap = rows;
   return 0;
 }
@@ -1177,13 +1229,6 @@ int launch_rows(K *kernel, const MlpArgs &a, cudaStream_t st) {
   kernel<<<(unsigned)std::min<long long>(sms, (a.n + 127) / 128), ML_THREADS, smem, st>>>(a);
   CB2_CUDA(cudaGetLastError());
   return 0;
-}
-
-// rows of a chunk of a sum over n rows into `tiles` output tiles: at least 256,
-// and the chunks cover the SMs about twice
-int split_chunk(long long n, int tiles) {
-  const long long nz = std::max<long long>(1, std::min<long long>((n + 255) / 256, (2 * 148 + tiles - 1) / tiles));
-  return (int)(((n + nz - 1) / nz + GK - 1) / GK * GK);
 }
 
 // C = opA opB on the tensor cores (k_tc_gemm).  split_k: K is cut into
@@ -1247,19 +1292,23 @@ int mlp_backward_fused(cb2_mlp *nt, const float *X, const float *T, size_t n) {
   CB2_CUDA(cudaMemsetAsync(nt->grad, 0, nt->np * sizeof(float), st));
   int rc = nt->O <= 5 ? launch_rows(k_mlp_fwd<true, 5>, a, st) : launch_rows(k_mlp_fwd<true, 8>, a, st);
   if (rc) return rc;
-  k_loss_sum<<<1, 256, 0, st>>>(4 * ((a.n + 127) / 128), nt->part, 1.0 / ((double)n * nt->O), nt->loss);
   if ((rc = launch_rows(k_mlp_bwd, a, st))) return rc;
   WgradArgs w{};
   w.n = a.n; w.F = a.F; w.H = a.H; w.O = a.O;
   w.X = X; w.Z1 = nt->Z1; w.Z2 = nt->Z2; w.dY = nt->dY; w.dZ1 = nt->dH; w.dZ2 = nt->dZ;
-  w.gW1 = nt->grad + nt->oW1; w.gb1 = nt->grad + nt->ob1; w.gW2 = nt->grad + nt->oW2; w.gb2 = nt->grad + nt->ob2;
-  w.gW3 = nt->grad + nt->oW3; w.gb3 = nt->grad + nt->ob3;
+  w.gW1 = nt->grad + nt->oW1; w.gW2 = nt->grad + nt->oW2; w.gW3 = nt->grad + nt->oW3;
+  w.bias = nt->bias;
   w.status = nt->status; w.wait_ns = kWaitNsGemm;
   const int ny = (a.H + 127) / 128;
   w.kchunk = split_chunk(a.n, ny);
   const size_t smem = 2 * (size_t)wg_stage(a.H) + 64 + 1024;
   CB2_CUDA(raise_smem_limit(k_mlp_wgrad, smem));
-  k_mlp_wgrad<<<dim3((unsigned)((a.n + w.kchunk - 1) / w.kchunk), ny), WG_THREADS, smem, st>>>(w);
+  const unsigned nx = (unsigned)((a.n + w.kchunk - 1) / w.kchunk);
+  k_mlp_wgrad<<<dim3(nx, ny), WG_THREADS, smem, st>>>(w);
+  k_mlp_sums<<<cdiv(2 * a.H + a.O, 32) + 1, 256, 0, st>>>((int)nx, a.H, a.O, nt->bias, nt->grad + nt->ob1,
+                                                          nt->grad + nt->ob2, nt->grad + nt->ob3,
+                                                          4 * ((a.n + 127) / 128), nt->part,
+                                                          1.0 / ((double)n * nt->O), nt->loss);
   CB2_CUDA(cudaGetLastError());
   return 0;
 }
