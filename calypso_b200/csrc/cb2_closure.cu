@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 #include "cb2_internal.cuh"
@@ -1513,7 +1514,19 @@ static int mlp_status(cb2_mlp *n, double *loss = nullptr) {
 
 int cb2_mlp_forward(cb2_mlp *n, const float *dev_x, long long rows, float *dev_y) {
   if (!n || !dev_x || !dev_y || rows <= 0) return CB2_ERR_ARG;
-  if (int rc = mlp_forward(n, dev_x, (size_t)rows, dev_y, n->stream)) return rc;
+  // the fused pass writes the rows of a tile while other tiles are still to be
+  // read: an output that overlaps the input goes through a buffer (the
+  // general kernels have read the input when their last layer writes)
+  const size_t nx = (size_t)rows * n->F, ny = (size_t)rows * n->O;
+  const std::less<const float *> before;
+  const bool overlap = fused_ok(n) && before(dev_x, dev_y + ny) && before(dev_y, dev_x + nx);
+  float *y = dev_y;
+  if (overlap) {
+    if (int rc = mlp_reserve_y(n, (size_t)rows)) return rc;
+    y = n->Yp;
+  }
+  if (int rc = mlp_forward(n, dev_x, (size_t)rows, y, n->stream)) return rc;
+  if (overlap) CB2_CUDA(cudaMemcpyAsync(dev_y, y, ny * sizeof(float), cudaMemcpyDeviceToDevice, n->stream));
   return mlp_status(n);
 }
 

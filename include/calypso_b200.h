@@ -336,7 +336,7 @@ int cb2_mlp_num_params(const cb2_mlp *net);
 /* float32 master parameters W1[nhid][nin], b1, W2[nhid][nhid], b2, W3[nout][nhid], b3 */
 int cb2_mlp_get_params(cb2_mlp *net, float *host);
 int cb2_mlp_set_params(cb2_mlp *net, const float *host);
-/* device buffers: x = rows x nin, y = rows x nout (float32) */
+/* device buffers: x = rows x nin, y = rows x nout (float32); they may overlap */
 int cb2_mlp_forward(cb2_mlp *net, const float *dev_x, long long rows, float *dev_y);
 /* mean squared error against dev_t and its gradient (kept for
  * cb2_mlp_adam_step; also copied to host_grad when it is not NULL) */
