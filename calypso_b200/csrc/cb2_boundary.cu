@@ -178,6 +178,7 @@ int upload_rlm(Ctx &c, const cb2_sph_tables *t) {
   if (int rc = tables_alloc(c)) return rc;
   CB2_CUDA(cudaMemcpyAsync(c.d_bnd_tab, pairs.get(), 2 * (size_t)nj * sizeof(int), cudaMemcpyHostToDevice, c.stream));
   c.bnd_rlm_key.assign(lm, lm + 2 * (size_t)nj);
+  c.bnd_rlm_full = once;
   return 0;
 }
 
@@ -604,8 +605,9 @@ int cb2_leg_bwd(cb2_ctx *c, const cb2_sph_tables *t, int ncomp, int nvector, int
     int slots[13];
     for (int g = 0; g < ch.nv; g++) slots[g] = MADV + 3 * g;
     for (int s = 0; s < ch.ns; s++) slots[ch.nv + s] = MADV + 3 * ch.nv + s;
-    // modes the table leaves out are zero
-    if (nj < c->jmax)
+    // modes the table leaves out are zero (one that lists a mode twice leaves
+    // another out, however long it is)
+    if (!c->bnd_rlm_full)
       CB2_CUDA(cudaMemsetAsync(c->fld(MADV), 0, (size_t)nc * c->fsize() * sizeof(double), c->stream));
     k_rlm_slots<true><<<dim3(cdiv(nj, JT), cdiv(c->nr, JK)), kBnd, JK * JT * (nc | 1) * sizeof(double), c->stream>>>(
         nj, c->nr, ncomp, t->istep_rlm[0], t->istep_rlm[1], ch.comp0, FastDiv(nc), MADV, dt.jo, const_cast<double *>(dWR),

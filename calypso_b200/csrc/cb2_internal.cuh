@@ -130,6 +130,7 @@ struct Ctx {
   size_t bnd_a_bytes = 0, bnd_b_bytes = 0, bnd_grid_bytes = 0;
   int *d_bnd_tab = nullptr, *d_bnd_mtab = nullptr;   // one allocation (d_bnd_tab)
   std::vector<int> bnd_rlm_key, bnd_rtm_key;   // the values the two device tables were made from
+  bool bnd_rlm_full = false;                   // the rlm table lists every mode once
   int istep = 0;
   bool started = false;
   // the nonlinear terms of the current state are not computed yet
