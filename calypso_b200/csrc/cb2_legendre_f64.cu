@@ -278,18 +278,22 @@ k_leg_bwd_f64(const __grid_constant__ LegArgs a) {
 struct FwdTileSz {
   static constexpr int NC = 8, AP = NC + 4, BP = LNB + 4;
   static constexpr int SA = 64 * AP, SB = 2 * NC * BP, STG = 2 * SA + SB;
+  // nh: south nodes whose weights are staged
   static size_t smem(int nh) {
     return LST * (size_t)STG * sizeof(double) + sizeof(LegCols) + (size_t)((nh + NC - 1) / NC * NC) * sizeof(double2);
   }
 };
 
+// WSM: the weights of the south nodes sit in shared memory, which has room for
+// 10,512 of them; beyond that they are read where they are used.
+template <bool WSM>
 __global__ void __launch_bounds__(LTH, 3)
 k_leg_fwd_f64(const __grid_constant__ LegArgs a) {
   using Z = FwdTileSz;
   constexpr int NC = Z::NC, AP = Z::AP, BP = Z::BP;
   extern __shared__ __align__(16) double smf[];
   LegCols &tc = *reinterpret_cast<LegCols *>(smf + LST * Z::STG);
-  double2 *wa = reinterpret_cast<double2 *>(&tc + 1);   // (w, m / sin(theta)) of each south node, zero beyond
+  double2 *wa = reinterpret_cast<double2 *>(&tc + 1);
   const int m = blockIdx.z, t0 = blockIdx.x * 64, nl = a.L + 1 - m;
   if (t0 >= nl) return;
   const bool isD = (int)blockIdx.y >= a.tilesP;
@@ -298,8 +302,12 @@ k_leg_fwd_f64(const __grid_constant__ LegArgs a) {
   const int ncols = a.nr * (isD ? 4 * a.nvec : 2 * (a.nvec + a.nscal));
   leg_columns(a, m, isD, c0, a.r, tc);
   const int nchk = (a.nh + NC - 1) / NC;
-  for (int i = tid; i < nchk * NC; i += LTH)
-    wa[i] = (i < a.nh) ? make_double2(a.wgt[i], (double)m * a.asin_t[i]) : make_double2(0.0, 0.0);
+  // (w, m / sin(theta)) of a south node, zero beyond
+  auto weight = [&](int i) {
+    return (i < a.nh) ? make_double2(a.wgt[i], (double)m * a.asin_t[i]) : make_double2(0.0, 0.0);
+  };
+  if (WSM)
+    for (int i = tid; i < nchk * NC; i += LTH) wa[i] = weight(i);
   const size_t po = a.poff[m], st = isD ? a.four.sD() : a.four.sP();
   const double *rows = (isD ? a.four.D : a.four.P) + (size_t)m * a.nth * st + c0;
   const bool pair16 = (a.nh & 1) == 0;
@@ -359,7 +367,7 @@ k_leg_fwd_f64(const __grid_constant__ LegArgs a) {
 #pragma unroll
     for (int ks = 0; ks < NC / 4; ks++) {
       const int kk = ks * 4 + tq;
-      const double2 w = wa[ch * NC + kk];
+      const double2 w = WSM ? wa[ch * NC + kk] : weight(ch * NC + kk);
       double sym[2], ant[2];
 #pragma unroll
       for (int c = 0; c < 2; c++) {
@@ -440,6 +448,13 @@ void launch_bwd(Ctx &c, const LegArgs &a, int tiles) {
   k_leg_bwd_f64<MF><<<dim3(cdiv(c.nh, 16 * MF), tiles, c.L + 1), LTH, sm, c.stream>>>(a);
 }
 
+template <bool WSM>
+void launch_fwd(Ctx &c, const LegArgs &a, int tiles) {
+  const size_t sm = FwdTileSz::smem(WSM ? c.nh : 0);
+  raise_smem_limit(k_leg_fwd_f64<WSM>, sm);
+  k_leg_fwd_f64<WSM><<<dim3(cdiv(c.L + 1, 64), tiles, c.L + 1), LTH, sm, c.stream>>>(a);
+}
+
 }  // namespace
 
 // order-major float64 Fourier rows over a buffer of (L+1) nth nr (6 nvec + 2
@@ -462,9 +477,8 @@ void leg_bwd_f64(Ctx &c, const int *slots, const MLayout64 &out) {
 void leg_fwd_f64(Ctx &c, const MLayout64 &in, const int *slots) {
   const LegArgs a = leg_args(c, in, slots);
   const int tiles = a.tilesP + cdiv((long)c.nr * in.rpD(), LNB);
-  const size_t sm = FwdTileSz::smem(c.nh);
-  raise_smem_limit(k_leg_fwd_f64, sm);
-  k_leg_fwd_f64<<<dim3(cdiv(c.L + 1, 64), tiles, c.L + 1), LTH, sm, c.stream>>>(a);
+  if (FwdTileSz::smem(c.nh) <= 227 * 1024) launch_fwd<true>(c, a, tiles);
+  else launch_fwd<false>(c, a, tiles);
 }
 
 }  // namespace cb2
