@@ -1610,9 +1610,16 @@ k_fft_products_g(const __grid_constant__ GPlan pl, int L, MLayoutT<T> fin, MLayo
   }
 }
 
-// order-major Fourier rows -> grid (float64), for the standalone transform API
+// order-major Fourier rows -> grid (float64), for the standalone transform API.
+// The rows lie far apart in m, so a (cos, sin) pair is one access, made once:
+// the pairs wait in the other buffer of the transform for the pair scaling.
+// Bound by the latency of the passes (block_fft): in float64 eight blocks an SM,
+// as many as without the pair scaling.  13 components at nphi = 384 / L127 / Nr33
+// 852 us (the pairs read twice, five blocks) -> 629 us, and the way back 768 ->
+// 632 (six).
+template <typename T> constexpr int kGridBlocks = sizeof(T) == 8 ? 8 : 6;
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kGridBlocks<T>)
 k_fft_to_grid_m(FFTPlan pl, int L, MLayoutT<T> fin, double *grid, const typename C2<T>::t *tw) {
   using T2 = typename C2<T>::t;
   using PB = PairBits<T>;
@@ -1628,24 +1635,31 @@ k_fft_to_grid_m(FFTPlan pl, int L, MLayoutT<T> fin, double *grid, const typename
     if (threadIdx.x < 2) pmx[threadIdx.x] = 0;
     for (int q = threadIdx.x; q < N; q += blockDim.x) Z0[q] = T2{0, 0};
     __syncthreads();
-    // pair scaling (pair_exp): the second row brought to the size of the first
+    // pair scaling (pair_exp): the second row, if there is one, brought to the
+    // size of the first
+    T sy = (T)1, iy = (T)1;
     {
       U mx = 0, my = 0;
       for (int m = threadIdx.x; m <= mmax; m += blockDim.x) {
-        mx = max(mx, max(PB::abs_bits(*fin.at(m, th, k, c, 0)), PB::abs_bits(*fin.at(m, th, k, c, 1))));
-        if (has1)
-          my = max(my, max(PB::abs_bits(*fin.at(m, th, k, c + 1, 0)), PB::abs_bits(*fin.at(m, th, k, c + 1, 1))));
+        const T2 v = __ldg(reinterpret_cast<const T2 *>(fin.at(m, th, k, c, 0)));
+        const T2 w = has1 ? __ldg(reinterpret_cast<const T2 *>(fin.at(m, th, k, c + 1, 0))) : T2{0, 0};
+        Z1[2 * m] = v;
+        Z1[2 * m + 1] = w;
+        mx = max(mx, max(PB::abs_bits(v.x), PB::abs_bits(v.y)));
+        my = max(my, max(PB::abs_bits(w.x), PB::abs_bits(w.y)));
       }
-      mx = __reduce_max_sync(0xffffffffu, mx);
-      my = __reduce_max_sync(0xffffffffu, my);
-      if ((threadIdx.x & 31) == 0) { atomicMax(pmx, mx); atomicMax(pmx + 1, my); }
+      if (has1) {
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        my = __reduce_max_sync(0xffffffffu, my);
+        if ((threadIdx.x & 31) == 0) { atomicMax(pmx, mx); atomicMax(pmx + 1, my); }
+        __syncthreads();
+        sy = PB::factor(pmx[0], pmx[1], false);
+        iy = PB::factor(pmx[0], pmx[1], true);
+      }
     }
-    __syncthreads();
-    const T sy = PB::factor(pmx[0], pmx[1], false), iy = PB::factor(pmx[0], pmx[1], true);
     for (int m = threadIdx.x; m <= mmax; m += blockDim.x) {
-      const T a0 = *fin.at(m, th, k, c, 0), b0 = (m > 0) ? *fin.at(m, th, k, c, 1) : (T)0;
-      const T a1 = has1 ? *fin.at(m, th, k, c + 1, 0) * sy : (T)0;
-      const T b1 = (has1 && m > 0) ? *fin.at(m, th, k, c + 1, 1) * sy : (T)0;
+      const T2 v = Z1[2 * m], w = Z1[2 * m + 1];   // this thread's own
+      const T a0 = v.x, b0 = v.y, a1 = w.x * sy, b1 = w.y * sy;
       if (m == 0) {
         Z0[0] = T2{a0, a1};
       } else {
@@ -1666,7 +1680,7 @@ k_fft_to_grid_m(FFTPlan pl, int L, MLayoutT<T> fin, double *grid, const typename
 
 // grid (float64) -> order-major Fourier rows
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kGridBlocks<T>)
 k_grid_to_fft_m(FFTPlan pl, int L, const double *grid, MLayoutT<T> fout, const typename C2<T>::t *tw) {
   using T2 = typename C2<T>::t;
   using PB = PairBits<T>;
@@ -1689,17 +1703,23 @@ k_grid_to_fft_m(FFTPlan pl, int L, const double *grid, MLayoutT<T> fout, const t
       mx = max(mx, PB::abs_bits(x));
       my = max(my, PB::abs_bits(y));
     }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    my = __reduce_max_sync(0xffffffffu, my);
-    if ((threadIdx.x & 31) == 0) { atomicMax(pmx, mx); atomicMax(pmx + 1, my); }
-    __syncthreads();
-    // pair scaling (pair_exp): the second row brought to the size of the first
-    const T sy = PB::factor(pmx[0], pmx[1], false);
-    if (sy != (T)1) {
-      for (int q = threadIdx.x; q < N; q += blockDim.x) Z0[q].y *= sy;
-      __syncthreads();
+    if (has1) {
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      my = __reduce_max_sync(0xffffffffu, my);
+      if ((threadIdx.x & 31) == 0) { atomicMax(pmx, mx); atomicMax(pmx + 1, my); }
     }
-    const T ay = an * PB::factor(pmx[0], pmx[1], true);
+    __syncthreads();
+    // pair scaling (pair_exp): the second row, if there is one, brought to the
+    // size of the first
+    T ay = an;
+    if (has1) {
+      const T sy = PB::factor(pmx[0], pmx[1], false);
+      if (sy != (T)1) {
+        for (int q = threadIdx.x; q < N; q += blockDim.x) Z0[q].y *= sy;
+        __syncthreads();
+      }
+      ay = an * PB::factor(pmx[0], pmx[1], true);
+    }
     const T2 *z = block_fft<T, T2>(Z0, Z1, pl, tw, -1);
     for (int m = threadIdx.x; m <= L; m += blockDim.x) {
       T a0, b0, a1, b1;
@@ -1711,12 +1731,8 @@ k_grid_to_fft_m(FFTPlan pl, int L, const double *grid, MLayoutT<T> fout, const t
         const T yr = (T)0.5 * (zk.y + zn.y), yi = (T)-0.5 * (zk.x - zn.x);
         a0 = (T)2 * an * xr; b0 = (T)-2 * an * xi; a1 = (T)2 * ay * yr; b1 = (T)-2 * ay * yi;
       }
-      *fout.at(m, th, k, c, 0) = a0;
-      *fout.at(m, th, k, c, 1) = b0;
-      if (has1) {
-        *fout.at(m, th, k, c + 1, 0) = a1;
-        *fout.at(m, th, k, c + 1, 1) = b1;
-      }
+      *reinterpret_cast<T2 *>(fout.at(m, th, k, c, 0)) = T2{a0, b0};
+      if (has1) *reinterpret_cast<T2 *>(fout.at(m, th, k, c + 1, 0)) = T2{a1, b1};
     }
     __syncthreads();
   }
