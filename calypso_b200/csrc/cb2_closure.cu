@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <vector>
@@ -126,7 +127,6 @@ __global__ void k_add_tendency(size_t n, int nr, int jmax, const float *Y, const
 // next wait on.  Every wait is bounded; a wait that runs out sets bit 2 of
 // *status and the CTA drains its MMAs, frees its TMEM and returns.
 constexpr int GK = 32;                        // K per stage (64-byte rows)
-constexpr unsigned long long kWaitNsGemm = 200ull * 1000 * 1000;
 constexpr uint32_t GA_BYTES = 128 * GK * 2;   // one bf16 term of the A tile
 
 template <typename T> struct Terms { static constexpr int n = 2; };
@@ -1145,6 +1145,8 @@ struct cb2_mlp {
   double *loss = nullptr;
   int *status = nullptr;
   size_t ycap = 0;              // rows of Yp
+  // budget of each wait inside the products (ns), CB2_PIPE_WAIT_NS as for a context
+  unsigned long long wait_ns = tc::kWaitNs;
   cudaStream_t stream = nullptr;
   // the parameters are written on `stream` and read there and on the streams of
   // the contexts the network is attached to: `written` follows their last
@@ -1215,7 +1217,7 @@ MlpArgs mlp_args(const cb2_mlp *n, const float *X, size_t rows, int *status) {
   a.W1 = n->w + n->oW1; a.W2 = n->w + n->oW2; a.W3 = n->w + n->oW3;
   a.count = (float)(rows * (size_t)n->O);
   a.status = status;
-  a.wait_ns = kWaitNsGemm;
+  a.wait_ns = n->wait_ns;
   return a;
 }
 
@@ -1235,9 +1237,15 @@ int launch_rows(K *kernel, const MlpArgs &a, cudaStream_t st) {
 // C = opA opB on the tensor cores (k_tc_gemm).  split_k: K is cut into
 // chunks so that the grid covers the SMs about twice, C is cleared and the
 // chunks' partial products are added with atomics.
+struct GemmRun {
+  cudaStream_t st;
+  int *status;
+  unsigned long long wait_ns;
+};
 template <typename TAT, typename TBT, bool TA, bool TB>
-void gemm(cudaStream_t st, int *status, int M, int N, int K, const TAT *A, int lda, const TBT *B, int ldb, float *C,
-          int ldc, bool split_k) {
+void gemm(const GemmRun &run, int M, int N, int K, const TAT *A, int lda, const TBT *B, int ldb, float *C, int ldc,
+          bool split_k) {
+  const cudaStream_t st = run.st;
   constexpr int NA = Terms<TAT>::n, NBT = Terms<TBT>::n;
   const int NT = std::min(256, ((N + 15) / 16) * 16);
   uint32_t cols = 64;
@@ -1259,7 +1267,7 @@ void gemm(cudaStream_t st, int *status, int M, int N, int K, const TAT *A, int l
   }
   dim3 grid((N + NT - 1) / NT, (M + 127) / 128, nz);
   k_tc_gemm<TAT, TBT, TA, TB><<<grid, 128, smem, st>>>(M, N, NT, K, A, lda, B, ldb, C, ldc, kchunk,
-                                                        split_k ? 1 : 0, cols, status, kWaitNsGemm);
+                                                        split_k ? 1 : 0, cols, run.status, run.wait_ns);
 }
 
 // forward pass of n rows of X (normalised features) into Y, on stream st
@@ -1273,12 +1281,13 @@ int mlp_forward(cb2_mlp *nt, const float *X, size_t n, float *Y, cudaStream_t st
   int rc = mlp_reserve(nt, n, false);
   if (rc) return rc;
   const int F = nt->F, H = nt->H, O = nt->O;
-  gemm<float, __nv_bfloat16, false, true>(st, status, (int)n, H, F, X, F, nt->w + nt->oW1, F, nt->Z1, H, false);
+  const GemmRun run{st, status, nt->wait_ns};
+  gemm<float, __nv_bfloat16, false, true>(run, (int)n, H, F, X, F, nt->w + nt->oW1, F, nt->Z1, H, false);
   k_bias_act<<<blocks(n * H), 256, 0, st>>>(n, H, nt->Z1, nt->master + nt->ob1, nt->H1, 1);
-  gemm<float, __nv_bfloat16, false, true>(st, status, (int)n, H, H, nt->H1, H, nt->w + nt->oW2, H, nt->Z2, H,
+  gemm<float, __nv_bfloat16, false, true>(run, (int)n, H, H, nt->H1, H, nt->w + nt->oW2, H, nt->Z2, H,
                                           false);
   k_bias_act<<<blocks(n * H), 256, 0, st>>>(n, H, nt->Z2, nt->master + nt->ob2, nt->H2, 1);
-  gemm<float, __nv_bfloat16, false, true>(st, status, (int)n, O, H, nt->H2, H, nt->w + nt->oW3, H, Y, O,
+  gemm<float, __nv_bfloat16, false, true>(run, (int)n, O, H, nt->H2, H, nt->w + nt->oW3, H, Y, O,
                                           false);
   k_bias_act<<<blocks(n * O), 256, 0, st>>>(n, O, Y, nt->master + nt->ob3, Y, 0);
   CB2_CUDA(cudaGetLastError());
@@ -1299,7 +1308,7 @@ int mlp_backward_fused(cb2_mlp *nt, const float *X, const float *T, size_t n) {
   w.X = X; w.Z1 = nt->Z1; w.Z2 = nt->Z2; w.dY = nt->dY; w.dZ1 = nt->dH; w.dZ2 = nt->dZ;
   w.gW1 = nt->grad + nt->oW1; w.gW2 = nt->grad + nt->oW2; w.gW3 = nt->grad + nt->oW3;
   w.bias = nt->bias;
-  w.status = nt->status; w.wait_ns = kWaitNsGemm;
+  w.status = nt->status; w.wait_ns = nt->wait_ns;
   const int ny = (a.H + 127) / 128;
   w.kchunk = split_chunk(a.n, ny);
   const size_t smem = 2 * (size_t)wg_stage(a.H) + 64 + 1024;
@@ -1325,20 +1334,21 @@ int mlp_backward(cb2_mlp *nt, const float *X, const float *T, size_t n) {
   }
   if ((rc = mlp_reserve_y(nt, n)) || (rc = mlp_forward(nt, X, n, nt->Yp, st))) return rc;
   const int F = nt->F, H = nt->H, O = nt->O;
+  const GemmRun run{st, nt->status, nt->wait_ns};
   const unsigned nb = blocks(n * O);
   k_mse<<<nb, 256, 0, st>>>(n, O, nt->Yp, T, nt->dY, nt->part);
   // layer 3
-  gemm<float, float, true, false>(st, nt->status, O, H, (int)n, nt->dY, O, nt->H2, H, nt->grad + nt->oW3, H, true);
+  gemm<float, float, true, false>(run, O, H, (int)n, nt->dY, O, nt->H2, H, nt->grad + nt->oW3, H, true);
   k_colsum<<<O, 256, 0, st>>>(n, O, nt->dY, nt->grad + nt->ob3);
-  gemm<float, __nv_bfloat16, false, false>(st, nt->status, (int)n, H, O, nt->dY, O, nt->w + nt->oW3, H, nt->dH, H, false);
+  gemm<float, __nv_bfloat16, false, false>(run, (int)n, H, O, nt->dY, O, nt->w + nt->oW3, H, nt->dH, H, false);
   k_act_grad<<<blocks(n * H), 256, 0, st>>>(n * H, nt->Z2, nt->dH, nt->dZ);
   // layer 2
-  gemm<float, float, true, false>(st, nt->status, H, H, (int)n, nt->dZ, H, nt->H1, H, nt->grad + nt->oW2, H, true);
+  gemm<float, float, true, false>(run, H, H, (int)n, nt->dZ, H, nt->H1, H, nt->grad + nt->oW2, H, true);
   k_colsum<<<H, 256, 0, st>>>(n, H, nt->dZ, nt->grad + nt->ob2);
-  gemm<float, __nv_bfloat16, false, false>(st, nt->status, (int)n, H, H, nt->dZ, H, nt->w + nt->oW2, H, nt->dH, H, false);
+  gemm<float, __nv_bfloat16, false, false>(run, (int)n, H, H, nt->dZ, H, nt->w + nt->oW2, H, nt->dH, H, false);
   k_act_grad<<<blocks(n * H), 256, 0, st>>>(n * H, nt->Z1, nt->dH, nt->dZ);
   // layer 1
-  gemm<float, float, true, false>(st, nt->status, H, F, (int)n, nt->dZ, H, X, F, nt->grad + nt->oW1, F, true);
+  gemm<float, float, true, false>(run, H, F, (int)n, nt->dZ, H, X, F, nt->grad + nt->oW1, F, true);
   k_colsum<<<H, 256, 0, st>>>(n, H, nt->dZ, nt->grad + nt->ob1);
   CB2_CUDA(cudaGetLastError());
   k_loss_sum<<<1, 256, 0, st>>>(nb, nt->part, 1.0 / ((double)n * O), nt->loss);
@@ -1411,6 +1421,7 @@ int cb2_mlp_create(int nin, int nhid, int nout, unsigned seed, cb2_mlp **out) {
   *out = nullptr;
   cb2_mlp *n = new cb2_mlp();
   n->F = nin; n->H = nhid; n->O = nout;
+  if (const char *pw = getenv("CB2_PIPE_WAIT_NS")) n->wait_ns = strtoull(pw, nullptr, 10);
   n->oW1 = 0; n->ob1 = n->oW1 + (size_t)nhid * nin; n->oW2 = n->ob1 + nhid;
   n->ob2 = n->oW2 + (size_t)nhid * nhid; n->oW3 = n->ob2 + nhid; n->ob3 = n->oW3 + (size_t)nout * nhid;
   n->np = n->ob3 + nout;

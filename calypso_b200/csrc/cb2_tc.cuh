@@ -31,10 +31,21 @@ __device__ inline void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 }
 
 // wait for the phase with the given parity to complete; false after
-// budget_ns (0: one try).  The pipelines' waits take the context's budget;
+// budget_ns (0: one look; a try may itself wait for some time).  The pipelines' waits take the context's budget;
 // the drains after an abort (copies and MMAs still in flight) take kWaitNs.
 __device__ inline bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned long long budget_ns = kWaitNs) {
   const uint32_t addr = smem_u32(bar);
+  if (budget_ns == 0) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    return done != 0;
+  }
   unsigned long long t0 = 0;
   for (uint32_t it = 0;; ++it) {
     uint32_t done;
@@ -46,7 +57,6 @@ __device__ inline bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned long l
         : "r"(addr), "r"(parity)
         : "memory");
     if (done) return true;
-    if (budget_ns == 0) return false;
     if (it == 64) t0 = globaltimer();
     if (it > 64) {
       if (globaltimer() - t0 > budget_ns) return false;

@@ -41,7 +41,8 @@ extern "C" {
                                  and later launches on the context do
                                  nothing: destroy it.  Each wait's budget is
                                  200 ms, or CB2_PIPE_WAIT_NS (nanoseconds)
-                                 from the environment at cb2_create */
+                                 from the environment at cb2_create (for a
+                                 closure network at cb2_mlp_create) */
 
 #define CB2_PREC_FP64 0       /* plain path: every stage in float64          */
 #define CB2_PREC_MIXED 1      /* Legendre split-fp16 tcgen05, fp32 FFT and
