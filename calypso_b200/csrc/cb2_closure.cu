@@ -282,9 +282,9 @@ k_tc_gemm(int M, int N, int NT, int K, const TAT *__restrict__ A, int lda, const
 // Three GEMMs with the activations between them in memory moved 1.6 GB for
 // 266240 rows (2031 us: the GEMMs, whose threads read a row each, 1510, bias
 // and SiLU 505); kept in tensor and shared memory the pass reads 64 and
-// writes 20 bytes a row and takes 196 us, bound by the SiLU epilogue (an
+// writes 20 bytes a row and takes 187 us, bound by the SiLU epilogue (an
 // __expf and a reciprocal per unit and layer) and the operand split.  A
-// training pass of 16384 rows: 29 + 39 + 55 + 3 us of kernels, before 500 us.
+// training pass of 16384 rows: 29 + 39 + 52 + 3 us of kernels, before 500 us.
 //
 // A training pass forms every product and activation with the terms, the order
 // and the rounding of the general kernels (k_tc_gemm, k_bias_act, k_mse,
@@ -367,14 +367,16 @@ __host__ __device__ inline MlpLayout mlp_layout(int H) {
 // iteration from the approximate reciprocal rounds as 1.0f / x does (compared
 // for every float of that range), without the division's range check a value,
 // which kept the 32 chains of a thread apart (closure forward of 266240 rows:
-// 333 us with 1.0f / x, 196 so).
+// 333 us with 1.0f / x, 196 so, 187 two values a time).
 __device__ inline float sigm(float z) { return 1.0f / (1.0f + __expf(-z)); }
 constexpr float kSigmLow = -87.0f;
-__device__ inline float sigm_mid(float z) {
-  const float x = 1.0f + __expf(-z);
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+// two values a time: the packed operations round each as the scalar ones
+__device__ inline float2 sigm_mid(float2 z) {
+  const float2 x = __fadd2_rn(float2{1.0f, 1.0f}, float2{__expf(-z.x), __expf(-z.y)});
+  float2 y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(x.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(x.y));
+  return __ffma2_rn(y, __ffma2_rn(float2{-x.x, -x.y}, y, float2{1.0f, 1.0f}), y);
 }
 template <int N>
 __device__ inline bool all_mid(const float *z) {
@@ -389,7 +391,11 @@ template <int N>
 __device__ inline void silu(float *z) {
   if (all_mid<N>(z)) {
 #pragma unroll
-    for (int j = 0; j < N; j++) z[j] = __fmul_rn(z[j], sigm_mid(z[j]));
+    for (int j = 0; j < N; j += 2) {
+      const float2 v{z[j], z[j + 1]}, h = __fmul2_rn(v, sigm_mid(v));
+      z[j] = h.x;
+      z[j + 1] = h.y;
+    }
   } else {
 #pragma unroll
     for (int j = 0; j < N; j++) z[j] = __fmul_rn(z[j], sigm(z[j]));
@@ -402,7 +408,11 @@ template <int N>
 __device__ inline void act_grad(float *d, const float *z) {
   if (all_mid<N>(z)) {
 #pragma unroll
-    for (int j = 0; j < N; j++) d[j] = act_grad(d[j], z[j], sigm_mid(z[j]));
+    for (int j = 0; j < N; j += 2) {
+      const float2 s = sigm_mid(float2{z[j], z[j + 1]});
+      d[j] = act_grad(d[j], z[j], s.x);
+      d[j + 1] = act_grad(d[j + 1], z[j + 1], s.y);
+    }
   } else {
 #pragma unroll
     for (int j = 0; j < N; j++) d[j] = act_grad(d[j], z[j], sigm(z[j]));
