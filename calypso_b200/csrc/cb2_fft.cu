@@ -1777,7 +1777,7 @@ static int attr_fft_t(Ctx &c) {
       }
   }
   CB2_CUDA(cudaMalloc(&c.d_twp32, t.size() * sizeof(float2)));
-  CB2_CUDA(cudaMemcpy(c.d_twp32, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
+  CB2_CUDA(cudaMemcpyAsync(c.d_twp32, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice, c.stream));
   return 0;
 }
 
@@ -1800,7 +1800,7 @@ static int attr_fft_4s(Ctx &c) {
       t[3 * P::M + n2 * P::WP + k1] = float2{(float)std::cos(ang), (float)std::sin(ang)};
     }
   CB2_CUDA(cudaMalloc(&c.d_twf4, t.size() * sizeof(float2)));
-  CB2_CUDA(cudaMemcpy(c.d_twf4, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
+  CB2_CUDA(cudaMemcpyAsync(c.d_twf4, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice, c.stream));
   return 0;
 }
 
@@ -1822,7 +1822,7 @@ static int attr_fft_4s64(Ctx &c) {
       t[3 * P::M + n2 * P::WP + k1] = double2{std::cos(ang), std::sin(ang)};
     }
   CB2_CUDA(cudaMalloc(&c.d_twf4_64, t.size() * sizeof(double2)));
-  CB2_CUDA(cudaMemcpy(c.d_twf4_64, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice));
+  CB2_CUDA(cudaMemcpyAsync(c.d_twf4_64, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice, c.stream));
   return 0;
 }
 

@@ -1542,7 +1542,7 @@ int mixed_setup(Ctx &c) {
   t->rows_all = R + t->NFmax;   // every NFmax-row box stays in the array
   auto up = [&](int **d, const std::vector<int> &v) -> int {
     CB2_CUDA(cudaMalloc(d, v.size() * sizeof(int)));
-    CB2_CUDA(cudaMemcpy(*d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CB2_CUDA(cudaMemcpyAsync(*d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
     return 0;
   };
   int rc;
@@ -1569,7 +1569,7 @@ int mixed_setup(Ctx &c) {
   {
     std::vector<float> w(c.h_wgt.begin(), c.h_wgt.end());
     CB2_CUDA(cudaMalloc(&t->wgt32, w.size() * sizeof(float)));
-    CB2_CUDA(cudaMemcpy(t->wgt32, w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice));
+    CB2_CUDA(cudaMemcpyAsync(t->wgt32, w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice, c.stream));
   }
   CB2_CUDA(cudaMalloc(&t->rowmax_four, (size_t)(L + 1) * (26 * (size_t)c.nr + 8) * sizeof(float)));
   // the four-step FFT kernel (nph = 3 (L + 1), L + 1 a multiple of 16)
@@ -1880,8 +1880,11 @@ int multi_leg_setup(const std::vector<Ctx *> &shells, int bnvec, int bnscal, con
     m->grid = std::min(m->grid, std::max(m->ntiles_bwd, m->ntiles_fwd));
     cudaError_t e = cudaMalloc(&m->d_bwd, n * sizeof(BwdShell));
     if (e == cudaSuccess) e = cudaMalloc(&m->d_fwd, n * sizeof(FwdShell));
-    if (e == cudaSuccess) e = cudaMemcpy(m->d_bwd, hb.data(), n * sizeof(BwdShell), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(m->d_fwd, hf.data(), n * sizeof(FwdShell), cudaMemcpyHostToDevice);
+    // waited for: the launches run on a stream of the ensemble's
+    const cudaStream_t st = shells[0]->stream;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(m->d_bwd, hb.data(), n * sizeof(BwdShell), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(m->d_fwd, hf.data(), n * sizeof(FwdShell), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = raise_smem_limit(k_leg_bwd_ws<true>, (int)m->smem_bwd);
     if (e == cudaSuccess) e = raise_smem_limit(k_leg_fwd_ws<true>, (int)m->smem_fwd);
     if (e != cudaSuccess) rc = cuda_fail(e, "multi-shell Legendre tables");

@@ -187,15 +187,17 @@ __global__ void k_plm(int L, int nh, const double *colat, const size_t *poff,
   }
 }
 
+// on the context's stream, which the kernels that read the table run on and
+// which does not wait for the default one
 template <typename T>
-static int upload(T **dst, const std::vector<T> &v) {
+static int upload(cudaStream_t st, T **dst, const std::vector<T> &v) {
   CB2_CUDA(cudaMalloc(dst, v.size() * sizeof(T)));
-  CB2_CUDA(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+  CB2_CUDA(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
   return 0;
 }
 
 #define UP(dst, v) \
-  do { int _r = upload(&(dst), (v)); if (_r) return _r; } while (0)
+  do { int _r = upload(c.stream, &(dst), (v)); if (_r) return _r; } while (0)
 
 int setup_tables(Ctx &c) {
   const cb2_params &p = c.p;
