@@ -78,11 +78,17 @@ int autotune(Ctx &c) {
   };
   std::vector<Item> items;
   if (c.prec == CB2_PREC_FP64) {
-    // 384: the float64 four-step kernel (where nphi = 3 (L + 1)), 512: the general one
-    items.push_back({TUNE_FFT_THREADS, {384, 512}, stage_fft_f64});
+    // 384: the float64 four-step kernel (where nphi = 3 (L + 1)), 512: the
+    // general one, the only one on other grids
+    if (c.d_twf4_64) items.push_back({TUNE_FFT_THREADS, {384, 512}, stage_fft_f64});
   } else {
     items.push_back({TUNE_PACK_KC, {1, 2, 4}, stage_bwd_mixed});
-    items.push_back({TUNE_FFT_THREADS, {384, 512, 256, 128}, stage_fft_mixed});
+    // the four-step kernel, and the Stockham kernel of the zonal grids that
+    // have one; the general kernel chooses its own block
+    std::vector<int> fft;
+    if (c.d_twf4) fft.push_back(384);
+    if (c.d_twp32) fft.insert(fft.end(), {512, 256, 128});
+    if (!fft.empty()) items.push_back({TUNE_FFT_THREADS, fft, stage_fft_mixed});
   }
   if (c.cn_ready) items.push_back({TUNE_CN, {0, 1}, stage_cn});
   for (const Item &it : items) {

@@ -139,7 +139,10 @@ int cb2_energies_static(cb2_ctx *ctx, double out[7]);
  * 12 (perturbation) temperature; other slots are work fields. */
 int cb2_get_field(cb2_ctx *ctx, int slot, double *host);
 int cb2_set_field(cb2_ctx *ctx, int slot, const double *host);
-/* the same with device buffers on the context's device (no copy to host) */
+/* the same with device buffers on the context's device (no copy to host).
+ * Both only queue their work on the context's own stream, which does not wait
+ * for the default one: dev must be ready before a set, and is in use until
+ * cb2_sync (or a call that returns results) after either. */
 int cb2_get_field_device(cb2_ctx *ctx, int slot, double *dev);
 int cb2_set_field_device(cb2_ctx *ctx, int slot, const double *dev);
 
@@ -276,9 +279,11 @@ int cb2_free_pinned(void *p);
  * overwrites the work fields).  tuning[5]: float64 backward kernel (1, 2 or
  * 4), float64 forward kernel (1, 2 or 3) (kept: one kernel on the float64
  * tensor cores now serves every value), mixed pack radial tile, FFT kernel of
- * either precision (384: the four-step kernel, used where nphi = 3 (ltr + 1);
- * 128, 256, 512: the Stockham kernel, float32 with that many threads), and
- * 1 (the default) to run the explicit update, the radial solves and the
+ * either precision (384: the four-step kernel, used where nphi = 3 (ltr + 1)
+ * = 96, 192, 384 or 768; 128, 256, 512: in float32 the Stockham kernel of
+ * those four zonal grids with that many threads, whatever ltr, in float64 the
+ * general kernel; on other grids the general kernel runs in either precision
+ * and the entry chooses nothing), and 1 (the default) to run the explicit update, the radial solves and the
  * derived fields of the step as one kernel, 0 as separate kernels; -1
  * (fixed) where the one kernel cannot take the context (cb2_tuning_note
  * says why). */
@@ -343,6 +348,8 @@ int cb2_mlp_forward(cb2_mlp *net, const float *dev_x, long long rows, float *dev
  * cb2_mlp_adam_step; also copied to host_grad when it is not NULL) */
 int cb2_mlp_loss_grad(cb2_mlp *net, const float *dev_x, const float *dev_t, long long rows, double *loss,
                       float *host_grad);
+/* queued on the network's stream; every later call on the network, and every
+ * step of the context it is attached to, sees the new parameters */
 int cb2_mlp_adam_step(cb2_mlp *net, float lr, float beta1, float beta2, float eps);
 int cb2_mlp_sync(cb2_mlp *net);
 /* dst state := src state truncated to dst's L and restricted to dst's
