@@ -52,7 +52,7 @@ int grow(void **buf, size_t *have, size_t need) {
 // m-major index, so that consecutive entries are consecutive in the field
 // slots; mo: (mp, |m|, s, -) in the order of (|m|, s), so that the two orders
 // of a Fourier row follow each other; mpos: [|m|][s] -> mp (the last one the
-// table lists) or -1; jj and mq: by j_rlm and by mp.
+// table lists) or -1; mq: by mp.
 struct DevTab {
   const int2 *jo = nullptr;  // nidx_rlm(2)
   const int *mq = nullptr;   // nidx_rtm(3) x 2: |m|, s (0 cos / order +m, 1 sin / order -m)
@@ -290,7 +290,7 @@ constexpr int kBnd = 256;
 
 // rlm buffer <-> work slots (device order).  The slots run along jj, the
 // rlm buffer along the nq components of a mode (a run of 8 nq bytes): a block
-// takes JT modes of consecutive jj at one radial level and turns them round
+// takes JT modes of consecutive jj at JK radial levels and turns them round
 // in shared memory, so both sides move in whole runs: bound by the runs'
 // partial sectors.  At L255 / Nr65 / 11 components 150 us inwards (5.0 TB/s);
 // a thread per mode, whose 8-byte slot writes scattered over the orders, took
@@ -345,8 +345,8 @@ k_rlm_slots(int nj, int nr, int ncomp, int is0, int is1, int comp0, FastDiv nq, 
 
 // Order-major Fourier rows <-> rtm buffer where the radius runs faster than
 // the order (istep_rtm(1) <= istep_rtm(3), the reference's own order): a
-// block takes one colatitude of one order, the lanes along the buffer's
-// (k, component) runs.  One thread per (theta, k) and order with its
+// block takes one order at RTH colatitudes outwards (one inwards), the lanes
+// along the buffer's (k, component) runs.  One thread per (theta, k) and order with its
 // components in a loop (k_four_to_rtm / k_rtm_to_four, which stay for the
 // other stride orders) wrote 8 bytes of every line at a time: 1112 us
 // outwards at L255 / Nr65 / 11 components, now 295 us (5.6 TB/s); 323 us

@@ -39,11 +39,12 @@
 namespace cb2 {
 
 // Rows each thread keeps in flight (cp.async ring) and threads of a block.
-// Large shells: 4 rows, which leaves room for four blocks of 256 an SM (the
-// factors two rows ahead cost registers for three: L255 / Nr129 step 4980 us
-// for 4860).  Shells of at most CN_DEEP columns (two blocks of 256 an SM),
-// whose time is the latency of the rows: 8 rows, the factors two rows ahead,
-// and blocks of 64, to use every SM (step at L31 / Nr33 79 -> 76 -> 74 us).
+// Large shells: 4 rows, which leaves room for four blocks of 256 an SM (64
+// registers, 8 bytes of a thread spilt; with the factors two rows ahead the
+// registers are for three: L255 / Nr129 step 4980 us for 4860).  Shells of at
+// most CN_DEEP columns (two blocks of 256 an SM), whose time is the latency of
+// the rows: 8 rows, the factors two rows ahead, and blocks of 64, to use every
+// SM (step at L31 / Nr33 79 -> 76 -> 74 us).
 constexpr int CN_RING = 4, CN_RING_DEEP = 8, CN_DEEP = 2 * 148 * 256;
 __host__ __device__ constexpr int cn_threads(int ring) { return ring == CN_RING ? 256 : 64; }
 __host__ __device__ constexpr int cn_ahead(int ring) { return ring == CN_RING ? 1 : 2; }

@@ -19,13 +19,14 @@
 // X[3 - q] = X[q ^ 3]: within an 8-column fragment that is the value of the
 // lane 12 away, so one staged copy of X serves both.
 //
-// Bounds: at L255 / Nr129 / 4 vectors + 1 scalar the sums are 6.8e10 flop each
-// way, 1.9 ms at the 37 TF/s that mma f64 (and DFMA) reach on a B200; the
-// traffic is 0.55 ms.  The earlier kernels (a block per 2 radial levels over
+// Bounds: at L255 / Nr129 the sums are 6.8e10 flop backward (4 vectors + 1
+// scalar) and 6.5e10 forward (4 vectors), 1.84 and 1.76 ms at the 37 TF/s that
+// mma f64 (and DFMA) reach on a B200; the traffic is 0.55 ms.  The earlier kernels (a block per 2 radial levels over
 // theta-major rows, whose 16-byte pieces of an order lie 53 KB apart, the B
 // matrices of both products built in shared memory for each chunk) took 7.3 ms
-// backward and 8.8 ms forward; these take 3.02 ms and 3.28 ms, 64 % and 59 %
-// of the float64 rate.
+// backward and 8.8 ms forward; these take 3.02 ms and 3.28 ms, 61 % and 54 %
+// of that rate in useful flops, the matrix pipe 64 % and 60 % busy (padding of
+// the tiles counted).
 #include <algorithm>
 
 #include "cb2_internal.cuh"

@@ -801,7 +801,8 @@ struct CorCol {
 //  add_reftemp_advect_sph_MHD, set_MHD_terms_to_force).
 // A thread takes kl radial levels of one (l, m): the rows k - 1, k, k + 1 of
 // the seven differentiated fields slide through registers and the Coriolis
-// weights are read once.  Bound by HBM and the latency of the rows.  A thread
+// weights are read once.  Bound by HBM and the latency of the rows; at the 128
+// registers that four blocks an SM leave, 108 bytes of a thread spill.  A thread
 // per point read every row three times and the 16 table entries at each level
 // (L2 traffic three times that of DRAM): 432 -> 372 us at L255 / Nr129, 84 ->
 // 77 us at L127 / Nr97.

@@ -55,10 +55,11 @@ RESTART_FIELDS = [("velocity", 3), ("temperature", 1), ("magnetic_field", 3),
                   ("previous_momentum", 3), ("previous_induction", 3), ("previous_heat", 1)]
 RESTART_FIELDS_COMPS = [(n, c) for n, nc in RESTART_FIELDS for c in range(nc)]
 
-# kernel-variant tuning entries (cb2_get_tuning / cb2_set_tuning): float64
-# backward radial tile, float64 forward radial tile, mixed pack radial tile,
-# FFT kernel (384 four-step, else Stockham threads), fused Crank-Nicolson
-# step (1) or separate kernels (0)
+# kernel-variant tuning entries (cb2_get_tuning / cb2_set_tuning): two kept for
+# the float64 Legendre transforms, which have one kernel each and ignore them,
+# mixed pack radial tile, FFT kernel (384 four-step, else Stockham threads, on
+# the grids that have those), fused Crank-Nicolson step (1) or separate
+# kernels (0)
 TUNE_BWD_KT, TUNE_FWD_KT, TUNE_PACK_KC, TUNE_FFT_THREADS, TUNE_CN = range(5)
 TUNE_N = 5
 
