@@ -1500,16 +1500,17 @@ int cb2_mlp_get_params(cb2_mlp *n, float *host) {
   return 0;
 }
 
-// the network's stream behind every pass of an attached context that reads the
-// parameters, before they change
-static int params_begin(cb2_mlp *n) {
+// the network's stream behind every pass of an attached context, which reads the
+// parameters and uses the work buffers of the general kernels and Yp: before
+// either is written
+static int after_users(cb2_mlp *n) {
   for (ClosureState *cs : n->users) CB2_CUDA(cudaStreamWaitEvent(n->stream, cs->read, cudaEventWaitDefault));
   return 0;
 }
 
 int cb2_mlp_set_params(cb2_mlp *n, const float *host) {
   if (!n || !host) return CB2_ERR_ARG;
-  if (int rc = params_begin(n)) return rc;
+  if (int rc = after_users(n)) return rc;
   CB2_CUDA(cudaMemcpyAsync(n->master, host, n->np * sizeof(float), cudaMemcpyHostToDevice, n->stream));
   k_to_bf16<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->w);
   CB2_CUDA(cudaEventRecord(n->written, n->stream));
@@ -1542,6 +1543,8 @@ int cb2_mlp_forward(cb2_mlp *n, const float *dev_x, long long rows, float *dev_y
   const std::less<const float *> before;
   const bool overlap = fused_ok(n) && before(dev_x, dev_y + ny) && before(dev_y, dev_x + nx);
   float *y = dev_y;
+  if (overlap || !fused_ok(n))
+    if (int rc = after_users(n)) return rc;
   if (overlap) {
     if (int rc = mlp_reserve_y(n, (size_t)rows)) return rc;
     y = n->Yp;
@@ -1557,8 +1560,8 @@ int cb2_mlp_loss_grad(cb2_mlp *n, const float *dev_x, const float *dev_t, long l
                       float *host_grad) {
   if (!n || !dev_x || !dev_t || rows <= 0) return CB2_ERR_ARG;
   double l = 0.0;
-  int rc = mlp_backward(n, dev_x, dev_t, (size_t)rows);
-  if (rc || (rc = mlp_status(n, &l))) return rc;
+  int rc = fused_ok(n) ? 0 : after_users(n);
+  if (rc || (rc = mlp_backward(n, dev_x, dev_t, (size_t)rows)) || (rc = mlp_status(n, &l))) return rc;
   if (loss) *loss = l;
   if (host_grad) CB2_CUDA(cudaMemcpy(host_grad, n->grad, n->np * sizeof(float), cudaMemcpyDeviceToHost));
   return 0;
@@ -1566,7 +1569,7 @@ int cb2_mlp_loss_grad(cb2_mlp *n, const float *dev_x, const float *dev_t, long l
 
 int cb2_mlp_adam_step(cb2_mlp *n, float lr, float beta1, float beta2, float eps) {
   if (!n) return CB2_ERR_ARG;
-  if (int rc = params_begin(n)) return rc;
+  if (int rc = after_users(n)) return rc;
   n->t += 1;
   const float c1 = 1.0f - std::pow(beta1, (float)n->t), c2 = 1.0f - std::pow(beta2, (float)n->t);
   k_adam<<<blocks(n->np), 256, 0, n->stream>>>(n->np, n->master, n->grad, n->m, n->v, lr, beta1, beta2, eps, c1, c2, n->w);

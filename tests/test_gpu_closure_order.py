@@ -101,6 +101,28 @@ def test_update_waits_for_queued_steps(graph):
     assert np.array_equal(*got)
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_passes_wait_for_queued_steps(graph):
+    # a network of these widths has one set of work buffers for all its passes
+    got = []
+    x, t = batch(1000)
+    for drained in (True, False):
+        net = closure.MLP(16, WIDE, 5, seed=1)
+        g = shell_with(net)
+        net.loss_grad(x, t)          # buffers of their largest size
+        out = []
+        for call in (lambda: net.forward(x).cpu().numpy(), lambda: np.array(net.loss_grad(x, t))):
+            g.step(6, graph=graph)
+            if drained:
+                g.sync()
+            out.append(call())
+        got.append(out + [g.get_field(FORCES)])
+        g.close()
+        net.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
 def test_network_closed_before_its_context():
     net = closure.MLP(16, 64, 5, seed=1)
     g = shell_with(net)
